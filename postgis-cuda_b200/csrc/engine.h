@@ -145,7 +145,7 @@ struct gsj_ctx {
   uint64_t node_visits = 0;   // LBVH nodes visited by traversals (roofline accounting)
   uint64_t edge_pairs = 0;    // local edge pairs (na x nb) of the pairs refined (the refinement's work unit)
   gsj::RefineShape shape;
-  gsj::RefineGraph rgraph[12];   // [variant (plain, filtered, filtered FP32) x scratch bin or not x self bin or not]
+  gsj::RefineGraph rgraph[36];   // [variant (plain, filtered x what is wanted, filtered FP32 x the same) x scratch bin or not x self bin or not]
   // scratch pools
   gsj::DevBuf counters, cand, flag, area, ev, evb, heavy, selfidx, scratch, keep, opairs, oarea, oev, oevb, ocode, tmp, keys, keys2, idx,
       idx2, agg_area, agg_ev, agg_evb, agg_flag, qbb, uf, misc1, misc2, misc3,
@@ -191,9 +191,10 @@ uint64_t refine(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2*
                 uint8_t* flag, double* area, double4* ev, uint32_t* evb);
 // the same in two halves, for callers with a stream sync of their own after it: refine_enqueue puts the bins and the
 // copy of their counters on the stream; refine_result, after the caller's next sync, checks the error word and
-// returns the oversized-pair count (the outputs must not be used before it returned without throwing)
+// returns the oversized-pair count (the outputs must not be used before it returned without throwing). hits_only: the
+// caller reads the outputs of pairs with flag 1 alone (flag 2 then counts as 0)
 void refine_enqueue(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, int mode,
-                    uint8_t* flag, double* area, double4* ev, uint32_t* evb);
+                    uint8_t* flag, double* area, double4* ev, uint32_t* evb, bool hits_only = false);
 uint64_t refine_result(gsj_ctx* c);
 
 // refinement launch shapes (tune.cu)

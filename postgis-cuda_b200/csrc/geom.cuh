@@ -134,8 +134,11 @@ struct Box { double x0, y0, x1, y1; };
 
 // Local edge list (SoA; in shared memory for the fast bins, in global scratch for oversized pairs).
 // fl: bit 0 = synthetic (cut) edge, bit 1 / bit 2 = start / end vertex is a cut point.
-struct EList {
-  double* x0; double* y0; double* x1; double* y1; uint32_t* fl;
+template <class FL>
+struct EListT {
+  double* x0; double* y0; double* x1; double* y1; FL* fl;
 };
+using EList = EListT<uint32_t>;
+using EList8 = EListT<uint8_t>;
 
 }  // namespace gsj

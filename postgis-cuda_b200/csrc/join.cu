@@ -181,7 +181,7 @@ void run_join(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const RefineAr
     uint32_t* evb = rel ? c->evb.as<uint32_t>(np) : nullptr;
     // area is needed for the piece fold or the output; relate-only joins still fold (zero) areas.
     // The refinement's counters come back with the compaction's count: one host round trip for both.
-    refine_enqueue(c, P, R, pairs, np, rp, o.refine_mode, flag, area, ev, evb);
+    refine_enqueue(c, P, R, pairs, np, rp, o.refine_mode, flag, area, ev, evb, !agg);
     tr.mark_end();
     tm.start();
     uint32_t* keep = c->keep.as<uint32_t>(np);

@@ -12,7 +12,6 @@ __device__ __forceinline__ EList carve(unsigned char* base, int cap) {
   L.fl = reinterpret_cast<uint32_t*>(L.y1 + cap);
   return L;
 }
-__device__ __forceinline__ EList carve_f(unsigned char* base, int cap) { return carve(base, cap); }
 // edge (x0, y0)-(x1, y1) entirely outside box [bx0, bx1] x [by0, by1], by comparisons only
 __device__ __forceinline__ bool out_cmp(double x0, double y0, double x1, double y1, double bx0, double by0, double bx1, double by1) {
   return (x0 < bx0 && x1 < bx0) || (x0 > bx1 && x1 > bx1) || (y0 < by0 && y1 < by0) || (y0 > by1 && y1 > by1);
@@ -21,42 +20,47 @@ __device__ __forceinline__ bool edge_outside(double px, double py, double qx, do
   return fmax(px, qx) < o.x0 || fmin(px, qx) > o.x1 || fmax(py, qy) < o.y0 || fmin(py, qy) > o.y1;
 }
 
+// Whether the horizontal segment (ox, my) -> (mx, my) crosses the edge (x0, y0)-(x1, y1), which reaches the level my:
+// so != sc && su != sv of the four orientations (engine.cuh:382-397), where ox lies left of both end points by at least about
+// 1 (of the frame's unit). The side of (ox, my) is then the edge's direction in y, or in x for a level edge (the
+// determinant is at least |y1 - y0| beside terms of a few hundred times that, so its rounding cannot turn it), and the
+// orientations of the end points against the level segment are the signs of the plain products (their other term is 0).
+template <bool S32 = false>
+__device__ __forceinline__ bool ray_crosses(double x0, double y0, double x1, double y1, double ox, double mx, double my) {
+  const bool so = y0 != y1 ? y1 > y0 : x1 > x0, sc = S32 ? left_of32(x0, y0, x1, y1, mx, my) : left_of(x0, y0, x1, y1, mx, my);
+  const double a = mx - ox;
+  return so != sc && (a * (y0 - my) > 0) != (a * (y1 - my) > 0);
+}
+
 // all edges of geometry A meeting the overlap box, compacted in ring order with a warp ballot (engine.cuh:358-377).
 // PIP: the same pass also takes the crossing parity of the segment (A's bbox left edge - 1, my) -> (mx, my) over
 // every edge of A, as pip_full_warp does (an XOR over the edges, so the order is free), into *inside.
-template <bool F, bool PIP = false, bool S32 = false>
-static __device__ int collect(const Frame& A, const Box& ov, EList L, int cap, int lane, double mx = 0, double my = 0, bool* inside = nullptr) {
+template <bool F, bool PIP = false, bool S32 = false, class EL>
+static __device__ int collect(const Frame& A, const Box& ov, EL L, int cap, int lane, double mx = 0, double my = 0, bool* inside = nullptr) {
   const DLayer& S = *A.L;
   const unsigned lt = (1u << lane) - 1;
-  const double ox = A.shx - (double)1, oy = my;
+  const double ox = A.shx - (double)1;
   bool par = false;
   int cnt = 0;
+#pragma unroll 1
   for (uint32_t ra = A.r0; ra < A.r1; ra++) {
-    const uint64_t s = S.rvo[ra], e = S.rvo[ra + 1];
-    for (uint64_t base = s; base + 1 < e; base += 32) {
-      const uint64_t i = base + lane;
+    const uint64_t s = S.rvo[ra];
+    const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);   // a ring's vertices, indexed by 32 bits
+    const double2* v = S.xy + s;
+#pragma unroll 1
+    for (uint32_t base = 0; base + 1 < n; base += 32) {
+      const uint32_t i = base + lane;
       bool in = false;
       double x0 = 0, y0 = 0, x1 = 0, y1 = 0; uint32_t fl = 0;
-      if (i + 1 < e) {
-        A.v(i, x0, y0); A.v(i + 1, x1, y1);
+      if (i + 1 < n) {
+        const double2 p = v[i], q = v[i + 1];
+        x0 = A.shx + p.x; y0 = A.shy + p.y; x1 = A.shx + q.x; y1 = A.shy + q.y;
         if (S.synb) {
-          fl = (uint32_t)S.syn(i) | (S.syn(i > s ? i - 1 : e - 2) ? 2u : 0u) | (S.syn(i + 2 < e ? i + 1 : s) ? 4u : 0u);
+          fl = (uint32_t)S.syn(s + i) | (S.syn(s + (i > 0 ? i - 1 : n - 2)) ? 2u : 0u) | (S.syn(s + (i + 2 < n ? i + 1 : 0)) ? 4u : 0u);
         }
         in = F ? !out_cmp(x0, y0, x1, y1, ov.x0, ov.y0, ov.x1, ov.y1) : !edge_outside(x0, y0, x1, y1, ov);
         if (PIP && !((y0 > my) == (y1 > my) && y0 != my && y1 != my)) {
-          if (S32) {   // the same signs through the certified FP32 filter
-            const bool so = left_of32(x0, y0, x1, y1, ox, oy), sc = left_of32(x0, y0, x1, y1, mx, my);
-            if (so != sc) {
-              const bool su = orient_sign32(ox, oy, mx, my, x0, y0) > 0, sv = orient_sign32(ox, oy, mx, my, x1, y1) > 0;
-              if (su != sv) par = !par;
-            }
-          } else {
-            const bool so = left_of(x0, y0, x1, y1, ox, oy), sc = left_of(x0, y0, x1, y1, mx, my);
-            if (so != sc) {
-              const bool su = orient(ox, oy, mx, my, x0, y0) > 0, sv = orient(ox, oy, mx, my, x1, y1) > 0;
-              if (su != sv) par = !par;
-            }
-          }
+          if (ray_crosses<S32>(x0, y0, x1, y1, ox, mx, my)) par = !par;
         }
       }
       const unsigned m = __ballot_sync(0xffffffffu, in);
@@ -74,17 +78,15 @@ static __device__ int collect(const Frame& A, const Box& ov, EList L, int cap, i
 // crossing parity of segment (B's bbox left edge - 1, my) -> (mx, my) over all of B's edges (engine.cuh:382-397)
 static __device__ bool pip_full_warp(const Frame& B, double mx, double my, int lane) {
   const DLayer& S = *B.L;
-  const double ox = B.shx - (double)1, oy = my;
+  const double ox = B.shx - (double)1;
   bool par = false;
+#pragma unroll 1
   for (uint32_t r = B.r0; r < B.r1; r++) {
     const uint64_t s = S.rvo[r], e = S.rvo[r + 1];
+#pragma unroll 1
     for (uint64_t j = s + 1 + lane; j < e; j += 32) {
       double x0, y0, x1, y1; B.v(j - 1, x0, y0); B.v(j, x1, y1);
-      if ((y0 > my) == (y1 > my) && y0 != my && y1 != my) continue;
-      bool so = left_of(x0, y0, x1, y1, ox, oy), sc = left_of(x0, y0, x1, y1, mx, my);
-      if (so == sc) continue;
-      bool su = orient(ox, oy, mx, my, x0, y0) > 0, sv = orient(ox, oy, mx, my, x1, y1) > 0;
-      if (su != sv) par = !par;
+      if (!((y0 > my) == (y1 > my) && y0 != my && y1 != my) && ray_crosses(x0, y0, x1, y1, ox, mx, my)) par = !par;
     }
   }
   return (__popc(__ballot_sync(0xffffffffu, par)) & 1) != 0;
@@ -92,8 +94,8 @@ static __device__ bool pip_full_warp(const Frame& B, double mx, double my, int l
 
 // inside(x) = inside(c) xor crossings of c -> x with the local edges (engine.cuh:400-412)
 // S32: the four orientation signs through the certified FP32 filter (the same booleans)
-template <bool F, bool S32 = false>
-__device__ __forceinline__ bool inside_from_c(const EList& L, int cnt, double cx, double cy, bool in_c, double x, double y) {
+template <bool F, bool S32 = false, class EL>
+__device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, double cy, bool in_c, double x, double y) {
   bool in = in_c;
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);
   auto step = [&](int k) {
@@ -113,16 +115,18 @@ __device__ __forceinline__ bool inside_from_c(const EList& L, int cnt, double cx
     }
     return false;
   };
+#pragma unroll 1
   for (int k = 0; k < cnt; k++) step(k);
   return in;
 }
 
 // The same parity for one query point shared by the whole warp: lanes split the edges, a ballot counts crossings
 // (the parity does not depend on the order of the edges).
-template <bool S32 = false>
-static __device__ bool inside_from_c_warp(const EList& L, int cnt, double cx, double cy, bool in_c, double x, double y, int lane) {
+template <bool S32 = false, class EL>
+static __device__ bool inside_from_c_warp(const EL& L, int cnt, double cx, double cy, bool in_c, double x, double y, int lane) {
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);
   bool par = false;
+#pragma unroll 1
   for (int k = lane; k < cnt; k += 32) {
     const double ex0 = L.x0[k], ey0 = L.y0[k], ex1 = L.x1[k], ey1 = L.y1[k];
     if (out_cmp(ex0, ey0, ex1, ey1, sx0, sy0, sx1, sy1)) continue;

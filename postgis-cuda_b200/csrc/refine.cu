@@ -5,15 +5,15 @@
 // FP64 area and boundary-length sums have one fixed rounding order: bit-identical to the CPU oracle.
 //
 // Pairs whose local edge lists fit CAP run from shared memory; larger pairs are queued and re-run by
-// k_refine_scratch with per-warp lists in global scratch (the same device code, so the same results).
+// k_refine_scratch with per-warp lists in global scratch.
 //
-// Two variants of the same pair routine (template flag F):
-//  - plain (F = false): FP64 box tests, as the reference.
-//  - filtered (F = true): the box rejection tests that dominate the inner loops are written as plain comparisons
-//    (max(a, b) < x  <=>  a < x && b < x for finite values) instead of FP64 min/max, which on sm_100a issue on the
-//    XU pipe - the pipe the plain kernel saturates (ncu: XU 77 % of peak, FP64 25 %). The same booleans, so every
-//    decision and every FP64 value is unchanged. Containment probes are tested by the whole warp (crossing parity
-//    is order-free).
+// Two variants with the same decisions and the same FP64 values:
+//  - plain (F = false): the reference's sweeps, FP64 box tests (refine_pair_t<false>).
+//  - filtered (F = true): candidate edge pairs first, then only the work they need (refine_pair_m in the shared-memory
+//    bins, refine_pair_t<true, FLAT> in the scratch bin). Box rejection tests are plain comparisons (max(a, b) < x  <=>
+//    a < x && b < x for finite values) instead of FP64 min/max, which on sm_100a issue on the XU pipe. Containment probes
+//    are tested by the whole warp (crossing parity is order-free).
+#include <type_traits>
 #include "engine.h"
 #include "pairkit.cuh"
 
@@ -24,10 +24,8 @@ constexpr int RB_WARPS = 4;                      // warps per block
 constexpr size_t EDGE_BYTES = 4 * sizeof(double) + sizeof(uint32_t);
 constexpr size_t LIST_BYTES = CAP * EDGE_BYTES;  // one list
 constexpr size_t RB_SMEM = (size_t)RB_WARPS * 2 * LIST_BYTES;
-constexpr int CAP_F = 128;                       // filtered: local edges per polygon per warp
-constexpr size_t EDGE_BYTES_F = EDGE_BYTES;
-constexpr size_t LIST_BYTES_F = CAP_F * EDGE_BYTES_F;
-constexpr size_t RB_SMEM_F = (size_t)RB_WARPS * 2 * LIST_BYTES_F;
+constexpr int CAP_F = 128;                       // filtered: local edges per polygon per warp (a multiple of 32, below 256)
+constexpr size_t EDGE_BYTES_8 = 4 * sizeof(double) + 1;   // filtered shared-memory bins: flags in a byte
 
 struct PairGeo { Box ov; double tol, eps_par, snap, cx, cy; };
 
@@ -202,262 +200,273 @@ __device__ int flat_candidates(const EList& LA, int na, const EList& LB, int nb,
   return cnt;
 }
 
-// Candidate edge pairs of the shared-memory kernel as bit masks: row i holds the B edges j whose boxes come within
-// 2 tol of A edge i (the flat lists' test and set), column j the A edges i. A row visits its j, a column its i, in
-// increasing order by walking set bits, which is the order of the flat lists; the masks never overflow (up to
-// CAP_F edges per side) and cost no counting, scans or scatter. Word-major: word w of row i at rm[w * CAP_F + i].
-constexpr int MASK_WORDS = CAP_F / 32;
-struct MaskBuf { uint32_t* rm; uint32_t* cm; };
-constexpr size_t MASK_BYTES = 2 * (size_t)MASK_WORDS * CAP_F * sizeof(uint32_t);
+// Green's-theorem contribution of edge p->q within the other polygon + relate lengths (engine.cuh:416-515), in three
+// steps: the edge's cuts (split points and coincident intervals against the other polygon's edges), its segments
+// between consecutive split points, each segment's value.
+struct EdgeRef { double px, py, qx, qy, dx, dy, len2, len; uint32_t fl; };   // len: where lengths are wanted
+struct EdgeCuts {
+  double ts[MAXS]; int ns;
+  double ol0[MAXO], ol1[MAXO]; bool osame[MAXO]; int oidx[MAXO]; int no;
+};
+struct Segment { double t0, t1, mx, my; int net, first, net_real, n_real; bool valid, need; };
 
-// one stage of the in-register 32 x 32 bit transpose: lanes l and l ^ s swap the off-diagonal s x s blocks
-__device__ __forceinline__ uint32_t transpose_stage(uint32_t x, int s, uint32_t m, int lane) {
-  const uint32_t p = __shfl_xor_sync(0xffffffffu, x, s);
-  return (lane & s) ? ((x & ~m) | ((p >> s) & m)) : ((x & m) | ((p << s) & ~m));
-}
-// lane l holds row l of a 32 x 32 bit matrix (bit j = M[l][j]); returns column l (bit i = M[i][l])
-__device__ __forceinline__ uint32_t warp_transpose32(uint32_t x, int lane) {
-  x = transpose_stage(x, 16, 0x0000FFFFu, lane);
-  x = transpose_stage(x, 8, 0x00FF00FFu, lane);
-  x = transpose_stage(x, 4, 0x0F0F0F0Fu, lane);
-  x = transpose_stage(x, 2, 0x33333333u, lane);
-  return transpose_stage(x, 1, 0x55555555u, lane);
+template <class EL>
+__device__ __forceinline__ EdgeRef edge_ref(const EL& L, int i, bool rel) {
+  EdgeRef e;
+  e.px = L.x0[i]; e.py = L.y0[i]; e.qx = L.x1[i]; e.qy = L.y1[i]; e.fl = L.fl[i];
+  e.dx = e.qx - e.px; e.dy = e.qy - e.py;
+  e.len2 = e.dx * e.dx + e.dy * e.dy;
+  e.len = rel ? sqrt(e.len2) : 0.0;
+  return e;
 }
 
-// lane i (per 32 A edges) keeps its padded box in registers and tests every B edge j, read once for the whole warp
-// (a shared-memory broadcast); each 32 x 32 block of rows is transposed into columns by shuffles (COLS; the self
-// bin reads rows only). STRIDE: rows per mask word plane (the bin's list capacity).
-template <int STRIDE = CAP_F, bool COLS = true>
-__device__ void mask_candidates(const EList& LA, int na, const EList& LB, int nb, double pad, const MaskBuf& mb, int lane) {
-  const int nbw = (nb + 31) >> 5;
-  const double inf = __longlong_as_double(0x7ff0000000000000LL);
-  for (int ic = 0; ic < na; ic += 32) {
-    const int i = ic + lane;
-    double ax0 = inf, ay0 = inf, ax1 = -inf, ay1 = -inf;   // lanes past the end keep an empty box: no bits
-    if (i < na) {
-      const double px = LA.x0[i], py = LA.y0[i], qx = LA.x1[i], qy = LA.y1[i];
-      ax0 = (px < qx ? px : qx) - pad; ax1 = (px < qx ? qx : px) + pad;
-      ay0 = (py < qy ? py : qy) - pad; ay1 = (py < qy ? qy : py) + pad;
-    }
-    for (int w = 0; w < nbw; w++) {
-      const int j0 = w << 5, j1 = min(nb, j0 + 32);
-      uint32_t bits = 0;
-      for (int j = j0; j < j1; j++)
-        bits |= (out_cmp(LB.x0[j], LB.y0[j], LB.x1[j], LB.y1[j], ax0, ay0, ax1, ay1) ? 0u : 1u) << (j - j0);
-      if (i < na) mb.rm[w * STRIDE + i] = bits;
-      if constexpr (COLS) {
-        const uint32_t col = warp_transpose32(bits, lane);
-        if (j0 + lane < nb) mb.cm[(ic >> 5) * STRIDE + j0 + lane] = col;
-      }
-    }
-  }
-  __syncwarp();
-}
-
-// Green's-theorem contribution of edge p->q within the other polygon + relate lengths (engine.cuh:416-515).
-// each_k(visit) calls visit(k) for the other polygon's local edges k in increasing order: all of them, or only
-// those of a candidate list that holds every k passing the box test below (the same visits, the same results).
-template <bool F, bool S32, class EachK>
-__device__ double edge_contrib_k(double px, double py, double qx, double qy, const EList& L, int cnt, bool in_c, const PairGeo& G, bool real,
-                                 double* l_in, double* l_on, uint32_t* bits, uint32_t cut, EachK&& each_k) {
-  const double dx = qx - px, dy = qy - py;
-  const double len2 = dx * dx + dy * dy;
-  if (len2 == 0) return 0.0;
-  const double tol = G.tol;
-  const double tol2len2 = tol * tol * len2, eps2 = G.eps_par * G.eps_par;
-  double ts[MAXS]; int ns = 0;
-  double ol0[MAXO], ol1[MAXO]; bool osame[MAXO]; int oidx[MAXO]; int no = 0;
-  ts[ns++] = 0; ts[ns++] = 1;
+// the cuts that edge k of the other polygon makes
+template <bool F, class EL>
+__device__ __forceinline__ void edge_visit(EdgeCuts& C, const EdgeRef& e, const EL& L, int k, const PairGeo& G) {
+  const double px = e.px, py = e.py, qx = e.qx, qy = e.qy, dx = e.dx, dy = e.dy, len2 = e.len2, tol = G.tol;
+  const double ex0 = L.x0[k], ey0 = L.y0[k], ex1 = L.x1[k], ey1 = L.y1[k];
   const double bx0 = fmin(px, qx) - tol, bx1 = fmax(px, qx) + tol, by0 = fmin(py, qy) - tol, by1 = fmax(py, qy) + tol;
-  const double snap2 = G.snap * G.snap;
-  auto visit = [&](int k) {
-    const double ex0 = L.x0[k], ey0 = L.y0[k], ex1 = L.x1[k], ey1 = L.y1[k];
-    if (F ? out_cmp(ex0, ey0, ex1, ey1, bx0, by0, bx1, by1)
-          : (fmax(ex0, ex1) < bx0 || fmin(ex0, ex1) > bx1 || fmax(ey0, ey1) < by0 || fmin(ey0, ey1) > by1)) return false;
-    const uint32_t efl = L.fl[k];
-    const double fx = ex1 - ex0, fy = ey1 - ey0;
-    const double r = dx * fy - dy * fx;
-    const double flen2 = fx * fx + fy * fy;
-    const double c0 = orient(px, py, qx, qy, ex0, ey0), c1 = orient(px, py, qx, qy, ex1, ey1);
-    bool col = (c0 * c0 <= snap2 * len2 || ((efl & 2u) && c0 * c0 <= tol2len2)) && (c1 * c1 <= snap2 * len2 || ((efl & 4u) && c1 * c1 <= tol2len2));
-    if (!col && flen2 > 0) {
-      const double g0 = orient(ex0, ey0, ex1, ey1, px, py), g1 = orient(ex0, ey0, ex1, ey1, qx, qy), tf = tol * tol * flen2;
-      col = (g0 * g0 <= snap2 * flen2 || ((cut & 2u) && g0 * g0 <= tf)) && (g1 * g1 <= snap2 * flen2 || ((cut & 4u) && g1 * g1 <= tf));
+  if (F ? out_cmp(ex0, ey0, ex1, ey1, bx0, by0, bx1, by1)
+        : (fmax(ex0, ex1) < bx0 || fmin(ex0, ex1) > bx1 || fmax(ey0, ey1) < by0 || fmin(ey0, ey1) > by1)) return;
+  const double tol2len2 = tol * tol * len2, eps2 = G.eps_par * G.eps_par, snap2 = G.snap * G.snap;
+  const uint32_t efl = L.fl[k], cut = e.fl;
+  const double fx = ex1 - ex0, fy = ey1 - ey0;
+  const double r = dx * fy - dy * fx;
+  const double flen2 = fx * fx + fy * fy;
+  const double c0 = orient(px, py, qx, qy, ex0, ey0), c1 = orient(px, py, qx, qy, ex1, ey1);
+  bool col = (c0 * c0 <= snap2 * len2 || ((efl & 2u) && c0 * c0 <= tol2len2)) && (c1 * c1 <= snap2 * len2 || ((efl & 4u) && c1 * c1 <= tol2len2));
+  if (!col && flen2 > 0) {
+    const double g0 = orient(ex0, ey0, ex1, ey1, px, py), g1 = orient(ex0, ey0, ex1, ey1, qx, qy), tf = tol * tol * flen2;
+    col = (g0 * g0 <= snap2 * flen2 || ((cut & 2u) && g0 * g0 <= tf)) && (g1 * g1 <= snap2 * flen2 || ((cut & 4u) && g1 * g1 <= tf));
+  }
+  // the ends of a coincident interval, or the parameters of a crossing on both edges: n1 / d and n2 / d
+  const double wx = ex0 - px, wy = ey0 - py;
+  double n1, n2, d;
+  if (col) {
+    d = len2; n1 = wx * dx + wy * dy; n2 = (ex1 - px) * dx + (ey1 - py) * dy;
+  } else {
+    if (!(r * r > eps2 * len2 * flen2)) return;
+    d = r; n1 = wx * fy - wy * fx;
+    if (r > 0 ? (n1 <= 0 || n1 >= r) : (n1 >= 0 || n1 <= r)) return;
+    n2 = wx * dy - wy * dx;
+  }
+  // n / d is n for n = +-0 (up to the zero's sign, which no test reads) and exactly 1 for n = d: a coincident edge's ends need no division
+  n1 = n1 == 0.0 ? 0.0 : (n1 == d ? 1.0 : n1 / d);
+  n2 = n2 == 0.0 ? 0.0 : (n2 == d ? 1.0 : n2 / d);
+  if (col) {
+    const double lo = fmax((double)0, fmin(n1, n2)), hi = fmin((double)1, fmax(n1, n2));
+    if (hi > lo) {
+      if (lo > 0 && C.ns < MAXS) C.ts[C.ns++] = lo;
+      if (hi < 1 && C.ns < MAXS) C.ts[C.ns++] = hi;
+      if (C.no < MAXO) { C.ol0[C.no] = lo; C.ol1[C.no] = hi; C.osame[C.no] = (dx * fx + dy * fy) > 0; C.oidx[C.no] = k; C.no++; }
     }
-    if (col) {
-      double tc = (ex0 - px) * dx + (ey0 - py) * dy, te = (ex1 - px) * dx + (ey1 - py) * dy;
-      if (F) {   // n / len2 is n for n = +-0 and exactly 1 for n = len2 (> 0): a coincident edge's ends need no division
-        tc = tc == 0.0 ? tc : (tc == len2 ? 1.0 : tc / len2);
-        te = te == 0.0 ? te : (te == len2 ? 1.0 : te / len2);
-      } else {
-        tc = tc / len2; te = te / len2;
-      }
-      const double lo = fmax((double)0, fmin(tc, te)), hi = fmin((double)1, fmax(tc, te));
-      if (hi > lo) {
-        if (lo > 0 && ns < MAXS) ts[ns++] = lo;
-        if (hi < 1 && ns < MAXS) ts[ns++] = hi;
-        if (no < MAXO) { ol0[no] = lo; ol1[no] = hi; osame[no] = (dx * fx + dy * fy) > 0; oidx[no] = k; no++; }
-      }
-    } else if (r * r > eps2 * len2 * flen2) {
-      const double wx = ex0 - px, wy = ey0 - py;
-      const double tn = wx * fy - wy * fx;
-      if (r > 0 ? (tn <= 0 || tn >= r) : (tn >= 0 || tn <= r)) return false;
-      const double t = tn / r, u = (wx * dy - wy * dx) / r;
+  } else {
+    bool in = n2 >= 0 && n2 <= 1;
+    if (!in) {
       const double du = tol / (flen2 > 0 ? sqrt(flen2) : (double)1);
-      if (u >= -du && u <= 1 + du && ns < MAXS) ts[ns++] = t;
+      in = n2 >= -du && n2 <= 1 + du;
     }
-    return false;
-  };
-  each_k(visit);
-  for (int a = 1; a < ns; a++) { double v = ts[a]; int b = a - 1; while (b >= 0 && ts[b] > v) { ts[b + 1] = ts[b]; b--; } ts[b + 1] = v; }
+    if (in && C.ns < MAXS) C.ts[C.ns++] = n1;
+  }
+}
+__device__ __forceinline__ void edge_cuts_begin(EdgeCuts& C) { C.ts[0] = 0; C.ts[1] = 1; C.ns = 2; C.no = 0; }
+__device__ __forceinline__ void edge_cuts_sort(EdgeCuts& C) {
+#pragma unroll 1
+  for (int a = 1; a < C.ns; a++) {
+    const double v = C.ts[a];
+    int b = a - 1;
+#pragma unroll 1
+    while (b >= 0 && C.ts[b] > v) { C.ts[b + 1] = C.ts[b]; b--; }
+    C.ts[b + 1] = v;
+  }
+}
+
+// segment k of the edge: its midpoint, the coincident intervals over it, and whether the inside test of the midpoint
+// is read by its value (lens: lengths are wanted and the edge is real; AREA: the area term is wanted)
+template <bool AREA = true, class EL>
+__device__ __forceinline__ Segment edge_segment(const EdgeCuts& C, const EdgeRef& e, const EL& L, int k, const PairGeo& G, bool lens) {
+  Segment s;
+  s.t0 = C.ts[k]; s.t1 = C.ts[k + 1];
+  s.valid = s.t1 > s.t0;
+  const double tm = (double)0.5 * (s.t0 + s.t1);
+  s.mx = e.px + e.dx * tm; s.my = e.py + e.dy * tm;
+  s.net = 0; s.first = -1; s.net_real = 0; s.n_real = 0;
+#pragma unroll 1
+  for (int o = 0; o < C.no; o++)
+    if (tm > C.ol0[o] && tm < C.ol1[o]) {
+      const int sgn = C.osame[o] ? 1 : -1;
+      s.net += sgn; if (s.first < 0) s.first = o;
+      if (!(L.fl[C.oidx[o]] & 1u)) { s.net_real += sgn; s.n_real++; }
+    }
+  const bool half = s.net == 1 || s.net == -1;
+  const bool in_ov = s.mx >= G.ov.x0 && s.mx <= G.ov.x1 && s.my >= G.ov.y0 && s.my <= G.ov.y1;
+  s.need = s.valid && in_ov && ((AREA && (s.first < 0 || !half)) || (lens && s.net_real == 0 && !(s.n_real == 0 && half)));
+  return s;
+}
+// adds the segment's length to l_in / l_on and its term to acc (AREA); vin: the midpoint is inside (false where not needed)
+template <bool AREA = true, class EL>
+__device__ __forceinline__ void edge_segment_add(const Segment& s, const EdgeCuts& C, const EdgeRef& e, const EL& L, const PairGeo& G, bool lens, int vin,
+                                                 double& acc, double& l_in, double& l_on, uint32_t& bits) {
+  const int net = s.net;
+  if (lens) {
+    const double seg = e.len * (s.t1 - s.t0);
+    if (s.net_real != 0) { l_on += seg; bits |= (s.net_real > 0 ? REL_COIN_SAME : REL_COIN_OPP) | REL_TOUCH; }
+    else if (s.n_real == 0 && (net == 1 || net == -1)) l_in += 0.5 * seg;
+    else if (vin) l_in += seg;
+  }
+  if constexpr (!AREA) return;
+  double w;
+  if (s.first < 0) w = vin ? 1.0 : 0.0;
+  else if (net == 1 || net == -1) w = 0.5;
+  else if (net == 0) w = vin ? 1.0 : 0.0;
+  else {
+    const int fo = C.oidx[s.first];
+    const bool sb = left_of(L.x0[fo], L.y0[fo], L.x1[fo], L.y1[fo], s.mx, s.my);
+    const bool m_left = C.osame[s.first] ? sb : !sb;
+    int other = m_left ? vin - net : vin + net;
+    other = other < 0 ? 0 : (other > 1 ? 1 : other);
+    w = 0.5 * (vin + other);
+  }
+  if (w != 0.0) {
+    const double ax = e.px + e.dx * s.t0 - G.cx, ay = e.py + e.dy * s.t0 - G.cy, bx = e.px + e.dx * s.t1 - G.cx, by = e.py + e.dy * s.t1 - G.cy;
+    acc += w * (double)(ax * by - ay * bx);
+  }
+}
+
+// One edge by one lane. each_k(visit) calls visit(k) for the other polygon's local edges k in increasing order: all of
+// them, or only those of a candidate list that holds every k passing the box test (the same visits, the same results).
+template <bool F, class EL, class EachK>
+__device__ double edge_contrib_k(const EL& LS, int i, const EL& L, int cnt, bool in_c, const PairGeo& G, bool rel, double& l_in, double& l_on, uint32_t& bits,
+                                 EachK&& each_k) {
+  const EdgeRef e = edge_ref(LS, i, rel);
+  if (e.len2 == 0) return 0.0;
+  const bool lens = rel && !(e.fl & 1u);
+  EdgeCuts C;
+  edge_cuts_begin(C);
+  each_k([&](int k) { edge_visit<F>(C, e, L, k, G); });
+  edge_cuts_sort(C);
   double acc = 0.0;
-  for (int k = 0; k + 1 < ns; k++) {
-    const double t0 = ts[k], t1 = ts[k + 1];
-    if (!(t1 > t0)) continue;
-    const double tm = (double)0.5 * (t0 + t1);
-    const double mx = px + dx * tm, my = py + dy * tm;
-    const bool in_ov = mx >= G.ov.x0 && mx <= G.ov.x1 && my >= G.ov.y0 && my <= G.ov.y1;
-    int net = 0, first = -1, net_real = 0, n_real = 0;
-    for (int o = 0; o < no; o++)
-      if (tm > ol0[o] && tm < ol1[o]) {
-        const int sgn = osame[o] ? 1 : -1;
-        net += sgn; if (first < 0) first = o;
-        if (!(L.fl[oidx[o]] & 1u)) { net_real += sgn; n_real++; }
-      }
-    // the inside test of the midpoint, evaluated once and only where a branch below reads it
-    const bool lens = l_in && real;
-    const bool need = first < 0 || (net != 1 && net != -1) || (lens && net_real == 0 && !(n_real == 0 && (net == 1 || net == -1)));
-    const int vin = (need && in_ov && inside_from_c<F, S32>(L, cnt, G.cx, G.cy, in_c, mx, my)) ? 1 : 0;
-    if (lens) {
-      const double seg = sqrt(len2) * (t1 - t0);
-      if (net_real != 0) { *l_on += seg; *bits |= (net_real > 0 ? REL_COIN_SAME : REL_COIN_OPP) | REL_TOUCH; }
-      else if (n_real == 0 && (net == 1 || net == -1)) *l_in += 0.5 * seg;
-      else if (vin) *l_in += seg;
-    }
-    double w;
-    if (first < 0) w = vin ? 1.0 : 0.0;
-    else if (net == 1 || net == -1) w = 0.5;
-    else if (net == 0) w = vin ? 1.0 : 0.0;
-    else {
-      const int fo = oidx[first];
-      const bool sb = left_of(L.x0[fo], L.y0[fo], L.x1[fo], L.y1[fo], mx, my);
-      const bool m_left = osame[first] ? sb : !sb;
-      int other = m_left ? vin - net : vin + net;
-      other = other < 0 ? 0 : (other > 1 ? 1 : other);
-      w = 0.5 * (vin + other);
-    }
-    if (w != 0.0) {
-      const double ax = px + dx * t0 - G.cx, ay = py + dy * t0 - G.cy, bx = px + dx * t1 - G.cx, by = py + dy * t1 - G.cy;
-      acc += w * (double)(ax * by - ay * bx);
-    }
+#pragma unroll 1
+  for (int k = 0; k + 1 < C.ns; k++) {
+    const Segment s = edge_segment(C, e, L, k, G, lens);
+    if (!s.valid) continue;
+    const int vin = s.need && inside_from_c<F>(L, cnt, G.cx, G.cy, in_c, s.mx, s.my) ? 1 : 0;
+    edge_segment_add(s, C, e, L, G, lens, vin, acc, l_in, l_on, bits);
   }
   return acc;
 }
-
-template <bool F>
-__device__ __forceinline__ double edge_contrib(double px, double py, double qx, double qy, const EList& L, int cnt, bool in_c, const PairGeo& G,
-                                               bool real, double* l_in, double* l_on, uint32_t* bits, uint32_t cut) {
-  return edge_contrib_k<F, false>(px, py, qx, qy, L, cnt, in_c, G, real, l_in, l_on, bits, cut, [&](auto&& visit) {
+template <bool F, class EL>
+__device__ __forceinline__ double edge_contrib(const EL& LS, int i, const EL& L, int cnt, bool in_c, const PairGeo& G, bool rel, double& l_in, double& l_on,
+                                               uint32_t& bits) {
+  return edge_contrib_k<F>(LS, i, L, cnt, in_c, G, rel, l_in, l_on, bits, [&](auto&& visit) {
+#pragma unroll 1
     for (int k = 0; k < cnt; k++) visit(k);
   });
 }
 
 __device__ __forceinline__ double pair_snap(double2 oa, double2 ea) {   // engine.cuh:524-527
-  double m = fmax(fmax(fabs(oa.x), fabs(oa.x + ea.x)), fmax(fabs(oa.y), fabs(oa.y + ea.y)));
-  return 0.5 * (nextafter(m, INFINITY) - m);
+  const double m = fmax(fmax(fabs(oa.x), fabs(oa.x + ea.x)), fmax(fabs(oa.y), fabs(oa.y + ea.y)));
+  return 0.5 * (__longlong_as_double(__double_as_longlong(m) + 1) - m);   // the next double up: m >= 0
 }
 
-// One pair, whole warp. Returns false when a local list exceeded cap (nothing written).
-// MASK (the filtered shared-memory kernel): candidate edge pairs as bit masks (mb).
-// FLAT (the filtered scratch kernel): candidate lists in global scratch; a pair whose list would exceed fb->cap is
-// handed back (false) and runs with the full sweeps.
-// SELF (> 0, filtered shared-memory bin only): the pair is a geometry with itself in one layer; the caller passes
-// one list of SELF edges as both LA and LB. B's gather and B's contribution pass would repeat A's exactly (the same
-// edges in the same frame, the same candidates in the same order, so the same values): A's pass runs once and each
-// lane adds its recorded values a second time, in the same order, which is the sum the two passes make.
-template <bool F, bool FLAT = false, bool BUCKETS = false, bool MASK = false, bool S32 = false, int SELF = 0>
-__device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList LA, EList LB, int cap,
-                              int lane, uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const FlatBuf* fb = nullptr,
-                              const MaskBuf* mb = nullptr, unsigned long long* ep = nullptr) {
+// a lane's share of a pair's sums: twice the signed area, lengths of A inside / on B and of B inside / on A
+struct PairSums { double s2 = 0.0, ai = 0.0, ao = 0.0, bi = 0.0, bo = 0.0; };
+template <bool AREA = true, bool REL = true>
+__device__ __forceinline__ void pair_result(const PairSums& S, bool sums, bool hit, bool rtouch, uint32_t bits, uint8_t& o_flag, double& o_area, double4& o_ev,
+                                            uint32_t& o_evb) {
+  double ar = 0.0; double4 e4 = make_double4(0, 0, 0, 0); uint32_t eb4 = rtouch ? REL_TOUCH : 0;
+  if (sums) {
+    double s2 = S.s2;
+    if (REL) e4 = make_double4(S.ai, S.ao, S.bi, S.bo);
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {   // warp_sum of the five, side by side
+      if (AREA) s2 += __shfl_down_sync(0xffffffffu, s2, o);
+      if (REL) {
+        e4.x += __shfl_down_sync(0xffffffffu, e4.x, o); e4.y += __shfl_down_sync(0xffffffffu, e4.y, o);
+        e4.z += __shfl_down_sync(0xffffffffu, e4.z, o); e4.w += __shfl_down_sync(0xffffffffu, e4.w, o);
+      }
+    }
+    ar = 0.5 * s2;
+    eb4 = __reduce_or_sync(0xffffffffu, bits);
+  }
+  const bool ev_any = e4.x != 0 || e4.y != 0 || e4.z != 0 || e4.w != 0;
+  o_flag = hit ? 1 : ((ar != 0.0 || ev_any) ? 2 : 0);
+  o_area = ar; o_ev = e4; o_evb = eb4;
+}
+
+// geometry of a pair in the frame of A's origin: overlap box, tolerances, the probe point c
+__device__ __forceinline__ PairGeo pair_geo(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, Frame& A, Frame& B) {
   const double2 oa = P.origin[a], ob = R.origin[b], ea = P.ext[a], eb = R.ext[b];
   const double sx = ob.x - oa.x, sy = ob.y - oa.y;
   const double pad = 4.0 * fmax(rp.tol_abs, (double)rp.tol_rel * fmax(fmax(ea.x, ea.y), fmax(eb.x, eb.y)));
   PairGeo G;
   G.ov = Box{fmax(0.0, sx) - pad, fmax(0.0, sy) - pad, fmin(ea.x, sx + eb.x) + pad, fmin(ea.y, sy + eb.y) + pad};
-  const Frame A = frame_of(P, a, oa.x, oa.y), B = frame_of(R, b, oa.x, oa.y);
+  A = frame_of(P, a, oa.x, oa.y); B = frame_of(R, b, oa.x, oa.y);
   G.tol = fmax(rp.tol_abs, (double)rp.tol_rel * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0));
   G.eps_par = rp.eps_par;
   G.snap = rp.snap_half_ulp ? pair_snap(oa, ea) : 0.0;
   G.cx = (double)(G.ov.x0 + 0.381966 * (G.ov.x1 - G.ov.x0));
   G.cy = (double)(G.ov.y0 + 0.414213 * (G.ov.y1 - G.ov.y0));
-  int na = 0, nb = 0;
-  bool inB_c = false, inA_c = false;
-  for (int side = 0; side < (SELF ? 1 : 2); side++) {   // one inlined copy of the gather
-    bool in = false;
-    // MASK: the containment parity of the probe point c is taken in the gather's pass over each polygon's edges
-    const int n = collect<F, MASK, S32>(side ? B : A, G.ov, side ? LB : LA, cap, lane, G.cx, G.cy, &in);
-    if (side) { nb = n; inB_c = in; } else { na = n; inA_c = in; }
+  return G;
+}
+
+// filtered variants, no real boundary contact: intersects iff a real-edge vertex of one lies inside the other
+// (engine.cuh:577-594); one probe at a time, the warp splitting the other polygon's edges (crossing parity is
+// order-free). any: some probe vertex lies inside.
+template <bool S32, class EL>
+__device__ bool contains_warp(const Frame& A, const Frame& B, const EL& LA, int na, const EL& LB, int nb, bool inA_c, bool inB_c, const PairGeo& G, int lane,
+                              bool& any) {
+  bool h = false;
+#pragma unroll 1
+  for (int side = 0; side < 2 && !h; side++) {
+    const Frame& S = side ? B : A;
+    const EL& LO = side ? LA : LB;
+    const int no_ = side ? na : nb;
+    const bool inc = side ? inA_c : inB_c;
+#pragma unroll 1
+    for (uint32_t r = S.r0; r < S.r1 && !h; r++) {
+      double x, y; const bool real = probe_vertex(S, r, x, y);
+      if (!real) S.v(S.L->rvo[r], x, y);
+      if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c_warp<S32>(LO, no_, G.cx, G.cy, inc, x, y, lane)) {
+        any = true; h = real;
+      }
+    }
   }
-  if constexpr (SELF > 0) { nb = na; inB_c = inA_c; }
+  return h;
+}
+
+// One pair, whole warp. Returns false when a local list exceeded cap (nothing written).
+// FLAT (the filtered scratch kernel): candidate lists in global scratch; a pair whose list would exceed fb->cap is
+// handed back (false) and runs with the full sweeps.
+// SELF (FLAT only): the pair is a geometry with itself in one layer; the caller passes one list as both LA and LB.
+// B's gather and B's contribution pass would repeat A's exactly (the same edges in the same frame, the same candidates
+// in the same order, so the same values): A's pass runs once and each lane adds its recorded values a second time, in
+// the same order, which is the sum the two passes make.
+template <bool F, bool FLAT = false, bool BUCKETS = false, bool SELF = false>
+__device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList LA, EList LB, int cap,
+                              int lane, uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const FlatBuf* fb = nullptr,
+                              unsigned long long* ep = nullptr) {
+  Frame A, B;
+  const PairGeo G = pair_geo(P, R, a, b, rp, A, B);
+  int na = 0, nb = 0;
+#pragma unroll 1
+  for (int side = 0; side < (SELF ? 1 : 2); side++) {   // one inlined copy of the gather
+    const int n = collect<F>(side ? B : A, G.ov, side ? LB : LA, cap, lane);
+    if (side) nb = n; else na = n;
+  }
+  if constexpr (SELF) nb = na;
   if (na > cap || nb > cap) return false;
   __syncwarp();
-  constexpr int MW = SELF ? SELF / 32 : MASK_WORDS, MS = SELF ? SELF : CAP_F;   // mask words per row, row stride
   int ncp = -1;   // candidate edge pairs (FLAT); -1: sweep every edge pair
-  if constexpr (MASK) {
-    mask_candidates<MS, SELF == 0>(LA, na, LB, nb, 2.0 * G.tol, *mb, lane);
-  } else if constexpr (FLAT) {
+  if constexpr (FLAT) {
     ncp = flat_candidates<BUCKETS>(LA, na, LB, nb, 2.0 * G.tol, G.ov, *fb, lane);
     if (ncp > fb->cap) return false;
   }
   // boundary contact
   bool hit = false, hit_any = false;
-  auto seg_loop = [&](int i) {
-    const double px0 = LA.x0[i], py0 = LA.y0[i], px1 = LA.x1[i], py1 = LA.y1[i];
-    const uint32_t fa = LA.fl[i];
-    const double ax0 = fmin(px0, px1), ax1 = fmax(px0, px1), ay0 = fmin(py0, py1), ay1 = fmax(py0, py1);
-    auto test = [&](int j) {
-      const double qx0 = LB.x0[j], qy0 = LB.y0[j], qx1 = LB.x1[j], qy1 = LB.y1[j];
-      if (F ? out_cmp(qx0, qy0, qx1, qy1, ax0, ay0, ax1, ay1)
-            : (fmax(qx0, qx1) < ax0 || fmin(qx0, qx1) > ax1 || fmax(qy0, qy1) < ay0 || fmin(qy0, qy1) > ay1)) return false;
-      if (seg_isect(px0, py0, px1, py1, qx0, qy0, qx1, qy1)) {
-        hit_any = true;
-        if (!((fa | LB.fl[j]) & 1u)) { hit = true; return true; }
-      }
-      return false;
-    };
-    for (int j = 0; j < nb; j++) if (test(j)) break;
-  };
-  if constexpr (MASK) {
-    // each lane walks its A edge's candidates, one per round; the warp stops at the first real contact
-    const int nbw = (nb + 31) >> 5;
-    for (int ic = 0; ic < na && !hit; ic += 32) {
-      const int i = ic + lane;
-      uint32_t w[MW];
-      #pragma unroll
-      for (int q = 0; q < MW; q++) w[q] = (i < na && q < nbw) ? mb->rm[q * MS + i] : 0u;
-      double px0 = 0, py0 = 0, px1 = 0, py1 = 0;
-      uint32_t fa = 0;
-      if (i < na) { px0 = LA.x0[i]; py0 = LA.y0[i]; px1 = LA.x1[i]; py1 = LA.y1[i]; fa = LA.fl[i]; }
-      const double ax0 = px0 < px1 ? px0 : px1, ax1 = px0 < px1 ? px1 : px0, ay0 = py0 < py1 ? py0 : py1, ay1 = py0 < py1 ? py1 : py0;
-      for (;;) {
-        int j = -1;
-        #pragma unroll
-        for (int q = 0; q < MW; q++)
-          if (j < 0 && w[q]) { j = (q << 5) + __ffs(w[q]) - 1; w[q] &= w[q] - 1; }
-        if (!__any_sync(0xffffffffu, j >= 0)) break;
-        if (j >= 0) {
-          const double qx0 = LB.x0[j], qy0 = LB.y0[j], qx1 = LB.x1[j], qy1 = LB.y1[j];
-          if (!out_cmp(qx0, qy0, qx1, qy1, ax0, ay0, ax1, ay1) &&
-              (S32 ? seg_isect32(px0, py0, px1, py1, qx0, qy0, qx1, qy1) : seg_isect(px0, py0, px1, py1, qx0, qy0, qx1, qy1))) {
-            hit_any = true;
-            if (!((fa | LB.fl[j]) & 1u)) hit = true;
-          }
-        }
-        if (__any_sync(0xffffffffu, hit)) { hit = true; break; }
-      }
-    }
-  } else if constexpr (FLAT) {
+  if constexpr (FLAT) {
     // one candidate per lane; the warp stops at the first real contact (hit_any is then implied)
+#pragma unroll 1
     for (int base = 0; base < ncp; base += 32) {
       const int e = base + lane;
       if (e < ncp) {
@@ -474,44 +483,49 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
       if (__any_sync(0xffffffffu, hit)) { hit = true; break; }
     }
   } else {
+    auto seg_loop = [&](int i) {
+      const double px0 = LA.x0[i], py0 = LA.y0[i], px1 = LA.x1[i], py1 = LA.y1[i];
+      const uint32_t fa = LA.fl[i];
+      const double ax0 = fmin(px0, px1), ax1 = fmax(px0, px1), ay0 = fmin(py0, py1), ay1 = fmax(py0, py1);
+      auto test = [&](int j) {
+        const double qx0 = LB.x0[j], qy0 = LB.y0[j], qx1 = LB.x1[j], qy1 = LB.y1[j];
+        if (F ? out_cmp(qx0, qy0, qx1, qy1, ax0, ay0, ax1, ay1)
+              : (fmax(qx0, qx1) < ax0 || fmin(qx0, qx1) > ax1 || fmax(qy0, qy1) < ay0 || fmin(qy0, qy1) > ay1)) return false;
+        if (seg_isect(px0, py0, px1, py1, qx0, qy0, qx1, qy1)) {
+          hit_any = true;
+          if (!((fa | LB.fl[j]) & 1u)) { hit = true; return true; }
+        }
+        return false;
+      };
+#pragma unroll 1
+      for (int j = 0; j < nb; j++) if (test(j)) break;
+    };
+#pragma unroll 1
     for (int i = lane; i < na && !hit; i += 32) seg_loop(i);
   }
   hit = __any_sync(0xffffffffu, hit);
   hit_any = __any_sync(0xffffffffu, hit_any || hit);
   const bool rtouch = hit;
-  if (!MASK && (!hit || rp.want_area || rp.want_relate))
+  bool inB_c = false, inA_c = false;
+  if (!hit || rp.want_area || rp.want_relate)
+#pragma unroll 1
     for (int side = 0; side < 2; side++) {
       const bool in = pip_full_warp(side ? A : B, G.cx, G.cy, lane);
       if (side) inA_c = in; else inB_c = in;
     }
   bool contain_any = false;
   if (!hit) {
-    // no real boundary contact: intersects iff a real-edge vertex of one lies inside the other (engine.cuh:577-594)
-    bool h = false, ha = false;
     if constexpr (F) {
-      // one probe at a time, the warp splitting the other polygon's edges (crossing parity is order-free)
-      for (int side = 0; side < 2 && !h; side++) {
-        const Frame& S = side ? B : A;
-        const DLayer& SL = side ? R : P;
-        const EList& LO = side ? LA : LB;
-        const int no_ = side ? na : nb;
-        const bool inc = side ? inA_c : inB_c;
-        for (uint32_t r = S.r0; r < S.r1 && !h; r++) {
-          double x, y; const bool real = probe_vertex(S, r, x, y);
-          if (!real) S.v(SL.rvo[r], x, y);
-          if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c_warp<S32>(LO, no_, G.cx, G.cy, inc, x, y, lane)) {
-            ha = true; h = real;
-          }
-        }
-      }
-      hit = h;
-      contain_any = ha;
-    } else {
+      hit = contains_warp<false>(A, B, LA, na, LB, nb, inA_c, inB_c, G, lane, contain_any);
+    } else {   // no real boundary contact: intersects iff a real-edge vertex of one lies inside the other (engine.cuh:577-594)
+      bool h = false, ha = false;
+#pragma unroll 1
       for (uint32_t r = A.r0 + lane; r < A.r1 && !h; r += 32) {
         double x, y; const bool real = probe_vertex(A, r, x, y);
         if (!real) A.v(P.rvo[r], x, y);
         if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c<F>(LB, nb, G.cx, G.cy, inB_c, x, y)) { ha = true; h = real; }
       }
+#pragma unroll 1
       for (uint32_t r = B.r0 + lane; r < B.r1 && !h; r += 32) {
         double x, y; const bool real = probe_vertex(B, r, x, y);
         if (!real) B.v(R.rvo[r], x, y);
@@ -521,99 +535,55 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
       contain_any = __any_sync(0xffffffffu, ha);
     }
   }
-  double ar = 0.0; double4 e4 = make_double4(0, 0, 0, 0); uint32_t eb4 = 0;
-  if ((hit || hit_any || contain_any) && (rp.want_area || rp.want_relate)) {
-    double s2 = 0.0, ai = 0, ao = 0, bi = 0, bo = 0;
-    uint32_t bits = rtouch ? REL_TOUCH : 0;
+  PairSums S;
+  uint32_t bits = rtouch ? REL_TOUCH : 0;
+  const bool sums = (hit || hit_any || contain_any) && (rp.want_area || rp.want_relate);
+  if (sums) {
     const bool rel = rp.want_relate != 0;
-    if constexpr (MASK && SELF > 0) {   // A's pass once, then each lane's recorded values added again in order
-      const int nbw = (nb + 31) >> 5;
-      double rec[MW];
-      double lin = 0.0, lon = 0.0;
-      int k = 0;
-      for (int i = lane; i < na; i += 32, k++) {
-        const uint32_t f = LA.fl[i];
-        rec[k] = edge_contrib_k<F, S32>(LA.x0[i], LA.y0[i], LA.x1[i], LA.y1[i], LB, nb, inB_c, G, !(f & 1u), rel ? &lin : nullptr, &lon, &bits, f,
-                                   [&](auto&& visit) {
-                                     for (int q = 0; q < nbw; q++)
-                                       for (uint32_t m = mb->rm[q * MS + i]; m; m &= m - 1) visit((q << 5) + __ffs(m) - 1);
-                                   });
-        s2 += rec[k];
-      }
-      for (int q = 0; q < k; q++) s2 += rec[q];
-      ai = bi = lin; ao = bo = lon;
-    } else if constexpr (MASK) {   // visit only each edge's candidates, in increasing order, by walking the set bits
-      const int nbw = (nb + 31) >> 5, naw = (na + 31) >> 5;
-      for (int pass = 0; pass < 2; pass++) {
-        const EList& LS = pass ? LB : LA;
-        const EList& LO = pass ? LA : LB;
-        const int nself = pass ? nb : na, nother = pass ? na : nb, nw = pass ? naw : nbw;
-        const uint32_t* mrow = pass ? mb->cm : mb->rm;
-        const bool inc = pass ? inA_c : inB_c;
-        double lin = 0.0, lon = 0.0;   // this pass's lengths (each starts from 0, so the sums are the same)
-        for (int i = lane; i < nself; i += 32) {
-          const uint32_t f = LS.fl[i];
-          s2 += edge_contrib_k<F, S32>(LS.x0[i], LS.y0[i], LS.x1[i], LS.y1[i], LO, nother, inc, G, !(f & 1u), rel ? &lin : nullptr, &lon, &bits, f,
-                                  [&](auto&& visit) {
-                                    for (int q = 0; q < nw; q++)
-                                      for (uint32_t m = mrow[q * CAP_F + i]; m; m &= m - 1) visit((q << 5) + __ffs(m) - 1);
-                                  });
-        }
-        if (pass) { bi = lin; bo = lon; } else { ai = lin; ao = lon; }
-      }
-    } else if constexpr (FLAT && SELF > 0) {   // the self pair's A pass, recorded per edge, then added again in order
+    if constexpr (FLAT && SELF) {   // the self pair's A pass, recorded per edge, then added again in order
       const uint32_t* cp = fb->cp;
-      double lin = 0.0, lon = 0.0;
+#pragma unroll 1
       for (int i = lane; i < na; i += 32) {
-        const uint32_t f = LA.fl[i];
         const int r0 = (int)fb->sa[i], r1 = (int)fb->sa[i + 1];
-        const double v = edge_contrib_k<F, S32>(LA.x0[i], LA.y0[i], LA.x1[i], LA.y1[i], LB, nb, inB_c, G, !(f & 1u), rel ? &lin : nullptr, &lon, &bits, f,
-                                           [&](auto&& visit) {
-                                             for (int e = r0; e < r1; e++) visit((int)(cp[e] >> 16));
-                                           });
+        const double v = edge_contrib_k<F>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits, [&](auto&& visit) {
+#pragma unroll 1
+          for (int e = r0; e < r1; e++) visit((int)(cp[e] >> 16));
+        });
         fb->rec[i] = v;
-        s2 += v;
+        S.s2 += v;
       }
-      for (int i = lane; i < na; i += 32) s2 += fb->rec[i];
-      ai = bi = lin; ao = bo = lon;
+#pragma unroll 1
+      for (int i = lane; i < na; i += 32) S.s2 += fb->rec[i];
+      S.bi = S.ai; S.bo = S.ao;
     } else if constexpr (FLAT) {   // visit only each edge's candidates, in the same increasing order; one call site for both passes
       const uint32_t* cp = fb->cp;
       const uint16_t* pj = fb->pj;
+#pragma unroll 1
       for (int pass = 0; pass < 2; pass++) {
         const EList& LS = pass ? LB : LA;
         const EList& LO = pass ? LA : LB;
         const int nself = pass ? nb : na, nother = pass ? na : nb;
         const bool inc = pass ? inA_c : inB_c;
         double lin = 0.0, lon = 0.0;   // this pass's lengths (each starts from 0, so the sums are the same)
+#pragma unroll 1
         for (int i = lane; i < nself; i += 32) {
-          const uint32_t f = LS.fl[i];
           const int r0 = pass ? (i ? (int)fb->sb[i - 1] : 0) : (int)fb->sa[i];
           const int r1 = pass ? (int)fb->sb[i] : (int)fb->sa[i + 1];
-          s2 += edge_contrib_k<F, S32>(LS.x0[i], LS.y0[i], LS.x1[i], LS.y1[i], LO, nother, inc, G, !(f & 1u), rel ? &lin : nullptr, &lon, &bits, f,
-                                  [&](auto&& visit) {
-                                    for (int e = r0; e < r1; e++) visit(pass ? (int)(cp[pj[e]] & 0xFFFFu) : (int)(cp[e] >> 16));
-                                  });
+          S.s2 += edge_contrib_k<F>(LS, i, LO, nother, inc, G, rel, lin, lon, bits, [&](auto&& visit) {
+#pragma unroll 1
+            for (int e = r0; e < r1; e++) visit(pass ? (int)(cp[pj[e]] & 0xFFFFu) : (int)(cp[e] >> 16));
+          });
         }
-        if (pass) { bi = lin; bo = lon; } else { ai = lin; ao = lon; }
+        if (pass) { S.bi = lin; S.bo = lon; } else { S.ai = lin; S.ao = lon; }
       }
     } else {
-      for (int i = lane; i < na; i += 32) {
-        const uint32_t f = LA.fl[i];
-        s2 += edge_contrib<F>(LA.x0[i], LA.y0[i], LA.x1[i], LA.y1[i], LB, nb, inB_c, G, !(f & 1u), rel ? &ai : nullptr, &ao, &bits, f);
-      }
-      for (int i = lane; i < nb; i += 32) {
-        const uint32_t f = LB.fl[i];
-        s2 += edge_contrib<F>(LB.x0[i], LB.y0[i], LB.x1[i], LB.y1[i], LA, na, inA_c, G, !(f & 1u), rel ? &bi : nullptr, &bo, &bits, f);
-      }
+#pragma unroll 1
+      for (int i = lane; i < na; i += 32) S.s2 += edge_contrib<F>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits);
+#pragma unroll 1
+      for (int i = lane; i < nb; i += 32) S.s2 += edge_contrib<F>(LB, i, LA, na, inA_c, G, rel, S.bi, S.bo, bits);
     }
-    s2 = warp_sum(s2); ai = warp_sum(ai); ao = warp_sum(ao); bi = warp_sum(bi); bo = warp_sum(bo);
-    ar = 0.5 * s2;
-    e4 = make_double4(ai, ao, bi, bo);
-    eb4 = __reduce_or_sync(0xffffffffu, bits);
-  } else if (rtouch) eb4 = REL_TOUCH;
-  const bool ev_any = e4.x != 0 || e4.y != 0 || e4.z != 0 || e4.w != 0;
-  o_flag = hit ? 1 : ((ar != 0.0 || ev_any) ? 2 : 0);
-  o_area = ar; o_ev = e4; o_evb = eb4;
+  }
+  pair_result(S, sums, hit, rtouch, bits, o_flag, o_area, o_ev, o_evb);
   if (ep && lane == 0) *ep += (unsigned long long)na * (unsigned long long)nb;   // local edge pairs: the refinement's work unit
   return true;
 }
@@ -624,15 +594,418 @@ __device__ bool refine_pair(const DLayer& P, const DLayer& R, uint32_t a, uint32
   return refine_pair_t<false>(P, R, a, b, rp, LA, LB, cap, lane, o_flag, o_area, o_ev, o_evb);
 }
 
-template <bool F> struct Cfg;
-template <> struct Cfg<false> { static constexpr int cap = CAP; static constexpr size_t list = LIST_BYTES, smem = RB_SMEM, edge = EDGE_BYTES; static constexpr int minb = 3; };
-template <> struct Cfg<true> { static constexpr int cap = CAP_F; static constexpr size_t list = LIST_BYTES_F, smem = RB_SMEM_F + RB_WARPS * MASK_BYTES, edge = EDGE_BYTES_F; static constexpr int minb = 4; };
+// ---- the shared-memory bins' pair routine (filtered variants) -----------------------------------------------------------
+// Per warp: the two edge lists, the boxes of B's edges on a 15-bit grid over the overlap box (qb), a queue of candidate edge
+// pairs (q), the coincident pairs as bit masks (row i of A: the B edges that coincide with part of A's edge i, column j the A
+// edges that do with B's edge j; word w of row i at rm[w * stride + i]) and the split points of both polygons' edges
+// (the unused tails of the list arrays). cand: bit i of A (then bit j of B) set when any edge of the other polygon
+// comes within 2 tol of the edge.
+//
+// The routine is bound by instruction issue, dependent latency (16 warps per SM) and instruction fetch, so the work is laid out to keep
+// lanes busy side by side and the code small: edge pairs whose boxes come within 2 tol are queued and classified 32 at a
+// time, one per lane, from the four orientations of the pair, which decide the contact and every cut the two edges make in each
+// other. The contribution passes are left with the coincident pairs, one per shared edge. The inside tests of a
+// pass's segments are taken one at a time by the whole warp, and edges that follow one another with no edge of the
+// other polygon within 2 tol share one test (edge_pass).
+// Loops are kept rolled on purpose: the kernel runs nearly straight through its code, and above about 48 KB of it the
+// warps wait for instructions (100k parcels, this kernel: 71 KB 5.66 ms, 54 KB 3.82 ms, 49 KB 2.86 ms, with the
+// instruction-fetch stall at 8.6, 4.3 and 0.9 cycles an instruction).
+// 100k-parcel relate self-join, against lanes that each visited their own edge's candidates: this bin 3.45 -> 2.86 ms, the
+// self bin 1.44 -> 0.76 ms; two 60k layers, area: 4.35 -> 3.16 ms (14.5 -> 20.5 lanes active per instruction).
+constexpr int QCAP = 64;
+struct MaskBuf { uint32_t* rm; uint32_t* cm; uint2* qb; uint32_t* cand; uint16_t* q; };
 
-template <bool F>
-__device__ __forceinline__ EList carve_t(unsigned char* base, int cap) { return F ? carve_f(base, cap) : carve(base, cap); }
+// the box of an edge on the 15-bit grid, packed so that one subtraction per axis tests both ends: bit 31 of (B - A) is
+// B's upper end >= A's lower end, bit 15 A's upper end >= B's lower end (fields of 16 bits, no borrow between them).
+// Every step is monotone in the coordinate, so boxes that meet are never told apart; coordinates outside the overlap
+// box clamp to its sides.
+struct QGrid { double x0, y0; float sx, sy; };
+struct QBox { int x0, y0, x1, y1; };
+__device__ __forceinline__ QGrid qgrid(const Box& ov) {
+  QGrid g{ov.x0, ov.y0, 0.f, 0.f};
+  const float w = (float)(ov.x1 - ov.x0), h = (float)(ov.y1 - ov.y0);
+  if (w > 1e-30f) g.sx = 1.f / w;
+  if (h > 1e-30f) g.sy = 1.f / h;
+  return g;
+}
+__device__ __forceinline__ int qcell(double v, double o, float s) { return __float2int_rd(__saturatef((float)(v - o) * s) * 32767.f); }
+template <class EL>
+__device__ __forceinline__ QBox qbox(const QGrid& g, const EL& L, int i) {
+  const int px = qcell(L.x0[i], g.x0, g.sx), py = qcell(L.y0[i], g.y0, g.sy), qx = qcell(L.x1[i], g.x0, g.sx), qy = qcell(L.y1[i], g.y0, g.sy);
+  return QBox{min(px, qx), min(py, qy), max(px, qx), max(py, qy)};
+}
+
+// Split points found by the classification: edge and parameter, in the tails of a list's arrays (n of MS entries in
+// use): the parameters behind x0 and x1, the edges behind y0 and y1. 2 (MS - n) of them fit.
+template <int MS, class EL>
+__device__ __forceinline__ double* split_slot(const EL& L, int n, int s) { return L.x0 + n + (s < MS - n ? s : s + 2 * MS - (MS - n)); }
+struct Splits { int a, b; bool full; };   // split points of A's and of B's edges so far (uniform); full: some did not fit
+
+// Classifies one candidate edge pair (i of A, j of B) per lane: real / any contact (seg_isect on the four orientations
+// of the pair, behind the same box test), and for either edge what edge_visit finds for it: coincidence (a bit in the
+// masks) or a split point. The two edges' conditions are the same but for their box tests, the order of a product and
+// the end tolerances; r, tn and un change sign together when the edges swap roles, so un / r is B's parameter.
+template <int MS, bool SELF, bool CUTS, class EL>
+__device__ __forceinline__ void classify_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const MaskBuf& mb, uint32_t e, bool act, int lane,
+                                               Splits& sp, bool& hit, bool& hit_any) {
+  const int i = (int)(e >> 8), j = (int)(e & 255u);
+  bool sa = false, sb = false;
+  double t = 0, u = 0;
+  if (act) {
+    const double px = LA.x0[i], py = LA.y0[i], qx = LA.x1[i], qy = LA.y1[i];
+    const double ex0 = LB.x0[j], ey0 = LB.y0[j], ex1 = LB.x1[j], ey1 = LB.y1[j];
+    const uint32_t fa = LA.fl[i], fb = LB.fl[j];
+    const double c0 = orient(px, py, qx, qy, ex0, ey0), c1 = orient(px, py, qx, qy, ex1, ey1);
+    const double g0 = orient(ex0, ey0, ex1, ey1, px, py), g1 = orient(ex0, ey0, ex1, ey1, qx, qy);
+    const double ax0 = px < qx ? px : qx, ax1 = px < qx ? qx : px, ay0 = py < qy ? py : qy, ay1 = py < qy ? qy : py;
+    const double bx0 = ex0 < ex1 ? ex0 : ex1, bx1 = ex0 < ex1 ? ex1 : ex0, by0 = ey0 < ey1 ? ey0 : ey1, by1 = ey0 < ey1 ? ey1 : ey0;
+    const bool near = !(bx1 < ax0 || bx0 > ax1 || by1 < ay0 || by0 > ay1);
+    if (!SELF && near) {
+      bool is = ((g0 > 0 && g1 < 0) || (g0 < 0 && g1 > 0)) && ((c0 > 0 && c1 < 0) || (c0 < 0 && c1 > 0));
+      is = is || (g0 == 0 && px >= bx0 && px <= bx1 && py >= by0 && py <= by1) || (g1 == 0 && qx >= bx0 && qx <= bx1 && qy >= by0 && qy <= by1) ||
+           (c0 == 0 && ex0 >= ax0 && ex0 <= ax1 && ey0 >= ay0 && ey0 <= ay1) || (c1 == 0 && ex1 >= ax0 && ex1 <= ax1 && ey1 >= ay0 && ey1 <= ay1);
+      if (is) { hit_any = true; if (!((fa | fb) & 1u)) hit = true; }
+    }
+    if constexpr (CUTS) {
+      const double tol = G.tol;
+      bool ka = near, kb = near;   // the box tests of the two edges, padded by tol
+      if (!near) {
+        ka = !(bx1 < ax0 - tol || bx0 > ax1 + tol || by1 < ay0 - tol || by0 > ay1 + tol);
+        kb = !(ax1 < bx0 - tol || ax0 > bx1 + tol || ay1 < by0 - tol || ay0 > by1 + tol);
+      }
+      const double dx = qx - px, dy = qy - py, fx = ex1 - ex0, fy = ey1 - ey0;
+      const double len2 = dx * dx + dy * dy, flen2 = fx * fx + fy * fy, snap2 = G.snap * G.snap, eps2 = G.eps_par * G.eps_par;
+      // an end's distance passes within the snap distance, a cut point's within tol as well
+      const double ca = snap2 * len2, cat = fmax(ca, tol * tol * len2), cb = snap2 * flen2, cbt = fmax(cb, tol * tol * flen2);
+      const bool onA = c0 * c0 <= ((fb & 2u) ? cat : ca) && c1 * c1 <= ((fb & 4u) ? cat : ca);
+      const bool onB = g0 * g0 <= ((fa & 2u) ? cbt : cb) && g1 * g1 <= ((fa & 4u) ? cbt : cb);
+      ka = ka && len2 != 0; kb = kb && flen2 != 0;
+      if (onA || onB) {
+        if (ka && (onA || flen2 > 0)) atomicOr(&mb.rm[(j >> 5) * MS + i], 1u << (j & 31));
+        if (kb && (onB || len2 > 0)) atomicOr(SELF ? &mb.rm[(i >> 5) * MS + j] : &mb.cm[(i >> 5) * MS + j], 1u << (i & 31));
+      }
+      const double r = dx * fy - dy * fx, wx = ex0 - px, wy = ey0 - py, tn = wx * fy - wy * fx, un = wx * dy - wy * dx;
+      sa = ka && !(onA || (flen2 > 0 && onB)) && r * r > eps2 * len2 * flen2 && (r > 0 ? (tn > 0 && tn < r) : (tn < 0 && tn > r));
+      sb = kb && !(onB || (len2 > 0 && onA)) && r * r > eps2 * flen2 * len2 && (r > 0 ? (un > 0 && un < r) : (un < 0 && un > r));
+      if (sa || sb) {
+#pragma unroll 1
+        for (int z = 0; z < 2; z++) {   // one site for the division and the square root: t, then u; beyond an end: within its tolerance?
+          const double q = (z ? un : tn) / r, f2 = z ? flen2 : len2;
+          bool in = q >= 0 && q <= 1;
+          if (!in) { const double d = tol / (f2 > 0 ? sqrt(f2) : (double)1); in = q >= -d && q <= 1 + d; }
+          if (z) { u = q; sa = sa && in; } else { t = q; sb = sb && in; }
+        }
+      }
+    }
+  }
+  if constexpr (!CUTS) return;
+  const unsigned ma = __ballot_sync(0xffffffffu, sa), mB = __ballot_sync(0xffffffffu, sb);
+  if (ma | mB) {
+    const unsigned lt = (1u << lane) - 1;
+    const int na2 = sp.a + __popc(ma), b0 = SELF ? na2 : sp.b, nb2 = b0 + __popc(mB);
+    sp.full = sp.full || na2 > 2 * (MS - na) || nb2 > 2 * (MS - (SELF ? na : nb));
+    if (!sp.full) {
+      if (sa) {
+        double* d = split_slot<MS>(LA, na, sp.a + __popc(ma & lt));
+        d[0] = t;
+        *reinterpret_cast<int*>(d + MS) = i;
+      }
+      if (sb) {
+        double* d = split_slot<MS>(SELF ? LA : LB, SELF ? na : nb, b0 + __popc(mB & lt));
+        d[0] = u;
+        *reinterpret_cast<int*>(d + MS) = j;
+      }
+    }
+    sp.a = SELF ? nb2 : na2;
+    sp.b = SELF ? 0 : nb2;
+  }
+}
+
+// the interval that edge k of the other polygon, coincident with part of edge e, covers of it (edge_visit's arithmetic)
+template <class EL>
+__device__ __forceinline__ void edge_cover(EdgeCuts& C, const EdgeRef& e, const EL& L, int k) {
+  double tc = 0, te = 0;
+#pragma unroll 1
+  for (int z = 0; z < 2; z++) {   // one site for the division; exact twins, the shared edges of a tiling, need none
+    const double n = ((z ? L.x1 : L.x0)[k] - e.px) * e.dx + ((z ? L.y1 : L.y0)[k] - e.py) * e.dy;
+    tc = te;
+    te = n == 0.0 ? 0.0 : (n == e.len2 ? 1.0 : n / e.len2);
+  }
+  const double lo = fmax((double)0, fmin(tc, te)), hi = fmin((double)1, fmax(tc, te));
+  if (!(hi > lo)) return;
+  if (lo > 0 && C.ns < MAXS) C.ts[C.ns++] = lo;
+  if (hi < 1 && C.ns < MAXS) C.ts[C.ns++] = hi;
+  if (C.no < MAXO) {
+    C.ol0[C.no] = lo; C.ol1[C.no] = hi; C.oidx[C.no] = k;
+    C.osame[C.no] = (e.dx * (L.x1[k] - L.x0[k]) + e.dy * (L.y1[k] - L.y0[k])) > 0;
+    C.no++;
+  }
+}
+
+// Candidate edge pairs (boxes within 2 tol of each other, or a little more on the grid) found and classified; CUTS: the cuts
+// are wanted, else the contact alone. A lane keeps the
+// grid box of one A edge (per 32) in registers and tests B's edges one after the other, each read once for the whole
+// warp (a shared-memory broadcast); the pairs go through the queue. Returns at the first real contact when nothing but
+// the flag is wanted. SELF: only j > i is searched (an edge always coincides with itself).
+template <int MS, bool SELF, bool CUTS, class EL>
+__device__ Splits find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const MaskBuf& mb, int lane, bool& hit, bool& hit_any) {
+  const int nbw = (nb + 31) >> 5;
+  const unsigned lt = (1u << lane) - 1;
+  const QGrid g = qgrid(G.ov);
+  const float pad = 2.f * (float)G.tol;
+  const int cx = 2 + (int)fminf(pad * g.sx * 32767.f, 32767.f), cy = 2 + (int)fminf(pad * g.sy * 32767.f, 32767.f);   // 2 tol in cells, rounded up
+  if constexpr (CUTS) {
+    uint4* z = reinterpret_cast<uint4*>(mb.rm);
+#pragma unroll 1
+    for (int t = lane; t < (SELF ? 1 : 2) * (MS / 32) * MS / 4; t += 32) z[t] = make_uint4(0u, 0u, 0u, 0u);
+    __syncwarp();
+  }
+#pragma unroll 1
+  for (int j = lane; j < nb; j += 32) {
+    const QBox b = qbox(g, LB, j);
+    mb.qb[j] = make_uint2(0x80008000u + (uint32_t)(b.x1 << 16 | (0x7FFF - b.x0)), 0x80008000u + (uint32_t)(b.y1 << 16 | (0x7FFF - b.y0)));
+    if (CUTS && SELF) mb.rm[(j >> 5) * MS + j] = 1u << (j & 31);
+  }
+  if (!SELF && lane < 2 * (MS / 32)) mb.cand[lane] = 0u;
+  __syncwarp();
+  Splits sp{0, 0, false};
+  int qn = 0, ic = 0, w = -1;   // ic, w: the 32 A edges and the 32 B edges being tested
+  uint32_t bits = 0, any = 0;
+  uint2 ab = make_uint2(0u, 0u);
+  for (bool more = na > 0 && nb > 0; more || qn > 0;) {
+    while (more && qn < 32) {
+      const unsigned m = __ballot_sync(0xffffffffu, bits != 0);
+      if (m) {   // each lane queues one of its pairs
+        if (bits) {
+          mb.q[qn + __popc(m & lt)] = (uint16_t)((ic + lane) << 8 | ((w << 5) + __ffs(bits) - 1));
+          bits &= bits - 1;
+        }
+        qn += __popc(m);
+        continue;
+      }
+      if (w < 0 || ++w >= nbw) {   // next 32 A edges
+        if (w >= nbw) {
+          if (!SELF && CUTS) {
+            const unsigned c = __ballot_sync(0xffffffffu, any != 0);
+            if (lane == 0) mb.cand[ic >> 5] = c;
+          }
+          ic += 32;
+          any = 0;
+          if (ic >= na) { more = false; break; }
+        }
+        w = SELF ? ic >> 5 : 0;
+        const int i = ic + lane;
+        if (i < na) {
+          const QBox b = qbox(g, LA, i);
+          ab = make_uint2((uint32_t)(max(b.x0 - cx, 0) << 16 | (0x7FFF - min(b.x1 + cx, 0x7FFF))),
+                          (uint32_t)(max(b.y0 - cy, 0) << 16 | (0x7FFF - min(b.y1 + cy, 0x7FFF))));
+        }
+      }
+      const uint2* qb = mb.qb + (w << 5);
+      const int n = min(32, nb - (w << 5));
+#pragma unroll 1
+      for (int j = 0; j < n; j += 4)   // up to 3 entries past the end are masked below
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+          const uint2 b = qb[j + q];
+          if (((b.x - ab.x) & (b.y - ab.y) & 0x80008000u) == 0x80008000u) bits |= 1u << (j + q);
+        }
+      if (n < 32) bits &= (1u << n) - 1u;
+      if (ic + lane >= na) bits = 0;
+      if (SELF) { if (w == (ic >> 5)) bits &= ~((2u << lane) - 1u); }
+      else if constexpr (CUTS) {
+        any |= bits;
+        const uint32_t ob = __reduce_or_sync(0xffffffffu, bits);
+        if (lane == 0) mb.cand[MS / 32 + w] |= ob;
+      }
+    }
+    __syncwarp();
+    const uint32_t e = mb.q[lane];
+    const uint16_t rest = mb.q[32 + lane];
+    classify_pairs<MS, SELF, CUTS>(LA, na, LB, nb, G, mb, e, lane < qn, lane, sp, hit, hit_any);
+    if (!CUTS && __any_sync(0xffffffffu, hit)) break;
+    __syncwarp();
+    qn = max(qn - 32, 0);
+    if (lane < qn) mb.q[lane] = rest;
+    __syncwarp();
+  }
+  __syncwarp();
+  return sp;
+}
+
+// One polygon's contribution pass: lane l owns edges l, l + 32, ... and adds its values in that order. Each lane collects its
+// edge's split points and coincident intervals; the segments are then taken in step, the k-th of every edge at once,
+// and their inside tests by the whole warp, one after the other. Returns false when an edge's split points reach the
+// number that is kept (which of them are kept depends on the order in which they are met).
+// Edges with no edge of the other polygon within 2 tol have one segment and no cut. Two of them that share an end
+// point are connected by a path that keeps at least 2 tol away from the other polygon, so their midpoints lie on the same side of it: a run
+// of such edges takes one test. (The crossing-parity test returns the true side for points this far from the boundary:
+// its orientation signs can only be wrong for points within rounding, ~1e-7 of tol, of an edge's line.) tol below
+// 1e-12 of the overlap box (a caller's own tolerances) turns the sharing off.
+template <bool S32, int MS, bool SELF, bool AREA, bool REL, class EL>
+__device__ __forceinline__ bool edge_pass(const EL& LS, int nself, int nsplit, const EL& LO, int nother, const uint32_t* mrow, const uint32_t* cand, bool inc,
+                                          const PairGeo& G, bool share, int lane, double& s2, double& lin, double& lon, uint32_t& bits, double* rec) {
+  const int nw = (nother + 31) >> 5;
+  const unsigned le = (2u << lane) - 1u;
+#pragma unroll 1
+  for (int ic = 0, c = 0; ic < nself; ic += 32, c++) {
+    const int i = ic + lane;
+    EdgeRef e;
+    EdgeCuts C;
+    edge_cuts_begin(C);
+#pragma unroll 1
+    for (int k = 0; k < nsplit; k++) {
+      const double* d = split_slot<MS>(LS, nself, k);
+      if (*reinterpret_cast<const int*>(d + MS) == i && C.ns < MAXS) C.ts[C.ns++] = d[0];
+    }
+    e.px = e.py = e.qx = e.qy = e.dx = e.dy = e.len2 = e.len = 0.0; e.fl = 0;
+    if (i < nself) {
+      e = edge_ref(LS, i, REL);
+#pragma unroll 1
+      for (int w = 0; w < nw; w++)
+#pragma unroll 1
+        for (uint32_t m = mrow[w * MS + i]; m; m &= m - 1) edge_cover(C, e, LO, (w << 5) + __ffs(m) - 1);
+      edge_cuts_sort(C);
+    }
+    if (__any_sync(0xffffffffu, C.ns == MAXS)) return false;
+    if (e.len2 == 0) C.ns = 0;
+    const bool lens = REL && !(e.fl & 1u);
+    unsigned link = 0;   // bit l: edges l - 1 and l are free of the other polygon and share an end point
+    if constexpr (!SELF) {
+      const unsigned fr = share ? ~cand[c] : 0u;
+      const double prx = __shfl_up_sync(0xffffffffu, e.qx, 1), pry = __shfl_up_sync(0xffffffffu, e.qy, 1);
+      link = __ballot_sync(0xffffffffu, i < nself && lane > 0 && prx == e.px && pry == e.py) & fr & (fr << 1);
+    }
+    double acc = 0.0;
+#pragma unroll 1
+    for (int k = 0; __any_sync(0xffffffffu, k + 1 < C.ns); k++) {
+      Segment s;
+      s.valid = s.need = false;
+      s.mx = s.my = 0;
+      if (k + 1 < C.ns) s = edge_segment<AREA>(C, e, LO, k, G, lens);
+      int vin = 0;
+      const unsigned needm = __ballot_sync(0xffffffffu, s.need);
+      if (needm) {
+        // this lane's run of linked edges: [start, end); its first edge that needs the test takes it for all
+        const unsigned heads = k == 0 ? ~link : 0xffffffffu;
+        const int start = 31 - __clz(heads & le);
+        const unsigned after = heads & ~le;
+        const unsigned run = (after ? (after & (0u - after)) - 1u : 0xffffffffu) & ~((1u << start) - 1u);
+        const int tester = __ffs(needm & run) - 1;
+        unsigned in = 0;
+#pragma unroll 1
+        for (unsigned m = __ballot_sync(0xffffffffu, s.need && tester == lane); m; m &= m - 1) {
+          const int src = __ffs(m) - 1;
+          const double x = __shfl_sync(0xffffffffu, s.mx, src), y = __shfl_sync(0xffffffffu, s.my, src);
+          if (inside_from_c_warp<S32>(LO, nother, G.cx, G.cy, inc, x, y, lane)) in |= 1u << src;
+        }
+        vin = s.need && ((in >> tester) & 1u) ? 1 : 0;
+      }
+      if (s.valid) edge_segment_add<AREA>(s, C, e, LO, G, lens, vin, acc, lin, lon, bits);
+    }
+    if (AREA) s2 += acc;
+    if (AREA && rec) rec[c] = acc;
+  }
+  return true;
+}
+
+// What a pair's refinement has to give: the flag alone; the area; the DE-9IM evidence of intersecting pairs (flag 1; the others are
+// not told apart); everything. Each is compiled by itself: what is not wanted costs neither instructions nor
+// instruction-cache room.
+enum Want { W_FLAG = 0, W_AREA = 1, W_REL = 2, W_ALL = 3 };
+
+// One pair by one warp from shared memory. Returns false (nothing written) when a local list exceeded cap or the split
+// points the room kept for them.
+// SELF (> 0): the pair is a geometry with itself in one layer; the caller passes one list of up to SELF edges as both LA and LB. B's
+// gather and B's contribution pass would repeat A's exactly (the same edges in the same frame, the same cuts in the same
+// order, so the same values): A's pass runs once and each lane adds its recorded values a second time, in the same
+// order, which is the sum the two passes make. Every edge meets itself, so the contact needs no test.
+template <bool S32, int SELF, int W>
+__device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList8 LA, EList8 LB, int cap, int lane,
+                              uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const MaskBuf& mb, unsigned long long* ep) {
+  constexpr int MS = SELF ? SELF : CAP_F;   // row stride of the masks
+  constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
+  Frame A, B;
+  const PairGeo G = pair_geo(P, R, a, b, rp, A, B);
+  int na = 0, nb = 0;
+  bool inB_c = false, inA_c = false;
+#pragma unroll 1
+  for (int side = 0; side < (SELF ? 1 : 2); side++) {   // one inlined copy of the gather; it also takes the parity of the probe point c
+    bool in = false;
+    const int n = collect<true, true, S32>(side ? B : A, G.ov, side ? LB : LA, cap, lane, G.cx, G.cy, &in);
+    if (side) { nb = n; inB_c = in; } else { na = n; inA_c = in; }
+  }
+  if constexpr (SELF > 0) { nb = na; inB_c = inA_c; }
+  if (na > cap || nb > cap) return false;
+  __syncwarp();
+  bool hit = false, hit_any = false;
+  Splits sp{0, 0, false};
+  if constexpr (SELF > 0) {
+#pragma unroll 1
+    for (int i = lane; i < na; i += 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
+    if constexpr (W != W_FLAG) sp = find_pairs<MS, true, true>(LA, na, LB, nb, G, mb, lane, hit, hit_any);
+  } else {
+    sp = find_pairs<MS, false, W != W_FLAG>(LA, na, LB, nb, G, mb, lane, hit, hit_any);
+  }
+  if (sp.full) return false;
+  hit = __any_sync(0xffffffffu, hit);
+  hit_any = __any_sync(0xffffffffu, hit_any || hit);
+  const bool rtouch = hit;
+  if (!hit) hit = contains_warp<S32>(A, B, LA, na, LB, nb, inA_c, inB_c, G, lane, hit_any);
+  PairSums S;
+  uint32_t bits = rtouch ? REL_TOUCH : 0;
+  const bool sums = W != W_FLAG && (hit || (W != W_REL && hit_any));
+  if constexpr (W != W_FLAG)
+    if (sums) {
+      const bool share = G.tol >= 1e-12 * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0);
+      if constexpr (SELF > 0) {
+        double rec[SELF / 32];
+        if (!edge_pass<S32, MS, true, AREA, REL>(LA, na, sp.a, LB, nb, mb.rm, mb.cand, inB_c, G, false, lane, S.s2, S.ai, S.ao, bits, rec)) return false;
+#pragma unroll 1
+        for (int c = 0; AREA && c * 32 < na; c++) S.s2 += rec[c];
+        S.bi = S.ai; S.bo = S.ao;
+      } else {
+#pragma unroll 1
+        for (int pass = 0; pass < 2; pass++) {   // one inlined copy of the pass
+          double lin = 0.0, lon = 0.0;   // this pass's lengths (each starts from 0, so the sums are the same)
+          if (!edge_pass<S32, MS, false, AREA, REL>(pass ? LB : LA, pass ? nb : na, pass ? sp.b : sp.a, pass ? LA : LB, pass ? na : nb, pass ? mb.cm : mb.rm,
+                                                    mb.cand + (pass ? MS / 32 : 0), pass ? inA_c : inB_c, G, share, lane, S.s2, lin, lon, bits, nullptr))
+            return false;
+          if (pass) { S.bi = lin; S.bo = lon; } else { S.ai = lin; S.ao = lon; }
+        }
+      }
+    }
+  pair_result<AREA, REL>(S, sums, hit, rtouch, bits, o_flag, o_area, o_ev, o_evb);
+  if (lane == 0) *ep += (unsigned long long)na * (unsigned long long)nb;   // local edge pairs: the refinement's work unit
+  return true;
+}
+
+// shared memory of one warp of the filtered bins: lists (one for self pairs), row masks, column masks, grid boxes, cand,
+// queue, flags; every part starts on a multiple of 8 bytes
+__host__ __device__ constexpr size_t mask_warp_bytes(int cap, bool self) {
+  return (size_t)(self ? 1 : 2) * cap * EDGE_BYTES_8 + (size_t)(self ? 1 : 2) * (cap / 32) * cap * 4 + (size_t)cap * 8 + 2 * (cap / 32) * 4 + QCAP * 2;
+}
+static_assert(mask_warp_bytes(128, false) % 16 == 0 && mask_warp_bytes(192, true) % 16 == 0, "a warp's part starts on 16 bytes");
+template <int MS, bool SELF>
+__device__ __forceinline__ void carve_mask(unsigned char* base, EList8& LA, EList8& LB, MaskBuf& mb) {
+  double* d = reinterpret_cast<double*>(base);
+  auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + MS; L.x1 = d + 2 * MS; L.y1 = d + 3 * MS; d += 4 * MS; };
+  doubles(LA);
+  if (!SELF) doubles(LB);
+  mb.qb = reinterpret_cast<uint2*>(d);
+  mb.rm = reinterpret_cast<uint32_t*>(mb.qb + MS);
+  mb.cm = mb.rm + (MS / 32) * MS;
+  mb.cand = SELF ? mb.cm : mb.cm + (MS / 32) * MS;
+  mb.q = reinterpret_cast<uint16_t*>(mb.cand + 2 * (MS / 32));
+  LA.fl = reinterpret_cast<uint8_t*>(mb.q + QCAP);
+  if (SELF) LB = LA; else LB.fl = LA.fl + MS;
+}
+template <bool F> struct Cfg;
+template <> struct Cfg<false> { static constexpr int cap = CAP; static constexpr size_t smem = RB_SMEM; static constexpr int minb = 3; };
+template <> struct Cfg<true> { static constexpr int cap = CAP_F; static constexpr size_t smem = RB_WARPS * mask_warp_bytes(CAP_F, false); static constexpr int minb = 4; };
 
 // S32 (filtered only): the contact test's and the gather's orientation signs through the certified FP32 filter
-template <bool F, bool S32 = false>
+template <bool F, bool S32 = false, int W = W_ALL>
 __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
                                                                         RefineArgs rp, uint8_t* flag, double* area, double4* ev, uint32_t* evb,
                                                                         uint32_t* heavy, unsigned long long* nheavy, unsigned long long* next,
@@ -643,19 +1016,22 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   if (lane == 0) s_ep[wib] = 0;
   __syncwarp();
-  EList LA = carve_t<F>(smem + (size_t)wib * 2 * Cfg<F>::list, Cfg<F>::cap);
-  EList LB = carve_t<F>(smem + (size_t)wib * 2 * Cfg<F>::list + Cfg<F>::list, Cfg<F>::cap);
-  MaskBuf mbuf{nullptr, nullptr};
-  if constexpr (F) {   // after the lists of all warps: row masks, then column masks
-    unsigned char* mbase = smem + (size_t)RB_WARPS * 2 * Cfg<F>::list + (size_t)wib * MASK_BYTES;
-    mbuf.rm = reinterpret_cast<uint32_t*>(mbase);
-    mbuf.cm = mbuf.rm + MASK_WORDS * CAP_F;
+  EList LA, LB;
+  EList8 MA, MB;
+  MaskBuf mbuf;
+  if constexpr (F) {
+    carve_mask<CAP_F, false>(smem + (size_t)wib * mask_warp_bytes(CAP_F, false), MA, MB, mbuf);
+  } else {
+    LA = carve(smem + (size_t)wib * 2 * LIST_BYTES, CAP);
+    LB = carve(smem + (size_t)wib * 2 * LIST_BYTES + LIST_BYTES, CAP);
   }
   auto one = [&](uint64_t p) {
     const uint2 pr = pairs[p];
     if (skip_self && pr.x == pr.y) return;   // a geometry with itself: the self bin's
     uint8_t f; double ar; double4 e4; uint32_t b4;
-    const bool ok = refine_pair_t<F, false, false, F, S32>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &mbuf, &s_ep[wib]);
+    bool ok;
+    if constexpr (F) ok = refine_pair_m<S32, 0, W>(P, R, pr.x, pr.y, rp, MA, MB, bin_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
+    else ok = refine_pair_t<false>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &s_ep[wib]);
     if (lane == 0) {
       if (!ok) { heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)p; flag[p] = 0; }
       else {
@@ -691,10 +1067,8 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P
 // for the row masks; the largest that keeps 4 blocks of 4 warps per SM: 256 with 3 blocks measured 5 % slower),
 // row masks only, A's gather and contribution pass only (refine_pair_t SELF).
 constexpr int CAP_SELF = 192;
-constexpr size_t SELF_LIST = (size_t)CAP_SELF * EDGE_BYTES_F;
-constexpr size_t SELF_MASK = (size_t)(CAP_SELF / 32) * CAP_SELF * sizeof(uint32_t);
-constexpr size_t SELF_SMEM = (size_t)RB_WARPS * (SELF_LIST + SELF_MASK);
-constexpr int SELF_MINB = 4;   // blocks per SM: 4 x 46 KB of shared memory
+constexpr size_t SELF_SMEM = RB_WARPS * mask_warp_bytes(CAP_SELF, true);
+constexpr int SELF_MINB = 4;   // blocks per SM: 4 x 51 KB of shared memory
 
 // positions of the self pairs (a == b) among the candidate pairs, warp-aggregated (order free: outputs go by position)
 __global__ void k_self_index(const uint2* __restrict__ pairs, uint64_t np, uint32_t* sidx, unsigned long long* nself) {
@@ -712,7 +1086,7 @@ __global__ void k_self_index(const uint2* __restrict__ pairs, uint64_t np, uint3
   }
 }
 
-template <bool S32>
+template <bool S32, int W>
 __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer P, const uint2* __restrict__ pairs, const uint32_t* __restrict__ sidx,
                                                                           const unsigned long long* nself, RefineArgs rp, uint8_t* flag, double* area,
                                                                           double4* ev, uint32_t* evb, uint32_t* heavy, unsigned long long* nheavy,
@@ -723,10 +1097,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   if (lane == 0) s_ep[wib] = 0;
   __syncwarp();
-  const EList L = carve_f(smem + (size_t)wib * SELF_LIST, CAP_SELF);
+  EList8 L, L2;
   MaskBuf mbuf;
-  mbuf.rm = reinterpret_cast<uint32_t*>(smem + (size_t)RB_WARPS * SELF_LIST + (size_t)wib * SELF_MASK);
-  mbuf.cm = nullptr;
+  carve_mask<CAP_SELF, true>(smem + (size_t)wib * mask_warp_bytes(CAP_SELF, true), L, L2, mbuf);
   const uint64_t n = *nself;   // written by k_self_index, launched before this kernel
   for (int k = 0; k < runs; k++) {
     unsigned long long h0 = 0;
@@ -738,8 +1111,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
       const uint32_t p = sidx[h];
       const uint2 pr = pairs[p];
       uint8_t f; double ar; double4 e4; uint32_t b4;
-      const bool ok = refine_pair_t<true, false, false, true, S32, CAP_SELF>(P, P, pr.x, pr.y, rp, L, L, self_cap, lane, f, ar, e4, b4, nullptr, &mbuf,
-                                                                            &s_ep[wib]);
+      const bool ok = refine_pair_m<S32, CAP_SELF, W>(P, P, pr.x, pr.y, rp, L, L, self_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
       if (lane == 0) {
         if (!ok) { heavy[atomicAdd(nheavy, 1ull)] = p; flag[p] = 0; }
         else {
@@ -759,7 +1131,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
 // keeps its candidate list there (cph entries); a pair with more candidates runs the full sweeps instead.
 template <bool F>
 __host__ __device__ constexpr size_t scratch_per_warp(int cap, int cph) {
-  return ((2 * (size_t)cap * Cfg<F>::edge + (F ? (size_t)cph * 6 + 2 * ((size_t)cap + 1) * 4 + ((size_t)(2 * cap + 64) + NBK + 1) * 4 : 0)) + 15) &
+  return ((2 * (size_t)cap * EDGE_BYTES + (F ? (size_t)cph * 6 + 2 * ((size_t)cap + 1) * 4 + ((size_t)(2 * cap + 64) + NBK + 1) * 4 : 0)) + 15) &
          ~(size_t)15;
 }
 template <bool F>
@@ -773,10 +1145,10 @@ __global__ void __launch_bounds__(128) k_refine_scratch(DLayer P, DLayer R, cons
   unsigned long long ep = 0;
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   unsigned char* base = scratch + w * scratch_per_warp<F>(cap, cph);
-  EList LA = carve_t<F>(base, cap), LB = carve_t<F>(base + (size_t)cap * Cfg<F>::edge, cap);
+  EList LA = carve(base, cap), LB = carve(base + (size_t)cap * EDGE_BYTES, cap);
   FlatBuf fb;
   if constexpr (F) {   // cp (u32), sa, sb (u32), pj (u16) after the lists
-    fb.cp = reinterpret_cast<uint32_t*>(base + 2 * (size_t)cap * Cfg<F>::edge);
+    fb.cp = reinterpret_cast<uint32_t*>(base + 2 * (size_t)cap * EDGE_BYTES);
     fb.sa = fb.cp + cph;
     fb.sb = fb.sa + (cap + 1);
     fb.bl = fb.sb + (cap + 1);
@@ -798,12 +1170,12 @@ __global__ void __launch_bounds__(128) k_refine_scratch(DLayer P, DLayer R, cons
     bool ok;
     if constexpr (F) {   // candidate entries pack both edge indices in 16 bits each
       if (same_layer && pr.x == pr.y)   // a geometry with itself: one list, one contribution pass (B's list records it)
-        ok = cap <= 0xFFFF && refine_pair_t<F, true, true, false, false, 1>(P, P, pr.x, pr.y, rp, LA, LA, cap, lane, f, ar, e4, b4, &fb, nullptr, &ep);
+        ok = cap <= 0xFFFF && refine_pair_t<F, true, true, true>(P, P, pr.x, pr.y, rp, LA, LA, cap, lane, f, ar, e4, b4, &fb, &ep);
       else
-        ok = cap <= 0xFFFF && refine_pair_t<F, true, true>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, &fb, nullptr, &ep);
-      if (!ok) ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, nullptr, &ep);
+        ok = cap <= 0xFFFF && refine_pair_t<F, true, true>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, &fb, &ep);
+      if (!ok) ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
     } else {
-      ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, nullptr, &ep);
+      ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
     }
     if (lane == 0) {
       if (!ok) *err = 1;
@@ -834,13 +1206,14 @@ static ScratchGeom scratch_geom(const gsj_layer* P, const gsj_layer* R) {
 // shared-memory bin (pairs whose local lists fit bin_cap), then the scratch bin (the pairs the first bin listed as
 // oversized; it reads their count on the device, so no host round trip separates the bins); then one stream sync.
 // The executable graph is built once per context and variant and re-parameterised per call.
-template <bool F, bool S32 = false>
+template <bool F, bool S32 = false, int W = W_ALL>
 static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, uint8_t* flag,
                      double* area, double4* ev, uint32_t* evb) {
   cudaStream_t s = c->stream;
-  const int bit = S32 ? 4 : (F ? 2 : 1);
+  constexpr int variant = F ? 1 + 4 * S32 + W : 0;   // plain, filtered x W, filtered FP32 x W
+  const int bit = 1 << variant;
   if (!(c->refine_attr & bit)) {
-    GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F>::smem));
+    GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F>::smem));
     c->refine_attr |= bit;
   }
   const RefineShape& sh = c->shape;
@@ -861,13 +1234,14 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   } else {
     blocks = (int)std::min<uint64_t>((np + RB_WARPS - 1) / RB_WARPS, (uint64_t)c->sm_count * 8);
   }
-  // a pair can only be oversized when one of its polygons has more edges than the bin holds
-  const bool scr = std::max(P->max_geom_edges, R->max_geom_edges) > (uint32_t)bin_cap;
+  // a pair can only be oversized when one of its polygons has more edges than the bin holds; the filtered bins also hand
+  // on the rare pairs whose split points they cannot keep, so they always have a scratch bin behind them (a few warps)
+  const bool big = std::max(P->max_geom_edges, R->max_geom_edges) > (uint32_t)bin_cap, scr = F || big;
   const ScratchGeom sg = scratch_geom<F>(P, R);
   int sblocks = 0;
   unsigned char* sbuf = nullptr;
   if (scr) {   // warps: the shape's share of every SM, at most one per pair and at most 1 GiB of lists
-    uint64_t nwarps = std::min<uint64_t>((uint64_t)c->sm_count * sh.scratch_wpsm, std::max<uint64_t>(1, (1ull << 30) / sg.per));
+    uint64_t nwarps = std::min<uint64_t>((uint64_t)c->sm_count * (big ? sh.scratch_wpsm : 1), std::max<uint64_t>(1, (1ull << 30) / sg.per));
     nwarps = std::min<uint64_t>(nwarps, np);
     nwarps = (nwarps + 3) / 4 * 4;
     sblocks = (int)(nwarps / 4);
@@ -880,9 +1254,9 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   uint32_t* sidx = nullptr;
   const int self_cap = std::min(sh.bin_cap + sh.bin_cap / 2, CAP_SELF);   // 1.5 x the shape's shared-memory bin threshold
   if (self) {
-    const int sbit = S32 ? 16 : 8;
+    const int sbit = 1 << (16 + variant);
     if (!(c->refine_attr & sbit)) {
-      GSJ_CK(cudaFuncSetAttribute(k_refine_self<S32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SELF_SMEM));
+      GSJ_CK(cudaFuncSetAttribute(k_refine_self<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SELF_SMEM));
       c->refine_attr |= sbit;
     }
     sidx = c->selfidx.as<uint32_t>(np);
@@ -897,14 +1271,14 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   unsigned long long* h = c->h_refine.as<unsigned long long>(4);
   // counters: [0] oversized pairs, [1] error word, [2] pair counter, [3] local edge pairs, [4] scratch pair counter,
   // [5] self pairs, [6] self pair counter
-  auto a_main = kernel_args(k_refine<F, S32>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
+  auto a_main = kernel_args(k_refine<F, S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
                             self ? 1 : 0);
   auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, sbuf, sg.cap, sg.cph, err, ctr + 3,
                            ctr + 4, P == R ? 1 : 0);
   auto a_idx = kernel_args(k_self_index, pairs, np, sidx, ctr + 5);
-  auto a_self = kernel_args(k_refine_self<S32>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
+  auto a_self = kernel_args(k_refine_self<S32, W>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
   cudaKernelNodeParams km{}, ks{}, ki{}, kf{};
-  km.func = (void*)k_refine<F, S32>;
+  km.func = (void*)k_refine<F, S32, W>;
   km.gridDim = dim3(blocks);
   km.blockDim = dim3(RB_WARPS * 32);
   km.sharedMemBytes = (unsigned)Cfg<F>::smem;
@@ -917,12 +1291,12 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   ki.gridDim = dim3(iblocks);
   ki.blockDim = dim3(256);
   ki.kernelParams = a_idx.ptr;
-  kf.func = (void*)k_refine_self<S32>;
+  kf.func = (void*)k_refine_self<S32, W>;
   kf.gridDim = dim3(fblocks);
   kf.blockDim = dim3(RB_WARPS * 32);
   kf.sharedMemBytes = (unsigned)SELF_SMEM;
   kf.kernelParams = a_self.ptr;
-  RefineGraph& g = c->rgraph[((S32 ? 2 : (F ? 1 : 0)) * 2 + (scr ? 1 : 0)) * 2 + (self ? 1 : 0)];
+  RefineGraph& g = c->rgraph[variant * 4 + (scr ? 2 : 0) + (self ? 1 : 0)];
   if (!g.exec) {   // the graph is kept with its executable: the node handles used for the updates belong to it
     if (!g.graph) {
       GSJ_CK(cudaGraphCreate(&g.graph, 0));
@@ -953,10 +1327,18 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
 }
 
 void refine_enqueue(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, int mode,
-                    uint8_t* flag, double* area, double4* ev, uint32_t* evb) {
+                    uint8_t* flag, double* area, double4* ev, uint32_t* evb, bool hits_only) {
   if (!np) return;
-  if (mode == GSJ_REFINE_FILTERED_FP32) refine_t<true, true>(c, P, R, pairs, np, rp, flag, area, ev, evb);
-  else if (mode == GSJ_REFINE_FILTERED) refine_t<true>(c, P, R, pairs, np, rp, flag, area, ev, evb);
+  const int w = !rp.want_relate ? (rp.want_area ? W_AREA : W_FLAG) : (hits_only && !area ? W_REL : W_ALL);
+  auto go = [&](auto s32) {
+    constexpr bool S32 = decltype(s32)::value;
+    if (w == W_FLAG) refine_t<true, S32, W_FLAG>(c, P, R, pairs, np, rp, flag, area, ev, evb);
+    else if (w == W_AREA) refine_t<true, S32, W_AREA>(c, P, R, pairs, np, rp, flag, area, ev, evb);
+    else if (w == W_REL) refine_t<true, S32, W_REL>(c, P, R, pairs, np, rp, flag, area, ev, evb);
+    else refine_t<true, S32, W_ALL>(c, P, R, pairs, np, rp, flag, area, ev, evb);
+  };
+  if (mode == GSJ_REFINE_FILTERED_FP32) go(std::true_type{});
+  else if (mode == GSJ_REFINE_FILTERED) go(std::false_type{});
   else refine_t<false>(c, P, R, pairs, np, rp, flag, area, ev, evb);
 }
 

@@ -1,0 +1,85 @@
+"""The shared-memory bins of the refinement at the sizes where they hand pairs on: an edge cut more often than its split
+list holds, more split points than the room behind the edge lists, edge lists at multiples of the mask words, an
+overlap box of no height, tolerances of zero. Every variant has to give the oracle's rows bit for bit."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import gsj
+import pyoracle as O
+from shapes import S, make_set, square
+
+pytestmark = pytest.mark.gpu
+MODES = [gsj.GSJ_REFINE_PLAIN, gsj.GSJ_REFINE_FILTERED, gsj.GSJ_REFINE_FILTERED_FP32]
+
+
+def comb(teeth, w, h, x0=0.0, y0=0.0, flip=False):
+    """A comb of upright teeth on a bar: 4 teeth + 3 edges; flip: lying on its side."""
+    pts = [(x0, y0), (x0 + w, y0)]
+    for t in reversed(range(teeth)):
+        a, b = x0 + w * (t + 0.25) / teeth, x0 + w * (t + 0.75) / teeth
+        pts += [(b, y0 + 0.1 * h), (b, y0 + h), (a, y0 + h), (a, y0 + 0.1 * h)]
+    pts += [(x0, y0 + 0.1 * h), (x0, y0)]
+    return [(y, x) for x, y in reversed(pts)] if flip else pts
+
+
+def ngon(n, r, cx=0.0, cy=0.0):
+    a = 2 * np.pi * np.arange(n) / n
+    p = [(cx + r * np.cos(t), cy + r * np.sin(t)) for t in a]
+    return p + p[:1]
+
+
+SHAPES = {
+    # a bar across every tooth: 2 x teeth splits on its long edges (an edge keeps 22 beside its ends)
+    **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28)},
+    # crossed combs: more split points than fit behind the lists
+    "combs_9": ([[comb(9, 10 * S, 10 * S)]], [[comb(9, 10 * S, 10 * S, flip=True)]]),
+    "combs_28": ([[comb(28, 10 * S, 10 * S)]], [[comb(28, 10 * S, 10 * S, flip=True)]]),
+    # level neighbours: the overlap box is as thin as its pad
+    "touch": ([[square(0, 0, S)]], [[square(0, S, S)], [square(S, S, S)]]),
+    "twins": ([[square(0, 0, S)], [comb(9, S, S)]], [[square(0, 0, S)], [comb(9, S, S)]]),
+}
+for _n in (31, 32, 33, 64, 96, 127, 128, 129):
+    SHAPES[f"ngon_{_n}"] = ([[ngon(_n, S)]], [[ngon(_n, S, 0.3 * S, 0.2 * S)], [ngon(7, 0.2 * S)]])
+
+
+def rows(r):
+    i = np.lexsort((r.pairs[:, 1], r.pairs[:, 0]))
+    return r.pairs[i], None if r.area is None else r.area[i], None if r.code is None else r.code[i]
+
+
+@pytest.mark.parametrize("name", sorted(SHAPES))
+@pytest.mark.parametrize("area,relate", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_handed_on_pairs(engine, name, area, relate):
+    A, B = (make_set(g) for g in SHAPES[name])
+    both = make_set([*SHAPES[name][0], *SHAPES[name][1]])
+    for P, R, up in ((A, B, False), (B, A, False), (both, both, True)):
+        p, oa, oc, _ = O.join(O.OSet(P), O.OSet(R), O.params(area, relate), upper=up)
+        lp = engine.upload_polygons(P)
+        lr = lp if R is P else engine.upload_polygons(R)
+        for m in MODES:
+            gp, ga, gc = rows(engine.join(lp, lr, want_area=bool(area), want_relate=bool(relate), upper=up, refine_mode=m))
+            assert np.array_equal(gp, p)
+            assert not area or np.array_equal(ga, oa)
+            assert not relate or np.array_equal(gc, oc)
+
+
+@pytest.mark.parametrize("tol", [0.0, 1e-11, 1e-7])
+def test_own_tolerances(engine, tol):
+    """Tolerances of zero turn the shared inside tests off, wide ones make whole edges candidates: as the plain kernels."""
+    from gsj import gen
+    P, R = gen.layer_parcels(1500, (-118.30, 33.95, -118.25, 34.00), seed=5), gen.layer_parcels(900, (-118.30, 33.95, -118.25, 34.00), seed=6)
+    lp, lr = engine.upload_polygons(P), engine.upload_polygons(R)
+    for a, b in ((lp, lr), (lp, lp)):
+        pairs = np.ascontiguousarray(engine.candidates(a, b))
+        got = []
+        for m in MODES:
+            n = len(pairs)
+            out = [np.zeros(n, np.uint8), np.zeros(n), np.zeros((n, 4)), np.zeros(n, np.uint32)]
+            rp = gsj.refine_params(True, True)
+            rp.tol_abs, rp.tol_rel = tol, 0.0
+            engine._check(gsj.lib().gsj_refine_pairs(engine.ctx, a.h, b.h, pairs.ctypes.data, n, ctypes.byref(rp), m, *[x.ctypes.data for x in out]))
+            got.append(out)
+        for out in got[1:]:
+            assert all(np.array_equal(x, y) for x, y in zip(got[0], out))
