@@ -359,64 +359,92 @@ __global__ void k_pt_dwithin(const double2* __restrict__ pts, DLayer R, const ui
 }
 
 // The same decision with a warp per (point, piece): lanes take consecutive edges of each ring (coalesced vertex
-// loads), each edge evaluated by exactly the code above; "within" is an any-of and the crossing parity an XOR over
-// the edges, so the ballots give the thread kernel's answer. A warp stops after the chunk in which some lane found
-// an edge within d (the answer is then 1 whatever the parity). The per-point set-up (scales, band) of 32 pairs is
-// computed one pair per lane and handed to the warp with shuffles, the same values bit for bit.
+// loads); "within" is an any-of and the crossing parity an XOR over the edges, so the ballots give the thread kernel's
+// answer. A warp stops after the chunk in which some lane found an edge within d (the answer is then 1 whatever the parity).
+// The set-up of 32 pairs (scales, band, reach, the piece's first ring) is computed one pair per lane and handed to the
+// warp with shuffles. Only edges whose box comes within the pair's reach - d plus the widest band an edge of the piece
+// can have, with a margin of 1e-6 that covers the rounding of the distance - are measured (they are measured by exactly the
+// code above): most chunks of 32 edges have none and cost a box test and the parity.
+// The geodesic is needed only where no edge is surely within d and some edge's distance lies in the band around d (a pair in
+// thousands): such a pair is put on a list for the GEO form, which measures it again. Without the geodesic's
+// registers 24 instead of 16 warps fit an SM.
+// Bound by issue and FP64 / memory latency. 2.1M pairs of 1M points x 200k parcels: measuring every edge with the geodesic inlined
+// 3.87 ms (914 warp instructions a pair), the reach test 2.65 ms, the geodesic on a list
+// 1.65 ms at 6 blocks an SM (8 blocks, with spills in the loop: 1.91 ms).
 __device__ __forceinline__ double shfl_d(double v, int k) { return __shfl_sync(0xffffffffu, v, k); }
-__global__ void __launch_bounds__(128, 4) k_pt_dwithin_warp(const double2* __restrict__ pts, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
-                                                          double d, uint8_t* hit) {
+template <bool GEO>
+__global__ void __launch_bounds__(128, GEO ? 4 : 6) k_pt_dwithin_warp(const double2* __restrict__ pts, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
+                                                                    double d, uint8_t* hit, uint32_t* geo, unsigned long long* ngeo) {
   const int lane = threadIdx.x & 31;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+  if (GEO) np = *ngeo;   // written by the first form, launched before this one on the same stream
   for (uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; i0 < np; i0 += nw * 32) {
-    uint2 mpr = make_uint2(0, 0);
-    double mx = 0, my = 0, mkx = 0, mky = 0, mtl = 0, mdelta = 0;
+    double mx = 0, my = 0, mox = 0, moy = 0, mkx = 0, mky = 0, mtl = 0, mdelta = 0, mrx = 0, mry = 0;
+    uint32_t mr0 = 0, mr1 = 0, mn = 0, mp = 0;
+    uint64_t ms = 0;
     if (i0 + lane < np) {
-      mpr = pairs[i0 + lane];
-      const double2 pt = pts[mpr.x];
-      mx = pt.x; my = pt.y;
+      mp = GEO ? geo[i0 + lane] : (uint32_t)(i0 + lane);
+      const uint2 pr = pairs[mp];
+      const double2 pt = pts[pr.x], o = R.origin[pr.y], ext = R.ext[pr.y];
+      mr0 = R.gro[pr.y]; mr1 = R.gro[pr.y + 1];
+      if (mr0 < mr1) { ms = R.rvo[mr0]; mn = (uint32_t)(R.rvo[mr0 + 1] - ms); }
+      mx = pt.x; my = pt.y; mox = o.x; moy = o.y;
       m_per_deg(pt.y, mkx, mky);
       const double gy = d / mky;
       mtl = fabs(tan(pt.y * DEG)) + 0.01;
       mdelta = 2.0 * gy * DEG * (mtl + 0.04) + 1e-9;
+      const double wx = ext.x * mkx, wy = ext.y * mky, reach = (d + geog_band(d, mdelta, (wx * wx + wy * wy) * 1.001, 0.0, mtl)) * (1.0 + 1e-6);
+      mrx = reach / mkx; mry = reach / mky;
     }
     const int cnt = np - i0 < 32 ? (int)(np - i0) : 32;
+    bool mhit = false, mgeo = false;
+#pragma unroll 1
     for (int k = 0; k < cnt; k++) {
-      const uint32_t g = __shfl_sync(0xffffffffu, mpr.y, k);
-      const double2 pt = make_double2(shfl_d(mx, k), shfl_d(my, k));
-      const double kx = shfl_d(mkx, k), ky = shfl_d(mky, k), tl = shfl_d(mtl, k), delta = shfl_d(mdelta, k);
-      const double2 o = R.origin[g];
-      const Frame B = frame_of(R, g, o.x, o.y);
-      const double px = pt.x - o.x, py = pt.y - o.y;
-      const double ox = B.shx - 1.0;
-      bool par = false, h = false;
-      for (uint32_t r = B.r0; r < B.r1; r++) {
-        const uint64_t s0 = R.rvo[r], e = R.rvo[r + 1];
-        for (uint64_t base = s0 + 1; base < e; base += 32) {
-          const uint64_t j = base + lane;
-          if (j < e) {
-            double x0, y0, x1, y1; B.v(j - 1, x0, y0); B.v(j, x1, y1);
-            if (!R.syn(j - 1)) {
-              const double d2 = pt_seg_d2(px * kx, py * ky, x0 * kx, y0 * ky, x1 * kx, y1 * ky);
-              const double ex = (x1 - x0) * kx, ey = (y1 - y0) * ky;
+      const uint32_t r0 = __shfl_sync(0xffffffffu, mr0, k), r1 = __shfl_sync(0xffffffffu, mr1, k);
+      const double px = shfl_d(mx - mox, k), py = shfl_d(my - moy, k), rx = shfl_d(mrx, k), ry = shfl_d(mry, k);
+      const double bx0 = px - rx, bx1 = px + rx, by0 = py - ry, by1 = py + ry;
+      uint64_t s = __shfl_sync(0xffffffffu, (unsigned long long)ms, k);
+      uint32_t n = __shfl_sync(0xffffffffu, mn, k);
+      bool par = false, h = false, g = false;
+#pragma unroll 1
+      for (uint32_t r = r0; r < r1; r++) {
+        if (r > r0) { s = R.rvo[r]; n = (uint32_t)(R.rvo[r + 1] - s); }
+        const double2* v = R.xy + s;
+#pragma unroll 1
+        for (uint32_t base = 0; base + 1 < n; base += 32) {
+          const uint32_t j = base + lane;
+          double2 a = make_double2(0, 0), b = a;
+          bool near = false;
+          if (j + 1 < n) {
+            a = v[j]; b = v[j + 1];
+            near = !out_cmp(a.x, a.y, b.x, b.y, bx0, by0, bx1, by1) && !R.syn(s + j);
+            if (!((a.y > py) == (b.y > py) && a.y != py && b.y != py)) par = par != ray_crosses(a.x, a.y, b.x, b.y, -1.0, px, py);
+          }
+          if (__any_sync(0xffffffffu, near)) {
+            const double kx = shfl_d(mkx, k), ky = shfl_d(mky, k), tl = shfl_d(mtl, k), delta = shfl_d(mdelta, k);
+            const double ptx = GEO ? shfl_d(mx, k) : 0, pty = GEO ? shfl_d(my, k) : 0, ogx = GEO ? shfl_d(mox, k) : 0, ogy = GEO ? shfl_d(moy, k) : 0;
+            if (near) {
+              const double d2 = pt_seg_d2(px * kx, py * ky, a.x * kx, a.y * ky, b.x * kx, b.y * ky);
+              const double ex = (b.x - a.x) * kx, ey = (b.y - a.y) * ky;
               const double band = geog_band(d, delta, ex * ex + ey * ey, 0.0, tl), dlo = d - band, dhi = d + band;
-              if (d2 <= dlo * dlo || (d2 <= dhi * dhi && geog_dist_inl(o.x + x0, o.y + y0, o.x + x1, o.y + y1, pt.x, pt.y, pt.x, pt.y, true) <= d)) h = true;
-            }
-            if (!((y0 > py) == (y1 > py) && y0 != py && y1 != py)) {
-              const bool so = left_of(x0, y0, x1, y1, ox, py), sp = left_of(x0, y0, x1, y1, px, py);
-              if (so != sp) {
-                const bool su = orient(ox, py, px, py, x0, y0) > 0, sv = orient(ox, py, px, py, x1, y1) > 0;
-                if (su != sv) par = !par;
+              if (d2 <= dlo * dlo) h = true;
+              else if (d2 <= dhi * dhi) {
+                if constexpr (GEO) h = h || geog_dist_inl(ogx + a.x, ogy + a.y, ogx + b.x, ogy + b.y, ptx, pty, ptx, pty, true) <= d;
+                else g = true;
               }
             }
+            if (__any_sync(0xffffffffu, h)) break;
           }
-          if (__any_sync(0xffffffffu, h)) break;
         }
         if (__any_sync(0xffffffffu, h)) break;
       }
-      const bool within = __any_sync(0xffffffffu, h);
-      const bool inside = (__popc(__ballot_sync(0xffffffffu, par)) & 1) != 0;
-      if (lane == 0) hit[i0 + k] = (within || inside) ? 1 : 0;
+      const bool res = __any_sync(0xffffffffu, h) || (__popc(__ballot_sync(0xffffffffu, par)) & 1) != 0;
+      const bool open = !GEO && __any_sync(0xffffffffu, g) && !res;
+      if (lane == k) { mhit = res; mgeo = open; }
+    }
+    if (i0 + lane < np) {
+      hit[mp] = mhit ? 1 : 0;
+      if (!GEO && mgeo) geo[atomicAdd(ngeo, 1ull)] = mp;
     }
   }
 }
@@ -1300,13 +1328,7 @@ __global__ void __launch_bounds__(128) k_pt_erode_warp(const double2* __restrict
           bool syn = false;
           if (valid) {
             vx(j, x0, y0); vx(j + 1, x1, y1);
-            if (!((y0 > 0) == (y1 > 0) && y0 != 0 && y1 != 0)) {
-              const bool so = left_of(x0, y0, x1, y1, ox, 0.0), sp = left_of(x0, y0, x1, y1, 0.0, 0.0);
-              if (so != sp) {
-                const bool su = orient(ox, 0.0, 0.0, 0.0, x0, y0) > 0, sv = orient(ox, 0.0, 0.0, 0.0, x1, y1) > 0;
-                if (su != sv) par = !par;
-              }
-            }
+            if (!((y0 > 0) == (y1 > 0) && y0 != 0 && y1 != 0)) par = par != ray_crosses(x0, y0, x1, y1, ox, 0.0, 0.0);
             L = hypot(x1 - x0, y1 - y0);
             syn = R.syn(j);
             if (!syn && L != 0) { ux = (x1 - x0) / L; uy = (y1 - y0) / L; }
@@ -1393,8 +1415,12 @@ void points_buffer_host(gsj_ctx* c, const gsj_layer* pts, const gsj_layer* R, do
     }
     else if (o.refine_mode == GSJ_REFINE_PLAIN) { k_pt_dwithin<<<grid_for(np, 128), 128, 0, s>>>(pts->pts, R->d, pairs, np, d, hit); c->launches++; }
     else {
-      const int G = (int)std::min<uint64_t>((np + 127) / 128, (uint64_t)c->sm_count * 16);   // a warp per 32 pairs
-      k_pt_dwithin_warp<<<G, 128, 0, s>>>(pts->pts, R->d, pairs, np, d, hit); c->launches++;
+      const int G = (int)std::min<uint64_t>((np + 127) / 128, (uint64_t)c->sm_count * 32);   // a warp per 32 pairs
+      uint32_t* geo = c->heavy.as<uint32_t>(np);
+      unsigned long long* ngeo = c->counters.as<unsigned long long>(8);
+      GSJ_CK(cudaMemsetAsync(ngeo, 0, sizeof(*ngeo), s));
+      k_pt_dwithin_warp<false><<<G, 128, 0, s>>>(pts->pts, R->d, pairs, np, d, hit, geo, ngeo); c->launches++;
+      k_pt_dwithin_warp<true><<<std::min(G, c->sm_count * 4), 128, 0, s>>>(pts->pts, R->d, pairs, np, d, hit, geo, ngeo); c->launches++;
     }
     GSJ_CK(cudaGetLastError());
     st.refine_ms += tm.stop();

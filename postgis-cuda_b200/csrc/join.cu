@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cub/cub.cuh>
 #include "engine.h"
+#include "pairkit.cuh"
 
 namespace gsj {
 
@@ -248,33 +249,48 @@ void run_join(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const RefineAr
 }
 
 // ---- points in polygons (k_pip_pairs, engine.cuh:1079-1106) ---------------------------------------------------
-__global__ void k_pip(const double2* __restrict__ pts, DLayer R, const uint2* __restrict__ pairs, uint64_t np, uint8_t* hit) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= np) return;
-  const uint2 pr = pairs[i];
-  const double2 pt = pts[pr.x], o = R.origin[pr.y];
-  const Frame B = frame_of(R, pr.y, o.x, o.y);
-  const double px = (double)(pt.x - o.x), py = (double)(pt.y - o.y);
-  const double ox = B.shx - (double)1;
+// 8 lanes per (point, piece): they take every 8th edge of the piece's rings, so a group reads 128 consecutive bytes of
+// vertices a step. A first sweep only marks the edges that reach the point's level (about two of a ring), a second one tests
+// the marked edges, so that the lanes of a warp run the orientations side by side. "On the boundary" is an any-of and the
+// crossing parity an XOR over the edges: each lane keeps its own and the group combines them once at the end.
+// Bound by memory latency and issue. 1.95M pairs of 1M points x 200k parcels: a thread per pair, testing as it walks
+// (8 of 32 lanes active), 0.92 ms; 8 lanes testing as they walk 0.95 ms; 0.84 ms in two sweeps.
+constexpr int PIP_LANES = 8;
+__global__ void __launch_bounds__(128) k_pip(const double2* __restrict__ pts, DLayer R, const uint2* __restrict__ pairs, uint64_t np, uint8_t* hit) {
+  const uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / PIP_LANES;
+  const int sub = threadIdx.x % PIP_LANES;
   bool par = false, on = false;
-  for (uint32_t r = B.r0; r < B.r1 && !on; r++) {
-    const uint64_t s0 = R.rvo[r], e = R.rvo[r + 1];
-    double x0, y0; B.v(s0, x0, y0);
-    for (uint64_t j = s0 + 1; j < e; j++) {
-      double x1, y1; B.v(j, x1, y1);
-      if (!((y0 > py) == (y1 > py) && y0 != py && y1 != py)) {
-        const double o_ = orient(x0, y0, x1, y1, px, py);
-        if (o_ == 0 && !R.syn(j - 1) && onseg(x0, y0, x1, y1, px, py)) { on = true; break; }
-        bool so = left_of(x0, y0, x1, y1, ox, py), sp = left_of(x0, y0, x1, y1, px, py);
-        if (so != sp) {
-          bool su = orient(ox, py, px, py, x0, y0) > 0, sv = orient(ox, py, px, py, x1, y1) > 0;
-          if (su != sv) par = !par;
+  if (i < np) {
+    const uint2 pr = pairs[i];
+    const double2 pt = pts[pr.x], o = R.origin[pr.y];
+    const double px = (double)(pt.x - o.x), py = (double)(pt.y - o.y);   // the piece's own frame: its left side is at 0
+    const uint32_t r0 = R.gro[pr.y], r1 = R.gro[pr.y + 1];
+    for (uint32_t r = r0; r < r1; r++) {
+      const uint64_t s0 = R.rvo[r];
+      const uint32_t n = (uint32_t)(R.rvo[r + 1] - s0);
+      const double2* v = R.xy + s0;
+      for (uint32_t base = sub; base + 1 < n; base += 32 * PIP_LANES) {   // 32 edges of the lane
+        uint32_t mark = 0;
+#pragma unroll 4
+        for (uint32_t t = 0; t < 32; t++) {
+          const uint32_t j = base + t * PIP_LANES;
+          if (j + 1 >= n) break;
+          const double y0 = v[j].y, y1 = v[j + 1].y;
+          if (!((y0 > py) == (y1 > py) && y0 != py && y1 != py)) mark |= 1u << t;
+        }
+        for (; mark; mark &= mark - 1) {
+          const uint32_t j = base + (__ffs(mark) - 1) * PIP_LANES;
+          const double2 a = v[j], b = v[j + 1];
+          on = on || (orient(a.x, a.y, b.x, b.y, px, py) == 0 && !R.syn(s0 + j) && onseg(a.x, a.y, b.x, b.y, px, py));
+          par = par != ray_crosses(a.x, a.y, b.x, b.y, -1.0, px, py);
         }
       }
-      x0 = x1; y0 = y1;
     }
   }
-  hit[i] = on ? 2 : (par ? 1 : 0);
+  const int shift = (threadIdx.x & 31) & ~(PIP_LANES - 1);
+  const unsigned m = (1u << PIP_LANES) - 1;
+  const unsigned mo = (__ballot_sync(0xffffffffu, on) >> shift) & m, mp = (__ballot_sync(0xffffffffu, par) >> shift) & m;
+  if (i < np && sub == 0) hit[i] = mo ? 2 : (uint8_t)(__popc(mp) & 1);
 }
 __global__ void k_u8_nonzero(const uint8_t* f, uint64_t n, uint32_t* keep) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -325,8 +341,7 @@ void run_points(gsj_ctx* c, const gsj_layer* pts, const gsj_layer* R, const gsj_
     if (!np) continue;
     tm.start();
     uint8_t* hit = c->flag.as<uint8_t>(np);
-    // one thread per (point, piece) in both modes: a warp per pair measured slower (1.59 vs 1.37 ms for 2M pairs)
-    k_pip<<<grid_for(np, 128), 128, 0, s>>>(pts->pts, R->d, pairs, np, hit); c->launches++;
+    k_pip<<<grid_for(np * PIP_LANES, 128), 128, 0, s>>>(pts->pts, R->d, pairs, np, hit); c->launches++;
     GSJ_CK(cudaGetLastError());
     st.refine_ms += tm.stop();
     tm.start();

@@ -1,0 +1,54 @@
+"""Point kernels at the sizes where their lane groups and marks end: rings around multiples of 8, 32 and 256 edges, points on
+vertices, on edges and at the search distance give or take its band. Every variant gives the oracle's rows."""
+import numpy as np
+import pytest
+
+import gsj
+import pyoracle as O
+from shapes import S, X0, Y0, cw, make_set
+from test_gpu_bins import ngon
+
+pytestmark = pytest.mark.gpu
+MODES = [gsj.GSJ_REFINE_PLAIN, gsj.GSJ_REFINE_FILTERED, gsj.GSJ_REFINE_FILTERED_FP32]
+SIZES = [3, 7, 8, 9, 31, 32, 33, 64, 255, 256, 257, 300]
+D = 5.0
+
+
+def layer():
+    """A polygon of each size, every other one with a hole, and points around them."""
+    geoms, pts = [], []
+    rng = np.random.default_rng(3)
+    for k, n in enumerate(SIZES):
+        cx, cy, r = 4 * S * k, 0.0, S
+        ring = ngon(n, r, cx, cy)
+        geoms.append([ring, cw(ngon(5, 0.3 * r, cx, cy))] if k % 2 else [ring])
+        ring = np.array(ring)
+        a, b = ring[:-1], ring[1:]
+        out = (0.5 * (a + b) - [cx, cy])
+        out /= np.linalg.norm(out, axis=1, keepdims=True)
+        at = D / 111000.0
+        pts += [a, 0.5 * (a + b), 0.25 * a + 0.75 * b, np.column_stack([rng.uniform(cx - 1.5 * r, cx + 1.5 * r, 200), np.repeat(a[:1, 1], 200)])]
+        pts += [0.5 * (a + b) + out * at * f for f in (0.5, 0.99, 0.9999, 1.0, 1.0001, 1.003, 1.01, 1.2)]
+        pts += [rng.uniform([cx - 2 * r, -2 * r], [cx + 2 * r, 2 * r], (200, 2))]
+    return make_set(geoms), np.concatenate(pts) + [X0, Y0]
+
+
+@pytest.fixture(scope="module")
+def both(engine):
+    g, p = layer()
+    return g, p, engine.upload_polygons(g), engine.upload_points(p)
+
+
+@pytest.mark.parametrize("mode", MODES)
+def test_points_in_polygons(engine, both, mode):
+    g, p, lg, lp = both
+    op, ow, _ = O.pip(p, O.OSet(g))
+    gp, gw, _ = engine.join_points(lp, lg, refine_mode=mode)
+    assert np.array_equal(gp, op) and np.array_equal(gw, ow)
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("d", [0.5, D, 2 * D])
+def test_points_within(engine, both, mode, d):
+    g, p, lg, lp = both
+    assert np.array_equal(engine.points_dwithin(lp, lg, d, refine_mode=mode)[0], O.pt_dwithin(p, O.OSet(g), d))
