@@ -179,14 +179,16 @@ _COPY_POOL = None
 
 
 def _copy_out(ptr, count, dtype):
-    """count elements from a host pointer the library owns only during a sink call, into a new numpy array. Large
-    arrays are copied in 8 slices on a small thread pool (ctypes.memmove releases the GIL), so a sink's copy of a
-    few hundred MB of rows is not one thread's memcpy."""
+    """count elements from a host pointer the library owns only during a sink call, into a new numpy array. Arrays of 32 MB
+    and more (the size from which malloc maps fresh pages each time) are copied in 8 slices on a small thread pool
+    (ctypes.memmove releases the GIL): 91 MB of rows 17 ms by one thread, 4 ms by 8. Below that one thread is faster: the
+    staging buffer then stays in one core's caches, and the next device copy into it runs at link speed (9 MB:
+    0.17 ms against 1.2 ms after 8 threads have read it)."""
     global _COPY_POOL
     out = np.empty(count, dtype)
     nbytes = out.nbytes
     src = ctypes.cast(ptr, ctypes.c_void_p).value
-    if nbytes < (8 << 20):
+    if nbytes < (32 << 20):
         if nbytes:
             ctypes.memmove(out.ctypes.data, src, nbytes)
         return out
@@ -401,16 +403,14 @@ class Engine:
         cp, cw = [], []
 
         def sink(user, pairs, where, n):
-            cp.append(np.ctypeslib.as_array(pairs, (n * 2,)).copy())
-            cw.append(np.ctypeslib.as_array(where, (n,)).copy())
+            cp.append(_copy_out(pairs, n * 2, np.uint32))
+            cw.append(_copy_out(where, n, np.uint8))
             return 0
 
         cb = POINTS_SINK(sink)
         st = JoinStats()
         self._check(lib().gsj_join_points(self.ctx, pts.h, R.h, ctypes.byref(o), cb, None, ctypes.byref(st)))
-        pairs = np.concatenate(cp).reshape(-1, 2) if cp else np.zeros((0, 2), np.uint32)
-        where = np.concatenate(cw) if cw else np.zeros(0, np.uint8)
-        return pairs, where, st.as_dict()
+        return _join_chunks(cp, np.uint32).reshape(-1, 2), _join_chunks(cw, np.uint8), st.as_dict()
 
     def cluster(self, P: Layer, nparent: int | None = None, refine_mode=GSJ_REFINE_FILTERED, shard=0, nshards=1):
         nparent = P.info["nparent"] if nparent is None else nparent
@@ -431,15 +431,14 @@ class Engine:
         chunks = []
 
         def sink(user, pairs, n):
-            chunks.append(np.ctypeslib.as_array(pairs, (n * 2,)).copy())
+            chunks.append(_copy_out(pairs, n * 2, np.uint32))
             return 0
 
         cb = PAIRS_SINK(sink)
         st = JoinStats()
         o = opts if opts is not None else join_opts()
         self._check(fn(self.ctx, *args, ctypes.byref(o), cb, None, ctypes.byref(st)))
-        pairs = np.concatenate(chunks).reshape(-1, 2) if chunks else np.zeros((0, 2), np.uint32)
-        return pairs, st.as_dict()
+        return _join_chunks(chunks, np.uint32).reshape(-1, 2), st.as_dict()
 
     def dwithin(self, P: Layer, R: Layer, d: float, same=False, upper=None, refine_mode=GSJ_REFINE_FILTERED):
         o = join_opts(upper=same if upper is None else upper, refine_mode=refine_mode)
