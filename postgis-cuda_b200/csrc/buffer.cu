@@ -15,6 +15,8 @@ namespace gsj {
 constexpr double WGS84_A = 6378137.0, WGS84_F = 1.0 / 298.257223563, WGS84_E2 = WGS84_F * (2.0 - WGS84_F);
 constexpr double DEG = 3.14159265358979323846 / 180.0;
 
+__device__ __forceinline__ double shfl_d(double v, int k) { return __shfl_sync(0xffffffffu, v, k); }
+
 // ---- geodesy (restating buffer.cuh:29-180) --------------------------------------------------------------------
 __device__ __forceinline__ void m_per_deg(double lat, double& kx, double& ky) {   // meters per degree of lon / lat
   const double s = sin(lat * DEG), c = cos(lat * DEG);
@@ -283,25 +285,132 @@ constexpr int DW_CAP = 128, DW_WARPS = 4;
 constexpr size_t DW_EDGE = 4 * sizeof(double) + sizeof(uint32_t);
 __host__ __device__ constexpr size_t dw_warp_bytes(size_t cap) { return 2 * cap * DW_EDGE + DW_QCAP * sizeof(uint2); }   // lists, queue
 constexpr size_t DW_SMEM = (size_t)DW_WARPS * dw_warp_bytes(DW_CAP);
+constexpr size_t DW_WARP_F = 2 * (size_t)DW_CAP * (4 * sizeof(double) + 1) + DW_CAP * sizeof(uint2) + QCAP * sizeof(uint16_t);   // lists, grid boxes, queue
+constexpr size_t DW_SMEM_F = (size_t)DW_WARPS * DW_WARP_F;
+constexpr int DW_MINB = 4;   // filtered: 128 registers a thread (5 blocks, with spills: 2.77 ms where 4 take 2.48)
 
-template <bool QUEUED>
-__global__ void __launch_bounds__(DW_WARPS * 32, 4) k_dwithin(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
-                                                           uint8_t* flag, uint32_t* heavy, unsigned long long* nheavy) {
+// plain: the reference's scheme
+__global__ void __launch_bounds__(DW_WARPS * 32, 4) k_dwithin_plain(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
+                                                                    uint8_t* flag, uint32_t* heavy, unsigned long long* nheavy) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   unsigned char* wbase = smem + (size_t)wib * dw_warp_bytes(DW_CAP);
   EList LA = carve(wbase, DW_CAP), LB = carve(wbase + (size_t)DW_CAP * DW_EDGE, DW_CAP);
-  uint2* Q = reinterpret_cast<uint2*>(wbase + 2 * (size_t)DW_CAP * DW_EDGE);
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nw) {
     const uint2 pr = pairs[p];
     if (same && P.pid(pr.x) == R.pid(pr.y)) { if (lane == 0) flag[p] = 1; continue; }   // pieces of one geometry (buffer.cuh:247-250)
-    const int r = dw_pair<QUEUED>(P, R, pr.x, pr.y, d, LA, LB, DW_CAP, lane, nullptr, Q);
+    const int r = dw_pair<false>(P, R, pr.x, pr.y, d, LA, LB, DW_CAP, lane, nullptr, nullptr);
     if (lane == 0) {
       if (r < 0) { heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)p; flag[p] = 0; }
       else flag[p] = (uint8_t)r;
     }
     __syncwarp();
+  }
+}
+
+// filtered: dw_pair's decision without the geodesic. The frames and search distances of 32 pairs (sines, cosines and a tangent
+// each) are computed one pair per lane and handed to the warp with shuffles; the edge pairs whose boxes come within the
+// search distance are measured 32 at a time. A pair without a surely-within edge pair but with one in the band around
+// d goes to the list of oversized pairs, whose kernel has the geodesic (a pair in thousands), unless one polygon
+// contains the other.
+// Bound by issue and instruction fetch: 150k-parcel self-join at 5 m, 666k pairs: 4.02 ms with the set-up in every lane and two
+// inlined copies of the measuring and the geodesic (314 KB of code, instruction-fetch stall 4.2 cycles an instruction), 2.05 ms.
+__global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
+                                                                   uint8_t* flag, uint32_t* heavy, unsigned long long* nheavy) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  double* x = reinterpret_cast<double*>(smem + (size_t)wib * DW_WARP_F);
+  EList8 LA{x, x + DW_CAP, x + 2 * DW_CAP, x + 3 * DW_CAP, nullptr}, LB{x + 4 * DW_CAP, x + 5 * DW_CAP, x + 6 * DW_CAP, x + 7 * DW_CAP, nullptr};
+  uint2* qb = reinterpret_cast<uint2*>(x + 8 * DW_CAP);
+  uint16_t* q = reinterpret_cast<uint16_t*>(qb + DW_CAP);
+  LA.fl = reinterpret_cast<uint8_t*>(q + QCAP);
+  LB.fl = LA.fl + DW_CAP;
+  const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, span = (np + nw - 1) / nw < 32 ? (np + nw - 1) / nw : 32;   // few pairs: spread over all warps
+  for (uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * span; i0 < np; i0 += nw * span) {
+    const int cnt = np - i0 < span ? (int)(np - i0) : (int)span;
+    uint2 mpr = make_uint2(0, 0);
+    Box mov{0, 0, 0, 0};
+    double mgx = 0, mgy = 0, mkx = 0, mky = 0, mtl = 0, mdelta = 0;
+    int mres = -2;   // -2: to be decided by the warp, else the flag
+    if (lane < cnt) {
+      mpr = pairs[i0 + lane];
+      if (same && P.pid(mpr.x) == R.pid(mpr.y)) mres = 1;   // pieces of one geometry (buffer.cuh:247-250)
+      else {
+        const double2 oa = P.origin[mpr.x], ob = R.origin[mpr.y], ea = P.ext[mpr.x], eb = R.ext[mpr.y];
+        const double sx = ob.x - oa.x, sy = ob.y - oa.y;
+        deg_cover(fmin(oa.y, ob.y), fmax(oa.y + ea.y, ob.y + eb.y), d, true, mgx, mgy);
+        mov = Box{fmax(-mgx, sx - mgx), fmax(-mgy, sy - mgy), fmin(ea.x + mgx, sx + eb.x + mgx), fmin(ea.y + mgy, sy + eb.y + mgy)};
+        if (mov.x0 > mov.x1 || mov.y0 > mov.y1) mres = 0;
+        const double phi0 = oa.y + 0.5 * (mov.y0 + mov.y1);
+        m_per_deg(phi0, mkx, mky);
+        mtl = fabs(tan(phi0 * DEG)) + 0.01;
+        mdelta = 2.0 * 0.5 * (mov.y1 - mov.y0) * DEG * (mtl + 0.04) + 1e-9;
+      }
+    }
+#pragma unroll 1
+    for (int k = 0; k < cnt; k++) {
+      if (__shfl_sync(0xffffffffu, mres, k) != -2) continue;
+      const uint32_t a = __shfl_sync(0xffffffffu, mpr.x, k), b = __shfl_sync(0xffffffffu, mpr.y, k);
+      const Box ov{shfl_d(mov.x0, k), shfl_d(mov.y0, k), shfl_d(mov.x1, k), shfl_d(mov.y1, k)};
+      const double2 oa = P.origin[a];
+      const Frame A = frame_of(P, a, oa.x, oa.y), B = frame_of(R, b, oa.x, oa.y);
+      int na = 0, nb = 0;
+#pragma unroll 1
+      for (int side = 0; side < 2; side++) {   // one inlined copy of the gather
+        const int n = collect<true>(side ? B : A, ov, side ? LB : LA, DW_CAP, lane);
+        if (side) nb = n; else na = n;
+      }
+      __syncwarp();
+      int res = -1;   // -1: the list of oversized pairs
+      if (na <= DW_CAP && nb <= DW_CAP) {
+        const double gx = shfl_d(mgx, k), gy = shfl_d(mgy, k), kx = shfl_d(mkx, k), ky = shfl_d(mky, k), tl = shfl_d(mtl, k), delta = shfl_d(mdelta, k);
+        bool hit = false, open = false;
+        scan_edge_pairs<false>(
+            LA, na, LB, nb, ov, gx, gy, qb, q, lane, [](int, uint32_t) {}, [](int) {},
+            [&](uint32_t e, bool act) {
+              const int i = (int)(e >> 8), j = (int)(e & 255u);
+              if (act && !((LA.fl[i] | LB.fl[j]) & 1u)) {
+                const double ex0 = LA.x0[i], ey0 = LA.y0[i], ex1 = LA.x1[i], ey1 = LA.y1[i];
+                const double fx0 = LB.x0[j], fy0 = LB.y0[j], fx1 = LB.x1[j], fy1 = LB.y1[j];
+                const double bx0 = fmin(ex0, ex1) - gx, bx1 = fmax(ex0, ex1) + gx, by0 = fmin(ey0, ey1) - gy, by1 = fmax(ey0, ey1) + gy;
+                if (!out_cmp(fx0, fy0, fx1, fy1, bx0, by0, bx1, by1)) {
+                  if (seg_isect(ex0, ey0, ex1, ey1, fx0, fy0, fx1, fy1)) hit = true;
+                  else {
+                    double d2 = 1e300;
+#pragma unroll 1
+                    for (int z = 0; z < 4; z++) {   // seg_seg_d2 with one site for the point-segment distance
+                      const bool pa = z < 2;        // the point is A's
+                      const double ptx = (pa ? (z ? ex1 : ex0) : (z == 3 ? fx1 : fx0)) * kx, pty = (pa ? (z ? ey1 : ey0) : (z == 3 ? fy1 : fy0)) * ky;
+                      const double t = pt_seg_d2(ptx, pty, (pa ? fx0 : ex0) * kx, (pa ? fy0 : ey0) * ky, (pa ? fx1 : ex1) * kx, (pa ? fy1 : ey1) * ky);
+                      if (t < d2) d2 = t;
+                    }
+                    const double exm = (ex1 - ex0) * kx, eym = (ey1 - ey0) * ky, fxm = (fx1 - fx0) * kx, fym = (fy1 - fy0) * ky;
+                    const double band = geog_band(d, delta, exm * exm + eym * eym, fxm * fxm + fym * fym, tl), dlo = d - band, dhi = d + band;
+                    if (d2 <= dlo * dlo) hit = true;
+                    else if (d2 <= dhi * dhi) open = true;
+                  }
+                }
+              }
+              return __any_sync(0xffffffffu, hit);
+            });
+        res = __any_sync(0xffffffffu, hit) ? 1 : 0;
+        if (!res) {   // no boundary within d: within d iff one contains the other (a real vertex of one inside the other piece)
+          const double cx = ov.x0 + 0.381966 * (ov.x1 - ov.x0), cy = ov.y0 + 0.414213 * (ov.y1 - ov.y0);
+          bool in[2], any = false;
+#pragma unroll 1
+          for (int side = 0; side < 2; side++) in[side] = pip_full_warp(side ? B : A, cx, cy, lane);
+          res = contains_warp<false>(A, B, LA, na, LB, nb, in[0], in[1], ov, cx, cy, lane, any) ? 1 : 0;
+          if (!res && __any_sync(0xffffffffu, open)) res = -1;
+        }
+      }
+      if (lane == k) mres = res;
+      __syncwarp();
+    }
+    if (lane < cnt) {
+      flag[i0 + lane] = mres > 0 ? 1 : 0;
+      if (mres < 0) heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)(i0 + lane);
+    }
   }
 }
 template <bool QUEUED>
@@ -371,7 +480,6 @@ __global__ void k_pt_dwithin(const double2* __restrict__ pts, DLayer R, const ui
 // Bound by issue and FP64 / memory latency. 2.1M pairs of 1M points x 200k parcels: measuring every edge with the geodesic inlined
 // 3.87 ms (914 warp instructions a pair), the reach test 2.65 ms, the geodesic on a list
 // 1.65 ms at 6 blocks an SM (8 blocks, with spills in the loop: 1.91 ms).
-__device__ __forceinline__ double shfl_d(double v, int k) { return __shfl_sync(0xffffffffu, v, k); }
 template <bool GEO>
 __global__ void __launch_bounds__(128, GEO ? 4 : 6) k_pt_dwithin_warp(const double2* __restrict__ pts, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
                                                                     double d, uint8_t* hit, uint32_t* geo, unsigned long long* ngeo) {
@@ -539,8 +647,8 @@ void dwithin_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double d, 
     qbb = e;
   }
   if (!c->dw_attr) {
-    GSJ_CK(cudaFuncSetAttribute(k_dwithin<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
-    GSJ_CK(cudaFuncSetAttribute(k_dwithin<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
+    GSJ_CK(cudaFuncSetAttribute(k_dwithin_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
+    GSJ_CK(cudaFuncSetAttribute(k_dwithin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM_F));
     c->dw_attr = 1;
   }
   const bool queued = o.refine_mode != GSJ_REFINE_PLAIN;
@@ -564,8 +672,8 @@ void dwithin_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double d, 
     int* err = reinterpret_cast<int*>(ctr + 1);
     GSJ_CK(cudaMemsetAsync(ctr, 0, 16, s));
     const int blocks = (int)std::min<uint64_t>((np + DW_WARPS - 1) / DW_WARPS, (uint64_t)c->sm_count * 8);
-    if (queued) k_dwithin<true><<<blocks, DW_WARPS * 32, DW_SMEM, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
-    else k_dwithin<false><<<blocks, DW_WARPS * 32, DW_SMEM, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
+    if (queued) k_dwithin<<<blocks, DW_WARPS * 32, DW_SMEM_F, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
+    else k_dwithin_plain<<<blocks, DW_WARPS * 32, DW_SMEM, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
     c->launches++;
     GSJ_CK(cudaGetLastError());
     unsigned long long* h = c->h_counters.as<unsigned long long>(2);

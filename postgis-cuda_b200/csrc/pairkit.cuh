@@ -154,4 +154,126 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// the box of an edge on the 15-bit grid, packed so that one subtraction per axis tests both ends: bit 31 of (B - A) is
+// B's upper end >= A's lower end, bit 15 A's upper end >= B's lower end (fields of 16 bits, no borrow between them).
+// Every step is monotone in the coordinate, so boxes that meet are never told apart; coordinates outside the overlap
+// box clamp to its sides.
+struct QGrid { double x0, y0; float sx, sy; };
+struct QBox { int x0, y0, x1, y1; };
+__device__ __forceinline__ QGrid qgrid(const Box& ov) {
+  QGrid g{ov.x0, ov.y0, 0.f, 0.f};
+  const float w = (float)(ov.x1 - ov.x0), h = (float)(ov.y1 - ov.y0);
+  if (w > 1e-30f) g.sx = 1.f / w;
+  if (h > 1e-30f) g.sy = 1.f / h;
+  return g;
+}
+__device__ __forceinline__ int qcell(double v, double o, float s) { return __float2int_rd(__saturatef((float)(v - o) * s) * 32767.f); }
+template <class EL>
+__device__ __forceinline__ QBox qbox(const QGrid& g, const EL& L, int i) {
+  const int px = qcell(L.x0[i], g.x0, g.sx), py = qcell(L.y0[i], g.y0, g.sy), qx = qcell(L.x1[i], g.x0, g.sx), qy = qcell(L.y1[i], g.y0, g.sy);
+  return QBox{min(px, qx), min(py, qy), max(px, qx), max(py, qy)};
+}
+
+// Finds the pairs (i of A, j of B) of local edges whose boxes come within (padx, pady) of each other, or a little more
+// (TRI: one list, j > i only), and hands them to wave(i << 8 | j, act) 32 at a time, one per lane; wave is called by
+// the whole warp and ends the search by returning true (for all lanes). on_block(w, bits): lane i's pairs with B's 32
+// edges from 32 w on, on_row(ic): A's 32 edges from ic on are done. Lists of up to 255 edges.
+// A lane keeps the grid box of one A edge (per 32) in registers and tests B's edges one after the other, each read once
+// for the whole warp (a shared-memory broadcast): 7 integer instructions a pair against ~24 with FP64 boxes. The pairs
+// go through a queue, since a lane's own edge has few: the waves are full.
+constexpr int QCAP = 64;
+template <bool TRI, class EL, class Block, class Row, class Wave>
+__device__ __forceinline__ void scan_edge_pairs(const EL& LA, int na, const EL& LB, int nb, const Box& box, double padx, double pady, uint2* qb, uint16_t* q,
+                                                int lane, Block&& on_block, Row&& on_row, Wave&& wave) {
+  const int nbw = (nb + 31) >> 5;
+  const unsigned lt = (1u << lane) - 1;
+  const QGrid g = qgrid(box);
+  const int cx = 2 + (int)fminf((float)padx * g.sx * 32767.f, 32767.f), cy = 2 + (int)fminf((float)pady * g.sy * 32767.f, 32767.f);   // in cells, rounded up
+#pragma unroll 1
+  for (int j = lane; j < nb; j += 32) {
+    const QBox b = qbox(g, LB, j);
+    qb[j] = make_uint2(0x80008000u + (uint32_t)(b.x1 << 16 | (0x7FFF - b.x0)), 0x80008000u + (uint32_t)(b.y1 << 16 | (0x7FFF - b.y0)));
+  }
+  __syncwarp();
+  int qn = 0, ic = 0, w = -1;   // ic, w: the 32 A edges and the 32 B edges being tested
+  uint32_t bits = 0;
+  uint2 ab = make_uint2(0u, 0u);
+#pragma unroll 1
+  for (bool more = na > 0 && nb > 0; more || qn > 0;) {
+#pragma unroll 1
+    while (more && qn < 32) {
+      const unsigned m = __ballot_sync(0xffffffffu, bits != 0);
+      if (m) {   // each lane queues one of its pairs
+        if (bits) {
+          q[qn + __popc(m & lt)] = (uint16_t)((ic + lane) << 8 | ((w << 5) + __ffs(bits) - 1));
+          bits &= bits - 1;
+        }
+        qn += __popc(m);
+        continue;
+      }
+      if (w < 0 || ++w >= nbw) {   // next 32 A edges
+        if (w >= nbw) {
+          on_row(ic);
+          ic += 32;
+          if (ic >= na) { more = false; break; }
+        }
+        w = TRI ? ic >> 5 : 0;
+        const int i = ic + lane;
+        if (i < na) {
+          const QBox b = qbox(g, LA, i);
+          ab = make_uint2((uint32_t)(max(b.x0 - cx, 0) << 16 | (0x7FFF - min(b.x1 + cx, 0x7FFF))),
+                          (uint32_t)(max(b.y0 - cy, 0) << 16 | (0x7FFF - min(b.y1 + cy, 0x7FFF))));
+        }
+      }
+      const uint2* qw = qb + (w << 5);
+      const int n = min(32, nb - (w << 5));
+#pragma unroll 1
+      for (int j = 0; j < n; j += 4)   // up to 3 entries past the end are masked below
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          const uint2 b = qw[j + k];
+          if (((b.x - ab.x) & (b.y - ab.y) & 0x80008000u) == 0x80008000u) bits |= 1u << (j + k);
+        }
+      if (n < 32) bits &= (1u << n) - 1u;
+      if (ic + lane >= na) bits = 0;
+      if (TRI && w == (ic >> 5)) bits &= ~((2u << lane) - 1u);
+      on_block(w, bits);
+    }
+    __syncwarp();
+    const uint32_t e = q[lane];
+    const uint16_t rest = q[32 + lane];
+    if (wave(e, lane < qn)) break;
+    __syncwarp();
+    qn = max(qn - 32, 0);
+    if (lane < qn) q[lane] = rest;
+    __syncwarp();
+  }
+  __syncwarp();
+}
+
+// filtered variants, no real boundary contact: intersects iff a real-edge vertex of one lies inside the other
+// (engine.cuh:577-594); one probe at a time, the warp splitting the other polygon's edges (crossing parity is
+// order-free). any: some probe vertex lies inside.
+template <bool S32, class EL>
+__device__ bool contains_warp(const Frame& A, const Frame& B, const EL& LA, int na, const EL& LB, int nb, bool inA_c, bool inB_c, const Box& ov, double cx,
+                              double cy, int lane, bool& any) {
+  bool h = false;
+#pragma unroll 1
+  for (int side = 0; side < 2 && !h; side++) {
+    const Frame& S = side ? B : A;
+    const EL& LO = side ? LA : LB;
+    const int no_ = side ? na : nb;
+    const bool inc = side ? inA_c : inB_c;
+#pragma unroll 1
+    for (uint32_t r = S.r0; r < S.r1 && !h; r++) {
+      double x, y; const bool real = probe_vertex(S, r, x, y);
+      if (!real) S.v(S.L->rvo[r], x, y);
+      if (x >= ov.x0 && x <= ov.x1 && y >= ov.y0 && y <= ov.y1 && inside_from_c_warp<S32>(LO, no_, cx, cy, inc, x, y, lane)) {
+        any = true; h = real;
+      }
+    }
+  }
+  return h;
+}
+
 }  // namespace gsj

@@ -410,31 +410,6 @@ __device__ __forceinline__ PairGeo pair_geo(const DLayer& P, const DLayer& R, ui
   return G;
 }
 
-// filtered variants, no real boundary contact: intersects iff a real-edge vertex of one lies inside the other
-// (engine.cuh:577-594); one probe at a time, the warp splitting the other polygon's edges (crossing parity is
-// order-free). any: some probe vertex lies inside.
-template <bool S32, class EL>
-__device__ bool contains_warp(const Frame& A, const Frame& B, const EL& LA, int na, const EL& LB, int nb, bool inA_c, bool inB_c, const PairGeo& G, int lane,
-                              bool& any) {
-  bool h = false;
-#pragma unroll 1
-  for (int side = 0; side < 2 && !h; side++) {
-    const Frame& S = side ? B : A;
-    const EL& LO = side ? LA : LB;
-    const int no_ = side ? na : nb;
-    const bool inc = side ? inA_c : inB_c;
-#pragma unroll 1
-    for (uint32_t r = S.r0; r < S.r1 && !h; r++) {
-      double x, y; const bool real = probe_vertex(S, r, x, y);
-      if (!real) S.v(S.L->rvo[r], x, y);
-      if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c_warp<S32>(LO, no_, G.cx, G.cy, inc, x, y, lane)) {
-        any = true; h = real;
-      }
-    }
-  }
-  return h;
-}
-
 // One pair, whole warp. Returns false when a local list exceeded cap (nothing written).
 // FLAT (the filtered scratch kernel): candidate lists in global scratch; a pair whose list would exceed fb->cap is
 // handed back (false) and runs with the full sweeps.
@@ -516,7 +491,7 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
   bool contain_any = false;
   if (!hit) {
     if constexpr (F) {
-      hit = contains_warp<false>(A, B, LA, na, LB, nb, inA_c, inB_c, G, lane, contain_any);
+      hit = contains_warp<false>(A, B, LA, na, LB, nb, inA_c, inB_c, G.ov, G.cx, G.cy, lane, contain_any);
     } else {   // no real boundary contact: intersects iff a real-edge vertex of one lies inside the other (engine.cuh:577-594)
       bool h = false, ha = false;
 #pragma unroll 1
@@ -612,28 +587,7 @@ __device__ bool refine_pair(const DLayer& P, const DLayer& R, uint32_t a, uint32
 // instruction-fetch stall at 8.6, 4.3 and 0.9 cycles an instruction).
 // 100k-parcel relate self-join, against lanes that each visited their own edge's candidates: this bin 3.45 -> 2.86 ms, the
 // self bin 1.44 -> 0.76 ms; two 60k layers, area: 4.35 -> 3.16 ms (14.5 -> 20.5 lanes active per instruction).
-constexpr int QCAP = 64;
 struct MaskBuf { uint32_t* rm; uint32_t* cm; uint2* qb; uint32_t* cand; uint16_t* q; };
-
-// the box of an edge on the 15-bit grid, packed so that one subtraction per axis tests both ends: bit 31 of (B - A) is
-// B's upper end >= A's lower end, bit 15 A's upper end >= B's lower end (fields of 16 bits, no borrow between them).
-// Every step is monotone in the coordinate, so boxes that meet are never told apart; coordinates outside the overlap
-// box clamp to its sides.
-struct QGrid { double x0, y0; float sx, sy; };
-struct QBox { int x0, y0, x1, y1; };
-__device__ __forceinline__ QGrid qgrid(const Box& ov) {
-  QGrid g{ov.x0, ov.y0, 0.f, 0.f};
-  const float w = (float)(ov.x1 - ov.x0), h = (float)(ov.y1 - ov.y0);
-  if (w > 1e-30f) g.sx = 1.f / w;
-  if (h > 1e-30f) g.sy = 1.f / h;
-  return g;
-}
-__device__ __forceinline__ int qcell(double v, double o, float s) { return __float2int_rd(__saturatef((float)(v - o) * s) * 32767.f); }
-template <class EL>
-__device__ __forceinline__ QBox qbox(const QGrid& g, const EL& L, int i) {
-  const int px = qcell(L.x0[i], g.x0, g.sx), py = qcell(L.y0[i], g.y0, g.sy), qx = qcell(L.x1[i], g.x0, g.sx), qy = qcell(L.y1[i], g.y0, g.sy);
-  return QBox{min(px, qx), min(py, qy), max(px, qx), max(py, qy)};
-}
 
 // Split points found by the classification: edge and parameter, in the tails of a list's arrays (n of MS entries in
 // use): the parameters behind x0 and x1, the edges behind y0 and y1. 2 (MS - n) of them fit.
@@ -743,93 +697,42 @@ __device__ __forceinline__ void edge_cover(EdgeCuts& C, const EdgeRef& e, const 
 }
 
 // Candidate edge pairs (boxes within 2 tol of each other, or a little more on the grid) found and classified; CUTS: the cuts
-// are wanted, else the contact alone. A lane keeps the
-// grid box of one A edge (per 32) in registers and tests B's edges one after the other, each read once for the whole
-// warp (a shared-memory broadcast); the pairs go through the queue. Returns at the first real contact when nothing but
-// the flag is wanted. SELF: only j > i is searched (an edge always coincides with itself).
+// are wanted, else the contact alone (the search then ends at the first real one). SELF: an edge always coincides
+// with itself, only j > i is searched.
 template <int MS, bool SELF, bool CUTS, class EL>
 __device__ Splits find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const MaskBuf& mb, int lane, bool& hit, bool& hit_any) {
-  const int nbw = (nb + 31) >> 5;
-  const unsigned lt = (1u << lane) - 1;
-  const QGrid g = qgrid(G.ov);
-  const float pad = 2.f * (float)G.tol;
-  const int cx = 2 + (int)fminf(pad * g.sx * 32767.f, 32767.f), cy = 2 + (int)fminf(pad * g.sy * 32767.f, 32767.f);   // 2 tol in cells, rounded up
   if constexpr (CUTS) {
     uint4* z = reinterpret_cast<uint4*>(mb.rm);
 #pragma unroll 1
     for (int t = lane; t < (SELF ? 1 : 2) * (MS / 32) * MS / 4; t += 32) z[t] = make_uint4(0u, 0u, 0u, 0u);
+    if (!SELF && lane < 2 * (MS / 32)) mb.cand[lane] = 0u;
     __syncwarp();
-  }
+    if (SELF)
 #pragma unroll 1
-  for (int j = lane; j < nb; j += 32) {
-    const QBox b = qbox(g, LB, j);
-    mb.qb[j] = make_uint2(0x80008000u + (uint32_t)(b.x1 << 16 | (0x7FFF - b.x0)), 0x80008000u + (uint32_t)(b.y1 << 16 | (0x7FFF - b.y0)));
-    if (CUTS && SELF) mb.rm[(j >> 5) * MS + j] = 1u << (j & 31);
+      for (int j = lane; j < nb; j += 32) mb.rm[(j >> 5) * MS + j] = 1u << (j & 31);
   }
-  if (!SELF && lane < 2 * (MS / 32)) mb.cand[lane] = 0u;
-  __syncwarp();
   Splits sp{0, 0, false};
-  int qn = 0, ic = 0, w = -1;   // ic, w: the 32 A edges and the 32 B edges being tested
-  uint32_t bits = 0, any = 0;
-  uint2 ab = make_uint2(0u, 0u);
-  for (bool more = na > 0 && nb > 0; more || qn > 0;) {
-    while (more && qn < 32) {
-      const unsigned m = __ballot_sync(0xffffffffu, bits != 0);
-      if (m) {   // each lane queues one of its pairs
-        if (bits) {
-          mb.q[qn + __popc(m & lt)] = (uint16_t)((ic + lane) << 8 | ((w << 5) + __ffs(bits) - 1));
-          bits &= bits - 1;
+  uint32_t any = 0;
+  scan_edge_pairs<SELF>(
+      LA, na, LB, nb, G.ov, 2.0 * G.tol, 2.0 * G.tol, mb.qb, mb.q, lane,
+      [&](int w, uint32_t bits) {
+        if constexpr (!SELF && CUTS) {
+          any |= bits;
+          const uint32_t ob = __reduce_or_sync(0xffffffffu, bits);
+          if (lane == 0) mb.cand[MS / 32 + w] |= ob;
         }
-        qn += __popc(m);
-        continue;
-      }
-      if (w < 0 || ++w >= nbw) {   // next 32 A edges
-        if (w >= nbw) {
-          if (!SELF && CUTS) {
-            const unsigned c = __ballot_sync(0xffffffffu, any != 0);
-            if (lane == 0) mb.cand[ic >> 5] = c;
-          }
-          ic += 32;
+      },
+      [&](int ic) {
+        if constexpr (!SELF && CUTS) {
+          const unsigned c = __ballot_sync(0xffffffffu, any != 0);
+          if (lane == 0) mb.cand[ic >> 5] = c;
           any = 0;
-          if (ic >= na) { more = false; break; }
         }
-        w = SELF ? ic >> 5 : 0;
-        const int i = ic + lane;
-        if (i < na) {
-          const QBox b = qbox(g, LA, i);
-          ab = make_uint2((uint32_t)(max(b.x0 - cx, 0) << 16 | (0x7FFF - min(b.x1 + cx, 0x7FFF))),
-                          (uint32_t)(max(b.y0 - cy, 0) << 16 | (0x7FFF - min(b.y1 + cy, 0x7FFF))));
-        }
-      }
-      const uint2* qb = mb.qb + (w << 5);
-      const int n = min(32, nb - (w << 5));
-#pragma unroll 1
-      for (int j = 0; j < n; j += 4)   // up to 3 entries past the end are masked below
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          const uint2 b = qb[j + q];
-          if (((b.x - ab.x) & (b.y - ab.y) & 0x80008000u) == 0x80008000u) bits |= 1u << (j + q);
-        }
-      if (n < 32) bits &= (1u << n) - 1u;
-      if (ic + lane >= na) bits = 0;
-      if (SELF) { if (w == (ic >> 5)) bits &= ~((2u << lane) - 1u); }
-      else if constexpr (CUTS) {
-        any |= bits;
-        const uint32_t ob = __reduce_or_sync(0xffffffffu, bits);
-        if (lane == 0) mb.cand[MS / 32 + w] |= ob;
-      }
-    }
-    __syncwarp();
-    const uint32_t e = mb.q[lane];
-    const uint16_t rest = mb.q[32 + lane];
-    classify_pairs<MS, SELF, CUTS>(LA, na, LB, nb, G, mb, e, lane < qn, lane, sp, hit, hit_any);
-    if (!CUTS && __any_sync(0xffffffffu, hit)) break;
-    __syncwarp();
-    qn = max(qn - 32, 0);
-    if (lane < qn) mb.q[lane] = rest;
-    __syncwarp();
-  }
-  __syncwarp();
+      },
+      [&](uint32_t e, bool act) {
+        classify_pairs<MS, SELF, CUTS>(LA, na, LB, nb, G, mb, e, act, lane, sp, hit, hit_any);
+        return !CUTS && __any_sync(0xffffffffu, hit);
+      });
   return sp;
 }
 
@@ -951,7 +854,7 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
   hit = __any_sync(0xffffffffu, hit);
   hit_any = __any_sync(0xffffffffu, hit_any || hit);
   const bool rtouch = hit;
-  if (!hit) hit = contains_warp<S32>(A, B, LA, na, LB, nb, inA_c, inB_c, G, lane, hit_any);
+  if (!hit) hit = contains_warp<S32>(A, B, LA, na, LB, nb, inA_c, inB_c, G.ov, G.cx, G.cy, lane, hit_any);
   PairSums S;
   uint32_t bits = rtouch ? REL_TOUCH : 0;
   const bool sums = W != W_FLAG && (hit || (W != W_REL && hit_any));

@@ -1,4 +1,4 @@
-"""Point kernels at the sizes where their lane groups and marks end: rings around multiples of 8, 32 and 256 edges, points on
+"""Distance and point kernels at the sizes where their lane groups and marks end: rings around multiples of 8, 32 and 256 edges, points on
 vertices, on edges and at the search distance give or take its band. Every variant gives the oracle's rows."""
 import numpy as np
 import pytest
@@ -52,3 +52,24 @@ def test_points_in_polygons(engine, both, mode):
 def test_points_within(engine, both, mode, d):
     g, p, lg, lp = both
     assert np.array_equal(engine.points_dwithin(lp, lg, d, refine_mode=mode)[0], O.pt_dwithin(p, O.OSet(g), d))
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("d", [0.5, D, 2 * D])
+def test_polygons_within(engine, mode, d):
+    """Polygons of 3 to 129 edges (the lists hold 128) side by side at gaps around d, one inside another, and apart."""
+    sizes = [3, 31, 32, 33, 64, 127, 128, 129]
+    m = 1.0 / (111320.0 * np.cos(np.radians(Y0)))   # about a metre of longitude
+    A, B = [], []
+    for k, n in enumerate(sizes):
+        for q, f in enumerate((0.5, 0.99, 0.9999, 1.0001, 1.01, 1.5)):
+            cx, cy = 8 * S * k, 4 * S * q
+            A.append([ngon(n, S, cx, cy)])
+            B.append([ngon(sizes[(k + q) % len(sizes)], S, cx + 2 * S + f * d * m, cy)])
+        A.append([ngon(n, 0.2 * S, 8 * S * k, -4 * S)])
+        B.append([ngon(9, S, 8 * S * k, -4 * S)])
+    a, b = make_set(A), make_set(B)
+    la, lb = engine.upload_polygons(a), engine.upload_polygons(b)
+    for lr, rs, same in ((lb, b, False), (la, a, True)):
+        got, want = engine.dwithin(la, lr, d, same=same, refine_mode=mode)[0], O.dwithin(O.OSet(a), O.OSet(rs), d, same=same)[0]
+        assert set(map(tuple, got.tolist())) == set(map(tuple, want.tolist()))
