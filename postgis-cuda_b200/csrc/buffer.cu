@@ -24,6 +24,8 @@ __device__ __forceinline__ void m_per_deg(double lat, double& kx, double& ky) { 
   kx = WGS84_A / w * c * DEG;
   ky = WGS84_A * (1.0 - WGS84_E2) / (w2 * w) * DEG;
 }
+// the same out of line: the set-up routines call it several times, and its sine and cosine are 2.5 KB of code each time
+__device__ __noinline__ double2 m_per_deg_call(double lat) { double2 k; m_per_deg(lat, k.x, k.y); return k; }
 // degrees covering d meters over latitudes [y0, y1], larger (expand) or smaller (shrink)
 __device__ void deg_cover(double y0, double y1, double d, bool larger, double& dx, double& dy) {
   if (d <= 0) { dx = dy = 0; return; }
@@ -31,14 +33,12 @@ __device__ void deg_cover(double y0, double y1, double d, bool larger, double& d
   double lo = (y0 - pad <= 0 && y1 + pad >= 0) ? 0.0 : fmin(fabs(y0), fabs(y1)) - pad;
   const double hi = fmin(fmax(fabs(y0), fabs(y1)) + pad, 89.9);
   lo = fmax(lo, 0.0);
-  double kxa, kya, kxb, kyb;
-  m_per_deg(hi, kxa, kya);
-  m_per_deg(lo, kxb, kyb);
-  if (larger) { dx = d / kxa * (1 + 1e-6); dy = d / kyb * (1 + 1e-6); }
-  else { dx = d / kxb * (1 - 1e-6); dy = d / kya * (1 - 1e-6); }
+  const double2 ka = m_per_deg_call(hi), kb = m_per_deg_call(lo);
+  if (larger) { dx = d / ka.x * (1 + 1e-6); dy = d / kb.y * (1 + 1e-6); }
+  else { dx = d / kb.x * (1 - 1e-6); dy = d / ka.y * (1 - 1e-6); }
 }
 // point scale factor of the UTM zone chosen for a geometry centred at (glon, glat), at (lon, lat)
-__device__ double utm_k(double glon, double glat, double lon, double lat) {
+__device__ __noinline__ double utm_k(double glon, double glat, double lon, double lat) {
   if (glat > 70.0 || glat < -70.0) return 1.0;
   int zone = (int)floor((glon + 180.0) / 6.0);
   if (zone > 59) zone = 59;
@@ -715,21 +715,59 @@ struct BEl { double x0, y0, x1, y1; };                                  // eleme
 constexpr double FILLET_QUANTUM = 3.14159265358979323846 / 16.0;       // 8 segments per quarter circle (GEOS default)
 constexpr int ER_WARPS = 2, ER_CAPE = 64, ER_CAPL = 128, ER_MAX_DEPTH = 12;
 constexpr int ER_QCAP = 64;                                                // crossing candidates queued per warp
-constexpr int ER_RUN = 4, ER_RUNS = 64, ER_MINB = 4;   // k_erode_main: pairs per fetch, fetches per warp, blocks per SM
-constexpr size_t ER_SMEM_WARP = 2 * ER_CAPE * sizeof(BEd) + 2 * ER_CAPL * sizeof(BEl) + ER_QCAP * sizeof(uint2);
-constexpr size_t ER_SMEM = (size_t)ER_WARPS * ER_SMEM_WARP;
-struct ErScratch { BEd* EA; BEd* EB; BEl* LA; BEl* LB; uint2* Q; int capE, capL; };
+constexpr int ER_RUN = 8, ER_RUNS = 64, ER_MINB = 4;   // k_erode_main: pairs per fetch, fetches per warp, blocks per SM
+// a warp's lists: edges, elements, crossing queue, grid boxes of the edges' exclusion zones (qe) and of B's elements (qb: the
+// shared-memory kernels only)
+struct ErScratch { BEd* EA; BEd* EB; BEl* LA; BEl* LB; uint2* Q; uint2* qa; uint2* qe; uint2* qb; int capE, capL; };
 __host__ __device__ constexpr size_t er_scratch_bytes(size_t capE, size_t capL) {
-  return 2 * capE * sizeof(BEd) + 2 * capL * sizeof(BEl) + ER_QCAP * sizeof(uint2);
+  return 2 * capE * sizeof(BEd) + 2 * capL * sizeof(BEl) + ER_QCAP * sizeof(uint2) + 2 * capE * sizeof(uint2);
 }
+constexpr size_t ER_SMEM_WARP = er_scratch_bytes(ER_CAPE, ER_CAPL) + ER_CAPL * sizeof(uint2);
+constexpr size_t ER_SMEM = (size_t)ER_WARPS * ER_SMEM_WARP;
+__device__ __forceinline__ ErScratch er_carve(unsigned char* base, int capE, int capL) {
+  ErScratch sc;
+  sc.EA = reinterpret_cast<BEd*>(base); sc.EB = sc.EA + capE;
+  sc.LA = reinterpret_cast<BEl*>(sc.EB + capE); sc.LB = sc.LA + capL;
+  sc.Q = reinterpret_cast<uint2*>(sc.LB + capL);
+  sc.qa = sc.Q + ER_QCAP; sc.qe = sc.qa + capE; sc.qb = sc.qe + capE;
+  sc.capE = capE; sc.capL = capL;
+  return sc;
+}
+// an element list as the separate coordinate arrays of an edge list
+struct Stride4 { const double* p; __device__ __forceinline__ double operator[](int i) const { return p[4 * i]; } };
+struct BElView { Stride4 x0, y0, x1, y1; };
 struct ETile { uint32_t pair, depth; double4 box; };
 struct ErCtr { unsigned int ntile, nslab; int needE, needL; unsigned long long next; };   // next: k_erode_main's pair counter
 struct EFrame { double ox, oy, kx, ky; };
 
-__device__ bool in_excl(const BEd* E, int n, double r, double x, double y, double eps) {   // buffer.cuh:285-319
+// boxes of the exclusion zones of a side's edges on the window's grid (the edge's box widened by r, as in_excl tests it)
+__device__ __forceinline__ void excl_boxes(const BEd* E, int n, double r, const QGrid& g, uint2* q, int lane) {
+  for (int k = lane; k < n; k += 32) {
+    const BEd& e = E[k];
+    const int x0 = qcell(fmin(e.x0, e.x1) - r, g.x0, g.sx), x1 = qcell(fmax(e.x0, e.x1) + r, g.x0, g.sx);
+    const int y0 = qcell(fmin(e.y0, e.y1) - r, g.y0, g.sy), y1 = qcell(fmax(e.y0, e.y1) + r, g.y0, g.sy);
+    q[k] = make_uint2(0x80008000u + (uint32_t)(x1 << 16 | (0x7FFF - x0)), 0x80008000u + (uint32_t)(y1 << 16 | (0x7FFF - y0)));
+  }
+}
+// the point in an edge's exclusion zone (an any-of over the edges): 32 edges at a time are first told apart by their grid
+// boxes, 7 integer instructions an edge, and only those whose box holds the point's cell are tested
+// Out of line, as the other large steps below: the crossing and vertex tests would inline it seven times.
+__device__ __noinline__ bool in_excl(const BEd* E, const uint2* q, const QGrid& g, int n, double r, double x, double y, double eps) {   // buffer.cuh:285-319
   if (r <= 0) return false;
   const double ri = r - eps;
-  for (int k = 0; k < n; k++) {
+  const int cx = qcell(x, g.x0, g.sx), cy = qcell(y, g.y0, g.sy);
+  const uint32_t px = (uint32_t)(cx << 16 | (0x7FFF - cx)), py = (uint32_t)(cy << 16 | (0x7FFF - cy));
+  for (int kb = 0, k = 0; kb < n; kb += 32) {
+   uint32_t todo = 0;
+   const int nk = min(32, n - kb);
+#pragma unroll 4
+   for (int t = 0; t < nk; t++) {
+     const uint2 b = q[kb + t];
+     if (((b.x - px) & (b.y - py) & 0x80008000u) == 0x80008000u) todo |= 1u << t;
+   }
+#pragma unroll 1
+   for (; todo; todo &= todo - 1) {
+    k = kb + __ffs(todo) - 1;
     const BEd& e = E[k];
     if (x < fmin(e.x0, e.x1) - r || x > fmax(e.x0, e.x1) + r || y < fmin(e.y0, e.y1) - r || y > fmax(e.y0, e.y1) + r) continue;
     const double dx = x - e.x0, dy = y - e.y0;
@@ -757,10 +795,11 @@ __device__ bool in_excl(const BEd* E, int n, double r, double x, double y, doubl
       const double t2 = mx * e.ci + my * e.si; my = -mx * e.si + my * e.ci; mx = t2;
     }
     if (in) return true;
+   }
   }
   return false;
 }
-__device__ __forceinline__ bool inside_m(const BEd* E, int n, double cx, double cy, bool in_c, double x, double y) {   // buffer.cuh:322-334
+__device__ __noinline__ bool inside_m(const BEd* E, int n, double cx, double cy, bool in_c, double x, double y) {   // buffer.cuh:322-334
   bool in = in_c;
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);
   for (int k = 0; k < n; k++) {
@@ -780,14 +819,17 @@ __device__ __forceinline__ void fv(const DLayer& S, double shx, double shy, uint
 // c inside the parent: the piece whose box holds c decides by crossing parity (buffer.cuh:359-381)
 __device__ bool pip_parent(const DLayer& S, uint32_t g0, uint32_t g1, const EFrame& F, double cx, double cy, int lane) {
   bool in = false;
+#pragma unroll 1
   for (uint32_t g = g0; g < g1 && !in; g++) {
     const double2 o = S.origin[g], e = S.ext[g];
     const double bx0 = (o.x - F.ox) * F.kx, by0 = (o.y - F.oy) * F.ky, bx1 = (o.x + e.x - F.ox) * F.kx, by1 = (o.y + e.y - F.oy) * F.ky;
     if (cx < bx0 - 1e-6 || cx > bx1 + 1e-6 || cy < by0 - 1e-6 || cy > by1 + 1e-6) continue;
     const double shx = o.x - F.ox, shy = o.y - F.oy, ox = bx0 - 1.0;
     bool par = false;
+#pragma unroll 1
     for (uint32_t r = S.gro[g]; r < S.gro[g + 1]; r++) {
       const uint64_t s0 = S.rvo[r], ee = S.rvo[r + 1];
+#pragma unroll 1
       for (uint64_t j = s0 + 1 + lane; j < ee; j += 32) {
         double x0, y0, x1, y1; fv(S, shx, shy, j - 1, F, x0, y0); fv(S, shx, shy, j, F, x1, y1);
         if ((y0 > cy) == (y1 > cy) && y0 != cy && y1 != cy) continue;
@@ -806,12 +848,15 @@ __device__ int collect_side(const DLayer& S, uint32_t g0, uint32_t g1, const EFr
                             int lane) {
   const unsigned lt = (1u << lane) - 1;
   int cnt = 0;
+#pragma unroll 1
   for (uint32_t g = g0; g < g1; g++) {
     const double2 o = S.origin[g], ex = S.ext[g];
     if ((o.x + ex.x - F.ox) * F.kx < cx0 || (o.x - F.ox) * F.kx > cx1 || (o.y + ex.y - F.oy) * F.ky < cy0 || (o.y - F.oy) * F.ky > cy1) continue;
     const double shx = o.x - F.ox, shy = o.y - F.oy;
+#pragma unroll 1
     for (uint32_t r = S.gro[g]; r < S.gro[g + 1]; r++) {
       const uint64_t s0 = S.rvo[r], e = S.rvo[r + 1];
+#pragma unroll 1
       for (uint64_t base = s0; base + 1 < e; base += 32) {
         const uint64_t i = base + lane;
         bool v = false; BEd ed;
@@ -831,16 +876,37 @@ __device__ int collect_side(const DLayer& S, uint32_t g0, uint32_t g1, const EFr
 }
 // unit directions, successor edge and end-vertex region (convex disk / reflex fillet) (buffer.cuh:411-439)
 __device__ void prepare_side(BEd* E, int n, double r, int lane) {
+#pragma unroll 1
   for (int k = lane; k < n; k += 32) {
     const double dx = E[k].x1 - E[k].x0, dy = E[k].y1 - E[k].y0, L = sqrt(dx * dx + dy * dy);
     E[k].ux = dx / L; E[k].uy = dy / L; E[k].L = L;
   }
   __syncwarp();
-  for (int k = lane; k < n; k += 32) {
-    const double ex1 = E[k].x1, ey1 = E[k].y1, eux = E[k].ux, euy = E[k].uy;
+#pragma unroll 1
+  for (int kb = 0; kb < n; kb += 32) {
+    const int k = kb + lane;
+    double ex1 = 0, ey1 = 0, eux = 0, euy = 0;
     int s = -1;
-    if (k + 1 < n && E[k + 1].x0 == ex1 && E[k + 1].y0 == ey1) s = k + 1;
-    else for (int j = 0; j < n; j++) if (j != k && E[j].x0 == ex1 && E[j].y0 == ey1) { s = j; break; }
+    if (k < n) {
+      ex1 = E[k].x1; ey1 = E[k].y1; eux = E[k].ux; euy = E[k].uy;
+      if (k + 1 < n && E[k + 1].x0 == ex1 && E[k + 1].y0 == ey1) s = k + 1;
+    }
+    // the first edge that starts where the edge ends, where that is not the next one (a ring's last edge): searched by
+    // the whole warp
+#pragma unroll 1
+    for (unsigned m = __ballot_sync(0xffffffffu, k < n && s < 0); m; m &= m - 1) {
+      const int src = __ffs(m) - 1;
+      const double sx = shfl_d(ex1, src), sy = shfl_d(ey1, src);
+      int f = -1;
+#pragma unroll 1
+      for (int j0 = 0; j0 < n && f < 0; j0 += 32) {
+        const int j = j0 + lane;
+        const unsigned w = __ballot_sync(0xffffffffu, j < n && j != kb + src && E[j].x0 == sx && E[j].y0 == sy);
+        if (w) f = j0 + __ffs(w) - 1;
+      }
+      if (lane == src) s = f;
+    }
+    if (k >= n) continue;
     int vt = 0; double ci = 1, si = 0;
     if (s >= 0 && r > 0) {
       const double fux = E[s].ux, fuy = E[s].uy;
@@ -863,6 +929,7 @@ __device__ void prepare_side(BEd* E, int n, double r, int lane) {
 __device__ int build_elements(const BEd* E, int n, double r, double wx0, double wy0, double wx1, double wy1, double eps, BEl* L, int cap, int lane) {
   const unsigned lt = (1u << lane) - 1;
   int cnt = 0;
+#pragma unroll 1
   for (int base = 0; base < n; base += 32) {
     const int k = base + lane;
     const bool valid = k < n;
@@ -874,6 +941,7 @@ __device__ int build_elements(const BEd* E, int n, double r, double wx0, double 
       nkx = -e.uy; nky = e.ux; wxr = nkx; wyr = nky; px = e.x1 + r * nkx; py = e.y1 + r * nky;
       if (e.vt >= 2) { nsx = -E[e.succ].uy; nsy = E[e.succ].ux; }
     }
+#pragma unroll 1
     for (int it = 0; it < mx; it++) {
       bool has = it < ne; BEl el;
       if (has) {
@@ -914,21 +982,21 @@ __device__ int seg_points(const BEl& p, const BEl& q, double* xs, double* ys) { 
   return 3;
 }
 
-// X_A meets X_B within the window (intersected with tile when given): 1 / 0, or -1 when a list overflowed
-// (needE / needL = sizes required, *wout = the window tested) (buffer.cuh:499-588). mirror: B is A (same layer,
-// same pieces, same radius), so B's edge and element lists, centre test and vertex pass are A's and are not
-// built twice; every value they would hold is computed from the same inputs by the same code.
-__device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, double ra_nom, double rb_nom, const ErScratch& sc, int lane, int* needE,
-                       int* needL, const double4* tile, double4* wout, bool mirror) {
-  if (ga.x >= ga.y || gb.x >= gb.y) return 0;
+// The window of a pair, its radii and frame: tens of sines, cosines and tangents, computed for several pairs at once, one per lane.
+struct ErSet { double wx0, wy0, wx1, wy1, rA, rB, kx, ky, fe; };   // wx0 > wx1: the pair cannot meet
+__device__ ErSet er_set(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, double ra_nom, double rb_nom, const double4* tile, bool mirror) {
+  ErSet e{1, 0, 0, 0, 0, 0, 0, 0, 0};
+  if (ga.x >= ga.y || gb.x >= gb.y) return e;
   double abx0 = 1e300, aby0 = 1e300, abx1 = -1e300, aby1 = -1e300, bbx0 = 1e300, bby0 = 1e300, bbx1 = -1e300, bby1 = -1e300;
+#pragma unroll 1
   for (uint32_t g = ga.x; g < ga.y; g++) {
-    const double2 o = P.origin[g], e = P.ext[g];
-    abx0 = fmin(abx0, o.x); aby0 = fmin(aby0, o.y); abx1 = fmax(abx1, o.x + e.x); aby1 = fmax(aby1, o.y + e.y);
+    const double2 o = P.origin[g], x = P.ext[g];
+    abx0 = fmin(abx0, o.x); aby0 = fmin(aby0, o.y); abx1 = fmax(abx1, o.x + x.x); aby1 = fmax(aby1, o.y + x.y);
   }
+#pragma unroll 1
   for (uint32_t g = gb.x; g < gb.y; g++) {
-    const double2 o = R.origin[g], e = R.ext[g];
-    bbx0 = fmin(bbx0, o.x); bby0 = fmin(bby0, o.y); bbx1 = fmax(bbx1, o.x + e.x); bby1 = fmax(bby1, o.y + e.y);
+    const double2 o = R.origin[g], x = R.ext[g];
+    bbx0 = fmin(bbx0, o.x); bby0 = fmin(bby0, o.y); bbx1 = fmax(bbx1, o.x + x.x); bby1 = fmax(bby1, o.y + x.y);
   }
   double dax, day, dbx, dby;
   deg_cover(aby0, aby1, ra_nom * 0.998, false, dax, day);   // shrink by a lower bound of the true radius
@@ -936,48 +1004,95 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, dou
   double wx0 = fmax(abx0 + dax, bbx0 + dbx), wx1 = fmin(abx1 - dax, bbx1 - dbx);
   double wy0 = fmax(aby0 + day, bby0 + dby), wy1 = fmin(aby1 - day, bby1 - dby);
   if (tile) { wx0 = fmax(wx0, tile->x); wy0 = fmax(wy0, tile->y); wx1 = fmin(wx1, tile->z); wy1 = fmin(wy1, tile->w); }
-  if (wx0 > wx1 || wy0 > wy1) return 0;
-  if (wout) *wout = make_double4(wx0, wy0, wx1, wy1);
+  if (wx0 > wx1 || wy0 > wy1) return e;
+  e.wx0 = wx0; e.wy0 = wy0; e.wx1 = wx1; e.wy1 = wy1;
   const double clon = 0.5 * (wx0 + wx1), clat = 0.5 * (wy0 + wy1);
-  const double rA = ra_nom > 0 ? ra_nom / utm_k(0.5 * (abx0 + abx1), 0.5 * (aby0 + aby1), clon, clat) : 0.0;
-  const double rB = mirror ? rA : rb_nom > 0 ? rb_nom / utm_k(0.5 * (bbx0 + bbx1), 0.5 * (bby0 + bby1), clon, clat) : 0.0;
-  EFrame F; { const double2 o = P.origin[ga.x]; F.ox = o.x; F.oy = o.y; } m_per_deg(clat, F.kx, F.ky);
-  const double Wx0 = (wx0 - F.ox) * F.kx, Wx1 = (wx1 - F.ox) * F.kx, Wy0 = (wy0 - F.oy) * F.ky, Wy1 = (wy1 - F.oy) * F.ky;
+  e.rA = ra_nom > 0 ? ra_nom / utm_k(0.5 * (abx0 + abx1), 0.5 * (aby0 + aby1), clon, clat) : 0.0;
+  e.rB = mirror ? e.rA : rb_nom > 0 ? rb_nom / utm_k(0.5 * (bbx0 + bbx1), 0.5 * (bby0 + bby1), clon, clat) : 0.0;
+  const double2 k = m_per_deg_call(clat);
+  e.kx = k.x; e.ky = k.y;
+  e.fe = 1.0 + 2.0 * 0.5 * (wy1 - wy0) * DEG * (fabs(tan(clat * DEG)) + 0.05);
+  return e;
+}
+
+// Bound by FP64 latency at 8 warps an SM (the lists take 21 KB a warp, the code ~220 registers) and instruction fetch. 200k-parcel
+// self-join at 1 m, k_erode_main and k_erode_tiles: 6.5 ms with the set-up in every lane, sweeps of all edges for every
+// exclusion test and 218 KB of inlined code; 3.3 ms now.
+// X_A meets X_B within the window (S: er_set's, not empty): 1 / 0, or -1 when a list overflowed
+// (needE / needL = sizes required) (buffer.cuh:499-588). mirror: B is A (same layer, same pieces, same radius), so B's
+// edge and element lists, centre test and vertex pass are A's and are not built twice; every value they would hold is
+// computed from the same inputs by the same code. GRID: lists of up to 255 elements, searched by grid boxes.
+template <bool GRID>
+__device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, const ErSet& S, const ErScratch& sc, int lane, int* needE, int* needL,
+                       bool mirror) {
+  const double rA = S.rA, rB = S.rB;
+  EFrame F; { const double2 o = P.origin[ga.x]; F.ox = o.x; F.oy = o.y; } F.kx = S.kx; F.ky = S.ky;
+  const double Wx0 = (S.wx0 - F.ox) * F.kx, Wx1 = (S.wx1 - F.ox) * F.kx, Wy0 = (S.wy0 - F.oy) * F.ky, Wy1 = (S.wy1 - F.oy) * F.ky;
   const double ext = fmax(fmax(fabs(Wx0), fabs(Wx1)), fmax(fabs(Wy0), fabs(Wy1))) + fmax(rA, rB);
   const double eps = 1e-9 + 1e-12 * ext;
-  const double fe = 1.0 + 2.0 * 0.5 * (wy1 - wy0) * DEG * (fabs(tan(clat * DEG)) + 0.05);
-  const double ma = rA * fe + 1e-6, mb = rB * fe + 1e-6;
-  const int na = collect_side(P, ga.x, ga.y, F, Wx0 - ma, Wy0 - ma, Wx1 + ma, Wy1 + ma, sc.EA, sc.capE, lane);
+  const double ma = rA * S.fe + 1e-6, mb = rB * S.fe + 1e-6;
+  int ne[2], nl[2];
+#pragma unroll 1
+  for (int side = 0; side < (mirror ? 1 : 2); side++) {   // one inlined copy of each step
+    const double m = side ? mb : ma;
+    ne[side] = collect_side(side ? R : P, side ? gb.x : ga.x, side ? gb.y : ga.y, F, Wx0 - m, Wy0 - m, Wx1 + m, Wy1 + m, side ? sc.EB : sc.EA, sc.capE, lane);
+  }
+  const int na = ne[0], nb = mirror ? na : ne[1];
   BEd* const EBw = mirror ? sc.EA : sc.EB;
-  const int nb = mirror ? na : collect_side(R, gb.x, gb.y, F, Wx0 - mb, Wy0 - mb, Wx1 + mb, Wy1 + mb, EBw, sc.capE, lane);
   if (na > sc.capE || nb > sc.capE) { if (needE) *needE = max(na, nb); return -1; }
   __syncwarp();
-  prepare_side(sc.EA, na, rA, lane);
-  if (!mirror) prepare_side(EBw, nb, rB, lane);
-  const int la = build_elements(sc.EA, na, rA, Wx0, Wy0, Wx1, Wy1, eps, sc.LA, sc.capL, lane);
-  const int lb = mirror ? la : build_elements(EBw, nb, rB, Wx0, Wy0, Wx1, Wy1, eps, sc.LB, sc.capL, lane);
+#pragma unroll 1
+  for (int side = 0; side < (mirror ? 1 : 2); side++) {
+    BEd* const E = side ? sc.EB : sc.EA;
+    prepare_side(E, side ? nb : na, side ? rB : rA, lane);
+    nl[side] = build_elements(E, side ? nb : na, side ? rB : rA, Wx0, Wy0, Wx1, Wy1, eps, side ? sc.LB : sc.LA, sc.capL, lane);
+  }
+  const int la = nl[0], lb = mirror ? la : nl[1];
   if (la > sc.capL || lb > sc.capL) { if (needE) *needE = max(na, nb); if (needL) *needL = max(la, lb); return -1; }
   __syncwarp();
   const BEd* EA = sc.EA; const BEd* EB = EBw; const BEl* LA = sc.LA; const BEl* LB = mirror ? sc.LA : sc.LB;
+  const QGrid g = qgrid(Box{Wx0, Wy0, Wx1, Wy1});
+  excl_boxes(EA, na, rA, g, sc.qa, lane);
+  if (!mirror) excl_boxes(EB, nb, rB, g, sc.qe, lane);
+  const uint2* qA = sc.qa; const uint2* qB = mirror ? sc.qa : sc.qe;
+  __syncwarp();
   auto inW = [&](double x, double y) { return x >= Wx0 - eps && x <= Wx1 + eps && y >= Wy0 - eps && y <= Wy1 + eps; };
   // (a) the eroded boundaries cross outside both exclusion zones. The la x lb element grid is scanned 32 cells a
   // wave; cells whose boxes overlap are queued and tested 32 at a time, one per lane, so that the warp runs the
   // exclusion tests side by side (the answer is an any-of, so the order of the tests does not change it).
   bool hit = false;
   if (la && lb) {
-    const unsigned lt = (1u << lane) - 1;
-    uint2* Q = sc.Q;
-    auto cross = [&](uint2 e) {
-      const BEl p = LA[e.x], q = LB[e.y];
+    auto cross = [&](int i, int j) {
+      const BEl p = LA[i], q = LB[j];
       if (!seg_isect(p.x0, p.y0, p.x1, p.y1, q.x0, q.y0, q.x1, q.y1)) return false;
       double xs[3], ys[3]; const int k = seg_points(p, q, xs, ys);
+#pragma unroll 1
       for (int t = 0; t < k; t++)
-        if (inW(xs[t], ys[t]) && !in_excl(EA, na, rA, xs[t], ys[t], eps) && (mirror || !in_excl(EB, nb, rB, xs[t], ys[t], eps))) return true;
+        if (inW(xs[t], ys[t]) && !in_excl(EA, qA, g, na, rA, xs[t], ys[t], eps) && (mirror || !in_excl(EB, qB, g, nb, rB, xs[t], ys[t], eps))) return true;
       return false;
     };
+    if constexpr (GRID) {
+      auto view = [](const BEl* L) { return BElView{{&L->x0}, {&L->y0}, {&L->x1}, {&L->y1}}; };
+      scan_edge_pairs<false>(
+          view(LA), la, view(LB), lb, Box{Wx0, Wy0, Wx1, Wy1}, 0.0, 0.0, sc.qb, reinterpret_cast<uint16_t*>(sc.Q), lane, [](int, uint32_t) {}, [](int) {},
+          [&](uint32_t e, bool act) {
+            const int i = (int)(e >> 8), j = (int)(e & 255u);
+            if (act) {
+              const BEl p = LA[i], q = LB[j];
+              if (!(fmax(q.x0, q.x1) < fmin(p.x0, p.x1) || fmin(q.x0, q.x1) > fmax(p.x0, p.x1) || fmax(q.y0, q.y1) < fmin(p.y0, p.y1) ||
+                    fmin(q.y0, q.y1) > fmax(p.y0, p.y1)))
+                hit = cross(i, j);
+            }
+            return __any_sync(0xffffffffu, hit);
+          });
+      if (__any_sync(0xffffffffu, hit)) return 1;
+    } else {
+    const unsigned lt = (1u << lane) - 1;
+    uint2* Q = sc.Q;
     const uint64_t tot = (uint64_t)la * (uint64_t)lb;
     const int di = 32 / lb, dj = 32 % lb;
     int i = lane / lb, j = lane % lb, qn = 0;
+#pragma unroll 1
     for (uint64_t base = 0; base < tot; base += 32) {
       bool c = false;
       if (i < la) {
@@ -992,7 +1107,7 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, dou
       if (j >= lb) { j -= lb; i++; }
       if (qn >= 32) {
         __syncwarp();
-        if (__any_sync(0xffffffffu, cross(Q[lane]))) return 1;
+        if (__any_sync(0xffffffffu, cross((int)Q[lane].x, (int)Q[lane].y))) return 1;
         const int rest = qn - 32;
         const uint2 t = lane < rest ? Q[32 + lane] : make_uint2(0, 0);
         __syncwarp();
@@ -1002,13 +1117,15 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, dou
       }
     }
     __syncwarp();
-    if (__any_sync(0xffffffffu, lane < qn && cross(Q[lane]))) return 1;
+    if (__any_sync(0xffffffffu, lane < qn && cross((int)Q[lane].x, (int)Q[lane].y))) return 1;
     __syncwarp();
+    }
   }
   // (b), (c) a vertex of one eroded boundary inside the other eroded polygon
   const double cx = Wx0 + 0.381966 * (Wx1 - Wx0), cy = Wy0 + 0.414213 * (Wy1 - Wy0);
   const bool inA_c = pip_parent(P, ga.x, ga.y, F, cx, cy, lane);
   const bool inB_c = mirror ? inA_c : pip_parent(R, gb.x, gb.y, F, cx, cy, lane);
+#pragma unroll 1
   for (int side = 0; side < (mirror ? 1 : 2); side++) {
     const BEd* ES = side ? EB : EA; const BEd* EO = side ? EA : EB;
     const BEl* LS = side ? LB : LA;
@@ -1016,17 +1133,20 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, dou
     const double rs = side ? rB : rA, ro = side ? rA : rB;
     const bool inO_c = side ? inA_c : inB_c;
     auto vio = [&](double x, double y) {
-      return inW(x, y) && !in_excl(ES, ns, rs, x, y, eps) && inside_m(EO, no, cx, cy, inO_c, x, y) && !in_excl(EO, no, ro, x, y, eps);
+      return inW(x, y) && !in_excl(ES, side ? qB : qA, g, ns, rs, x, y, eps) && inside_m(EO, no, cx, cy, inO_c, x, y) && !in_excl(EO, side ? qA : qB, g, no, ro, x, y, eps);
     };
+#pragma unroll 1
     for (int i = lane; i < ls && !hit; i += 32) {
       const BEl p = LS[i];
       if (vio(p.x0, p.y0) || vio(p.x1, p.y1)) { hit = true; break; }
       const double px0 = fmin(p.x0, p.x1), px1 = fmax(p.x0, p.x1), py0 = fmin(p.y0, p.y1), py1 = fmax(p.y0, p.y1);
+#pragma unroll 1
       for (int j = i + 1; j < ls && !hit; j++) {
         const BEl q = LS[j];
         if (fmax(q.x0, q.x1) < px0 || fmin(q.x0, q.x1) > px1 || fmax(q.y0, q.y1) < py0 || fmin(q.y0, q.y1) > py1) continue;
         if (!seg_isect(p.x0, p.y0, p.x1, p.y1, q.x0, q.y0, q.x1, q.y1)) continue;
         double xs[3], ys[3]; const int k = seg_points(p, q, xs, ys);
+#pragma unroll 1
         for (int t = 0; t < k && !hit; t++) if (vio(xs[t], ys[t])) hit = true;
       }
     }
@@ -1036,15 +1156,7 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, dou
 }
 
 __device__ __forceinline__ uint2 piece_range(const uint32_t* pf, uint32_t p) { return pf ? make_uint2(pf[p], pf[p + 1]) : make_uint2(p, p + 1); }
-__device__ __forceinline__ ErScratch er_smem(unsigned char* raw, int wib) {
-  unsigned char* base = raw + (size_t)wib * ER_SMEM_WARP;
-  ErScratch sc;
-  sc.EA = reinterpret_cast<BEd*>(base); sc.EB = sc.EA + ER_CAPE;
-  sc.LA = reinterpret_cast<BEl*>(sc.EB + ER_CAPE); sc.LB = sc.LA + ER_CAPL;
-  sc.Q = reinterpret_cast<uint2*>(sc.LB + ER_CAPL);
-  sc.capE = ER_CAPE; sc.capL = ER_CAPL;
-  return sc;
-}
+__device__ __forceinline__ ErScratch er_smem(unsigned char* raw, int wib) { return er_carve(raw + (size_t)wib * ER_SMEM_WARP, ER_CAPE, ER_CAPL); }
 // pf[q] = first piece whose parent is >= q, q in [0, np] (parents non-decreasing)
 __global__ void k_piece_first(const uint32_t* __restrict__ parent, uint32_t n, uint32_t np, uint32_t* pf) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1111,12 +1223,20 @@ __global__ void __launch_bounds__(ER_WARPS * 32) k_erode_main(DLayer P, DLayer R
     if (lane == 0) p0 = atomicAdd(next, (unsigned long long)ER_RUN);
     p0 = __shfl_sync(0xffffffffu, p0, 0);
     if (p0 >= np) break;
-    const uint64_t p1 = p0 + ER_RUN < np ? p0 + ER_RUN : np;
-    for (uint64_t p = p0; p < p1; p++) {
-      const uint2 pr = pairs[p];
-      const int r = er_pair(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), ra, rb, sc, lane, nullptr, nullptr, nullptr, nullptr,
-                            self_layer && pr.x == pr.y);
-      if (lane == 0) { flag[p] = r > 0 ? 1 : 0; if (r < 0) heavy[atomicAdd(nheavy, 1u)] = (uint32_t)p; }
+    const int cnt = np - p0 < ER_RUN ? (int)(np - p0) : ER_RUN;
+    ErSet mine{};
+    uint2 mpr = make_uint2(0, 0);
+    if (lane < cnt) {
+      mpr = pairs[p0 + lane];
+      mine = er_set(P, R, piece_range(pfP, mpr.x), piece_range(pfR, mpr.y), ra, rb, nullptr, self_layer && mpr.x == mpr.y);
+    }
+#pragma unroll 1
+    for (int q = 0; q < cnt; q++) {
+      const uint2 pr = make_uint2(__shfl_sync(0xffffffffu, mpr.x, q), __shfl_sync(0xffffffffu, mpr.y, q));
+      const ErSet S{shfl_d(mine.wx0, q), shfl_d(mine.wy0, q), shfl_d(mine.wx1, q), shfl_d(mine.wy1, q), shfl_d(mine.rA, q),
+                    shfl_d(mine.rB, q),  shfl_d(mine.kx, q),  shfl_d(mine.ky, q),  shfl_d(mine.fe, q)};
+      const int r = S.wx0 > S.wx1 ? 0 : er_pair<true>(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), S, sc, lane, nullptr, nullptr, self_layer && pr.x == pr.y);
+      if (lane == 0) { flag[p0 + q] = r > 0 ? 1 : 0; if (r < 0) heavy[atomicAdd(nheavy, 1u)] = (uint32_t)(p0 + q); }
       __syncwarp();
     }
   }
@@ -1151,9 +1271,12 @@ __global__ void __launch_bounds__(ER_WARPS * 32) k_erode_tiles(DLayer P, DLayer 
   for (uint64_t i = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < ni; i += nw) {
     ETile t = items[i];
     if (flag[t.pair]) continue;   // another tile already found an intersection
-    int ne = 0, nl = 0; double4 win = t.box;
+    int ne = 0, nl = 0;
     const uint2 pr = pairs[t.pair];
-    const int r = er_pair(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), ra, rb, sc, lane, &ne, &nl, &t.box, &win, self_layer && pr.x == pr.y);
+    const bool mirror = self_layer && pr.x == pr.y;
+    const ErSet S = er_set(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), ra, rb, &t.box, mirror);
+    const double4 win = make_double4(S.wx0, S.wy0, S.wx1, S.wy1);
+    const int r = S.wx0 > S.wx1 ? 0 : er_pair<true>(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), S, sc, lane, &ne, &nl, mirror);
     if (lane == 0) {
       if (r > 0) flag[t.pair] = 1;
       else if (r < 0) er_overflow(t.pair, t.depth, win, fmax(ra, rb), ne, nl, next, slab, c);
@@ -1166,18 +1289,15 @@ __global__ void k_erode_slab(DLayer P, DLayer R, const uint32_t* pfP, const uint
                              double ra, double rb, bool self_layer, uint8_t* flag, unsigned char* scratch, int capE, int capL, ETile* again, ErCtr* c) {
   const int lane = threadIdx.x & 31;
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-  unsigned char* base = scratch + w * er_scratch_bytes(capE, capL);
-  ErScratch sc;
-  sc.EA = reinterpret_cast<BEd*>(base); sc.EB = sc.EA + capE;
-  sc.LA = reinterpret_cast<BEl*>(sc.EB + capE); sc.LB = sc.LA + capL;
-  sc.Q = reinterpret_cast<uint2*>(sc.LB + capL);
-  sc.capE = capE; sc.capL = capL;
+  const ErScratch sc = er_carve(scratch + w * er_scratch_bytes(capE, capL), capE, capL);   // qb lies past the end: unused here
   for (uint64_t i = w; i < ni; i += nw) {
     ETile t = items[i];
     if (flag[t.pair]) continue;
     int ne = 0, nl = 0;
     const uint2 pr = pairs[t.pair];
-    const int r = er_pair(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), ra, rb, sc, lane, &ne, &nl, &t.box, nullptr, self_layer && pr.x == pr.y);
+    const bool mirror = self_layer && pr.x == pr.y;
+    const ErSet S = er_set(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), ra, rb, &t.box, mirror);
+    const int r = S.wx0 > S.wx1 ? 0 : er_pair<false>(P, R, piece_range(pfP, pr.x), piece_range(pfR, pr.y), S, sc, lane, &ne, &nl, mirror);
     if (lane == 0) {
       if (r > 0) flag[t.pair] = 1;
       else if (r < 0) { again[atomicAdd(&c->nslab, 1u)] = t; atomicMax(&c->needE, ne); atomicMax(&c->needL, nl); }

@@ -6,7 +6,7 @@ import pytest
 import gsj
 import pyoracle as O
 from shapes import S, X0, Y0, cw, make_set
-from test_gpu_bins import ngon
+from test_gpu_bins import comb, ngon
 
 pytestmark = pytest.mark.gpu
 MODES = [gsj.GSJ_REFINE_PLAIN, gsj.GSJ_REFINE_FILTERED, gsj.GSJ_REFINE_FILTERED_FP32]
@@ -72,4 +72,27 @@ def test_polygons_within(engine, mode, d):
     la, lb = engine.upload_polygons(a), engine.upload_polygons(b)
     for lr, rs, same in ((lb, b, False), (la, a, True)):
         got, want = engine.dwithin(la, lr, d, same=same, refine_mode=mode)[0], O.dwithin(O.OSet(a), O.OSet(rs), d, same=same)[0]
+        assert set(map(tuple, got.tolist())) == set(map(tuple, want.tolist()))
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("r", [1.0, 4.0, 20.0])
+def test_eroded(engine, mode, r):
+    """Eroded polygons of 3 to 130 edges (the lists hold 64 edges and 128 elements), convex and with reflex corners,
+    each with itself and with shifted copies whose eroded forms just meet or just do not."""
+    sizes = [3, 31, 32, 33, 63, 64, 65, 130]
+    m = 1.0 / (111320.0 * np.cos(np.radians(Y0)))
+    A, B = [], []
+    for k, n in enumerate(sizes):
+        for q, f in enumerate((0.0, 0.3, 1.9, 1.99, 2.01, 2.1)):
+            cx, cy = 8 * S * k, 4 * S * q
+            A.append([ngon(n, S, cx, cy)])
+            B.append([ngon(n, S, cx + 2 * S - f * r * m if f else cx, cy)])
+        A.append([comb(max(2, n // 5), 2 * S, 2 * S, 8 * S * k, -4 * S)])
+        B.append([comb(max(2, n // 5), 2 * S, 2 * S, 8 * S * k + 0.1 * S, -4 * S - 0.2 * S)])
+    a, b = make_set(A), make_set(B)
+    la, lb = engine.upload_polygons(a), engine.upload_polygons(b)
+    for lr, rs, same in ((lb, b, False), (la, a, True)):
+        got, want = engine.erode(la, lr, r, r, same=same, refine_mode=mode)[0], O.erode(O.OSet(a), O.OSet(rs), r, r, same=same)
+        want = want[0] if isinstance(want, tuple) else want
         assert set(map(tuple, got.tolist())) == set(map(tuple, want.tolist()))
