@@ -366,8 +366,10 @@ __global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DL
       if (na <= DW_CAP && nb <= DW_CAP) {
         const double gx = shfl_d(mgx, k), gy = shfl_d(mgy, k), kx = shfl_d(mkx, k), ky = shfl_d(mky, k), tl = shfl_d(mtl, k), delta = shfl_d(mdelta, k);
         bool hit = false, open = false;
-        scan_edge_pairs<false>(
-            LA, na, LB, nb, ov, gx, gy, qb, q, lane, [](int, uint32_t) {}, [](int) {},
+        fill_boxes(LB, nb, qgrid(ov), qb, lane, 32);
+        __syncwarp();
+        scan_edge_pairs<false, 8>(
+            LA, na, LB, nb, ov, gx, gy, qb, q, 0, 32, lane, [](int, uint32_t) {}, [](int) {},
             [&](uint32_t e, bool act) {
               const int i = (int)(e >> 8), j = (int)(e & 255u);
               if (act && !((LA.fl[i] | LB.fl[j]) & 1u)) {
@@ -1073,8 +1075,10 @@ __device__ int er_pair(const DLayer& P, const DLayer& R, uint2 ga, uint2 gb, con
     };
     if constexpr (GRID) {
       auto view = [](const BEl* L) { return BElView{{&L->x0}, {&L->y0}, {&L->x1}, {&L->y1}}; };
-      scan_edge_pairs<false>(
-          view(LA), la, view(LB), lb, Box{Wx0, Wy0, Wx1, Wy1}, 0.0, 0.0, sc.qb, reinterpret_cast<uint16_t*>(sc.Q), lane, [](int, uint32_t) {}, [](int) {},
+      fill_boxes(view(LB), lb, g, sc.qb, lane, 32);
+      __syncwarp();
+      scan_edge_pairs<false, 8>(
+          view(LA), la, view(LB), lb, Box{Wx0, Wy0, Wx1, Wy1}, 0.0, 0.0, sc.qb, reinterpret_cast<uint16_t*>(sc.Q), 0, 32, lane, [](int, uint32_t) {}, [](int) {},
           [&](uint32_t e, bool act) {
             const int i = (int)(e >> 8), j = (int)(e & 255u);
             if (act) {

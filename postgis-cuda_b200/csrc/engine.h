@@ -131,7 +131,7 @@ struct RefineShape { int run = 4, runs = 32, bin_cap = 128, scratch_wpsm = 32; }
 // context and re-parameterised per call.
 struct RefineGraph {
   cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t n_main = nullptr, n_scr = nullptr, n_idx = nullptr, n_self = nullptr;
+  cudaGraphNode_t n_main = nullptr, n_scr = nullptr, n_idx = nullptr, n_self = nullptr, n_big = nullptr;
 };
 }  // namespace gsj
 
@@ -147,13 +147,13 @@ struct gsj_ctx {
   gsj::RefineShape shape;
   gsj::RefineGraph rgraph[36];   // [variant (plain, filtered x what is wanted, filtered FP32 x the same) x scratch bin or not x self bin or not]
   // scratch pools
-  gsj::DevBuf counters, cand, flag, area, ev, evb, heavy, selfidx, scratch, keep, opairs, oarea, oev, oevb, ocode, tmp, keys, keys2, idx,
+  gsj::DevBuf counters, cand, flag, area, ev, evb, heavy, heavy2, selfidx, scratch, keep, opairs, oarea, oev, oevb, ocode, tmp, keys, keys2, idx,
       idx2, agg_area, agg_ev, agg_evb, agg_flag, qbb, uf, misc1, misc2, misc3,
       er_pf, er_keep, er_off, er_pairs, er_flag, er_heavy, er_tiles, er_tiles2, er_slab, er_again, er_scr, er_ctr, er_tmp,
       enc_in, enc_cnt, enc_pre, enc_blk, enc_out;
   // every scratch pool, e.g. to bind them to the stream or release them before the stream goes
   template <class Fn> void each_buf(Fn&& fn) {
-    for (gsj::DevBuf* b : {&counters, &cand, &flag, &area, &ev, &evb, &heavy, &selfidx, &scratch, &keep, &opairs, &oarea, &oev, &oevb, &ocode, &tmp, &keys, &keys2, &idx, &idx2, &agg_area, &agg_ev, &agg_evb, &agg_flag, &qbb, &uf, &misc1, &misc2, &misc3, &er_pf, &er_keep, &er_off, &er_pairs, &er_flag, &er_heavy, &er_tiles, &er_tiles2, &er_slab, &er_again, &er_scr, &er_ctr, &er_tmp, &enc_in, &enc_cnt, &enc_pre, &enc_blk, &enc_out}) fn(*b);
+    for (gsj::DevBuf* b : {&counters, &cand, &flag, &area, &ev, &evb, &heavy, &heavy2, &selfidx, &scratch, &keep, &opairs, &oarea, &oev, &oevb, &ocode, &tmp, &keys, &keys2, &idx, &idx2, &agg_area, &agg_ev, &agg_evb, &agg_flag, &qbb, &uf, &misc1, &misc2, &misc3, &er_pf, &er_keep, &er_off, &er_pairs, &er_flag, &er_heavy, &er_tiles, &er_tiles2, &er_slab, &er_again, &er_scr, &er_ctr, &er_tmp, &enc_in, &enc_cnt, &enc_pre, &enc_blk, &enc_out}) fn(*b);
   }
   gsj::PinnedBuf h_counters, h_refine, h_pairs, h_area, h_code, h_where, h_enc;
   bool refine_pending = false;   // a refinement's counters are on their way to h_refine (refine_enqueue)

@@ -32,6 +32,26 @@ __device__ __forceinline__ bool ray_crosses(double x0, double y0, double x1, dou
   return so != sc && (a * (y0 - my) > 0) != (a * (y1 - my) > 0);
 }
 
+// Edge i of a ring of n vertices (the first is vertex s of the layer) in a pair frame: its ends and cut flags, whether it
+// meets the overlap box, and its crossing of the level ray to (mx, my) into par (PIP).
+struct GatherEdge { double x0, y0, x1, y1; uint32_t fl; bool in; };
+template <bool F, bool PIP, bool S32>
+__device__ __forceinline__ GatherEdge gather_edge(const Frame& A, const Box& ov, uint64_t s, uint32_t n, uint32_t i, double mx, double my, bool& par) {
+  const DLayer& S = *A.L;
+  GatherEdge e{0, 0, 0, 0, 0u, false};
+  if (i + 1 >= n) return e;
+  const double2 p = S.xy[s + i], q = S.xy[s + i + 1];
+  e.x0 = A.shx + p.x; e.y0 = A.shy + p.y; e.x1 = A.shx + q.x; e.y1 = A.shy + q.y;
+  if (S.synb) {
+    e.fl = (uint32_t)S.syn(s + i) | (S.syn(s + (i > 0 ? i - 1 : n - 2)) ? 2u : 0u) | (S.syn(s + (i + 2 < n ? i + 1 : 0)) ? 4u : 0u);
+  }
+  e.in = F ? !out_cmp(e.x0, e.y0, e.x1, e.y1, ov.x0, ov.y0, ov.x1, ov.y1) : !edge_outside(e.x0, e.y0, e.x1, e.y1, ov);
+  if (PIP && !((e.y0 > my) == (e.y1 > my) && e.y0 != my && e.y1 != my)) {
+    if (ray_crosses<S32>(e.x0, e.y0, e.x1, e.y1, A.shx - (double)1, mx, my)) par = !par;
+  }
+  return e;
+}
+
 // all edges of geometry A meeting the overlap box, compacted in ring order with a warp ballot (engine.cuh:358-377).
 // PIP: the same pass also takes the crossing parity of the segment (A's bbox left edge - 1, my) -> (mx, my) over
 // every edge of A, as pip_full_warp does (an XOR over the edges, so the order is free), into *inside.
@@ -39,34 +59,19 @@ template <bool F, bool PIP = false, bool S32 = false, class EL>
 static __device__ int collect(const Frame& A, const Box& ov, EL L, int cap, int lane, double mx = 0, double my = 0, bool* inside = nullptr) {
   const DLayer& S = *A.L;
   const unsigned lt = (1u << lane) - 1;
-  const double ox = A.shx - (double)1;
   bool par = false;
   int cnt = 0;
 #pragma unroll 1
   for (uint32_t ra = A.r0; ra < A.r1; ra++) {
     const uint64_t s = S.rvo[ra];
     const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);   // a ring's vertices, indexed by 32 bits
-    const double2* v = S.xy + s;
 #pragma unroll 1
     for (uint32_t base = 0; base + 1 < n; base += 32) {
-      const uint32_t i = base + lane;
-      bool in = false;
-      double x0 = 0, y0 = 0, x1 = 0, y1 = 0; uint32_t fl = 0;
-      if (i + 1 < n) {
-        const double2 p = v[i], q = v[i + 1];
-        x0 = A.shx + p.x; y0 = A.shy + p.y; x1 = A.shx + q.x; y1 = A.shy + q.y;
-        if (S.synb) {
-          fl = (uint32_t)S.syn(s + i) | (S.syn(s + (i > 0 ? i - 1 : n - 2)) ? 2u : 0u) | (S.syn(s + (i + 2 < n ? i + 1 : 0)) ? 4u : 0u);
-        }
-        in = F ? !out_cmp(x0, y0, x1, y1, ov.x0, ov.y0, ov.x1, ov.y1) : !edge_outside(x0, y0, x1, y1, ov);
-        if (PIP && !((y0 > my) == (y1 > my) && y0 != my && y1 != my)) {
-          if (ray_crosses<S32>(x0, y0, x1, y1, ox, mx, my)) par = !par;
-        }
-      }
-      const unsigned m = __ballot_sync(0xffffffffu, in);
+      const GatherEdge e = gather_edge<F, PIP, S32>(A, ov, s, n, base + lane, mx, my, par);
+      const unsigned m = __ballot_sync(0xffffffffu, e.in);
       const int pos = cnt + __popc(m & lt);
-      if (in && pos < cap) {
-        L.x0[pos] = x0; L.y0[pos] = y0; L.x1[pos] = x1; L.y1[pos] = y1; L.fl[pos] = fl;
+      if (e.in && pos < cap) {
+        L.x0[pos] = e.x0; L.y0[pos] = e.y0; L.x1[pos] = e.x1; L.y1[pos] = e.y1; L.fl[pos] = e.fl;
       }
       cnt += __popc(m);
     }
@@ -174,38 +179,43 @@ __device__ __forceinline__ QBox qbox(const QGrid& g, const EL& L, int i) {
   return QBox{min(px, qx), min(py, qy), max(px, qx), max(py, qy)};
 }
 
+// the boxes of a list's edges as B boxes, guard bits set; t of nt: the calling thread among those that fill them
+template <class EL>
+__device__ __forceinline__ void fill_boxes(const EL& L, int n, const QGrid& g, uint2* qb, int t, int nt) {
+#pragma unroll 1
+  for (int j = t; j < n; j += nt) {
+    const QBox b = qbox(g, L, j);
+    qb[j] = make_uint2(0x80008000u + (uint32_t)(b.x1 << 16 | (0x7FFF - b.x0)), 0x80008000u + (uint32_t)(b.y1 << 16 | (0x7FFF - b.y0)));
+  }
+}
+
 // Finds the pairs (i of A, j of B) of local edges whose boxes come within (padx, pady) of each other, or a little more
-// (TRI: one list, j > i only), and hands them to wave(i << 8 | j, act) 32 at a time, one per lane; wave is called by
+// (TRI: one list, j > i only), and hands them to wave(i << SH | j, act) 32 at a time, one per lane; wave is called by
 // the whole warp and ends the search by returning true (for all lanes). on_block(w, bits): lane i's pairs with B's 32
-// edges from 32 w on, on_row(ic): A's 32 edges from ic on are done. Lists of up to 255 edges.
+// edges from 32 w on, on_row(ic): A's 32 edges from ic on are done. qb: B's boxes (fill_boxes over the same box); the
+// warp takes the 32 A edges from ic0 on, then those from ic0 + step on. Lists of up to 1 << SH edges (Q: the queue's type).
 // A lane keeps the grid box of one A edge (per 32) in registers and tests B's edges one after the other, each read once
 // for the whole warp (a shared-memory broadcast): 7 integer instructions a pair against ~24 with FP64 boxes. The pairs
 // go through a queue, since a lane's own edge has few: the waves are full.
 constexpr int QCAP = 64;
-template <bool TRI, class EL, class Block, class Row, class Wave>
-__device__ __forceinline__ void scan_edge_pairs(const EL& LA, int na, const EL& LB, int nb, const Box& box, double padx, double pady, uint2* qb, uint16_t* q,
-                                                int lane, Block&& on_block, Row&& on_row, Wave&& wave) {
+template <bool TRI, int SH, class EL, class Q, class Block, class Row, class Wave>
+__device__ __forceinline__ void scan_edge_pairs(const EL& LA, int na, const EL& LB, int nb, const Box& box, double padx, double pady, const uint2* qb, Q* q,
+                                                int ic0, int step, int lane, Block&& on_block, Row&& on_row, Wave&& wave) {
   const int nbw = (nb + 31) >> 5;
   const unsigned lt = (1u << lane) - 1;
   const QGrid g = qgrid(box);
   const int cx = 2 + (int)fminf((float)padx * g.sx * 32767.f, 32767.f), cy = 2 + (int)fminf((float)pady * g.sy * 32767.f, 32767.f);   // in cells, rounded up
-#pragma unroll 1
-  for (int j = lane; j < nb; j += 32) {
-    const QBox b = qbox(g, LB, j);
-    qb[j] = make_uint2(0x80008000u + (uint32_t)(b.x1 << 16 | (0x7FFF - b.x0)), 0x80008000u + (uint32_t)(b.y1 << 16 | (0x7FFF - b.y0)));
-  }
-  __syncwarp();
-  int qn = 0, ic = 0, w = -1;   // ic, w: the 32 A edges and the 32 B edges being tested
+  int qn = 0, ic = ic0, w = -1;   // ic, w: the 32 A edges and the 32 B edges being tested
   uint32_t bits = 0;
   uint2 ab = make_uint2(0u, 0u);
 #pragma unroll 1
-  for (bool more = na > 0 && nb > 0; more || qn > 0;) {
+  for (bool more = ic0 < na && nb > 0; more || qn > 0;) {
 #pragma unroll 1
     while (more && qn < 32) {
       const unsigned m = __ballot_sync(0xffffffffu, bits != 0);
       if (m) {   // each lane queues one of its pairs
         if (bits) {
-          q[qn + __popc(m & lt)] = (uint16_t)((ic + lane) << 8 | ((w << 5) + __ffs(bits) - 1));
+          q[qn + __popc(m & lt)] = (Q)((ic + lane) << SH | ((w << 5) + __ffs(bits) - 1));
           bits &= bits - 1;
         }
         qn += __popc(m);
@@ -214,7 +224,7 @@ __device__ __forceinline__ void scan_edge_pairs(const EL& LA, int na, const EL& 
       if (w < 0 || ++w >= nbw) {   // next 32 A edges
         if (w >= nbw) {
           on_row(ic);
-          ic += 32;
+          ic += step;
           if (ic >= na) { more = false; break; }
         }
         w = TRI ? ic >> 5 : 0;
@@ -241,7 +251,7 @@ __device__ __forceinline__ void scan_edge_pairs(const EL& LA, int na, const EL& 
     }
     __syncwarp();
     const uint32_t e = q[lane];
-    const uint16_t rest = q[32 + lane];
+    const Q rest = q[32 + lane];
     if (wave(e, lane < qn)) break;
     __syncwarp();
     qn = max(qn - 32, 0);

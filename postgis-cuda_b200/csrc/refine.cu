@@ -4,8 +4,8 @@
 // its lane ownership kept (lane l owns local edges l, l+32, ...; A's then B's; shfl_down tree 16..1), so the
 // FP64 area and boundary-length sums have one fixed rounding order: bit-identical to the CPU oracle.
 //
-// Pairs whose local edge lists fit CAP run from shared memory; larger pairs are queued and re-run by
-// k_refine_scratch with per-warp lists in global scratch.
+// Pairs whose local edge lists fit CAP run from shared memory, a warp each; larger pairs are queued and re-run by
+// k_refine_block (filtered: a block each) and, beyond its lists, k_refine_scratch (per-warp lists in global scratch).
 //
 // Two variants with the same decisions and the same FP64 values:
 //  - plain (F = false): the reference's sweeps, FP64 box tests (refine_pair_t<false>).
@@ -571,11 +571,9 @@ __device__ bool refine_pair(const DLayer& P, const DLayer& R, uint32_t a, uint32
 
 // ---- the shared-memory bins' pair routine (filtered variants) -----------------------------------------------------------
 // Per warp: the two edge lists, the boxes of B's edges on a 15-bit grid over the overlap box (qb), a queue of candidate edge
-// pairs (q), the coincident pairs as bit masks (row i of A: the B edges that coincide with part of A's edge i, column j the A
-// edges that do with B's edge j; word w of row i at rm[w * stride + i]) and the split points of both polygons' edges
-// (the unused tails of the list arrays). cand: bit i of A (then bit j of B) set when any edge of the other polygon
-// comes within 2 tol of the edge.
-//
+// pairs (q) and the cuts of both polygons' edges as linked lists (head of each edge, nodes val / nxt): a split point's
+// parameter, or an edge of the other polygon that coincides with part of the edge. cand: bit i of A (then bit j of B) set
+// when any edge of the other polygon comes within 2 tol of the edge.
 // The routine is bound by instruction issue, dependent latency (16 warps per SM) and instruction fetch, so the work is laid out to keep
 // lanes busy side by side and the code small: edge pairs whose boxes come within 2 tol are queued and classified 32 at a
 // time, one per lane, from the four orientations of the pair, which decide the contact and every cut the two edges make in each
@@ -585,25 +583,23 @@ __device__ bool refine_pair(const DLayer& P, const DLayer& R, uint32_t a, uint32
 // Loops are kept rolled on purpose: the kernel runs nearly straight through its code, and above about 48 KB of it the
 // warps wait for instructions (100k parcels, this kernel: 71 KB 5.66 ms, 54 KB 3.82 ms, 49 KB 2.86 ms, with the
 // instruction-fetch stall at 8.6, 4.3 and 0.9 cycles an instruction).
+// Cuts as linked lists instead of masks and a pool of split points: 500k-parcel relate self-join 21.2 -> 20.4 ms.
 // 100k-parcel relate self-join, against lanes that each visited their own edge's candidates: this bin 3.45 -> 2.86 ms, the
 // self bin 1.44 -> 0.76 ms; two 60k layers, area: 4.35 -> 3.16 ms (14.5 -> 20.5 lanes active per instruction).
-struct MaskBuf { uint32_t* rm; uint32_t* cm; uint2* qb; uint32_t* cand; uint16_t* q; };
-
-// Split points found by the classification: edge and parameter, in the tails of a list's arrays (n of MS entries in
-// use): the parameters behind x0 and x1, the edges behind y0 and y1. 2 (MS - n) of them fit.
-template <int MS, class EL>
-__device__ __forceinline__ double* split_slot(const EL& L, int n, int s) { return L.x0 + n + (s < MS - n ? s : s + 2 * MS - (MS - n)); }
-struct Splits { int a, b; bool full; };   // split points of A's and of B's edges so far (uniform); full: some did not fit
+constexpr int NIL = 0x7FFF, COVER = 0x8000;   // nxt: end of list; bit 15: the node names a coincident edge
+template <class Q>
+struct CutLists { uint2* qb; double* val; uint32_t* headA; uint32_t* headB; uint32_t* cand; uint16_t* nxt; Q* q; uint32_t* count; int cap; };
+struct Nodes { int n; bool full; };   // nodes in use (a warp's own lists; a block counts in *count); full: some did not fit
 
 // Classifies one candidate edge pair (i of A, j of B) per lane: real / any contact (seg_isect on the four orientations
 // of the pair, behind the same box test), and for either edge what edge_visit finds for it: coincidence (a bit in the
 // masks) or a split point. The two edges' conditions are the same but for their box tests, the order of a product and
 // the end tolerances; r, tn and un change sign together when the edges swap roles, so un / r is B's parameter.
-template <int MS, bool SELF, bool CUTS, class EL>
-__device__ __forceinline__ void classify_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const MaskBuf& mb, uint32_t e, bool act, int lane,
-                                               Splits& sp, bool& hit, bool& hit_any) {
-  const int i = (int)(e >> 8), j = (int)(e & 255u);
-  bool sa = false, sb = false;
+template <bool SELF, bool CUTS, int SH, class Q, class EL>
+__device__ __forceinline__ void classify_pairs(const EL& LA, const EL& LB, const PairGeo& G, const CutLists<Q>& cl, uint32_t e, bool act, int lane, Nodes& nd,
+                                               bool& hit, bool& hit_any) {
+  const int i = (int)(e >> SH), j = (int)(e & ((1u << SH) - 1u));
+  bool sa = false, sb = false, va = false, vb = false;   // split point of A's / B's edge; coincident part of A's / B's edge
   double t = 0, u = 0;
   if (act) {
     const double px = LA.x0[i], py = LA.y0[i], qx = LA.x1[i], qy = LA.y1[i];
@@ -634,13 +630,11 @@ __device__ __forceinline__ void classify_pairs(const EL& LA, int na, const EL& L
       const bool onA = c0 * c0 <= ((fb & 2u) ? cat : ca) && c1 * c1 <= ((fb & 4u) ? cat : ca);
       const bool onB = g0 * g0 <= ((fa & 2u) ? cbt : cb) && g1 * g1 <= ((fa & 4u) ? cbt : cb);
       ka = ka && len2 != 0; kb = kb && flen2 != 0;
-      if (onA || onB) {
-        if (ka && (onA || flen2 > 0)) atomicOr(&mb.rm[(j >> 5) * MS + i], 1u << (j & 31));
-        if (kb && (onB || len2 > 0)) atomicOr(SELF ? &mb.rm[(i >> 5) * MS + j] : &mb.cm[(i >> 5) * MS + j], 1u << (i & 31));
-      }
+      va = ka && (onA || (onB && flen2 > 0));
+      vb = kb && (onB || (onA && len2 > 0));
       const double r = dx * fy - dy * fx, wx = ex0 - px, wy = ey0 - py, tn = wx * fy - wy * fx, un = wx * dy - wy * dx;
-      sa = ka && !(onA || (flen2 > 0 && onB)) && r * r > eps2 * len2 * flen2 && (r > 0 ? (tn > 0 && tn < r) : (tn < 0 && tn > r));
-      sb = kb && !(onB || (len2 > 0 && onA)) && r * r > eps2 * flen2 * len2 && (r > 0 ? (un > 0 && un < r) : (un < 0 && un > r));
+      sa = ka && !va && r * r > eps2 * len2 * flen2 && (r > 0 ? (tn > 0 && tn < r) : (tn < 0 && tn > r));
+      sb = kb && !vb && r * r > eps2 * flen2 * len2 && (r > 0 ? (un > 0 && un < r) : (un < 0 && un > r));
       if (sa || sb) {
 #pragma unroll 1
         for (int z = 0; z < 2; z++) {   // one site for the division and the square root: t, then u; beyond an end: within its tolerance?
@@ -653,25 +647,30 @@ __device__ __forceinline__ void classify_pairs(const EL& LA, int na, const EL& L
     }
   }
   if constexpr (!CUTS) return;
-  const unsigned ma = __ballot_sync(0xffffffffu, sa), mB = __ballot_sync(0xffffffffu, sb);
+  const unsigned ma = __ballot_sync(0xffffffffu, sa || va), mB = __ballot_sync(0xffffffffu, sb || vb);
   if (ma | mB) {
     const unsigned lt = (1u << lane) - 1;
-    const int na2 = sp.a + __popc(ma), b0 = SELF ? na2 : sp.b, nb2 = b0 + __popc(mB);
-    sp.full = sp.full || na2 > 2 * (MS - na) || nb2 > 2 * (MS - (SELF ? na : nb));
-    if (!sp.full) {
-      if (sa) {
-        double* d = split_slot<MS>(LA, na, sp.a + __popc(ma & lt));
-        d[0] = t;
-        *reinterpret_cast<int*>(d + MS) = i;
+    const int total = __popc(ma) + __popc(mB);
+    int at = nd.n;
+    if (cl.count) {
+      if (lane == 0) at = (int)atomicAdd(cl.count, (uint32_t)total);
+      at = __shfl_sync(0xffffffffu, at, 0);
+    } else {
+      nd.n += total;
+    }
+    if (at + total > cl.cap) nd.full = true;
+    else {
+      if (sa || va) {
+        const int k = at + __popc(ma & lt);
+        cl.val[k] = va ? (double)j : t;
+        cl.nxt[k] = (uint16_t)(atomicExch(&cl.headA[i], (uint32_t)k) | (va ? COVER : 0));
       }
-      if (sb) {
-        double* d = split_slot<MS>(SELF ? LA : LB, SELF ? na : nb, b0 + __popc(mB & lt));
-        d[0] = u;
-        *reinterpret_cast<int*>(d + MS) = j;
+      if (sb || vb) {
+        const int k = at + __popc(ma) + __popc(mB & lt);
+        cl.val[k] = vb ? (double)i : u;
+        cl.nxt[k] = (uint16_t)(atomicExch(SELF ? &cl.headA[j] : &cl.headB[j], (uint32_t)k) | (vb ? COVER : 0));
       }
     }
-    sp.a = SELF ? nb2 : na2;
-    sp.b = SELF ? 0 : nb2;
   }
 }
 
@@ -697,43 +696,109 @@ __device__ __forceinline__ void edge_cover(EdgeCuts& C, const EdgeRef& e, const 
 }
 
 // Candidate edge pairs (boxes within 2 tol of each other, or a little more on the grid) found and classified; CUTS: the cuts
-// are wanted, else the contact alone (the search then ends at the first real one). SELF: an edge always coincides
-// with itself, only j > i is searched.
-template <int MS, bool SELF, bool CUTS, class EL>
-__device__ Splits find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const MaskBuf& mb, int lane, bool& hit, bool& hit_any) {
-  if constexpr (CUTS) {
-    uint4* z = reinterpret_cast<uint4*>(mb.rm);
-#pragma unroll 1
-    for (int t = lane; t < (SELF ? 1 : 2) * (MS / 32) * MS / 4; t += 32) z[t] = make_uint4(0u, 0u, 0u, 0u);
-    if (!SELF && lane < 2 * (MS / 32)) mb.cand[lane] = 0u;
-    __syncwarp();
-    if (SELF)
-#pragma unroll 1
-      for (int j = lane; j < nb; j += 32) mb.rm[(j >> 5) * MS + j] = 1u << (j & 31);
-  }
-  Splits sp{0, 0, false};
+// are wanted, else the contact alone (the search then ends at the first real one). SELF: only j > i is searched (an edge
+// always coincides with itself). One warp takes the 32 A edges from ic0 on, then those from ic0 + step on, ...
+template <int MS, bool SELF, bool CUTS, int SH, class Q, class EL>
+__device__ Nodes find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const CutLists<Q>& cl, int ic0, int step, int lane, bool& hit,
+                            bool& hit_any) {
+  Nodes nd{0, false};
   uint32_t any = 0;
-  scan_edge_pairs<SELF>(
-      LA, na, LB, nb, G.ov, 2.0 * G.tol, 2.0 * G.tol, mb.qb, mb.q, lane,
+  scan_edge_pairs<SELF, SH>(
+      LA, na, LB, nb, G.ov, 2.0 * G.tol, 2.0 * G.tol, cl.qb, cl.q, ic0, step, lane,
       [&](int w, uint32_t bits) {
         if constexpr (!SELF && CUTS) {
           any |= bits;
           const uint32_t ob = __reduce_or_sync(0xffffffffu, bits);
-          if (lane == 0) mb.cand[MS / 32 + w] |= ob;
+          if (lane == 0 && ob) atomicOr(&cl.cand[MS / 32 + w], ob);
         }
       },
       [&](int ic) {
         if constexpr (!SELF && CUTS) {
           const unsigned c = __ballot_sync(0xffffffffu, any != 0);
-          if (lane == 0) mb.cand[ic >> 5] = c;
+          if (lane == 0) cl.cand[ic >> 5] = c;
           any = 0;
         }
       },
       [&](uint32_t e, bool act) {
-        classify_pairs<MS, SELF, CUTS>(LA, na, LB, nb, G, mb, e, act, lane, sp, hit, hit_any);
+        classify_pairs<SELF, CUTS, SH>(LA, LB, G, cl, e, act, lane, nd, hit, hit_any);
         return !CUTS && __any_sync(0xffffffffu, hit);
       });
-  return sp;
+  return nd;
+}
+// the grid boxes of B's edges and, where cuts are wanted, empty lists; t of nt: the calling thread among those that share them
+template <int MS, bool SELF, bool CUTS, class Q, class EL>
+__device__ __forceinline__ void begin_pairs(const EL& LB, int na, int nb, const PairGeo& G, const CutLists<Q>& cl, int t, int nt) {
+  fill_boxes(LB, nb, qgrid(G.ov), cl.qb, t, nt);
+  if constexpr (CUTS) {
+#pragma unroll 1
+    for (int i = t; i < na; i += nt) cl.headA[i] = NIL;
+    if (!SELF) {
+#pragma unroll 1
+      for (int j = t; j < nb; j += nt) cl.headB[j] = NIL;
+      if (t < 2 * (MS / 32)) cl.cand[t] = 0u;
+    }
+  }
+}
+
+// Lane's edge i with its cuts: split points in any order (they are sorted), coincident edges in increasing order.
+// C.ns == MAXS: the split points reached the number that is kept (which are kept depends on the order they are met in).
+template <bool REL, bool SELF, class Q, class EL>
+__device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS, int i, bool valid, const EL& LO, const CutLists<Q>& cl, const uint32_t* head) {
+  edge_cuts_begin(C);
+  e.px = e.py = e.qx = e.qy = e.dx = e.dy = e.len2 = e.len = 0.0; e.fl = 0;
+  if (!valid) return;
+  e = edge_ref(LS, i, REL);
+  int nc = SELF ? 1 : 0, k = SELF ? i : 0x7FFFFFFF;   // coincident edges, the first of them
+#pragma unroll 1
+  for (uint32_t n = head[i]; n != NIL;) {
+    const uint32_t w = cl.nxt[n];
+    const double v = cl.val[n];
+    if (w & COVER) { nc++; k = min(k, (int)v); }
+    else if (C.ns < MAXS) C.ts[C.ns++] = v;
+    n = w & NIL;
+  }
+#pragma unroll 1
+  while (nc > 0) {
+    edge_cover(C, e, LO, k);
+    if (--nc == 0) break;
+    int next = SELF && i > k ? i : 0x7FFFFFFF;
+#pragma unroll 1
+    for (uint32_t n = head[i]; n != NIL;) {
+      const uint32_t w = cl.nxt[n];
+      const int c = (w & COVER) ? (int)cl.val[n] : 0x7FFFFFFF;
+      if (c > k) next = min(next, c);
+      n = w & NIL;
+    }
+    k = next;
+  }
+  edge_cuts_sort(C);
+}
+
+// The inside tests of 32 lanes' points (need, mx, my) against the polygon LO, one test at a time by the whole warp; lanes
+// linked to their predecessor (bit l of link: points l - 1 and l lie on the same side of LO) take its answer.
+template <bool S32, class EL>
+__device__ __forceinline__ bool inside_lanes(bool need, double mx, double my, unsigned link, const EL& LO, int nother, bool inc, const PairGeo& G, int lane) {
+  const unsigned needm = __ballot_sync(0xffffffffu, need), le = (2u << lane) - 1u;
+  if (!needm) return false;
+  // this lane's run of linked points: [start, end); its first that needs the test takes it for all
+  const unsigned heads = ~link;
+  const int start = 31 - __clz(heads & le);
+  const unsigned after = heads & ~le;
+  const unsigned run = (after ? (after & (0u - after)) - 1u : 0xffffffffu) & ~((1u << start) - 1u);
+  const int tester = __ffs(needm & run) - 1;
+  unsigned in = 0;
+#pragma unroll 1
+  for (unsigned m = __ballot_sync(0xffffffffu, need && tester == lane); m; m &= m - 1) {
+    const int src = __ffs(m) - 1;
+    const double x = __shfl_sync(0xffffffffu, mx, src), y = __shfl_sync(0xffffffffu, my, src);
+    if (inside_from_c_warp<S32>(LO, nother, G.cx, G.cy, inc, x, y, lane)) in |= 1u << src;
+  }
+  return need && ((in >> tester) & 1u);
+}
+// link mask of a chunk of edges (see edge_pass): fr = edges without candidates
+__device__ __forceinline__ unsigned edge_links(const EdgeRef& e, bool valid, unsigned fr, int lane) {
+  const double prx = __shfl_up_sync(0xffffffffu, e.qx, 1), pry = __shfl_up_sync(0xffffffffu, e.qy, 1);
+  return __ballot_sync(0xffffffffu, valid && lane > 0 && prx == e.px && pry == e.py) & fr & (fr << 1);
 }
 
 // One polygon's contribution pass: lane l owns edges l, l + 32, ... and adds its values in that order. Each lane collects its
@@ -745,40 +810,21 @@ __device__ Splits find_pairs(const EL& LA, int na, const EL& LB, int nb, const P
 // of such edges takes one test. (The crossing-parity test returns the true side for points this far from the boundary:
 // its orientation signs can only be wrong for points within rounding, ~1e-7 of tol, of an edge's line.) tol below
 // 1e-12 of the overlap box (a caller's own tolerances) turns the sharing off.
-template <bool S32, int MS, bool SELF, bool AREA, bool REL, class EL>
-__device__ __forceinline__ bool edge_pass(const EL& LS, int nself, int nsplit, const EL& LO, int nother, const uint32_t* mrow, const uint32_t* cand, bool inc,
-                                          const PairGeo& G, bool share, int lane, double& s2, double& lin, double& lon, uint32_t& bits, double* rec) {
-  const int nw = (nother + 31) >> 5;
-  const unsigned le = (2u << lane) - 1u;
+template <bool S32, bool SELF, bool AREA, bool REL, class Q, class EL>
+__device__ __forceinline__ bool edge_pass(const EL& LS, int nself, const EL& LO, int nother, const CutLists<Q>& cl, const uint32_t* head, const uint32_t* cand,
+                                          bool inc, const PairGeo& G, bool share, int lane, double& s2, double& lin, double& lon, uint32_t& bits,
+                                          double* rec) {
 #pragma unroll 1
   for (int ic = 0, c = 0; ic < nself; ic += 32, c++) {
     const int i = ic + lane;
     EdgeRef e;
     EdgeCuts C;
-    edge_cuts_begin(C);
-#pragma unroll 1
-    for (int k = 0; k < nsplit; k++) {
-      const double* d = split_slot<MS>(LS, nself, k);
-      if (*reinterpret_cast<const int*>(d + MS) == i && C.ns < MAXS) C.ts[C.ns++] = d[0];
-    }
-    e.px = e.py = e.qx = e.qy = e.dx = e.dy = e.len2 = e.len = 0.0; e.fl = 0;
-    if (i < nself) {
-      e = edge_ref(LS, i, REL);
-#pragma unroll 1
-      for (int w = 0; w < nw; w++)
-#pragma unroll 1
-        for (uint32_t m = mrow[w * MS + i]; m; m &= m - 1) edge_cover(C, e, LO, (w << 5) + __ffs(m) - 1);
-      edge_cuts_sort(C);
-    }
+    edge_cuts<REL, SELF>(e, C, LS, i, i < nself, LO, cl, head);
     if (__any_sync(0xffffffffu, C.ns == MAXS)) return false;
     if (e.len2 == 0) C.ns = 0;
     const bool lens = REL && !(e.fl & 1u);
-    unsigned link = 0;   // bit l: edges l - 1 and l are free of the other polygon and share an end point
-    if constexpr (!SELF) {
-      const unsigned fr = share ? ~cand[c] : 0u;
-      const double prx = __shfl_up_sync(0xffffffffu, e.qx, 1), pry = __shfl_up_sync(0xffffffffu, e.qy, 1);
-      link = __ballot_sync(0xffffffffu, i < nself && lane > 0 && prx == e.px && pry == e.py) & fr & (fr << 1);
-    }
+    unsigned link = 0;
+    if constexpr (!SELF) link = edge_links(e, i < nself, share ? ~cand[c] : 0u, lane);
     double acc = 0.0;
 #pragma unroll 1
     for (int k = 0; __any_sync(0xffffffffu, k + 1 < C.ns); k++) {
@@ -786,25 +832,8 @@ __device__ __forceinline__ bool edge_pass(const EL& LS, int nself, int nsplit, c
       s.valid = s.need = false;
       s.mx = s.my = 0;
       if (k + 1 < C.ns) s = edge_segment<AREA>(C, e, LO, k, G, lens);
-      int vin = 0;
-      const unsigned needm = __ballot_sync(0xffffffffu, s.need);
-      if (needm) {
-        // this lane's run of linked edges: [start, end); its first edge that needs the test takes it for all
-        const unsigned heads = k == 0 ? ~link : 0xffffffffu;
-        const int start = 31 - __clz(heads & le);
-        const unsigned after = heads & ~le;
-        const unsigned run = (after ? (after & (0u - after)) - 1u : 0xffffffffu) & ~((1u << start) - 1u);
-        const int tester = __ffs(needm & run) - 1;
-        unsigned in = 0;
-#pragma unroll 1
-        for (unsigned m = __ballot_sync(0xffffffffu, s.need && tester == lane); m; m &= m - 1) {
-          const int src = __ffs(m) - 1;
-          const double x = __shfl_sync(0xffffffffu, s.mx, src), y = __shfl_sync(0xffffffffu, s.my, src);
-          if (inside_from_c_warp<S32>(LO, nother, G.cx, G.cy, inc, x, y, lane)) in |= 1u << src;
-        }
-        vin = s.need && ((in >> tester) & 1u) ? 1 : 0;
-      }
-      if (s.valid) edge_segment_add<AREA>(s, C, e, LO, G, lens, vin, acc, lin, lon, bits);
+      const bool vin = inside_lanes<S32>(s.need, s.mx, s.my, k ? 0u : link, LO, nother, inc, G, lane);
+      if (s.valid) edge_segment_add<AREA>(s, C, e, LO, G, lens, vin ? 1 : 0, acc, lin, lon, bits);
     }
     if (AREA) s2 += acc;
     if (AREA && rec) rec[c] = acc;
@@ -825,7 +854,7 @@ enum Want { W_FLAG = 0, W_AREA = 1, W_REL = 2, W_ALL = 3 };
 // order, which is the sum the two passes make. Every edge meets itself, so the contact needs no test.
 template <bool S32, int SELF, int W>
 __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList8 LA, EList8 LB, int cap, int lane,
-                              uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const MaskBuf& mb, unsigned long long* ep) {
+                              uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const CutLists<uint16_t>& cl, unsigned long long* ep) {
   constexpr int MS = SELF ? SELF : CAP_F;   // row stride of the masks
   constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
   Frame A, B;
@@ -842,15 +871,17 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
   if (na > cap || nb > cap) return false;
   __syncwarp();
   bool hit = false, hit_any = false;
-  Splits sp{0, 0, false};
+  Nodes nd{0, false};
+  if constexpr (SELF == 0 || W != W_FLAG) {
+    begin_pairs<MS, (SELF > 0), W != W_FLAG>(LB, na, nb, G, cl, lane, 32);
+    __syncwarp();
+    nd = find_pairs<MS, (SELF > 0), W != W_FLAG, 8>(LA, na, LB, nb, G, cl, 0, 32, lane, hit, hit_any);
+  }
   if constexpr (SELF > 0) {
 #pragma unroll 1
     for (int i = lane; i < na; i += 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
-    if constexpr (W != W_FLAG) sp = find_pairs<MS, true, true>(LA, na, LB, nb, G, mb, lane, hit, hit_any);
-  } else {
-    sp = find_pairs<MS, false, W != W_FLAG>(LA, na, LB, nb, G, mb, lane, hit, hit_any);
   }
-  if (sp.full) return false;
+  if (nd.full) return false;
   hit = __any_sync(0xffffffffu, hit);
   hit_any = __any_sync(0xffffffffu, hit_any || hit);
   const bool rtouch = hit;
@@ -863,7 +894,7 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
       const bool share = G.tol >= 1e-12 * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0);
       if constexpr (SELF > 0) {
         double rec[SELF / 32];
-        if (!edge_pass<S32, MS, true, AREA, REL>(LA, na, sp.a, LB, nb, mb.rm, mb.cand, inB_c, G, false, lane, S.s2, S.ai, S.ao, bits, rec)) return false;
+        if (!edge_pass<S32, true, AREA, REL>(LA, na, LB, nb, cl, cl.headA, cl.cand, inB_c, G, false, lane, S.s2, S.ai, S.ao, bits, rec)) return false;
 #pragma unroll 1
         for (int c = 0; AREA && c * 32 < na; c++) S.s2 += rec[c];
         S.bi = S.ai; S.bo = S.ao;
@@ -871,8 +902,8 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
 #pragma unroll 1
         for (int pass = 0; pass < 2; pass++) {   // one inlined copy of the pass
           double lin = 0.0, lon = 0.0;   // this pass's lengths (each starts from 0, so the sums are the same)
-          if (!edge_pass<S32, MS, false, AREA, REL>(pass ? LB : LA, pass ? nb : na, pass ? sp.b : sp.a, pass ? LA : LB, pass ? na : nb, pass ? mb.cm : mb.rm,
-                                                    mb.cand + (pass ? MS / 32 : 0), pass ? inA_c : inB_c, G, share, lane, S.s2, lin, lon, bits, nullptr))
+          if (!edge_pass<S32, false, AREA, REL>(pass ? LB : LA, pass ? nb : na, pass ? LA : LB, pass ? na : nb, cl, pass ? cl.headB : cl.headA,
+                                                cl.cand + (pass ? MS / 32 : 0), pass ? inA_c : inB_c, G, share, lane, S.s2, lin, lon, bits, nullptr))
             return false;
           if (pass) { S.bi = lin; S.bo = lon; } else { S.ai = lin; S.ao = lon; }
         }
@@ -883,24 +914,30 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
   return true;
 }
 
-// shared memory of one warp of the filtered bins: lists (one for self pairs), row masks, column masks, grid boxes, cand,
-// queue, flags; every part starts on a multiple of 8 bytes
+// shared memory of one warp of the filtered bins: lists (one for self pairs), grid boxes, node values, heads, cand, node
+// links, queue, flags
+constexpr int NODES = 304;   // split points and coincident edges of both polygons (about 45 for parcel neighbours)
 __host__ __device__ constexpr size_t mask_warp_bytes(int cap, bool self) {
-  return (size_t)(self ? 1 : 2) * cap * EDGE_BYTES_8 + (size_t)(self ? 1 : 2) * (cap / 32) * cap * 4 + (size_t)cap * 8 + 2 * (cap / 32) * 4 + QCAP * 2;
+  const size_t sides = self ? 1 : 2;
+  return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + (size_t)NODES * 8 + sides * cap * 4 + 2 * (cap / 32) * 4 + (size_t)NODES * 2 + QCAP * 2;
 }
 static_assert(mask_warp_bytes(128, false) % 16 == 0 && mask_warp_bytes(192, true) % 16 == 0, "a warp's part starts on 16 bytes");
 template <int MS, bool SELF>
-__device__ __forceinline__ void carve_mask(unsigned char* base, EList8& LA, EList8& LB, MaskBuf& mb) {
+__device__ __forceinline__ void carve_mask(unsigned char* base, EList8& LA, EList8& LB, CutLists<uint16_t>& cl) {
   double* d = reinterpret_cast<double*>(base);
   auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + MS; L.x1 = d + 2 * MS; L.y1 = d + 3 * MS; d += 4 * MS; };
   doubles(LA);
   if (!SELF) doubles(LB);
-  mb.qb = reinterpret_cast<uint2*>(d);
-  mb.rm = reinterpret_cast<uint32_t*>(mb.qb + MS);
-  mb.cm = mb.rm + (MS / 32) * MS;
-  mb.cand = SELF ? mb.cm : mb.cm + (MS / 32) * MS;
-  mb.q = reinterpret_cast<uint16_t*>(mb.cand + 2 * (MS / 32));
-  LA.fl = reinterpret_cast<uint8_t*>(mb.q + QCAP);
+  cl.qb = reinterpret_cast<uint2*>(d);
+  cl.val = d + MS;
+  cl.headA = reinterpret_cast<uint32_t*>(cl.val + NODES);
+  cl.headB = SELF ? cl.headA : cl.headA + MS;
+  cl.cand = cl.headB + MS;
+  cl.nxt = reinterpret_cast<uint16_t*>(cl.cand + 2 * (MS / 32));
+  cl.q = cl.nxt + NODES;
+  cl.count = nullptr;
+  cl.cap = NODES;
+  LA.fl = reinterpret_cast<uint8_t*>(cl.q + QCAP);
   if (SELF) LB = LA; else LB.fl = LA.fl + MS;
 }
 template <bool F> struct Cfg;
@@ -921,7 +958,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P
   __syncwarp();
   EList LA, LB;
   EList8 MA, MB;
-  MaskBuf mbuf;
+  CutLists<uint16_t> mbuf;
   if constexpr (F) {
     carve_mask<CAP_F, false>(smem + (size_t)wib * mask_warp_bytes(CAP_F, false), MA, MB, mbuf);
   } else {
@@ -1001,7 +1038,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
   if (lane == 0) s_ep[wib] = 0;
   __syncwarp();
   EList8 L, L2;
-  MaskBuf mbuf;
+  CutLists<uint16_t> mbuf;
   carve_mask<CAP_SELF, true>(smem + (size_t)wib * mask_warp_bytes(CAP_SELF, true), L, L2, mbuf);
   const uint64_t n = *nself;   // written by k_self_index, launched before this kernel
   for (int k = 0; k < runs; k++) {
@@ -1028,6 +1065,196 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
   }
   __syncwarp();
   if (lane == 0 && s_ep[wib]) atomicAdd(epairs, s_ep[wib]);
+}
+
+// Block bin (filtered variants): the pairs the shared-memory bins hand on, a block of 4 warps per pair, lists of up to 512
+// edges a side in shared memory (54 KB a block, 4 blocks per SM). The routine is refine_pair_m's with the edges of the
+// gather, the search and the passes dealt out to the warps in chunks of 32; the sums keep their order: a lane's running sums
+// pass through shared memory from the warp of one chunk to that of the next. Larger pairs, or more than BIG_NODES cuts,
+// go on to the scratch bin.
+// Against the scratch bin's warp per pair with lists in global memory (10 % of the warps an SM holds, 37k instructions a
+// pair), whole refinement: two 120k layers with areas (7k such pairs) 7.82 -> 6.47 ms, 20k queries relate (3.9k) 1.70 ->
+// 1.32 ms, 100 queries (29: the latency of one pair) 0.27 -> 0.15 ms.
+constexpr int CAP_BIG = 512, BIG_WARPS = 4, BIG_NODES = 1024;
+constexpr size_t BIG_SMEM = 2 * CAP_BIG * EDGE_BYTES_8 + CAP_BIG * 8 + BIG_NODES * 8 + 2 * CAP_BIG * 4 + 2 * (CAP_BIG / 32) * 4 + 5 * 32 * 8 +
+                            BIG_WARPS * QCAP * 4 + BIG_NODES * 2 + 64;
+
+// the edges of A meeting the box, by the whole block, compacted in ring order; inside: the parity of (mx, my). cnt: one
+// word per warp and a spare set (the rounds alternate, so one barrier a round is enough)
+template <bool S32>
+__device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int cap, uint32_t* cnt, double mx, double my, bool& inside) {
+  const DLayer& S = *A.L;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  bool par = false;
+  int have = 0, flip = 0;
+#pragma unroll 1
+  for (uint32_t ra = A.r0; ra < A.r1; ra++) {
+    const uint64_t s = S.rvo[ra];
+    const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);
+#pragma unroll 1
+    for (uint32_t base = 0; base + 1 < n; base += BIG_WARPS * 32, flip ^= BIG_WARPS) {
+      const GatherEdge e = gather_edge<true, true, S32>(A, ov, s, n, base + threadIdx.x, mx, my, par);
+      const unsigned m = __ballot_sync(0xffffffffu, e.in);
+      if (lane == 0) cnt[flip + wid] = __popc(m);
+      __syncthreads();
+      int pos = have + __popc(m & ((1u << lane) - 1));
+      for (int w = 0; w < BIG_WARPS; w++) {
+        const int c = cnt[flip + w];
+        if (w < wid) pos += c;
+        have += c;
+      }
+      if (e.in && pos < cap) { L.x0[pos] = e.x0; L.y0[pos] = e.y0; L.x1[pos] = e.x1; L.y1[pos] = e.y1; L.fl[pos] = e.fl; }
+    }
+  }
+  inside = (__syncthreads_count(par) & 1) != 0;
+  return have;
+}
+
+template <bool S32, int W>
+__global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DLayer R, const uint2* __restrict__ pairs, const uint32_t* __restrict__ list,
+                                                                   const unsigned long long* nlist, RefineArgs rp, uint8_t* flag, double* area, double4* ev,
+                                                                   uint32_t* evb, uint32_t* heavy, unsigned long long* nheavy, unsigned long long* next,
+                                                                   unsigned long long* epairs) {
+  constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned long long s_h;
+  __shared__ uint32_t s_cnt[2 * BIG_WARPS], s_nodes, s_bits;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint64_t n = *nlist;   // written by the bins launched before this kernel
+  EList8 LA, LB;
+  CutLists<uint32_t> cl;
+  double* sums;   // s2, lin, lon of each lane (the pass that runs), then A's lin and lon
+  {
+    double* d = reinterpret_cast<double*>(smem);
+    auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + CAP_BIG; L.x1 = d + 2 * CAP_BIG; L.y1 = d + 3 * CAP_BIG; d += 4 * CAP_BIG; };
+    doubles(LA);
+    doubles(LB);
+    cl.qb = reinterpret_cast<uint2*>(d);
+    cl.val = d + CAP_BIG;
+    sums = cl.val + BIG_NODES;
+    cl.headA = reinterpret_cast<uint32_t*>(sums + 5 * 32);
+    cl.headB = cl.headA + CAP_BIG;
+    cl.cand = cl.headB + CAP_BIG;
+    cl.q = cl.cand + 2 * (CAP_BIG / 32) + wid * QCAP;
+    cl.nxt = reinterpret_cast<uint16_t*>(cl.cand + 2 * (CAP_BIG / 32) + BIG_WARPS * QCAP);
+    cl.count = &s_nodes;
+    cl.cap = BIG_NODES;
+    LA.fl = reinterpret_cast<uint8_t*>(cl.nxt + BIG_NODES);
+    LB.fl = LA.fl + CAP_BIG;
+  }
+  for (;;) {
+    __syncthreads();   // the previous pair's shared memory is no longer read
+    if (threadIdx.x == 0) { s_h = atomicAdd(next, 1ull); s_nodes = 0; s_bits = 0; }
+    __syncthreads();
+    if (s_h >= n) break;
+    const uint32_t p = list[s_h];
+    const uint2 pr = pairs[p];
+    Frame A, B;
+    const PairGeo G = pair_geo(P, R, pr.x, pr.y, rp, A, B);
+    int na = 0, nb = 0;
+    bool inA_c = false, inB_c = false;
+#pragma unroll 1
+    for (int side = 0; side < 2; side++) {
+      bool in = false;
+      const int c = collect_block<S32>(side ? B : A, G.ov, side ? LB : LA, CAP_BIG, s_cnt, G.cx, G.cy, in);
+      if (side) { nb = c; inB_c = in; } else { na = c; inA_c = in; }
+    }
+    bool over = na > CAP_BIG || nb > CAP_BIG;   // the same in every thread, here and below
+    bool hit = false, hit_any = false;
+    if (!over) {
+      begin_pairs<CAP_BIG, false, W != W_FLAG>(LB, na, nb, G, cl, threadIdx.x, BIG_WARPS * 32);
+      __syncthreads();
+      const Nodes nd = find_pairs<CAP_BIG, false, W != W_FLAG, 16>(LA, na, LB, nb, G, cl, wid * 32, BIG_WARPS * 32, lane, hit, hit_any);
+      hit = __syncthreads_or(hit);
+      hit_any = __syncthreads_or(hit_any || hit);
+      over = __syncthreads_or(nd.full);
+    }
+    const bool rtouch = hit;
+    if (!over && !hit) {   // every warp for itself, the same answer
+      hit = contains_warp<S32>(A, B, LA, na, LB, nb, inA_c, inB_c, G.ov, G.cx, G.cy, lane, hit_any);
+    }
+    const bool want = !over && W != W_FLAG && (hit || (W != W_REL && hit_any));
+    PairSums S;
+    uint32_t bits = rtouch ? REL_TOUCH : 0;
+    if constexpr (W != W_FLAG)
+      if (want) {
+        const bool share = G.tol >= 1e-12 * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0);
+#pragma unroll 1
+        for (int pass = 0; pass < 2 && !over; pass++) {
+          const EList8& LS = pass ? LB : LA;
+          const EList8& LO = pass ? LA : LB;
+          const int nself = pass ? nb : na, nother = pass ? na : nb;
+          const uint32_t* head = pass ? cl.headB : cl.headA;
+          const uint32_t* cand = cl.cand + (pass ? CAP_BIG / 32 : 0);
+          const bool inc = pass ? inA_c : inB_c;
+          if (wid == 0) {   // a lane's sums: s2 runs on, each pass's lengths start from 0
+            if (pass) { sums[96 + lane] = sums[32 + lane]; sums[128 + lane] = sums[64 + lane]; } else sums[lane] = 0.0;
+            sums[32 + lane] = 0.0; sums[64 + lane] = 0.0;
+          }
+          __syncthreads();
+#pragma unroll 1
+          for (int c0 = 0; c0 * 32 < nself && !over; c0 += BIG_WARPS) {
+            const int c = c0 + wid, i = c * 32 + lane;
+            EdgeRef e;
+            EdgeCuts C;
+            edge_cuts<REL, false>(e, C, LS, i, i < nself, LO, cl, head);
+            const bool full = C.ns == MAXS;
+            if (e.len2 == 0) C.ns = 0;
+            const bool lens = REL && !(e.fl & 1u);
+            const unsigned link = edge_links(e, i < nself, share && c * 32 < nself ? ~cand[c] : 0u, lane);
+            uint32_t vin = 0;   // bit k: segment k's midpoint is inside (fewer than MAXS segments)
+#pragma unroll 1
+            for (int k = 0; __any_sync(0xffffffffu, k + 1 < C.ns); k++) {
+              bool need = false;
+              double mx = 0, my = 0;
+              if (k + 1 < C.ns) {
+                const Segment s = edge_segment<AREA>(C, e, LO, k, G, lens);
+                need = s.need; mx = s.mx; my = s.my;
+              }
+              if (inside_lanes<S32>(need, mx, my, k ? 0u : link, LO, nother, inc, G, lane)) vin |= 1u << k;
+            }
+            over = __syncthreads_or(full);
+#pragma unroll 1
+            for (int w = 0; w < BIG_WARPS && !over; w++) {   // the chunks' terms in their order
+              if (w == wid && c * 32 < nself) {
+                double acc = 0.0, lin = sums[32 + lane], lon = sums[64 + lane];
+#pragma unroll 1
+                for (int k = 0; k + 1 < C.ns; k++) {
+                  const Segment s = edge_segment<AREA>(C, e, LO, k, G, lens);
+                  if (s.valid) edge_segment_add<AREA>(s, C, e, LO, G, lens, (vin >> k) & 1u ? 1 : 0, acc, lin, lon, bits);
+                }
+                __syncwarp();
+                if (i < nself) sums[lane] += acc;
+                sums[32 + lane] = lin; sums[64 + lane] = lon;
+              }
+              __syncthreads();
+            }
+          }
+        }
+        if (REL) {
+          const uint32_t b = __reduce_or_sync(0xffffffffu, bits);
+          if (lane == 0) atomicOr(&s_bits, b);
+          __syncthreads();
+          bits = s_bits;
+        }
+        S.s2 = sums[lane];
+        S.ai = sums[96 + lane]; S.ao = sums[128 + lane]; S.bi = sums[32 + lane]; S.bo = sums[64 + lane];
+      }
+    if (wid == 0) {
+      if (over) {
+        if (lane == 0) { heavy[atomicAdd(nheavy, 1ull)] = p; flag[p] = 0; }
+      } else {
+        uint8_t f; double ar; double4 e4; uint32_t b4;
+        pair_result<AREA, REL>(S, want, hit, rtouch, bits, f, ar, e4, b4);
+        if (lane == 0) {
+          flag[p] = f;
+          if (area) area[p] = ar;
+          if (ev) { ev[p] = e4; evb[p] = b4; }
+          atomicAdd(epairs, (unsigned long long)na * (unsigned long long)nb);
+        }
+      }
+    }
+  }
 }
 
 // oversized pairs: the same pair routine with per-warp edge lists in global scratch. The filtered variant also
@@ -1117,10 +1344,11 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   const int bit = 1 << variant;
   if (!(c->refine_attr & bit)) {
     GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F>::smem));
+    if (F) GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIG_SMEM));
     c->refine_attr |= bit;
   }
   const RefineShape& sh = c->shape;
-  unsigned long long* ctr = c->counters.as<unsigned long long>(8);
+  unsigned long long* ctr = c->counters.as<unsigned long long>(16);
   int* err = reinterpret_cast<int*>(ctr + 1);
   uint32_t* heavy = c->heavy.as<uint32_t>(np);
   const int bin_cap = std::min(sh.bin_cap, Cfg<F>::cap), run = sh.run, runs = sh.runs;
@@ -1137,9 +1365,13 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   } else {
     blocks = (int)std::min<uint64_t>((np + RB_WARPS - 1) / RB_WARPS, (uint64_t)c->sm_count * 8);
   }
-  // a pair can only be oversized when one of its polygons has more edges than the bin holds; the filtered bins also hand
-  // on the rare pairs whose split points they cannot keep, so they always have a scratch bin behind them (a few warps)
-  const bool big = std::max(P->max_geom_edges, R->max_geom_edges) > (uint32_t)bin_cap, scr = F || big;
+  // plain: a pair can only be oversized when one of its polygons has more edges than the bin holds. The filtered bins hand
+  // oversized pairs, and the rare ones whose cuts they cannot keep, to the block bin, and that bin to the scratch bin
+  // (the full number of warps only where a geometry can have more edges than the block bin holds)
+  const uint32_t most = std::max(P->max_geom_edges, R->max_geom_edges);
+  const bool big = most > (uint32_t)(F ? CAP_BIG : bin_cap), scr = F || big;
+  uint32_t* heavy2 = F ? c->heavy2.as<uint32_t>(np) : heavy;
+  const int bblocks = (int)std::min<uint64_t>(np, (uint64_t)c->sm_count * 4);
   const ScratchGeom sg = scratch_geom<F>(P, R);
   int sblocks = 0;
   unsigned char* sbuf = nullptr;
@@ -1173,14 +1405,20 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   }
   unsigned long long* h = c->h_refine.as<unsigned long long>(4);
   // counters: [0] oversized pairs, [1] error word, [2] pair counter, [3] local edge pairs, [4] scratch pair counter,
-  // [5] self pairs, [6] self pair counter
+  // [5] self pairs, [6] self pair counter, [7] the block bin's oversized pairs, [8] block pair counter
   auto a_main = kernel_args(k_refine<F, S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
                             self ? 1 : 0);
-  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, sbuf, sg.cap, sg.cph, err, ctr + 3,
+  auto a_big = kernel_args(k_refine_block<S32, W>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, heavy2, ctr + 7, ctr + 8, ctr + 3);
+  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, heavy2, F ? ctr + 7 : ctr, rp, flag, area, ev, evb, sbuf, sg.cap, sg.cph, err, ctr + 3,
                            ctr + 4, P == R ? 1 : 0);
   auto a_idx = kernel_args(k_self_index, pairs, np, sidx, ctr + 5);
   auto a_self = kernel_args(k_refine_self<S32, W>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
-  cudaKernelNodeParams km{}, ks{}, ki{}, kf{};
+  cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{};
+  kb.func = (void*)k_refine_block<S32, W>;
+  kb.gridDim = dim3(bblocks);
+  kb.blockDim = dim3(BIG_WARPS * 32);
+  kb.sharedMemBytes = (unsigned)BIG_SMEM;
+  kb.kernelParams = a_big.ptr;
   km.func = (void*)k_refine<F, S32, W>;
   km.gridDim = dim3(blocks);
   km.blockDim = dim3(RB_WARPS * 32);
@@ -1203,13 +1441,17 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   if (!g.exec) {   // the graph is kept with its executable: the node handles used for the updates belong to it
     if (!g.graph) {
       GSJ_CK(cudaGraphCreate(&g.graph, 0));
-      // shared-memory bin || (self index -> self bin), then the scratch bin after both
+      // shared-memory bin || (self index -> self bin), then the block bin after both, then the scratch bin
       GSJ_CK(cudaGraphAddKernelNode(&g.n_main, g.graph, nullptr, 0, &km));
       std::vector<cudaGraphNode_t> before{g.n_main};
       if (self) {
         GSJ_CK(cudaGraphAddKernelNode(&g.n_idx, g.graph, nullptr, 0, &ki));
         GSJ_CK(cudaGraphAddKernelNode(&g.n_self, g.graph, &g.n_idx, 1, &kf));
         before.push_back(g.n_self);
+      }
+      if (F) {
+        GSJ_CK(cudaGraphAddKernelNode(&g.n_big, g.graph, before.data(), before.size(), &kb));
+        before.assign(1, g.n_big);
       }
       if (scr) GSJ_CK(cudaGraphAddKernelNode(&g.n_scr, g.graph, before.data(), before.size(), &ks));
     }
@@ -1220,11 +1462,12 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
       GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_idx, &ki));
       GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_self, &kf));
     }
+    if (F) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big, &kb));
     if (scr) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_scr, &ks));
   }
-  GSJ_CK(cudaMemsetAsync(ctr, 0, 7 * sizeof(unsigned long long), s));
+  GSJ_CK(cudaMemsetAsync(ctr, 0, 9 * sizeof(unsigned long long), s));
   GSJ_CK(cudaGraphLaunch(g.exec, s));
-  c->launches += 1 + (scr ? 1 : 0) + (self ? 2 : 0);
+  c->launches += 1 + (F ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
   GSJ_CK(cudaMemcpyAsync(h, ctr, 32, cudaMemcpyDeviceToHost, s));
   c->refine_pending = true;
 }

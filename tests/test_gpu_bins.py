@@ -1,5 +1,5 @@
-"""The shared-memory bins of the refinement at the sizes where they hand pairs on: an edge cut more often than its split
-list holds, more split points than the room behind the edge lists, edge lists at multiples of the mask words, an
+"""The bins of the refinement at the sizes where they hand pairs on (a warp's bin, a block's, global scratch): an edge cut
+more often than its split list holds, more cuts than there is room for, edge lists around the bins' sizes, an
 overlap box of no height, tolerances of zero. Every variant has to give the oracle's rows bit for bit."""
 import ctypes
 
@@ -32,15 +32,16 @@ def ngon(n, r, cx=0.0, cy=0.0):
 
 SHAPES = {
     # a bar across every tooth: 2 x teeth splits on its long edges (an edge keeps 22 beside its ends)
-    **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28)},
-    # crossed combs: more split points than fit behind the lists
+    **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28, 100)},
+    # crossed combs: more split points than the lists hold
     "combs_9": ([[comb(9, 10 * S, 10 * S)]], [[comb(9, 10 * S, 10 * S, flip=True)]]),
     "combs_28": ([[comb(28, 10 * S, 10 * S)]], [[comb(28, 10 * S, 10 * S, flip=True)]]),
+    "combs_60": ([[comb(60, 10 * S, 10 * S)]], [[comb(60, 10 * S, 10 * S, flip=True)]]),
     # level neighbours: the overlap box is as thin as its pad
     "touch": ([[square(0, 0, S)]], [[square(0, S, S)], [square(S, S, S)]]),
     "twins": ([[square(0, 0, S)], [comb(9, S, S)]], [[square(0, 0, S)], [comb(9, S, S)]]),
 }
-for _n in (31, 32, 33, 64, 96, 127, 128, 129):
+for _n in (31, 32, 33, 64, 96, 127, 128, 129, 192, 193, 300, 511, 512, 513):
     SHAPES[f"ngon_{_n}"] = ([[ngon(_n, S)]], [[ngon(_n, S, 0.3 * S, 0.2 * S)], [ngon(7, 0.2 * S)]])
 
 
