@@ -916,37 +916,46 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
 
 // shared memory of one warp of the filtered bins: lists (one for self pairs), grid boxes, node values, heads, cand, node
 // links, queue, flags
-constexpr int NODES = 304;   // split points and coincident edges of both polygons (about 45 for parcel neighbours)
-__host__ __device__ constexpr size_t mask_warp_bytes(int cap, bool self) {
+// split points and coincident edges of both polygons (about 45 for parcel neighbours); of a self pair, beside each edge itself
+constexpr int NODES = 304, NODES_SELF = 160;
+// (the flag alone: lists, grid boxes, queue, flags)
+__host__ __device__ constexpr size_t mask_warp_bytes(int cap, bool self, bool cuts = true) {
   const size_t sides = self ? 1 : 2;
-  return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + (size_t)NODES * 8 + sides * cap * 4 + 2 * (cap / 32) * 4 + (size_t)NODES * 2 + QCAP * 2;
+  if (!cuts) return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + QCAP * 2;
+  const size_t nodes = self ? NODES_SELF : NODES;
+  return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + nodes * 8 + sides * cap * 4 + 2 * (cap / 32) * 4 + nodes * 2 + QCAP * 2;
 }
-static_assert(mask_warp_bytes(128, false) % 16 == 0 && mask_warp_bytes(192, true) % 16 == 0, "a warp's part starts on 16 bytes");
-template <int MS, bool SELF>
+static_assert(mask_warp_bytes(128, false) % 16 == 0 && mask_warp_bytes(256, true) % 16 == 0, "a warp's part starts on 16 bytes");
+template <int MS, bool SELF, bool CUTS>
 __device__ __forceinline__ void carve_mask(unsigned char* base, EList8& LA, EList8& LB, CutLists<uint16_t>& cl) {
+  constexpr int nodes = SELF ? NODES_SELF : NODES;
   double* d = reinterpret_cast<double*>(base);
   auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + MS; L.x1 = d + 2 * MS; L.y1 = d + 3 * MS; d += 4 * MS; };
   doubles(LA);
   if (!SELF) doubles(LB);
   cl.qb = reinterpret_cast<uint2*>(d);
   cl.val = d + MS;
-  cl.headA = reinterpret_cast<uint32_t*>(cl.val + NODES);
+  cl.headA = reinterpret_cast<uint32_t*>(cl.val + (CUTS ? nodes : 0));
   cl.headB = SELF ? cl.headA : cl.headA + MS;
   cl.cand = cl.headB + MS;
   cl.nxt = reinterpret_cast<uint16_t*>(cl.cand + 2 * (MS / 32));
-  cl.q = cl.nxt + NODES;
+  cl.q = CUTS ? cl.nxt + nodes : reinterpret_cast<uint16_t*>(cl.val);
   cl.count = nullptr;
-  cl.cap = NODES;
+  cl.cap = nodes;
   LA.fl = reinterpret_cast<uint8_t*>(cl.q + QCAP);
   if (SELF) LB = LA; else LB.fl = LA.fl + MS;
 }
-template <bool F> struct Cfg;
-template <> struct Cfg<false> { static constexpr int cap = CAP; static constexpr size_t smem = RB_SMEM; static constexpr int minb = 3; };
-template <> struct Cfg<true> { static constexpr int cap = CAP_F; static constexpr size_t smem = RB_WARPS * mask_warp_bytes(CAP_F, false); static constexpr int minb = 4; };
+template <bool F, int W> struct Cfg;
+template <int W> struct Cfg<false, W> { static constexpr int cap = CAP; static constexpr size_t smem = RB_SMEM, warp = 0; static constexpr int minb = 3; };
+template <int W> struct Cfg<true, W> {   // the flag alone needs no room for cuts and fewer registers: 5 blocks per SM
+  static constexpr int cap = CAP_F;
+  static constexpr size_t warp = mask_warp_bytes(CAP_F, false, W != W_FLAG), smem = RB_WARPS * warp;
+  static constexpr int minb = W == W_FLAG ? 5 : 4;
+};
 
 // S32 (filtered only): the contact test's and the gather's orientation signs through the certified FP32 filter
 template <bool F, bool S32 = false, int W = W_ALL>
-__global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
+__global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
                                                                         RefineArgs rp, uint8_t* flag, double* area, double4* ev, uint32_t* evb,
                                                                         uint32_t* heavy, unsigned long long* nheavy, unsigned long long* next,
                                                                         unsigned long long* epairs, int run, int runs, int bin_cap,
@@ -960,7 +969,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P
   EList8 MA, MB;
   CutLists<uint16_t> mbuf;
   if constexpr (F) {
-    carve_mask<CAP_F, false>(smem + (size_t)wib * mask_warp_bytes(CAP_F, false), MA, MB, mbuf);
+    carve_mask<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<F, W>::warp, MA, MB, mbuf);
   } else {
     LA = carve(smem + (size_t)wib * 2 * LIST_BYTES, CAP);
     LB = carve(smem + (size_t)wib * 2 * LIST_BYTES + LIST_BYTES, CAP);
@@ -1003,12 +1012,11 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F>::minb) k_refine(DLayer P
 }
 
 // Self bin (filtered variants, a layer joined with itself): the pairs of a geometry with itself, 24 % of a parcel
-// self-join's pairs and the costliest (every edge is local). One list of up to 192 edges per warp (a multiple of 32
-// for the row masks; the largest that keeps 4 blocks of 4 warps per SM: 256 with 3 blocks measured 5 % slower),
-// row masks only, A's gather and contribution pass only (refine_pair_t SELF).
-constexpr int CAP_SELF = 192;
+// self-join's pairs and the costliest (every edge is local). One list of up to 256 edges per warp (the largest that the
+// queue's bytes index and that keeps 4 blocks of 4 warps per SM), A's gather and contribution pass only (refine_pair_m SELF).
+constexpr int CAP_SELF = 256;
 constexpr size_t SELF_SMEM = RB_WARPS * mask_warp_bytes(CAP_SELF, true);
-constexpr int SELF_MINB = 4;   // blocks per SM: 4 x 51 KB of shared memory
+constexpr int SELF_MINB = 4;   // blocks per SM: 4 x 53 KB of shared memory
 
 // positions of the self pairs (a == b) among the candidate pairs, warp-aggregated (order free: outputs go by position)
 __global__ void k_self_index(const uint2* __restrict__ pairs, uint64_t np, uint32_t* sidx, unsigned long long* nself) {
@@ -1039,7 +1047,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
   __syncwarp();
   EList8 L, L2;
   CutLists<uint16_t> mbuf;
-  carve_mask<CAP_SELF, true>(smem + (size_t)wib * mask_warp_bytes(CAP_SELF, true), L, L2, mbuf);
+  carve_mask<CAP_SELF, true, true>(smem + (size_t)wib * mask_warp_bytes(CAP_SELF, true), L, L2, mbuf);
   const uint64_t n = *nself;   // written by k_self_index, launched before this kernel
   for (int k = 0; k < runs; k++) {
     unsigned long long h0 = 0;
@@ -1343,7 +1351,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   constexpr int variant = F ? 1 + 4 * S32 + W : 0;   // plain, filtered x W, filtered FP32 x W
   const int bit = 1 << variant;
   if (!(c->refine_attr & bit)) {
-    GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F>::smem));
+    GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
     if (F) GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIG_SMEM));
     c->refine_attr |= bit;
   }
@@ -1351,13 +1359,13 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   unsigned long long* ctr = c->counters.as<unsigned long long>(16);
   int* err = reinterpret_cast<int*>(ctr + 1);
   uint32_t* heavy = c->heavy.as<uint32_t>(np);
-  const int bin_cap = std::min(sh.bin_cap, Cfg<F>::cap), run = sh.run, runs = sh.runs;
+  const int bin_cap = std::min(sh.bin_cap, Cfg<F, W>::cap), run = sh.run, runs = sh.runs;
   int blocks;
   if constexpr (F) {
     // enough warps to cover every pair with `runs` fetches each, spread over all SMs; more than one wave of blocks
     // is rounded up to whole waves, so the last wave's blocks share the remaining pairs (the counter hands them out)
     // instead of leaving part of the GPU idle while a partial wave runs
-    const uint64_t per_block = (uint64_t)RB_WARPS * runs * run, wave = (uint64_t)c->sm_count * Cfg<F>::minb;
+    const uint64_t per_block = (uint64_t)RB_WARPS * runs * run, wave = (uint64_t)c->sm_count * Cfg<F, W>::minb;
     uint64_t cover = (np + per_block - 1) / per_block;
     if (cover > wave) cover = (cover + wave - 1) / wave * wave;
     const uint64_t spread = std::min<uint64_t>((np + (uint64_t)RB_WARPS * run - 1) / ((uint64_t)RB_WARPS * run), wave);
@@ -1387,7 +1395,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   const bool self = F && P == R;
   int iblocks = 1, fblocks = 1;
   uint32_t* sidx = nullptr;
-  const int self_cap = std::min(sh.bin_cap + sh.bin_cap / 2, CAP_SELF);   // 1.5 x the shape's shared-memory bin threshold
+  const int self_cap = std::min(2 * sh.bin_cap, CAP_SELF);   // twice the shape's shared-memory bin threshold: one list instead of two
   if (self) {
     const int sbit = 1 << (16 + variant);
     if (!(c->refine_attr & sbit)) {
@@ -1422,7 +1430,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   km.func = (void*)k_refine<F, S32, W>;
   km.gridDim = dim3(blocks);
   km.blockDim = dim3(RB_WARPS * 32);
-  km.sharedMemBytes = (unsigned)Cfg<F>::smem;
+  km.sharedMemBytes = (unsigned)Cfg<F, W>::smem;
   km.kernelParams = a_main.ptr;
   ks.func = (void*)k_refine_scratch<F>;
   ks.gridDim = dim3(std::max(sblocks, 1));
