@@ -7,6 +7,7 @@
 // Trigonometric functions are CUDA's (sin, cos, tan, atan, atan2; sqrt is exact).
 #include <algorithm>
 #include <cub/cub.cuh>
+#include "append.cuh"
 #include "engine.h"
 #include "pairkit.cuh"
 
@@ -560,25 +561,23 @@ __global__ void __launch_bounds__(128, GEO ? 4 : 6) k_pt_dwithin_warp(const doub
 }
 
 // ---- shared driver pieces ----------------------------------------------------------------------------------------
-__global__ void k_flag_keep(const uint8_t* __restrict__ f, uint64_t n, uint8_t want, uint32_t* keep) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) keep[i] = f[i] == want;
+__global__ void __launch_bounds__(APPEND_THREADS) k_append_keys(const uint2* __restrict__ pairs, const uint8_t* __restrict__ f, uint64_t n, uint8_t want,
+                                                               const uint32_t* parA, const uint32_t* parB, int bits, unsigned long long* keys,
+                                                               unsigned long long* count) {
+  append_items(n, count, [&](uint64_t i) { return f[i] == want; }, [&](uint64_t i, unsigned long long o) {
+    const uint2 p = pairs[i];
+    keys[o] = pair_key(parA ? parA[p.x] : p.x, parB ? parB[p.y] : p.y, bits);
+  });
 }
-__global__ void k_keys_kept(const uint2* __restrict__ pairs, const uint32_t* __restrict__ keep, const uint32_t* __restrict__ off, uint64_t n,
-                            const uint32_t* parA, const uint32_t* parB, unsigned long long* keys) {
-  const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !keep[i]) return;
-  const uint2 p = pairs[i];
-  keys[off[i]] = ((unsigned long long)(parA ? parA[p.x] : p.x) << 32) | (parB ? parB[p.y] : p.y);
-}
+// sorted keys -> pairs; head / off null: every key is there once
 __global__ void k_unique_heads(const unsigned long long* __restrict__ k, uint64_t n, uint32_t* head) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) head[i] = (i == 0 || k[i] != k[i - 1]) ? 1u : 0u;
 }
-__global__ void k_unique_scatter(const unsigned long long* __restrict__ k, const uint32_t* __restrict__ head, const uint32_t* __restrict__ off, uint64_t n,
+__global__ void k_unique_scatter(const unsigned long long* __restrict__ k, const uint32_t* __restrict__ head, const uint32_t* __restrict__ off, uint64_t n, int bits,
                                  uint2* out) {
   const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && head[i]) out[off[i]] = make_uint2((uint32_t)(k[i] >> 32), (uint32_t)k[i]);
+  if (i < n && (!head || head[i])) out[head ? off[i] : i] = key_pair(k[i], bits);
 }
 
 static uint64_t scan_count(gsj_ctx* c, const uint32_t* flags, uint32_t* off, uint64_t n) {
@@ -592,27 +591,35 @@ static uint64_t scan_count(gsj_ctx* c, const uint32_t* flags, uint32_t* off, uin
   return (uint64_t)h[0] + h[1];
 }
 
-// (a, b) pairs with flag == want -> unique (parent a, parent b) pairs, sorted; returns count, rows in c->opairs
+// (a, b) pairs with flag == want -> unique (parent a, parent b) pairs, sorted; returns count, rows in c->opairs.
+// nA, nB: parents of either side. Keys in as few bits as these need: 5 instead of 8 passes of the sort at 200k x 1M.
 static uint64_t fold_unique(gsj_ctx* c, const uint2* pairs, const uint8_t* flag, uint64_t np, uint8_t want, const uint32_t* parA, const uint32_t* parB,
-                            uint2** out) {
+                            uint64_t nA, uint64_t nB, uint2** out) {
   cudaStream_t s = c->stream;
-  uint32_t* keep = c->keep.as<uint32_t>(np);
-  uint32_t* off = c->idx.as<uint32_t>(np);
-  k_flag_keep<<<grid_for(np, 256), 256, 0, s>>>(flag, np, want, keep); c->launches++;
-  const uint64_t nk = scan_count(c, keep, off, np);
+  const int bits = key_bits(nB), total = bits + key_bits(nA);
+  unsigned long long* k1 = c->keys.as<unsigned long long>(np);
+  unsigned long long* cnt = c->counters.as<unsigned long long>(16);
+  GSJ_CK(cudaMemsetAsync(cnt, 0, 8, s));
+  k_append_keys<<<append_grid(np), APPEND_THREADS, 0, s>>>(pairs, flag, np, want, parA, parB, bits, k1, cnt); c->launches++;
+  unsigned long long* h = c->h_counters.as<unsigned long long>(2);
+  GSJ_CK(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, s));
+  GSJ_CK(cudaStreamSynchronize(s));
+  const uint64_t nk = h[0];
   *out = c->opairs.as<uint2>(nk);
   if (!nk) return 0;
-  unsigned long long* k1 = c->keys.as<unsigned long long>(nk);
   unsigned long long* k2 = c->keys2.as<unsigned long long>(nk);
-  k_keys_kept<<<grid_for(np, 256), 256, 0, s>>>(pairs, keep, off, np, parA, parB, k1); c->launches++;
   size_t tb = 0;
-  GSJ_CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, k1, k2, (int64_t)nk, 0, 64, s));
-  GSJ_CK(cub::DeviceRadixSort::SortKeys(c->tmp.get(tb), tb, k1, k2, (int64_t)nk, 0, 64, s));
-  uint32_t* head = c->misc1.as<uint32_t>(nk);
-  uint32_t* hoff = c->misc2.as<uint32_t>(nk);
-  k_unique_heads<<<grid_for(nk, 256), 256, 0, s>>>(k2, nk, head); c->launches++;
-  const uint64_t nu = scan_count(c, head, hoff, nk);
-  k_unique_scatter<<<grid_for(nk, 256), 256, 0, s>>>(k2, head, hoff, nk, *out); c->launches++;
+  GSJ_CK(cub::DeviceRadixSort::SortKeys(nullptr, tb, k1, k2, (int64_t)nk, 0, total, s));
+  GSJ_CK(cub::DeviceRadixSort::SortKeys(c->tmp.get(tb), tb, k1, k2, (int64_t)nk, 0, total, s));
+  uint32_t *head = nullptr, *hoff = nullptr;
+  uint64_t nu = nk;
+  if (parA || parB) {   // without parents every key is there once
+    head = c->misc1.as<uint32_t>(nk);
+    hoff = c->misc2.as<uint32_t>(nk);
+    k_unique_heads<<<grid_for(nk, 256), 256, 0, s>>>(k2, nk, head); c->launches++;
+    nu = scan_count(c, head, hoff, nk);
+  }
+  k_unique_scatter<<<grid_for(nk, 256), 256, 0, s>>>(k2, head, hoff, nk, bits, *out); c->launches++;
   GSJ_CK(cudaGetLastError());
   return nu;
 }
@@ -700,7 +707,7 @@ void dwithin_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double d, 
     st.refine_ms += tm.stop();
     tm.start();
     uint2* out = nullptr;
-    const uint64_t nu = fold_unique(c, pairs, flag, np, 1, P->d.parent, R->d.parent, &out);
+    const uint64_t nu = fold_unique(c, pairs, flag, np, 1, P->d.parent, R->d.parent, P->nparent, R->nparent, &out);
     st.compact_ms += tm.stop();
     emit(out, nu);
   }
@@ -1426,7 +1433,7 @@ void erode_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double ra, d
     st.refine_ms += tm.stop();
     tm.start();
     uint2* out = nullptr;
-    const uint64_t nu = fold_unique(c, ep, flag, ne, 1, nullptr, nullptr, &out);
+    const uint64_t nu = fold_unique(c, ep, flag, ne, 1, nullptr, nullptr, P->nparent, R->nparent, &out);
     st.compact_ms += tm.stop();
     emit(out, nu);
   };
@@ -1659,7 +1666,7 @@ void points_buffer_host(gsj_ctx* c, const gsj_layer* pts, const gsj_layer* R, do
     tm.start();
     uint2* out = nullptr;
     uint64_t nu = 0;
-    if (!erode) nu = fold_unique(c, pairs, hit, np, 1, nullptr, R->d.parent, &out);
+    if (!erode) nu = fold_unique(c, pairs, hit, np, 1, nullptr, R->d.parent, n, R->nparent, &out);
     else {   // OR the bits per (point, parent): inside some piece and near no real boundary (== 1)
       unsigned long long* k1 = c->keys.as<unsigned long long>(np);
       unsigned long long* k2 = c->keys2.as<unsigned long long>(np);

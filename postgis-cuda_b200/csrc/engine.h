@@ -195,6 +195,7 @@ uint64_t refine(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2*
 // caller reads the outputs of pairs with flag 1 alone (flag 2 then counts as 0)
 void refine_enqueue(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, int mode,
                     uint8_t* flag, double* area, double4* ev, uint32_t* evb, bool hits_only = false);
+constexpr int REFINE_ROWS = 9;   // a word of c->counters that refine_enqueue sets to 0 and does not use
 uint64_t refine_result(gsj_ctx* c);
 
 // refinement launch shapes (tune.cu)

@@ -4,15 +4,16 @@
 // per-request allocations.
 #include <algorithm>
 #include <cub/cub.cuh>
+#include "append.cuh"
 #include "engine.h"
 #include "pairkit.cuh"
 
 namespace gsj {
 
 // ---- small kernels -------------------------------------------------------------------------------------------
-__global__ void k_keep(const uint8_t* __restrict__ f, uint64_t n, int any_nonzero, uint32_t* keep) {
+__global__ void k_keep(const uint8_t* __restrict__ f, uint64_t n, uint32_t* keep) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) keep[i] = any_nonzero ? (f[i] != 0) : (f[i] == 1);
+  if (i < n) keep[i] = f[i] != 0;
 }
 
 // DE-9IM code from boundary evidence (engine.cuh:848-856)
@@ -39,6 +40,17 @@ __global__ void k_scatter_rows(const uint2* __restrict__ pairs, const uint32_t* 
   if (ocode) ocode[o] = de9im_code(ev[i], evb[i], blA[p.x], blB[p.y]);
 }
 
+// rows of the intersecting pairs (flag 1), in no set order, with their area and DE-9IM code
+__global__ void __launch_bounds__(APPEND_THREADS) k_append_rows(const uint2* __restrict__ pairs, const uint8_t* __restrict__ flag, uint64_t n, const double* area,
+                                                               const double4* ev, const uint32_t* evb, const double* blA, const double* blB, uint2* opairs,
+                                                               double* oarea, uint32_t* ocode, unsigned long long* count) {
+  append_items(n, count, [&](uint64_t i) { return flag[i] == 1; }, [&](uint64_t i, unsigned long long o) {
+    const uint2 p = pairs[i];
+    opairs[o] = p;
+    if (oarea) oarea[o] = area[i];
+    if (ocode) ocode[o] = de9im_code(ev[i], evb[i], blA[p.x], blB[p.y]);
+  });
+}
 // pieces kept for folding: sort keys (piece pair, then parent pair) and the per-pair payload
 __global__ void k_scatter_pieces(const uint2* __restrict__ pairs, const uint32_t* __restrict__ keep, const uint32_t* __restrict__ off, uint64_t n,
                                  const uint32_t* parA, const uint32_t* parB, unsigned long long* kpiece, uint32_t* idx) {
@@ -185,24 +197,30 @@ void run_join(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const RefineAr
     refine_enqueue(c, P, R, pairs, np, rp, o.refine_mode, flag, area, ev, evb, !agg);
     tr.mark_end();
     tm.start();
-    uint32_t* keep = c->keep.as<uint32_t>(np);
-    uint32_t* off = c->idx.as<uint32_t>(np);
-    k_keep<<<grid_for(np, 256), 256, 0, s>>>(flag, np, agg ? 1 : 0, keep); c->launches++;
-    exclusive_scan(c, keep, off, np);
-    uint64_t nk = read_last(c, off, keep, np);
+    JoinOut out{nullptr, nullptr, nullptr, 0};
+    uint32_t *keep = nullptr, *off = nullptr;
+    uint64_t nk = 0;
+    if (!agg) {   // rows written behind a counter of the refinement's; its count comes back with theirs
+      out.pairs = c->opairs.as<uint2>(np);
+      out.area = rp.want_area ? c->oarea.as<double>(np) : nullptr;
+      out.code = rel ? c->ocode.as<uint32_t>(np) : nullptr;
+      unsigned long long* cnt = c->counters.as<unsigned long long>(16) + REFINE_ROWS;
+      k_append_rows<<<append_grid(np), APPEND_THREADS, 0, s>>>(pairs, flag, np, area, ev, evb, P->d.blen, R->d.blen, out.pairs, out.area, out.code, cnt);
+      c->launches++;
+      unsigned long long* h = c->h_counters.as<unsigned long long>(2);
+      GSJ_CK(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, s));
+      GSJ_CK(cudaStreamSynchronize(s));
+      out.n = h[0];
+    } else {
+      keep = c->keep.as<uint32_t>(np);
+      off = c->idx.as<uint32_t>(np);
+      k_keep<<<grid_for(np, 256), 256, 0, s>>>(flag, np, keep); c->launches++;
+      exclusive_scan(c, keep, off, np);
+      nk = read_last(c, off, keep, np);
+    }
     st.heavy += refine_result(c);
     st.refine_ms += tr.elapsed();
-    JoinOut out{nullptr, nullptr, nullptr, 0};
-    if (!agg) {
-      out.pairs = c->opairs.as<uint2>(nk);
-      out.area = rp.want_area ? c->oarea.as<double>(nk) : nullptr;
-      out.code = rel ? c->ocode.as<uint32_t>(nk) : nullptr;
-      out.n = nk;
-      if (nk) {
-        k_scatter_rows<<<grid_for(np, 256), 256, 0, s>>>(pairs, keep, off, np, area, ev, evb, P->d.blen, R->d.blen, out.pairs, out.area, out.code);
-        c->launches++;
-      }
-    } else if (nk) {
+    if (nk) {
       // fold piece pairs into parent pairs in (parent pair, piece a, piece b) order
       unsigned long long* k1 = c->keys.as<unsigned long long>(nk);
       unsigned long long* k2 = c->keys2.as<unsigned long long>(nk);
@@ -292,28 +310,23 @@ __global__ void __launch_bounds__(128) k_pip(const double2* __restrict__ pts, DL
   const unsigned mo = (__ballot_sync(0xffffffffu, on) >> shift) & m, mp = (__ballot_sync(0xffffffffu, par) >> shift) & m;
   if (i < np && sub == 0) hit[i] = mo ? 2 : (uint8_t)(__popc(mp) & 1);
 }
-__global__ void k_u8_nonzero(const uint8_t* f, uint64_t n, uint32_t* keep) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) keep[i] = f[i] != 0;
-}
-__global__ void k_scatter_pts(const uint2* __restrict__ pairs, const uint8_t* __restrict__ hit, const uint32_t* keep, const uint32_t* off,
-                              uint64_t n, const uint32_t* parR, unsigned long long* key, uint8_t* val) {
-  uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !keep[i]) return;
-  uint2 p = pairs[i];
-  uint32_t o = off[i];
-  key[o] = ((unsigned long long)p.x << 32) | (parR ? parR[p.y] : p.y);
-  val[o] = hit[i];
+__global__ void __launch_bounds__(APPEND_THREADS) k_append_pts(const uint2* __restrict__ pairs, const uint8_t* __restrict__ hit, uint64_t n, const uint32_t* parR,
+                                                              int bits, unsigned long long* key, uint8_t* val, unsigned long long* count) {
+  append_items(n, count, [&](uint64_t i) { return hit[i] != 0; }, [&](uint64_t i, unsigned long long o) {
+    const uint2 p = pairs[i];
+    key[o] = pair_key(p.x, parR ? parR[p.y] : p.y, bits);
+    val[o] = hit[i];
+  });
 }
 // sorted (point, parent) keys: max fold per key (boundary wins over interior)
-__global__ void k_fold_max(const unsigned long long* __restrict__ k, const uint8_t* __restrict__ v, const uint32_t* start, uint64_t nseg, uint64_t n,
+__global__ void k_fold_max(const unsigned long long* __restrict__ k, const uint8_t* __restrict__ v, const uint32_t* start, uint64_t nseg, uint64_t n, int bits,
                            uint2* opairs, uint8_t* owhere) {
   uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nseg) return;
-  uint64_t b = start[s], e = s + 1 < nseg ? start[s + 1] : n;
+  uint64_t b = start ? start[s] : s, e = !start ? s + 1 : s + 1 < nseg ? start[s + 1] : n;   // start null: every key is one segment
   uint8_t m = 0;
   for (uint64_t q = b; q < e; q++) m = max(m, v[q]);
-  opairs[s] = make_uint2((uint32_t)(k[b] >> 32), (uint32_t)k[b]);
+  opairs[s] = key_pair(k[b], bits);
   owhere[s] = m;
 }
 
@@ -345,31 +358,36 @@ void run_points(gsj_ctx* c, const gsj_layer* pts, const gsj_layer* R, const gsj_
     GSJ_CK(cudaGetLastError());
     st.refine_ms += tm.stop();
     tm.start();
-    uint32_t* keep = c->keep.as<uint32_t>(np);
-    uint32_t* off = c->idx.as<uint32_t>(np);
-    k_u8_nonzero<<<grid_for(np, 256), 256, 0, s>>>(hit, np, keep); c->launches++;
-    exclusive_scan(c, keep, off, np);
-    uint64_t nk = read_last(c, off, keep, np);
+    const int bits = key_bits(R->nparent), total = bits + key_bits(pts->d.n);
+    unsigned long long* k1 = c->keys.as<unsigned long long>(np);
+    uint8_t* v1 = reinterpret_cast<uint8_t*>(c->misc1.as<uint32_t>(np / 4 + 1));
+    unsigned long long* cnt = c->counters.as<unsigned long long>(16);
+    GSJ_CK(cudaMemsetAsync(cnt, 0, 8, s));
+    k_append_pts<<<append_grid(np), APPEND_THREADS, 0, s>>>(pairs, hit, np, R->d.parent, bits, k1, v1, cnt); c->launches++;
+    unsigned long long* h = c->h_counters.as<unsigned long long>(2);
+    GSJ_CK(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, s));
+    GSJ_CK(cudaStreamSynchronize(s));
+    const uint64_t nk = h[0];
     uint2* opairs = c->opairs.as<uint2>(nk);
     uint8_t* owhere = reinterpret_cast<uint8_t*>(c->ocode.as<uint32_t>(nk / 4 + 1));
-    uint64_t nout = 0;
+    uint64_t nout = nk;
     if (nk) {
-      unsigned long long* k1 = c->keys.as<unsigned long long>(nk);
       unsigned long long* k2 = c->keys2.as<unsigned long long>(nk);
-      uint8_t* v1 = reinterpret_cast<uint8_t*>(c->misc1.as<uint32_t>(nk / 4 + 1));
       uint8_t* v2 = reinterpret_cast<uint8_t*>(c->misc2.as<uint32_t>(nk / 4 + 1));
-      k_scatter_pts<<<grid_for(np, 256), 256, 0, s>>>(pairs, hit, keep, off, np, R->d.parent, k1, v1); c->launches++;
       size_t tb = 0;
-      GSJ_CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k1, k2, v1, v2, (int64_t)nk, 0, 64, s));
-      GSJ_CK(cub::DeviceRadixSort::SortPairs(c->tmp.get(tb), tb, k1, k2, v1, v2, (int64_t)nk, 0, 64, s));
-      uint32_t* head = c->misc3.as<uint32_t>(nk);
-      uint32_t* hoff = c->idx2.as<uint32_t>(nk);
-      k_seg_heads<<<grid_for(nk, 256), 256, 0, s>>>(k2, nk, head); c->launches++;
-      exclusive_scan(c, head, hoff, nk);
-      nout = read_last(c, hoff, head, nk);
-      uint32_t* start = c->keep.as<uint32_t>(std::max<uint64_t>(np, nout));
-      k_seg_starts<<<grid_for(nk, 256), 256, 0, s>>>(head, hoff, nk, start); c->launches++;
-      k_fold_max<<<grid_for(nout, 256), 256, 0, s>>>(k2, v2, start, nout, nk, opairs, owhere); c->launches++;
+      GSJ_CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k1, k2, v1, v2, (int64_t)nk, 0, total, s));
+      GSJ_CK(cub::DeviceRadixSort::SortPairs(c->tmp.get(tb), tb, k1, k2, v1, v2, (int64_t)nk, 0, total, s));
+      uint32_t* start = nullptr;
+      if (R->d.parent) {   // without parents every key is there once
+        uint32_t* head = c->misc3.as<uint32_t>(nk);
+        uint32_t* hoff = c->idx2.as<uint32_t>(nk);
+        k_seg_heads<<<grid_for(nk, 256), 256, 0, s>>>(k2, nk, head); c->launches++;
+        exclusive_scan(c, head, hoff, nk);
+        nout = read_last(c, hoff, head, nk);
+        start = c->keep.as<uint32_t>(nout);
+        k_seg_starts<<<grid_for(nk, 256), 256, 0, s>>>(head, hoff, nk, start); c->launches++;
+      }
+      k_fold_max<<<grid_for(nout, 256), 256, 0, s>>>(k2, v2, start, nout, nk, bits, opairs, owhere); c->launches++;
       GSJ_CK(cudaGetLastError());
     }
     st.compact_ms += tm.stop();
@@ -406,18 +424,15 @@ constexpr uint32_t CLUSTER_ROUNDS = 8;
 // Cluster rounds (filtered mode): candidate i = t * R + r belongs to round r; it is refined only while its two
 // parents are still in different components. A skipped pair joins two geometries that are already connected, so
 // the components (and root[]) are those of the full intersects graph.
-__global__ void k_cl_select(const uint2* __restrict__ pairs, uint64_t n, uint32_t r, uint32_t R, const uint32_t* __restrict__ parent,
-                            uint32_t* par, uint32_t* keep) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = t * R + r;
-  if (i >= n) return;
-  const uint2 p = pairs[i];
-  const uint32_t a = parent ? parent[p.x] : p.x, b = parent ? parent[p.y] : p.y;
-  keep[t] = a != b && uf_find(par, a) != uf_find(par, b);
-}
-__global__ void k_cl_gather(const uint2* __restrict__ pairs, uint64_t n, uint32_t r, uint32_t R, const uint32_t* __restrict__ keep,
-                            const uint32_t* __restrict__ off, uint2* out) {
-  const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, i = t * R + r;
-  if (i < n && keep[t]) out[off[t]] = pairs[i];
+__global__ void __launch_bounds__(APPEND_THREADS) k_cl_select(const uint2* __restrict__ pairs, uint64_t n, uint32_t r, uint32_t R,
+                                                             const uint32_t* __restrict__ parent, uint32_t* par, uint2* out, unsigned long long* count) {
+  append_items((n - r + R - 1) / R, count,
+               [&](uint64_t t) {
+                 const uint2 p = pairs[t * R + r];
+                 const uint32_t a = parent ? parent[p.x] : p.x, b = parent ? parent[p.y] : p.y;
+                 return a != b && uf_find(par, a) != uf_find(par, b);
+               },
+               [&](uint64_t t, unsigned long long o) { out[o] = pairs[t * R + r]; });
 }
 __global__ void k_cl_union(const uint2* __restrict__ pairs, const uint8_t* __restrict__ flag, uint64_t n, const uint32_t* __restrict__ parent,
                            uint32_t* par, unsigned long long* hits) {
@@ -539,7 +554,7 @@ void cluster_host(gsj_ctx* c, const gsj_layer* P, uint32_t nparent, const gsj_jo
     Timer tm(s);
     bool whole = false;
     const std::vector<Batch> batches = make_batches(P, o, whole);
-    unsigned long long* hits = c->misc3.as<unsigned long long>(1);
+    unsigned long long* hits = c->misc3.as<unsigned long long>(2);   // hits, pairs selected in a round
     GSJ_CK(cudaMemsetAsync(hits, 0, sizeof(unsigned long long), s));
     for (const Batch& bt : batches) {
       if (o.cancel && *o.cancel) throw Error(GSJ_ERR_CANCELLED, "cancelled");
@@ -555,13 +570,13 @@ void cluster_host(gsj_ctx* c, const gsj_layer* P, uint32_t nparent, const gsj_jo
         if (o.cancel && *o.cancel) throw Error(GSJ_ERR_CANCELLED, "cancelled");
         tm.start();
         const uint64_t nt = (np - r + R - 1) / R;   // candidates r, r + R, ... < np
-        uint32_t* keep = c->keep.as<uint32_t>(nt);
-        uint32_t* off = c->idx.as<uint32_t>(nt);
-        k_cl_select<<<grid_for(nt, 256), 256, 0, s>>>(pairs, np, r, R, P->d.parent, par, keep); c->launches++;
-        exclusive_scan(c, keep, off, nt);
-        const uint64_t ns = read_last(c, off, keep, nt);
-        uint2* sel = c->opairs.as<uint2>(ns);
-        if (ns) { k_cl_gather<<<grid_for(nt, 256), 256, 0, s>>>(pairs, np, r, R, keep, off, sel); c->launches++; }
+        uint2* sel = c->opairs.as<uint2>(nt);
+        GSJ_CK(cudaMemsetAsync(hits + 1, 0, sizeof(unsigned long long), s));
+        k_cl_select<<<append_grid(nt), APPEND_THREADS, 0, s>>>(pairs, np, r, R, P->d.parent, par, sel, hits + 1); c->launches++;
+        unsigned long long* h = c->h_counters.as<unsigned long long>(2);
+        GSJ_CK(cudaMemcpyAsync(h, hits + 1, 8, cudaMemcpyDeviceToHost, s));
+        GSJ_CK(cudaStreamSynchronize(s));
+        const uint64_t ns = h[0];
         st.compact_ms += tm.stop();
         if (!ns) continue;
         tm.start();

@@ -1413,7 +1413,8 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   }
   unsigned long long* h = c->h_refine.as<unsigned long long>(4);
   // counters: [0] oversized pairs, [1] error word, [2] pair counter, [3] local edge pairs, [4] scratch pair counter,
-  // [5] self pairs, [6] self pair counter, [7] the block bin's oversized pairs, [8] block pair counter
+  // [5] self pairs, [6] self pair counter, [7] the block bin's oversized pairs, [8] block pair counter,
+  // [REFINE_ROWS] the caller's, set to 0 here
   auto a_main = kernel_args(k_refine<F, S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
                             self ? 1 : 0);
   auto a_big = kernel_args(k_refine_block<S32, W>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, heavy2, ctr + 7, ctr + 8, ctr + 3);
@@ -1473,7 +1474,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
     if (F) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big, &kb));
     if (scr) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_scr, &ks));
   }
-  GSJ_CK(cudaMemsetAsync(ctr, 0, 9 * sizeof(unsigned long long), s));
+  GSJ_CK(cudaMemsetAsync(ctr, 0, (REFINE_ROWS + 1) * sizeof(unsigned long long), s));
   GSJ_CK(cudaGraphLaunch(g.exec, s));
   c->launches += 1 + (F ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
   GSJ_CK(cudaMemcpyAsync(h, ctr, 32, cudaMemcpyDeviceToHost, s));

@@ -84,3 +84,21 @@ def test_own_tolerances(engine, tol):
             got.append(out)
         for out in got[1:]:
             assert all(np.array_equal(x, y) for x, y in zip(got[0], out))
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 127, 129, 1023, 1024, 1025, 4097])
+def test_every_row_arrives(engine, n):
+    """Rows are appended 1024 candidates a block: n squares apart give n rows, whatever the count."""
+    side = int(np.ceil(np.sqrt(n)))
+    g = make_set([[square(3 * S * (k % side), 3 * S * (k // side), S)] for k in range(n)])
+    la = engine.upload_polygons(g)
+    lp = engine.upload_points(g.xy[g.rvo[:-1].astype(np.int64)] + 0.5 * S)
+    same = np.repeat(np.arange(n, dtype=np.uint32)[:, None], 2, axis=1)
+    p, area, code = rows(engine.join(la, la, want_area=True, want_relate=True, upper=True))
+    assert np.array_equal(p, same) and np.allclose(area, S * S, rtol=1e-9) and (code == code[0]).all()
+    pp, where, _ = engine.join_points(lp, la)
+    assert np.array_equal(pp, same) and (where == 1).all()
+    assert np.array_equal(engine.dwithin(la, la, 5.0, same=True)[0], same)
+    assert np.array_equal(engine.points_dwithin(lp, la, 5.0)[0], same)
+    assert np.array_equal(engine.erode(la, la, 1.0, 1.0, same=True)[0], same)
+    assert np.array_equal(engine.cluster(la)[0], np.arange(n, dtype=np.uint32))
