@@ -32,15 +32,15 @@ __device__ __forceinline__ bool ray_crosses(double x0, double y0, double x1, dou
   return so != sc && (a * (y0 - my) > 0) != (a * (y1 - my) > 0);
 }
 
-// Edge i of a ring of n vertices (the first is vertex s of the layer) in a pair frame: its ends and cut flags, whether it
+// Edge i (p, q: its stored ends) of a ring of n vertices (the first is vertex s of the layer) in a pair frame: its ends and cut flags, whether it
 // meets the overlap box, and its crossing of the level ray to (mx, my) into par (PIP).
 struct GatherEdge { double x0, y0, x1, y1; uint32_t fl; bool in; };
 template <bool F, bool PIP, bool S32>
-__device__ __forceinline__ GatherEdge gather_edge(const Frame& A, const Box& ov, uint64_t s, uint32_t n, uint32_t i, double mx, double my, bool& par) {
+__device__ __forceinline__ GatherEdge gather_edge(const Frame& A, const Box& ov, uint64_t s, uint32_t n, uint32_t i, double2 p, double2 q, double mx, double my,
+                                                  bool& par) {
   const DLayer& S = *A.L;
   GatherEdge e{0, 0, 0, 0, 0u, false};
   if (i + 1 >= n) return e;
-  const double2 p = S.xy[s + i], q = S.xy[s + i + 1];
   e.x0 = A.shx + p.x; e.y0 = A.shy + p.y; e.x1 = A.shx + q.x; e.y1 = A.shy + q.y;
   if (S.synb) {
     e.fl = (uint32_t)S.syn(s + i) | (S.syn(s + (i > 0 ? i - 1 : n - 2)) ? 2u : 0u) | (S.syn(s + (i + 2 < n ? i + 1 : 0)) ? 4u : 0u);
@@ -61,13 +61,24 @@ static __device__ int collect(const Frame& A, const Box& ov, EL L, int cap, int 
   const unsigned lt = (1u << lane) - 1;
   bool par = false;
   int cnt = 0;
+  // the next 32 vertices are on their way while these are tested (500k-parcel relate self-join 19.15 -> 18.6 ms, 150k-parcel
+  // dwithin 2.53 -> 2.40 ms)
+  const uint64_t none = 0;
+  uint64_t s = A.r0 < A.r1 ? S.rvo[A.r0] : none, e1 = A.r0 < A.r1 ? S.rvo[A.r0 + 1] : none;
 #pragma unroll 1
   for (uint32_t ra = A.r0; ra < A.r1; ra++) {
-    const uint64_t s = S.rvo[ra];
-    const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);   // a ring's vertices, indexed by 32 bits
+    const uint32_t n = (uint32_t)(e1 - s);   // a ring's vertices, indexed by 32 bits
+    const uint64_t e2 = ra + 1 < A.r1 ? S.rvo[ra + 2] : none;
+    const double2* v = S.xy + s;
+    double2 p = make_double2(0, 0), q = p;
+    if (lane + 1 < n) { p = v[lane]; q = v[lane + 1]; }
 #pragma unroll 1
     for (uint32_t base = 0; base + 1 < n; base += 32) {
-      const GatherEdge e = gather_edge<F, PIP, S32>(A, ov, s, n, base + lane, mx, my, par);
+      double2 pn = make_double2(0, 0), qn = pn;
+      const uint32_t in = base + 32 + lane;
+      if (in + 1 < n) { pn = v[in]; qn = v[in + 1]; }
+      const GatherEdge e = gather_edge<F, PIP, S32>(A, ov, s, n, base + lane, p, q, mx, my, par);
+      p = pn; q = qn;
       const unsigned m = __ballot_sync(0xffffffffu, e.in);
       const int pos = cnt + __popc(m & lt);
       if (e.in && pos < cap) {
@@ -75,6 +86,7 @@ static __device__ int collect(const Frame& A, const Box& ov, EL L, int cap, int 
       }
       cnt += __popc(m);
     }
+    s = e1; e1 = e2;
   }
   if (PIP) *inside = (__popc(__ballot_sync(0xffffffffu, par)) & 1) != 0;
   return cnt;

@@ -1101,7 +1101,10 @@ __device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int
     const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);
 #pragma unroll 1
     for (uint32_t base = 0; base + 1 < n; base += BIG_WARPS * 32, flip ^= BIG_WARPS) {
-      const GatherEdge e = gather_edge<true, true, S32>(A, ov, s, n, base + threadIdx.x, mx, my, par);
+      const uint32_t i = base + threadIdx.x;
+      double2 p = make_double2(0, 0), q = p;
+      if (i + 1 < n) { p = S.xy[s + i]; q = S.xy[s + i + 1]; }
+      const GatherEdge e = gather_edge<true, true, S32>(A, ov, s, n, i, p, q, mx, my, par);
       const unsigned m = __ballot_sync(0xffffffffu, e.in);
       if (lane == 0) cnt[flip + wid] = __popc(m);
       __syncthreads();
