@@ -697,10 +697,10 @@ __device__ __forceinline__ void edge_cover(EdgeCuts& C, const EdgeRef& e, const 
 
 // Candidate edge pairs (boxes within 2 tol of each other, or a little more on the grid) found and classified; CUTS: the cuts
 // are wanted, else the contact alone (the search then ends at the first real one). SELF: only j > i is searched (an edge
-// always coincides with itself). One warp takes the 32 A edges from ic0 on, then those from ic0 + step on, ...
+// always coincides with itself); self: a geometry with itself searched in full, less each edge with itself. One warp takes the 32 A edges from ic0 on, then those from ic0 + step on, ...
 template <int MS, bool SELF, bool CUTS, int SH, class Q, class EL>
 __device__ Nodes find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const CutLists<Q>& cl, int ic0, int step, int lane, bool& hit,
-                            bool& hit_any) {
+                            bool& hit_any, bool self = false) {
   Nodes nd{0, false};
   uint32_t any = 0;
   scan_edge_pairs<SELF, SH>(
@@ -720,7 +720,7 @@ __device__ Nodes find_pairs(const EL& LA, int na, const EL& LB, int nb, const Pa
         }
       },
       [&](uint32_t e, bool act) {
-        classify_pairs<SELF, CUTS, SH>(LA, LB, G, cl, e, act, lane, nd, hit, hit_any);
+        classify_pairs<SELF, CUTS, SH>(LA, LB, G, cl, e, act && !(self && (e >> SH) == (e & ((1u << SH) - 1u))), lane, nd, hit, hit_any);
         return !CUTS && __any_sync(0xffffffffu, hit);
       });
   return nd;
@@ -742,13 +742,15 @@ __device__ __forceinline__ void begin_pairs(const EL& LB, int na, int nb, const 
 
 // Lane's edge i with its cuts: split points in any order (they are sorted), coincident edges in increasing order.
 // C.ns == MAXS: the split points reached the number that is kept (which are kept depends on the order they are met in).
-template <bool REL, bool SELF, class Q, class EL>
-__device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS, int i, bool valid, const EL& LO, const CutLists<Q>& cl, const uint32_t* head) {
+// self: the lists are one geometry's, whose edges each coincide with themselves (no node says so).
+template <bool REL, class Q, class EL>
+__device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS, int i, bool valid, const EL& LO, const CutLists<Q>& cl, const uint32_t* head,
+                                          bool self) {
   edge_cuts_begin(C);
   e.px = e.py = e.qx = e.qy = e.dx = e.dy = e.len2 = e.len = 0.0; e.fl = 0;
   if (!valid) return;
   e = edge_ref(LS, i, REL);
-  int nc = SELF ? 1 : 0, k = SELF ? i : 0x7FFFFFFF;   // coincident edges, the first of them
+  int nc = self ? 1 : 0, k = self ? i : 0x7FFFFFFF;   // coincident edges, the first of them
 #pragma unroll 1
   for (uint32_t n = head[i]; n != NIL;) {
     const uint32_t w = cl.nxt[n];
@@ -761,7 +763,7 @@ __device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS,
   while (nc > 0) {
     edge_cover(C, e, LO, k);
     if (--nc == 0) break;
-    int next = SELF && i > k ? i : 0x7FFFFFFF;
+    int next = self && i > k ? i : 0x7FFFFFFF;
 #pragma unroll 1
     for (uint32_t n = head[i]; n != NIL;) {
       const uint32_t w = cl.nxt[n];
@@ -819,7 +821,7 @@ __device__ __forceinline__ bool edge_pass(const EL& LS, int nself, const EL& LO,
     const int i = ic + lane;
     EdgeRef e;
     EdgeCuts C;
-    edge_cuts<REL, SELF>(e, C, LS, i, i < nself, LO, cl, head);
+    edge_cuts<REL>(e, C, LS, i, i < nself, LO, cl, head, SELF);
     if (__any_sync(0xffffffffu, C.ns == MAXS)) return false;
     if (e.len2 == 0) C.ns = 0;
     const bool lens = REL && !(e.fl & 1u);
@@ -1079,17 +1081,20 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
 // edges a side in shared memory (54 KB a block, 4 blocks per SM). The routine is refine_pair_m's with the edges of the
 // gather, the search and the passes dealt out to the warps in chunks of 32; the sums keep their order: a lane's running sums
 // pass through shared memory from the warp of one chunk to that of the next. Larger pairs, or more than BIG_NODES cuts,
-// go on to the scratch bin.
+// go on to the scratch bin; where a layer has geometries of more than 512 edges, a second form with 1024 edges a side and 8
+// warps (108 KB, 2 blocks per SM) stands between them: a pair of 700 edges took 0.4 ms by itself in the scratch bin.
 // Against the scratch bin's warp per pair with lists in global memory (10 % of the warps an SM holds, 37k instructions a
 // pair), whole refinement: two 120k layers with areas (7k such pairs) 7.82 -> 6.47 ms, 20k queries relate (3.9k) 1.70 ->
 // 1.32 ms, 100 queries (29: the latency of one pair) 0.27 -> 0.15 ms.
-constexpr int CAP_BIG = 512, BIG_WARPS = 4, BIG_NODES = 1024;
-constexpr size_t BIG_SMEM = 2 * CAP_BIG * EDGE_BYTES_8 + CAP_BIG * 8 + BIG_NODES * 8 + 2 * CAP_BIG * 4 + 2 * (CAP_BIG / 32) * 4 + 5 * 32 * 8 +
-                            BIG_WARPS * QCAP * 4 + BIG_NODES * 2 + 64;
+constexpr int CAP_BIG = 512, CAP_BIG2 = 1024;
+constexpr int block_warps(int cap) { return cap / 128; }
+constexpr size_t block_smem(size_t cap) {   // lists, grid boxes, 2 cap nodes, heads, cand, sums, queues
+  return 2 * cap * EDGE_BYTES_8 + cap * 8 + 2 * cap * 8 + 2 * cap * 4 + 2 * (cap / 32) * 4 + 5 * 32 * 8 + (cap / 128) * QCAP * 4 + 2 * cap * 2;
+}
 
 // the edges of A meeting the box, by the whole block, compacted in ring order; inside: the parity of (mx, my). cnt: one
 // word per warp and a spare set (the rounds alternate, so one barrier a round is enough)
-template <bool S32>
+template <bool S32, int NW>
 __device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int cap, uint32_t* cnt, double mx, double my, bool& inside) {
   const DLayer& S = *A.L;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1100,7 +1105,7 @@ __device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int
     const uint64_t s = S.rvo[ra];
     const uint32_t n = (uint32_t)(S.rvo[ra + 1] - s);
 #pragma unroll 1
-    for (uint32_t base = 0; base + 1 < n; base += BIG_WARPS * 32, flip ^= BIG_WARPS) {
+    for (uint32_t base = 0; base + 1 < n; base += NW * 32, flip ^= NW) {
       const uint32_t i = base + threadIdx.x;
       double2 p = make_double2(0, 0), q = p;
       if (i + 1 < n) { p = S.xy[s + i]; q = S.xy[s + i + 1]; }
@@ -1109,7 +1114,7 @@ __device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int
       if (lane == 0) cnt[flip + wid] = __popc(m);
       __syncthreads();
       int pos = have + __popc(m & ((1u << lane) - 1));
-      for (int w = 0; w < BIG_WARPS; w++) {
+      for (int w = 0; w < NW; w++) {
         const int c = cnt[flip + w];
         if (w < wid) pos += c;
         have += c;
@@ -1121,15 +1126,16 @@ __device__ int collect_block(const Frame& A, const Box& ov, const EList8& L, int
   return have;
 }
 
-template <bool S32, int W>
-__global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DLayer R, const uint2* __restrict__ pairs, const uint32_t* __restrict__ list,
+template <bool S32, int W, int CAP>
+__global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) k_refine_block(DLayer P, DLayer R, const uint2* __restrict__ pairs, const uint32_t* __restrict__ list,
                                                                    const unsigned long long* nlist, RefineArgs rp, uint8_t* flag, double* area, double4* ev,
                                                                    uint32_t* evb, uint32_t* heavy, unsigned long long* nheavy, unsigned long long* next,
-                                                                   unsigned long long* epairs) {
+                                                                   unsigned long long* epairs, int same_layer) {
+  constexpr int NW = block_warps(CAP), NODES_BLOCK = 2 * CAP;
   constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ unsigned long long s_h;
-  __shared__ uint32_t s_cnt[2 * BIG_WARPS], s_nodes, s_bits;
+  __shared__ uint32_t s_cnt[2 * NW], s_nodes, s_bits;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint64_t n = *nlist;   // written by the bins launched before this kernel
   EList8 LA, LB;
@@ -1137,21 +1143,21 @@ __global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DL
   double* sums;   // s2, lin, lon of each lane (the pass that runs), then A's lin and lon
   {
     double* d = reinterpret_cast<double*>(smem);
-    auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + CAP_BIG; L.x1 = d + 2 * CAP_BIG; L.y1 = d + 3 * CAP_BIG; d += 4 * CAP_BIG; };
+    auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + CAP; L.x1 = d + 2 * CAP; L.y1 = d + 3 * CAP; d += 4 * CAP; };
     doubles(LA);
     doubles(LB);
     cl.qb = reinterpret_cast<uint2*>(d);
-    cl.val = d + CAP_BIG;
-    sums = cl.val + BIG_NODES;
+    cl.val = d + CAP;
+    sums = cl.val + NODES_BLOCK;
     cl.headA = reinterpret_cast<uint32_t*>(sums + 5 * 32);
-    cl.headB = cl.headA + CAP_BIG;
-    cl.cand = cl.headB + CAP_BIG;
-    cl.q = cl.cand + 2 * (CAP_BIG / 32) + wid * QCAP;
-    cl.nxt = reinterpret_cast<uint16_t*>(cl.cand + 2 * (CAP_BIG / 32) + BIG_WARPS * QCAP);
+    cl.headB = cl.headA + CAP;
+    cl.cand = cl.headB + CAP;
+    cl.q = cl.cand + 2 * (CAP / 32) + wid * QCAP;
+    cl.nxt = reinterpret_cast<uint16_t*>(cl.cand + 2 * (CAP / 32) + NW * QCAP);
     cl.count = &s_nodes;
-    cl.cap = BIG_NODES;
-    LA.fl = reinterpret_cast<uint8_t*>(cl.nxt + BIG_NODES);
-    LB.fl = LA.fl + CAP_BIG;
+    cl.cap = NODES_BLOCK;
+    LA.fl = reinterpret_cast<uint8_t*>(cl.nxt + NODES_BLOCK);
+    LB.fl = LA.fl + CAP;
   }
   for (;;) {
     __syncthreads();   // the previous pair's shared memory is no longer read
@@ -1161,21 +1167,24 @@ __global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DL
     const uint32_t p = list[s_h];
     const uint2 pr = pairs[p];
     Frame A, B;
+    const bool self = same_layer && pr.x == pr.y;
     const PairGeo G = pair_geo(P, R, pr.x, pr.y, rp, A, B);
     int na = 0, nb = 0;
     bool inA_c = false, inB_c = false;
 #pragma unroll 1
     for (int side = 0; side < 2; side++) {
       bool in = false;
-      const int c = collect_block<S32>(side ? B : A, G.ov, side ? LB : LA, CAP_BIG, s_cnt, G.cx, G.cy, in);
+      const int c = collect_block<S32, NW>(side ? B : A, G.ov, side ? LB : LA, CAP, s_cnt, G.cx, G.cy, in);
       if (side) { nb = c; inB_c = in; } else { na = c; inA_c = in; }
     }
-    bool over = na > CAP_BIG || nb > CAP_BIG;   // the same in every thread, here and below
+    bool over = na > CAP || nb > CAP;   // the same in every thread, here and below
     bool hit = false, hit_any = false;
     if (!over) {
-      begin_pairs<CAP_BIG, false, W != W_FLAG>(LB, na, nb, G, cl, threadIdx.x, BIG_WARPS * 32);
+      begin_pairs<CAP, false, W != W_FLAG>(LB, na, nb, G, cl, threadIdx.x, NW * 32);
       __syncthreads();
-      const Nodes nd = find_pairs<CAP_BIG, false, W != W_FLAG, 16>(LA, na, LB, nb, G, cl, wid * 32, BIG_WARPS * 32, lane, hit, hit_any);
+      const Nodes nd = find_pairs<CAP, false, W != W_FLAG, 16>(LA, na, LB, nb, G, cl, wid * 32, NW * 32, lane, hit, hit_any, self);
+      if (self)
+        for (int i = threadIdx.x; i < na; i += NW * 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
       hit = __syncthreads_or(hit);
       hit_any = __syncthreads_or(hit_any || hit);
       over = __syncthreads_or(nd.full);
@@ -1196,7 +1205,7 @@ __global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DL
           const EList8& LO = pass ? LA : LB;
           const int nself = pass ? nb : na, nother = pass ? na : nb;
           const uint32_t* head = pass ? cl.headB : cl.headA;
-          const uint32_t* cand = cl.cand + (pass ? CAP_BIG / 32 : 0);
+          const uint32_t* cand = cl.cand + (pass ? CAP / 32 : 0);
           const bool inc = pass ? inA_c : inB_c;
           if (wid == 0) {   // a lane's sums: s2 runs on, each pass's lengths start from 0
             if (pass) { sums[96 + lane] = sums[32 + lane]; sums[128 + lane] = sums[64 + lane]; } else sums[lane] = 0.0;
@@ -1204,11 +1213,11 @@ __global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DL
           }
           __syncthreads();
 #pragma unroll 1
-          for (int c0 = 0; c0 * 32 < nself && !over; c0 += BIG_WARPS) {
+          for (int c0 = 0; c0 * 32 < nself && !over; c0 += NW) {
             const int c = c0 + wid, i = c * 32 + lane;
             EdgeRef e;
             EdgeCuts C;
-            edge_cuts<REL, false>(e, C, LS, i, i < nself, LO, cl, head);
+            edge_cuts<REL>(e, C, LS, i, i < nself, LO, cl, head, self);
             const bool full = C.ns == MAXS;
             if (e.len2 == 0) C.ns = 0;
             const bool lens = REL && !(e.fl & 1u);
@@ -1226,7 +1235,7 @@ __global__ void __launch_bounds__(BIG_WARPS * 32, 4) k_refine_block(DLayer P, DL
             }
             over = __syncthreads_or(full);
 #pragma unroll 1
-            for (int w = 0; w < BIG_WARPS && !over; w++) {   // the chunks' terms in their order
+            for (int w = 0; w < NW && !over; w++) {   // the chunks' terms in their order
               if (w == wid && c * 32 < nself) {
                 double acc = 0.0, lin = sums[32 + lane], lon = sums[64 + lane];
 #pragma unroll 1
@@ -1355,7 +1364,10 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   const int bit = 1 << variant;
   if (!(c->refine_attr & bit)) {
     GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
-    if (F) GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BIG_SMEM));
+    if (F) {
+      GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG)));
+      GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG2)));
+    }
     c->refine_attr |= bit;
   }
   const RefineShape& sh = c->shape;
@@ -1380,9 +1392,8 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   // oversized pairs, and the rare ones whose cuts they cannot keep, to the block bin, and that bin to the scratch bin
   // (the full number of warps only where a geometry can have more edges than the block bin holds)
   const uint32_t most = std::max(P->max_geom_edges, R->max_geom_edges);
-  const bool big = most > (uint32_t)(F ? CAP_BIG : bin_cap), scr = F || big;
-  uint32_t* heavy2 = F ? c->heavy2.as<uint32_t>(np) : heavy;
-  const int bblocks = (int)std::min<uint64_t>(np, (uint64_t)c->sm_count * 4);
+  const bool big = most > (uint32_t)(F ? CAP_BIG2 : bin_cap), scr = F || big, two = F && most > (uint32_t)CAP_BIG;
+  uint32_t* heavy2 = F ? c->heavy2.as<uint32_t>(np) : heavy;   // a pair leaves a bin's list before the next bin runs: the third list is the first's memory
   const ScratchGeom sg = scratch_geom<F>(P, R);
   int sblocks = 0;
   unsigned char* sbuf = nullptr;
@@ -1417,20 +1428,28 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   unsigned long long* h = c->h_refine.as<unsigned long long>(4);
   // counters: [0] oversized pairs, [1] error word, [2] pair counter, [3] local edge pairs, [4] scratch pair counter,
   // [5] self pairs, [6] self pair counter, [7] the block bin's oversized pairs, [8] block pair counter,
-  // [REFINE_ROWS] the caller's, set to 0 here
+  // [REFINE_ROWS] the caller's, set to 0 here, [10], [11] as [7], [8] of the second block bin
   auto a_main = kernel_args(k_refine<F, S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
                             self ? 1 : 0);
-  auto a_big = kernel_args(k_refine_block<S32, W>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, heavy2, ctr + 7, ctr + 8, ctr + 3);
-  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, heavy2, F ? ctr + 7 : ctr, rp, flag, area, ev, evb, sbuf, sg.cap, sg.cph, err, ctr + 3,
-                           ctr + 4, P == R ? 1 : 0);
+  auto a_big = kernel_args(k_refine_block<S32, W, CAP_BIG>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, heavy2, ctr + 7, ctr + 8, ctr + 3, P == R);
+  auto a_big2 = kernel_args(k_refine_block<S32, W, CAP_BIG2>, P->d, R->d, pairs, heavy2, ctr + 7, rp, flag, area, ev, evb, heavy, ctr + 10, ctr + 11, ctr + 3,
+                            P == R);
+  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, F && !two ? heavy2 : heavy, two ? ctr + 10 : F ? ctr + 7 : ctr, rp, flag, area, ev, evb, sbuf,
+                           sg.cap, sg.cph, err, ctr + 3, ctr + 4, P == R ? 1 : 0);
   auto a_idx = kernel_args(k_self_index, pairs, np, sidx, ctr + 5);
   auto a_self = kernel_args(k_refine_self<S32, W>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
-  cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{};
-  kb.func = (void*)k_refine_block<S32, W>;
-  kb.gridDim = dim3(bblocks);
-  kb.blockDim = dim3(BIG_WARPS * 32);
-  kb.sharedMemBytes = (unsigned)BIG_SMEM;
+  cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{}, kb2{};
+  kb.func = (void*)k_refine_block<S32, W, CAP_BIG>;
+  kb.gridDim = dim3((unsigned)std::min<uint64_t>(np, (uint64_t)c->sm_count * 4));
+  kb.blockDim = dim3(block_warps(CAP_BIG) * 32);
+  kb.sharedMemBytes = (unsigned)block_smem(CAP_BIG);
   kb.kernelParams = a_big.ptr;
+  kb2 = kb;
+  kb2.func = (void*)k_refine_block<S32, W, CAP_BIG2>;
+  kb2.gridDim = dim3((unsigned)std::min<uint64_t>(np, (uint64_t)c->sm_count * 2));
+  kb2.blockDim = dim3(block_warps(CAP_BIG2) * 32);
+  kb2.sharedMemBytes = (unsigned)block_smem(CAP_BIG2);
+  kb2.kernelParams = a_big2.ptr;
   km.func = (void*)k_refine<F, S32, W>;
   km.gridDim = dim3(blocks);
   km.blockDim = dim3(RB_WARPS * 32);
@@ -1449,7 +1468,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   kf.blockDim = dim3(RB_WARPS * 32);
   kf.sharedMemBytes = (unsigned)SELF_SMEM;
   kf.kernelParams = a_self.ptr;
-  RefineGraph& g = c->rgraph[variant * 4 + (scr ? 2 : 0) + (self ? 1 : 0)];
+  RefineGraph& g = c->rgraph[variant * 4 + (F ? two : scr) * 2 + (self ? 1 : 0)];
   if (!g.exec) {   // the graph is kept with its executable: the node handles used for the updates belong to it
     if (!g.graph) {
       GSJ_CK(cudaGraphCreate(&g.graph, 0));
@@ -1464,6 +1483,10 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
       if (F) {
         GSJ_CK(cudaGraphAddKernelNode(&g.n_big, g.graph, before.data(), before.size(), &kb));
         before.assign(1, g.n_big);
+        if (two) {
+          GSJ_CK(cudaGraphAddKernelNode(&g.n_big2, g.graph, before.data(), 1, &kb2));
+          before.assign(1, g.n_big2);
+        }
       }
       if (scr) GSJ_CK(cudaGraphAddKernelNode(&g.n_scr, g.graph, before.data(), before.size(), &ks));
     }
@@ -1475,11 +1498,12 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
       GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_self, &kf));
     }
     if (F) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big, &kb));
+    if (two) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big2, &kb2));
     if (scr) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_scr, &ks));
   }
-  GSJ_CK(cudaMemsetAsync(ctr, 0, (REFINE_ROWS + 1) * sizeof(unsigned long long), s));
+  GSJ_CK(cudaMemsetAsync(ctr, 0, 12 * sizeof(unsigned long long), s));
   GSJ_CK(cudaGraphLaunch(g.exec, s));
-  c->launches += 1 + (F ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
+  c->launches += 1 + (F ? 1 : 0) + (two ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
   GSJ_CK(cudaMemcpyAsync(h, ctr, 32, cudaMemcpyDeviceToHost, s));
   c->refine_pending = true;
 }

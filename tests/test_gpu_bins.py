@@ -32,7 +32,7 @@ def ngon(n, r, cx=0.0, cy=0.0):
 
 SHAPES = {
     # a bar across every tooth: 2 x teeth splits on its long edges (an edge keeps 22 beside its ends)
-    **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28, 100)},
+    **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28, 100, 200)},
     # crossed combs: more split points than the lists hold
     "combs_9": ([[comb(9, 10 * S, 10 * S)]], [[comb(9, 10 * S, 10 * S, flip=True)]]),
     "combs_28": ([[comb(28, 10 * S, 10 * S)]], [[comb(28, 10 * S, 10 * S, flip=True)]]),
@@ -41,7 +41,7 @@ SHAPES = {
     "touch": ([[square(0, 0, S)]], [[square(0, S, S)], [square(S, S, S)]]),
     "twins": ([[square(0, 0, S)], [comb(9, S, S)]], [[square(0, 0, S)], [comb(9, S, S)]]),
 }
-for _n in (31, 32, 33, 64, 96, 127, 128, 129, 192, 193, 300, 511, 512, 513):
+for _n in (31, 32, 33, 64, 96, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025):
     SHAPES[f"ngon_{_n}"] = ([[ngon(_n, S)]], [[ngon(_n, S, 0.3 * S, 0.2 * S)], [ngon(7, 0.2 * S)]])
 
 
