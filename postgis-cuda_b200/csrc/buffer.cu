@@ -286,9 +286,10 @@ constexpr int DW_CAP = 128, DW_WARPS = 4;
 constexpr size_t DW_EDGE = 4 * sizeof(double) + sizeof(uint32_t);
 __host__ __device__ constexpr size_t dw_warp_bytes(size_t cap) { return 2 * cap * DW_EDGE + DW_QCAP * sizeof(uint2); }   // lists, queue
 constexpr size_t DW_SMEM = (size_t)DW_WARPS * dw_warp_bytes(DW_CAP);
-constexpr size_t DW_WARP_F = 2 * (size_t)DW_CAP * (4 * sizeof(double) + 1) + DW_CAP * sizeof(uint2) + QCAP * sizeof(uint16_t);   // lists, grid boxes, queue
-constexpr size_t DW_SMEM_F = (size_t)DW_WARPS * DW_WARP_F;
-constexpr int DW_MINB = 4;   // filtered: 128 registers a thread (5 blocks, with spills: 2.77 ms where 4 take 2.48)
+// filtered: lists, grid boxes, queue of a warp; pairs of more than DW_CAP local edges a side take the same kernel with DW_CAP2
+constexpr size_t dw_warp_f(size_t cap) { return 2 * cap * (4 * sizeof(double) + 1) + cap * sizeof(uint2) + QCAP * sizeof(uint16_t); }
+constexpr int DW_CAP2 = 256;
+constexpr int dw_minb(int cap) { return cap == DW_CAP ? 4 : 2; }   // 128 registers a thread (5 blocks, with spills: 2.77 ms where 4 take 2.48); 2 x 77 KB
 
 // plain: the reference's scheme
 __global__ void __launch_bounds__(DW_WARPS * 32, 4) k_dwithin_plain(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
@@ -316,17 +317,23 @@ __global__ void __launch_bounds__(DW_WARPS * 32, 4) k_dwithin_plain(DLayer P, DL
 // d goes to the list of oversized pairs, whose kernel has the geodesic (a pair in thousands), unless one polygon
 // contains the other.
 // Bound by issue and instruction fetch: 150k-parcel self-join at 5 m, 666k pairs: 4.02 ms with the set-up in every lane and two
-// inlined copies of the measuring and the geodesic (314 KB of code, instruction-fetch stall 4.2 cycles an instruction), 2.05 ms.
-__global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
-                                                                   uint8_t* flag, uint32_t* heavy, unsigned long long* nheavy) {
+// inlined copies of the measuring and the geodesic (314 KB of code, instruction-fetch stall 4.2 cycles an instruction), 1.95 ms. The
+// 3.6k oversized pairs took 0.43 ms by a warp each from global lists; by the form with lists of 256 edges, which reads the
+// first form's list, the whole call fell from 3.55 to 3.44 ms.
+template <int CAP>
+__global__ void __launch_bounds__(DW_WARPS * 32, dw_minb(CAP)) k_dwithin(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, double d, int same,
+                                                                        uint8_t* flag, const uint32_t* list, const unsigned long long* nlist,
+                                                                        uint32_t* over, unsigned long long* nover, uint32_t* heavy,
+                                                                        unsigned long long* nheavy) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  double* x = reinterpret_cast<double*>(smem + (size_t)wib * DW_WARP_F);
-  EList8 LA{x, x + DW_CAP, x + 2 * DW_CAP, x + 3 * DW_CAP, nullptr}, LB{x + 4 * DW_CAP, x + 5 * DW_CAP, x + 6 * DW_CAP, x + 7 * DW_CAP, nullptr};
-  uint2* qb = reinterpret_cast<uint2*>(x + 8 * DW_CAP);
-  uint16_t* q = reinterpret_cast<uint16_t*>(qb + DW_CAP);
+  if (list) np = *nlist;   // written by the first form, launched before this one
+  double* x = reinterpret_cast<double*>(smem + (size_t)wib * dw_warp_f(CAP));
+  EList8 LA{x, x + CAP, x + 2 * CAP, x + 3 * CAP, nullptr}, LB{x + 4 * CAP, x + 5 * CAP, x + 6 * CAP, x + 7 * CAP, nullptr};
+  uint2* qb = reinterpret_cast<uint2*>(x + 8 * CAP);
+  uint16_t* q = reinterpret_cast<uint16_t*>(qb + CAP);
   LA.fl = reinterpret_cast<uint8_t*>(q + QCAP);
-  LB.fl = LA.fl + DW_CAP;
+  LB.fl = LA.fl + CAP;
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, span = (np + nw - 1) / nw < 32 ? (np + nw - 1) / nw : 32;   // few pairs: spread over all warps
   for (uint64_t i0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * span; i0 < np; i0 += nw * span) {
     const int cnt = np - i0 < span ? (int)(np - i0) : (int)span;
@@ -334,8 +341,10 @@ __global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DL
     Box mov{0, 0, 0, 0};
     double mgx = 0, mgy = 0, mkx = 0, mky = 0, mtl = 0, mdelta = 0;
     int mres = -2;   // -2: to be decided by the warp, else the flag
+    uint32_t mp = 0;
     if (lane < cnt) {
-      mpr = pairs[i0 + lane];
+      mp = list ? list[i0 + lane] : (uint32_t)(i0 + lane);
+      mpr = pairs[mp];
       if (same && P.pid(mpr.x) == R.pid(mpr.y)) mres = 1;   // pieces of one geometry (buffer.cuh:247-250)
       else {
         const double2 oa = P.origin[mpr.x], ob = R.origin[mpr.y], ea = P.ext[mpr.x], eb = R.ext[mpr.y];
@@ -359,12 +368,12 @@ __global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DL
       int na = 0, nb = 0;
 #pragma unroll 1
       for (int side = 0; side < 2; side++) {   // one inlined copy of the gather
-        const int n = collect<true>(side ? B : A, ov, side ? LB : LA, DW_CAP, lane);
+        const int n = collect<true>(side ? B : A, ov, side ? LB : LA, CAP, lane);
         if (side) nb = n; else na = n;
       }
       __syncwarp();
-      int res = -1;   // -1: the list of oversized pairs
-      if (na <= DW_CAP && nb <= DW_CAP) {
+      int res = -1;   // -1: oversized, -3: undecided without the geodesic
+      if (na <= CAP && nb <= CAP) {
         const double gx = shfl_d(mgx, k), gy = shfl_d(mgy, k), kx = shfl_d(mkx, k), ky = shfl_d(mky, k), tl = shfl_d(mtl, k), delta = shfl_d(mdelta, k);
         bool hit = false, open = false;
         fill_boxes(LB, nb, qgrid(ov), qb, lane, 32);
@@ -404,15 +413,16 @@ __global__ void __launch_bounds__(DW_WARPS * 32, DW_MINB) k_dwithin(DLayer P, DL
 #pragma unroll 1
           for (int side = 0; side < 2; side++) in[side] = pip_full_warp(side ? B : A, cx, cy, lane);
           res = contains_warp<false>(A, B, LA, na, LB, nb, in[0], in[1], ov, cx, cy, lane, any) ? 1 : 0;
-          if (!res && __any_sync(0xffffffffu, open)) res = -1;
+          if (!res && __any_sync(0xffffffffu, open)) res = -3;
         }
       }
       if (lane == k) mres = res;
       __syncwarp();
     }
     if (lane < cnt) {
-      flag[i0 + lane] = mres > 0 ? 1 : 0;
-      if (mres < 0) heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)(i0 + lane);
+      flag[mp] = mres > 0 ? 1 : 0;
+      if (mres == -1) over[atomicAdd(nover, 1ull)] = mp;
+      if (mres == -3) heavy[atomicAdd(nheavy, 1ull)] = mp;
     }
   }
 }
@@ -657,7 +667,8 @@ void dwithin_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double d, 
   }
   if (!c->dw_attr) {
     GSJ_CK(cudaFuncSetAttribute(k_dwithin_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM));
-    GSJ_CK(cudaFuncSetAttribute(k_dwithin, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DW_SMEM_F));
+    GSJ_CK(cudaFuncSetAttribute(k_dwithin<DW_CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DW_WARPS * dw_warp_f(DW_CAP))));
+    GSJ_CK(cudaFuncSetAttribute(k_dwithin<DW_CAP2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DW_WARPS * dw_warp_f(DW_CAP2))));
     c->dw_attr = 1;
   }
   const bool queued = o.refine_mode != GSJ_REFINE_PLAIN;
@@ -679,9 +690,17 @@ void dwithin_host(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, double d, 
     uint32_t* heavy = c->heavy.as<uint32_t>(np);
     unsigned long long* ctr = c->counters.as<unsigned long long>(8);
     int* err = reinterpret_cast<int*>(ctr + 1);
-    GSJ_CK(cudaMemsetAsync(ctr, 0, 16, s));
+    GSJ_CK(cudaMemsetAsync(ctr, 0, 24, s));   // pairs for the scratch kernel, error word, pairs for the second form
     const int blocks = (int)std::min<uint64_t>((np + DW_WARPS - 1) / DW_WARPS, (uint64_t)c->sm_count * 8);
-    if (queued) k_dwithin<<<blocks, DW_WARPS * 32, DW_SMEM_F, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
+    if (queued) {
+      uint32_t* over = c->heavy2.as<uint32_t>(np);
+      k_dwithin<DW_CAP><<<blocks, DW_WARPS * 32, DW_WARPS * dw_warp_f(DW_CAP), s>>>(P->d, R->d, pairs, np, d, same, flag, nullptr, nullptr, over, ctr + 2, heavy, ctr);
+      if (std::max(P->max_geom_edges, R->max_geom_edges) > (uint32_t)DW_CAP) {
+        k_dwithin<DW_CAP2><<<std::min(blocks, c->sm_count * 2), DW_WARPS * 32, DW_WARPS * dw_warp_f(DW_CAP2), s>>>(P->d, R->d, pairs, np, d, same, flag, over, ctr + 2,
+                                                                                                                 heavy, ctr, heavy, ctr);
+        c->launches++;
+      }
+    }
     else k_dwithin_plain<<<blocks, DW_WARPS * 32, DW_SMEM, s>>>(P->d, R->d, pairs, np, d, same, flag, heavy, ctr);
     c->launches++;
     GSJ_CK(cudaGetLastError());

@@ -551,7 +551,7 @@ void cluster_host(gsj_ctx* c, const gsj_layer* P, uint32_t nparent, const gsj_jo
       if (out.n) { k_uf_union<<<grid_for(out.n, 256), 256, 0, s>>>(out.pairs, out.n, par); c->launches++; }
     });
   } else {   // rounds that skip pairs whose parents are already connected
-    Timer tm(s);
+    Timer tm(s), tr(s), tu(s);
     bool whole = false;
     const std::vector<Batch> batches = make_batches(P, o, whole);
     unsigned long long* hits = c->misc3.as<unsigned long long>(2);   // hits, pairs selected in a round
@@ -566,8 +566,18 @@ void cluster_host(gsj_ctx* c, const gsj_layer* P, uint32_t nparent, const gsj_jo
       st.batches++;
       if (!np) continue;
       const uint32_t R = np < (1u << 16) ? 1 : CLUSTER_ROUNDS;
+      // one host wait a round, for the number of selected pairs: the refinement and the unions of a round are behind it
+      // on the stream, and their times and counters are read after the next wait
+      bool open = false;
+      auto finish = [&] {
+        if (!open) return;
+        st.heavy += refine_result(c);
+        st.refine_ms += tr.elapsed();
+        st.compact_ms += tu.elapsed();
+        open = false;
+      };
       for (uint32_t r = 0; r < R; r++) {
-        if (o.cancel && *o.cancel) throw Error(GSJ_ERR_CANCELLED, "cancelled");
+        if (o.cancel && *o.cancel) { GSJ_CK(cudaStreamSynchronize(s)); finish(); throw Error(GSJ_ERR_CANCELLED, "cancelled"); }
         tm.start();
         const uint64_t nt = (np - r + R - 1) / R;   // candidates r, r + R, ... < np
         uint2* sel = c->opairs.as<uint2>(nt);
@@ -575,19 +585,22 @@ void cluster_host(gsj_ctx* c, const gsj_layer* P, uint32_t nparent, const gsj_jo
         k_cl_select<<<append_grid(nt), APPEND_THREADS, 0, s>>>(pairs, np, r, R, P->d.parent, par, sel, hits + 1); c->launches++;
         unsigned long long* h = c->h_counters.as<unsigned long long>(2);
         GSJ_CK(cudaMemcpyAsync(h, hits + 1, 8, cudaMemcpyDeviceToHost, s));
-        GSJ_CK(cudaStreamSynchronize(s));
-        const uint64_t ns = h[0];
         st.compact_ms += tm.stop();
+        const uint64_t ns = h[0];
+        finish();
         if (!ns) continue;
-        tm.start();
+        tr.start();
         uint8_t* flag = c->flag.as<uint8_t>(ns);
-        st.heavy += refine(c, P, P, sel, ns, rp, o.refine_mode, flag, nullptr, nullptr, nullptr);
-        st.refine_ms += tm.stop();
-        tm.start();
+        refine_enqueue(c, P, P, sel, ns, rp, o.refine_mode, flag, nullptr, nullptr, nullptr, true);
+        tr.mark_end();
+        tu.start();
         k_cl_union<<<grid_for(ns, 256), 256, 0, s>>>(sel, flag, ns, P->d.parent, par, hits); c->launches++;
         k_uf_flatten<<<grid_for(nparent, 256), 256, 0, s>>>(par, nparent); c->launches++;
-        st.compact_ms += tm.stop();
+        tu.mark_end();
+        open = true;
       }
+      GSJ_CK(cudaStreamSynchronize(s));
+      finish();
     }
     unsigned long long hh = 0;
     GSJ_CK(cudaMemcpyAsync(&hh, hits, sizeof(hh), cudaMemcpyDeviceToHost, s));
