@@ -42,13 +42,15 @@ __global__ void k_scatter_rows(const uint2* __restrict__ pairs, const uint32_t* 
 
 // rows of the intersecting pairs (flag 1), in no set order, with their area and DE-9IM code
 __global__ void __launch_bounds__(APPEND_THREADS) k_append_rows(const uint2* __restrict__ pairs, const uint8_t* __restrict__ flag, uint64_t n, const double* area,
-                                                               const double4* ev, const uint32_t* evb, const double* blA, const double* blB, uint2* opairs,
-                                                               double* oarea, uint32_t* ocode, unsigned long long* count) {
+                                                               const double4* ev, const uint32_t* evb, const double* blA, const double* blB, const uint32_t* parA,
+                                                               const uint32_t* parB, uint2* opairs, double* oarea, uint32_t* ocode,
+                                                               unsigned long long* count) {
   append_items(n, count, [&](uint64_t i) { return flag[i] == 1; }, [&](uint64_t i, unsigned long long o) {
     const uint2 p = pairs[i];
     opairs[o] = p;
     if (oarea) oarea[o] = area[i];
-    if (ocode) ocode[o] = de9im_code(ev[i], evb[i], blA[p.x], blB[p.y]);
+    // lengths are kept per parent; pieces that are not folded (no_agg) take their parent's
+    if (ocode) ocode[o] = de9im_code(ev[i], evb[i], blA[parA ? parA[p.x] : p.x], blB[parB ? parB[p.y] : p.y]);
   });
 }
 // pieces kept for folding: sort keys (piece pair, then parent pair) and the per-pair payload
@@ -205,7 +207,8 @@ void run_join(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const RefineAr
       out.area = rp.want_area ? c->oarea.as<double>(np) : nullptr;
       out.code = rel ? c->ocode.as<uint32_t>(np) : nullptr;
       unsigned long long* cnt = c->counters.as<unsigned long long>(16) + REFINE_ROWS;
-      k_append_rows<<<append_grid(np), APPEND_THREADS, 0, s>>>(pairs, flag, np, area, ev, evb, P->d.blen, R->d.blen, out.pairs, out.area, out.code, cnt);
+      k_append_rows<<<append_grid(np), APPEND_THREADS, 0, s>>>(pairs, flag, np, area, ev, evb, P->d.blen, R->d.blen, P->d.parent, R->d.parent, out.pairs, out.area,
+                                                                   out.code, cnt);
       c->launches++;
       unsigned long long* h = c->h_counters.as<unsigned long long>(2);
       GSJ_CK(cudaMemcpyAsync(h, cnt, 8, cudaMemcpyDeviceToHost, s));

@@ -102,3 +102,15 @@ def test_every_row_arrives(engine, n):
     assert np.array_equal(engine.points_dwithin(lp, la, 5.0)[0], same)
     assert np.array_equal(engine.erode(la, la, 1.0, 1.0, same=True)[0], same)
     assert np.array_equal(engine.cluster(la)[0], np.arange(n, dtype=np.uint32))
+
+
+def test_unfolded_pieces_relate(engine):
+    """no_agg on subdivided layers: piece pairs, whose boundary lengths are their parents' (kept per parent, not per piece)."""
+    from gsj import gen
+    P = engine.subdivide(gen.layer_parcels(300, (-118.30, 33.95, -118.29, 33.96), seed=5), 12)
+    lp = engine.upload_polygons(P)
+    assert P.n > P.parent.max() + 1
+    got = [rows(engine.join(lp, lp, want_area=False, want_relate=True, no_agg=True, refine_mode=m)) for m in MODES]
+    assert got[0][0].max() == P.n - 1
+    for p, _, c in got[1:]:
+        assert np.array_equal(p, got[0][0]) and np.array_equal(c, got[0][2])
