@@ -131,7 +131,7 @@ struct RefineShape { int run = 4, runs = 32, bin_cap = 128, scratch_wpsm = 32; }
 // context and re-parameterised per call.
 struct RefineGraph {
   cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr;
-  cudaGraphNode_t n_main = nullptr, n_scr = nullptr, n_idx = nullptr, n_self = nullptr, n_big = nullptr, n_big2 = nullptr;
+  cudaGraphNode_t n_main = nullptr, n_scr = nullptr, n_idx = nullptr, n_self = nullptr, n_split = nullptr, n_big = nullptr, n_big2 = nullptr;
 };
 }  // namespace gsj
 
@@ -145,7 +145,7 @@ struct gsj_ctx {
   uint64_t node_visits = 0;   // LBVH nodes visited by traversals (roofline accounting)
   uint64_t edge_pairs = 0;    // local edge pairs (na x nb) of the pairs refined (the refinement's work unit)
   gsj::RefineShape shape;
-  gsj::RefineGraph rgraph[36];   // [variant (plain, filtered x what is wanted, filtered FP32 x the same) x second block bin (plain: scratch bin) or not x self bin or not]
+  gsj::RefineGraph rgraph[54];   // [variant (plain, filtered x what is wanted, filtered FP32 x the same) x bins for larger pairs, 0 - 2 x self bin or not]
   // scratch pools
   gsj::DevBuf counters, cand, flag, area, ev, evb, heavy, heavy2, selfidx, scratch, keep, opairs, oarea, oev, oevb, ocode, tmp, keys, keys2, idx,
       idx2, agg_area, agg_ev, agg_evb, agg_flag, qbb, uf, misc1, misc2, misc3,

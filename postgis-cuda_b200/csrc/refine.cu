@@ -5,7 +5,8 @@
 // FP64 area and boundary-length sums have one fixed rounding order: bit-identical to the CPU oracle.
 //
 // Pairs whose local edge lists fit CAP run from shared memory, a warp each; larger pairs are queued and re-run by
-// k_refine_block (filtered: a block each) and, beyond its lists, k_refine_scratch (per-warp lists in global scratch).
+// k_refine_block (filtered: a block each) and, beyond its lists, k_refine_scratch (per-warp lists in global scratch); the
+// filtered bin's pairs with an edge of many split points by k_refine_split.
 //
 // Two variants with the same decisions and the same FP64 values:
 //  - plain (F = false): the reference's sweeps, FP64 box tests (refine_pair_t<false>).
@@ -740,40 +741,54 @@ __device__ __forceinline__ void begin_pairs(const EL& LB, int na, int nb, const 
   }
 }
 
+// The cuts that all edges of the other polygon make, met in increasing order: the reference's own sweep, for an edge with more
+// split points than are kept (which are kept depends on the order) and for pairs with more cuts than the lists hold.
+template <class EL>
+__device__ __forceinline__ void edge_sweep(EdgeCuts& C, const EdgeRef& e, const EL& L, int cnt, const PairGeo& G) {
+  edge_cuts_begin(C);
+#pragma unroll 1
+  for (int k = 0; k < cnt; k++) edge_visit<true>(C, e, L, k, G);
+  edge_cuts_sort(C);
+}
+
 // Lane's edge i with its cuts: split points in any order (they are sorted), coincident edges in increasing order.
 // C.ns == MAXS: the split points reached the number that is kept (which are kept depends on the order they are met in).
-// self: the lists are one geometry's, whose edges each coincide with themselves (no node says so).
-template <bool REL, class Q, class EL>
-__device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS, int i, bool valid, const EL& LO, const CutLists<Q>& cl, const uint32_t* head,
-                                          bool self) {
+// self: the lists are one geometry's, whose edges each coincide with themselves (no node says so). SWEEP: such an edge's
+// cuts, and all edges' where the lists are not whole (sweep), are found by sweeping the other polygon's nother edges.
+template <bool REL, bool SWEEP, class Q, class EL>
+__device__ __forceinline__ void edge_cuts(EdgeRef& e, EdgeCuts& C, const EL& LS, int i, bool valid, const EL& LO, int nother, const CutLists<Q>& cl,
+                                          const uint32_t* head, bool self, bool sweep, const PairGeo& G) {
   edge_cuts_begin(C);
   e.px = e.py = e.qx = e.qy = e.dx = e.dy = e.len2 = e.len = 0.0; e.fl = 0;
   if (!valid) return;
   e = edge_ref(LS, i, REL);
-  int nc = self ? 1 : 0, k = self ? i : 0x7FFFFFFF;   // coincident edges, the first of them
-#pragma unroll 1
-  for (uint32_t n = head[i]; n != NIL;) {
-    const uint32_t w = cl.nxt[n];
-    const double v = cl.val[n];
-    if (w & COVER) { nc++; k = min(k, (int)v); }
-    else if (C.ns < MAXS) C.ts[C.ns++] = v;
-    n = w & NIL;
-  }
-#pragma unroll 1
-  while (nc > 0) {
-    edge_cover(C, e, LO, k);
-    if (--nc == 0) break;
-    int next = self && i > k ? i : 0x7FFFFFFF;
+  if (!SWEEP || !sweep) {
+    int nc = self ? 1 : 0, k = self ? i : 0x7FFFFFFF;   // coincident edges, the first of them
 #pragma unroll 1
     for (uint32_t n = head[i]; n != NIL;) {
       const uint32_t w = cl.nxt[n];
-      const int c = (w & COVER) ? (int)cl.val[n] : 0x7FFFFFFF;
-      if (c > k) next = min(next, c);
+      const double v = cl.val[n];
+      if (w & COVER) { nc++; k = min(k, (int)v); }
+      else if (C.ns < MAXS) C.ts[C.ns++] = v;
       n = w & NIL;
     }
-    k = next;
+#pragma unroll 1
+    while (nc > 0) {
+      edge_cover(C, e, LO, k);
+      if (--nc == 0) break;
+      int next = self && i > k ? i : 0x7FFFFFFF;
+#pragma unroll 1
+      for (uint32_t n = head[i]; n != NIL;) {
+        const uint32_t w = cl.nxt[n];
+        const int c = (w & COVER) ? (int)cl.val[n] : 0x7FFFFFFF;
+        if (c > k) next = min(next, c);
+        n = w & NIL;
+      }
+      k = next;
+    }
   }
-  edge_cuts_sort(C);
+  if (SWEEP && (sweep || C.ns == MAXS)) edge_sweep(C, e, LO, nother, G);
+  else edge_cuts_sort(C);
 }
 
 // The inside tests of 32 lanes' points (need, mx, my) against the polygon LO, one test at a time by the whole warp; lanes
@@ -806,13 +821,13 @@ __device__ __forceinline__ unsigned edge_links(const EdgeRef& e, bool valid, uns
 // One polygon's contribution pass: lane l owns edges l, l + 32, ... and adds its values in that order. Each lane collects its
 // edge's split points and coincident intervals; the segments are then taken in step, the k-th of every edge at once,
 // and their inside tests by the whole warp, one after the other. Returns false when an edge's split points reach the
-// number that is kept (which of them are kept depends on the order in which they are met).
+// number that is kept (SWEEP: never; the edge is swept).
 // Edges with no edge of the other polygon within 2 tol have one segment and no cut. Two of them that share an end
 // point are connected by a path that keeps at least 2 tol away from the other polygon, so their midpoints lie on the same side of it: a run
 // of such edges takes one test. (The crossing-parity test returns the true side for points this far from the boundary:
 // its orientation signs can only be wrong for points within rounding, ~1e-7 of tol, of an edge's line.) tol below
 // 1e-12 of the overlap box (a caller's own tolerances) turns the sharing off.
-template <bool S32, bool SELF, bool AREA, bool REL, class Q, class EL>
+template <bool S32, bool SELF, bool AREA, bool REL, bool SWEEP, class Q, class EL>
 __device__ __forceinline__ bool edge_pass(const EL& LS, int nself, const EL& LO, int nother, const CutLists<Q>& cl, const uint32_t* head, const uint32_t* cand,
                                           bool inc, const PairGeo& G, bool share, int lane, double& s2, double& lin, double& lon, uint32_t& bits,
                                           double* rec) {
@@ -821,8 +836,8 @@ __device__ __forceinline__ bool edge_pass(const EL& LS, int nself, const EL& LO,
     const int i = ic + lane;
     EdgeRef e;
     EdgeCuts C;
-    edge_cuts<REL>(e, C, LS, i, i < nself, LO, cl, head, SELF);
-    if (__any_sync(0xffffffffu, C.ns == MAXS)) return false;
+    edge_cuts<REL, SWEEP>(e, C, LS, i, i < nself, LO, nother, cl, head, SELF, false, G);
+    if (!SWEEP && __any_sync(0xffffffffu, C.ns == MAXS)) return false;
     if (e.len2 == 0) C.ns = 0;
     const bool lens = REL && !(e.fl & 1u);
     unsigned link = 0;
@@ -848,14 +863,15 @@ __device__ __forceinline__ bool edge_pass(const EL& LS, int nself, const EL& LO,
 // instruction-cache room.
 enum Want { W_FLAG = 0, W_AREA = 1, W_REL = 2, W_ALL = 3 };
 
-// One pair by one warp from shared memory. Returns false (nothing written) when a local list exceeded cap or the split
-// points the room kept for them.
+// One pair by one warp from shared memory. DONE, or, with nothing written, LONG: a local list exceeded cap or the cuts the
+// room kept for them; SPLIT (not with SWEEP): an edge has more split points than are kept.
 // SELF (> 0): the pair is a geometry with itself in one layer; the caller passes one list of up to SELF edges as both LA and LB. B's
 // gather and B's contribution pass would repeat A's exactly (the same edges in the same frame, the same cuts in the same
 // order, so the same values): A's pass runs once and each lane adds its recorded values a second time, in the same
 // order, which is the sum the two passes make. Every edge meets itself, so the contact needs no test.
-template <bool S32, int SELF, int W>
-__device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList8 LA, EList8 LB, int cap, int lane,
+enum Done { LONG = 0, DONE = 1, SPLIT = 2 };
+template <bool S32, int SELF, int W, bool SWEEP = false>
+__device__ Done refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList8 LA, EList8 LB, int cap, int lane,
                               uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const CutLists<uint16_t>& cl, unsigned long long* ep) {
   constexpr int MS = SELF ? SELF : CAP_F;   // row stride of the masks
   constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
@@ -870,7 +886,7 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
     if (side) { nb = n; inB_c = in; } else { na = n; inA_c = in; }
   }
   if constexpr (SELF > 0) { nb = na; inB_c = inA_c; }
-  if (na > cap || nb > cap) return false;
+  if (na > cap || nb > cap) return LONG;
   __syncwarp();
   bool hit = false, hit_any = false;
   Nodes nd{0, false};
@@ -883,7 +899,7 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
 #pragma unroll 1
     for (int i = lane; i < na; i += 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
   }
-  if (nd.full) return false;
+  if (nd.full) return LONG;
   hit = __any_sync(0xffffffffu, hit);
   hit_any = __any_sync(0xffffffffu, hit_any || hit);
   const bool rtouch = hit;
@@ -896,7 +912,7 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
       const bool share = G.tol >= 1e-12 * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0);
       if constexpr (SELF > 0) {
         double rec[SELF / 32];
-        if (!edge_pass<S32, true, AREA, REL>(LA, na, LB, nb, cl, cl.headA, cl.cand, inB_c, G, false, lane, S.s2, S.ai, S.ao, bits, rec)) return false;
+        if (!edge_pass<S32, true, AREA, REL, false>(LA, na, LB, nb, cl, cl.headA, cl.cand, inB_c, G, false, lane, S.s2, S.ai, S.ao, bits, rec)) return LONG;
 #pragma unroll 1
         for (int c = 0; AREA && c * 32 < na; c++) S.s2 += rec[c];
         S.bi = S.ai; S.bo = S.ao;
@@ -904,16 +920,16 @@ __device__ bool refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
 #pragma unroll 1
         for (int pass = 0; pass < 2; pass++) {   // one inlined copy of the pass
           double lin = 0.0, lon = 0.0;   // this pass's lengths (each starts from 0, so the sums are the same)
-          if (!edge_pass<S32, false, AREA, REL>(pass ? LB : LA, pass ? nb : na, pass ? LA : LB, pass ? na : nb, cl, pass ? cl.headB : cl.headA,
-                                                cl.cand + (pass ? MS / 32 : 0), pass ? inA_c : inB_c, G, share, lane, S.s2, lin, lon, bits, nullptr))
-            return false;
+          if (!edge_pass<S32, false, AREA, REL, SWEEP>(pass ? LB : LA, pass ? nb : na, pass ? LA : LB, pass ? na : nb, cl, pass ? cl.headB : cl.headA,
+                                                       cl.cand + (pass ? MS / 32 : 0), pass ? inA_c : inB_c, G, share, lane, S.s2, lin, lon, bits, nullptr))
+            return SPLIT;
           if (pass) { S.bi = lin; S.bo = lon; } else { S.ai = lin; S.ao = lon; }
         }
       }
     }
   pair_result<AREA, REL>(S, sums, hit, rtouch, bits, o_flag, o_area, o_ev, o_evb);
   if (lane == 0) *ep += (unsigned long long)na * (unsigned long long)nb;   // local edge pairs: the refinement's work unit
-  return true;
+  return DONE;
 }
 
 // shared memory of one warp of the filtered bins: lists (one for self pairs), grid boxes, node values, heads, cand, node
@@ -955,6 +971,8 @@ template <int W> struct Cfg<true, W> {   // the flag alone needs no room for cut
   static constexpr int minb = W == W_FLAG ? 5 : 4;
 };
 
+constexpr int NSPLIT = 12;   // counter of k_refine_split's pairs, behind nheavy
+
 // S32 (filtered only): the contact test's and the gather's orientation signs through the certified FP32 filter
 template <bool F, bool S32 = false, int W = W_ALL>
 __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
@@ -980,11 +998,14 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLaye
     const uint2 pr = pairs[p];
     if (skip_self && pr.x == pr.y) return;   // a geometry with itself: the self bin's
     uint8_t f; double ar; double4 e4; uint32_t b4;
-    bool ok;
-    if constexpr (F) ok = refine_pair_m<S32, 0, W>(P, R, pr.x, pr.y, rp, MA, MB, bin_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
-    else ok = refine_pair_t<false>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &s_ep[wib]);
+    Done d;
+    if constexpr (F) d = refine_pair_m<S32, 0, W>(P, R, pr.x, pr.y, rp, MA, MB, bin_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
+    else d = refine_pair_t<false>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &s_ep[wib]) ? DONE : LONG;
     if (lane == 0) {
-      if (!ok) { heavy[atomicAdd(nheavy, 1ull)] = (uint32_t)p; flag[p] = 0; }
+      if (d != DONE) {   // the list's front, or its back for k_refine_split
+        heavy[d == LONG ? atomicAdd(nheavy, 1ull) : np - 1 - atomicAdd(nheavy + NSPLIT, 1ull)] = (uint32_t)p;
+        flag[p] = 0;
+      }
       else {
         flag[p] = f;
         if (area) area[p] = ar;
@@ -1010,6 +1031,44 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLaye
     for (uint64_t p = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < np; p += nw) one(p);
   }
   __syncwarp();
+  if (lane == 0 && s_ep[wib]) atomicAdd(epairs, s_ep[wib]);
+}
+
+// The pairs of the shared-memory bin with an edge of more split points than are kept (a straight edge across a stair-stepped or
+// finely divided outline): the same routine, which sweeps such an edge. By itself, because the sweep's code in the bin cost every pair
+// more than it saved these (400k-parcel relate self-join, refinement 14.7 -> 15.3-16.3 ms in six forms: instruction fetch). 20k strips
+// across outlines of 96 edges, 24 cuts on an edge, area, whole call: 20.1 ms when the scratch bin took them, 4.3 ms by the block bin,
+// 2.15 ms here. 20k strips across 600 edges with 150 cuts (the block bins sweep too): 118.9 -> 11.1 ms.
+template <bool S32, int W>
+__global__ void __launch_bounds__(RB_WARPS * 32, Cfg<true, W>::minb) k_refine_split(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np, RefineArgs rp,
+                                                                                   uint8_t* flag, double* area, double4* ev, uint32_t* evb,
+                                                                                   const uint32_t* list, const unsigned long long* nlist,
+                                                                                   unsigned long long* next, unsigned long long* epairs) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ unsigned long long s_ep[RB_WARPS];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  if (lane == 0) s_ep[wib] = 0;
+  __syncwarp();
+  EList8 LA, LB;
+  CutLists<uint16_t> cl;
+  carve_mask<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<true, W>::warp, LA, LB, cl);
+  const uint64_t n = *nlist;   // written by k_refine, launched before this kernel
+  for (;;) {
+    unsigned long long h = 0;
+    if (lane == 0) h = atomicAdd(next, 1ull);
+    h = __shfl_sync(0xffffffffu, h, 0);
+    if (h >= n) break;
+    const uint32_t p = list[np - 1 - h];
+    const uint2 pr = pairs[p];
+    uint8_t f; double ar; double4 e4; uint32_t b4;
+    refine_pair_m<S32, 0, W, true>(P, R, pr.x, pr.y, rp, LA, LB, CAP_F, lane, f, ar, e4, b4, cl, &s_ep[wib]);   // DONE: its lists fitted before
+    if (lane == 0) {
+      flag[p] = f;
+      if (area) area[p] = ar;
+      if (ev) { ev[p] = e4; evb[p] = b4; }
+    }
+    __syncwarp();
+  }
   if (lane == 0 && s_ep[wib]) atomicAdd(epairs, s_ep[wib]);
 }
 
@@ -1061,9 +1120,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
       const uint32_t p = sidx[h];
       const uint2 pr = pairs[p];
       uint8_t f; double ar; double4 e4; uint32_t b4;
-      const bool ok = refine_pair_m<S32, CAP_SELF, W>(P, P, pr.x, pr.y, rp, L, L, self_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
+      const Done d = refine_pair_m<S32, CAP_SELF, W>(P, P, pr.x, pr.y, rp, L, L, self_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
       if (lane == 0) {
-        if (!ok) { heavy[atomicAdd(nheavy, 1ull)] = p; flag[p] = 0; }
+        if (d != DONE) { heavy[atomicAdd(nheavy, 1ull)] = p; flag[p] = 0; }
         else {
           flag[p] = f;
           if (area) area[p] = ar;
@@ -1080,9 +1139,9 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
 // Block bin (filtered variants): the pairs the shared-memory bins hand on, a block of 4 warps per pair, lists of up to 512
 // edges a side in shared memory (54 KB a block, 4 blocks per SM). The routine is refine_pair_m's with the edges of the
 // gather, the search and the passes dealt out to the warps in chunks of 32; the sums keep their order: a lane's running sums
-// pass through shared memory from the warp of one chunk to that of the next. Larger pairs, or more than BIG_NODES cuts,
-// go on to the scratch bin; where a layer has geometries of more than 512 edges, a second form with 1024 edges a side and 8
-// warps (108 KB, 2 blocks per SM) stands between them: a pair of 700 edges took 0.4 ms by itself in the scratch bin.
+// pass through shared memory from the warp of one chunk to that of the next. Larger pairs go on to a second form with 1024
+// edges a side and 8 warps (108 KB, 2 blocks per SM), and from there to the scratch bin: a pair of 700 edges took 0.4 ms by
+// itself in the scratch bin.
 // Against the scratch bin's warp per pair with lists in global memory (10 % of the warps an SM holds, 37k instructions a
 // pair), whole refinement: two 120k layers with areas (7k such pairs) 7.82 -> 6.47 ms, 20k queries relate (3.9k) 1.70 ->
 // 1.32 ms, 100 queries (29: the latency of one pair) 0.27 -> 0.15 ms.
@@ -1177,8 +1236,8 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
       const int c = collect_block<S32, NW>(side ? B : A, G.ov, side ? LB : LA, CAP, s_cnt, G.cx, G.cy, in);
       if (side) { nb = c; inB_c = in; } else { na = c; inA_c = in; }
     }
-    bool over = na > CAP || nb > CAP;   // the same in every thread, here and below
-    bool hit = false, hit_any = false;
+    const bool over = na > CAP || nb > CAP;   // the same in every thread, as sweep
+    bool hit = false, hit_any = false, sweep = false;
     if (!over) {
       begin_pairs<CAP, false, W != W_FLAG>(LB, na, nb, G, cl, threadIdx.x, NW * 32);
       __syncthreads();
@@ -1187,7 +1246,7 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
         for (int i = threadIdx.x; i < na; i += NW * 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
       hit = __syncthreads_or(hit);
       hit_any = __syncthreads_or(hit_any || hit);
-      over = __syncthreads_or(nd.full);
+      sweep = __syncthreads_or(nd.full);
     }
     const bool rtouch = hit;
     if (!over && !hit) {   // every warp for itself, the same answer
@@ -1200,7 +1259,7 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
       if (want) {
         const bool share = G.tol >= 1e-12 * fmax(G.ov.x1 - G.ov.x0, G.ov.y1 - G.ov.y0);
 #pragma unroll 1
-        for (int pass = 0; pass < 2 && !over; pass++) {
+        for (int pass = 0; pass < 2; pass++) {
           const EList8& LS = pass ? LB : LA;
           const EList8& LO = pass ? LA : LB;
           const int nself = pass ? nb : na, nother = pass ? na : nb;
@@ -1213,12 +1272,11 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
           }
           __syncthreads();
 #pragma unroll 1
-          for (int c0 = 0; c0 * 32 < nself && !over; c0 += NW) {
+          for (int c0 = 0; c0 * 32 < nself; c0 += NW) {
             const int c = c0 + wid, i = c * 32 + lane;
             EdgeRef e;
             EdgeCuts C;
-            edge_cuts<REL>(e, C, LS, i, i < nself, LO, cl, head, self);
-            const bool full = C.ns == MAXS;
+            edge_cuts<REL, true>(e, C, LS, i, i < nself, LO, nother, cl, head, self, sweep, G);
             if (e.len2 == 0) C.ns = 0;
             const bool lens = REL && !(e.fl & 1u);
             const unsigned link = edge_links(e, i < nself, share && c * 32 < nself ? ~cand[c] : 0u, lane);
@@ -1233,9 +1291,8 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
               }
               if (inside_lanes<S32>(need, mx, my, k ? 0u : link, LO, nother, inc, G, lane)) vin |= 1u << k;
             }
-            over = __syncthreads_or(full);
 #pragma unroll 1
-            for (int w = 0; w < NW && !over; w++) {   // the chunks' terms in their order
+            for (int w = 0; w < NW; w++) {   // the chunks' terms in their order
               if (w == wid && c * 32 < nself) {
                 double acc = 0.0, lin = sums[32 + lane], lon = sums[64 + lane];
 #pragma unroll 1
@@ -1366,6 +1423,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
     GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
     if (F) {
       GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG)));
+      if (W != W_FLAG) GSJ_CK(cudaFuncSetAttribute(k_refine_split<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
       GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG2)));
     }
     c->refine_attr |= bit;
@@ -1388,17 +1446,18 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   } else {
     blocks = (int)std::min<uint64_t>((np + RB_WARPS - 1) / RB_WARPS, (uint64_t)c->sm_count * 8);
   }
-  // plain: a pair can only be oversized when one of its polygons has more edges than the bin holds. The filtered bins hand
-  // oversized pairs, and the rare ones whose cuts they cannot keep, to the block bin, and that bin to the scratch bin
-  // (the full number of warps only where a geometry can have more edges than the block bin holds)
+  // The filtered bins of a warp per pair hand pairs with more local edges a side than they hold, or more cuts than they have room for, to the
+  // block bin, and that bin pairs with more local edges to the next: the bins that no geometry of the layers can need are not
+  // launched (stage: 0 - 2, how many behind the first block bin; plain: behind the shared-memory bin).
   const uint32_t most = std::max(P->max_geom_edges, R->max_geom_edges);
-  const bool big = most > (uint32_t)(F ? CAP_BIG2 : bin_cap), scr = F || big, two = F && most > (uint32_t)CAP_BIG;
+  const bool two = F && most > (uint32_t)CAP_BIG, scr = most > (uint32_t)(F ? CAP_BIG2 : bin_cap), spl = F && W != W_FLAG;
+  const int stage = (two ? 1 : 0) + (scr ? 1 : 0);
   uint32_t* heavy2 = F ? c->heavy2.as<uint32_t>(np) : heavy;   // a pair leaves a bin's list before the next bin runs: the third list is the first's memory
   const ScratchGeom sg = scratch_geom<F>(P, R);
   int sblocks = 0;
   unsigned char* sbuf = nullptr;
   if (scr) {   // warps: the shape's share of every SM, at most one per pair and at most 1 GiB of lists
-    uint64_t nwarps = std::min<uint64_t>((uint64_t)c->sm_count * (big ? sh.scratch_wpsm : 1), std::max<uint64_t>(1, (1ull << 30) / sg.per));
+    uint64_t nwarps = std::min<uint64_t>((uint64_t)c->sm_count * sh.scratch_wpsm, std::max<uint64_t>(1, (1ull << 30) / sg.per));
     nwarps = std::min<uint64_t>(nwarps, np);
     nwarps = (nwarps + 3) / 4 * 4;
     sblocks = (int)(nwarps / 4);
@@ -1428,17 +1487,19 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   unsigned long long* h = c->h_refine.as<unsigned long long>(4);
   // counters: [0] oversized pairs, [1] error word, [2] pair counter, [3] local edge pairs, [4] scratch pair counter,
   // [5] self pairs, [6] self pair counter, [7] the block bin's oversized pairs, [8] block pair counter,
-  // [REFINE_ROWS] the caller's, set to 0 here, [10], [11] as [7], [8] of the second block bin
+  // [REFINE_ROWS] the caller's, set to 0 here, [10], [11] as [7], [8] of the second block bin, [NSPLIT] pairs with an edge of
+  // many split points, [NSPLIT + 1] counter of these
   auto a_main = kernel_args(k_refine<F, S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr, ctr + 2, ctr + 3, run, runs, bin_cap,
                             self ? 1 : 0);
   auto a_big = kernel_args(k_refine_block<S32, W, CAP_BIG>, P->d, R->d, pairs, heavy, ctr, rp, flag, area, ev, evb, heavy2, ctr + 7, ctr + 8, ctr + 3, P == R);
   auto a_big2 = kernel_args(k_refine_block<S32, W, CAP_BIG2>, P->d, R->d, pairs, heavy2, ctr + 7, rp, flag, area, ev, evb, heavy, ctr + 10, ctr + 11, ctr + 3,
                             P == R);
-  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, F && !two ? heavy2 : heavy, two ? ctr + 10 : F ? ctr + 7 : ctr, rp, flag, area, ev, evb, sbuf,
-                           sg.cap, sg.cph, err, ctr + 3, ctr + 4, P == R ? 1 : 0);
+  auto a_scr = kernel_args(k_refine_scratch<F>, P->d, R->d, pairs, heavy, F ? ctr + 10 : ctr, rp, flag, area, ev, evb, sbuf, sg.cap, sg.cph, err, ctr + 3, ctr + 4,
+                           P == R ? 1 : 0);
   auto a_idx = kernel_args(k_self_index, pairs, np, sidx, ctr + 5);
   auto a_self = kernel_args(k_refine_self<S32, W>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
-  cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{}, kb2{};
+  auto a_split = kernel_args(k_refine_split<S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr + NSPLIT, ctr + NSPLIT + 1, ctr + 3);
+  cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{}, kb2{}, kp{};
   kb.func = (void*)k_refine_block<S32, W, CAP_BIG>;
   kb.gridDim = dim3((unsigned)std::min<uint64_t>(np, (uint64_t)c->sm_count * 4));
   kb.blockDim = dim3(block_warps(CAP_BIG) * 32);
@@ -1455,6 +1516,10 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   km.blockDim = dim3(RB_WARPS * 32);
   km.sharedMemBytes = (unsigned)Cfg<F, W>::smem;
   km.kernelParams = a_main.ptr;
+  kp = km;
+  kp.func = (void*)k_refine_split<S32, W>;
+  kp.gridDim = dim3((unsigned)std::min<uint64_t>((np + RB_WARPS - 1) / RB_WARPS, (uint64_t)c->sm_count * Cfg<F, W>::minb));
+  kp.kernelParams = a_split.ptr;
   ks.func = (void*)k_refine_scratch<F>;
   ks.gridDim = dim3(std::max(sblocks, 1));
   ks.blockDim = dim3(128);
@@ -1468,11 +1533,12 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   kf.blockDim = dim3(RB_WARPS * 32);
   kf.sharedMemBytes = (unsigned)SELF_SMEM;
   kf.kernelParams = a_self.ptr;
-  RefineGraph& g = c->rgraph[variant * 4 + (F ? two : scr) * 2 + (self ? 1 : 0)];
+  RefineGraph& g = c->rgraph[variant * 6 + stage * 2 + (self ? 1 : 0)];
   if (!g.exec) {   // the graph is kept with its executable: the node handles used for the updates belong to it
     if (!g.graph) {
       GSJ_CK(cudaGraphCreate(&g.graph, 0));
-      // shared-memory bin || (self index -> self bin), then the block bin after both, then the scratch bin
+      // shared-memory bin || (self index -> self bin), then the block bins after both, then the scratch bin; beside these the pairs
+      // with an edge of many split points
       GSJ_CK(cudaGraphAddKernelNode(&g.n_main, g.graph, nullptr, 0, &km));
       std::vector<cudaGraphNode_t> before{g.n_main};
       if (self) {
@@ -1480,13 +1546,14 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
         GSJ_CK(cudaGraphAddKernelNode(&g.n_self, g.graph, &g.n_idx, 1, &kf));
         before.push_back(g.n_self);
       }
+      if (spl) GSJ_CK(cudaGraphAddKernelNode(&g.n_split, g.graph, &g.n_main, 1, &kp));
       if (F) {
         GSJ_CK(cudaGraphAddKernelNode(&g.n_big, g.graph, before.data(), before.size(), &kb));
         before.assign(1, g.n_big);
-        if (two) {
-          GSJ_CK(cudaGraphAddKernelNode(&g.n_big2, g.graph, before.data(), 1, &kb2));
-          before.assign(1, g.n_big2);
-        }
+      }
+      if (two) {
+        GSJ_CK(cudaGraphAddKernelNode(&g.n_big2, g.graph, before.data(), 1, &kb2));
+        before.assign(1, g.n_big2);
       }
       if (scr) GSJ_CK(cudaGraphAddKernelNode(&g.n_scr, g.graph, before.data(), before.size(), &ks));
     }
@@ -1497,13 +1564,14 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
       GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_idx, &ki));
       GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_self, &kf));
     }
+    if (spl) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_split, &kp));
     if (F) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big, &kb));
     if (two) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_big2, &kb2));
     if (scr) GSJ_CK(cudaGraphExecKernelNodeSetParams(g.exec, g.n_scr, &ks));
   }
-  GSJ_CK(cudaMemsetAsync(ctr, 0, 12 * sizeof(unsigned long long), s));
+  GSJ_CK(cudaMemsetAsync(ctr, 0, 14 * sizeof(unsigned long long), s));
   GSJ_CK(cudaGraphLaunch(g.exec, s));
-  c->launches += 1 + (F ? 1 : 0) + (two ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
+  c->launches += 1 + (F ? 1 : 0) + (spl ? 1 : 0) + (two ? 1 : 0) + (scr ? 1 : 0) + (self ? 2 : 0);
   GSJ_CK(cudaMemcpyAsync(h, ctr, 32, cudaMemcpyDeviceToHost, s));
   c->refine_pending = true;
 }

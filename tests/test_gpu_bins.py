@@ -30,6 +30,11 @@ def ngon(n, r, cx=0.0, cy=0.0):
     return p + p[:1]
 
 
+def fine(n):
+    """A square whose lower side is divided into n edges."""
+    return [(S * k / n, 0.0) for k in range(n)] + [(S, 0.0), (S, S), (0.0, S), (0.0, 0.0)]
+
+
 SHAPES = {
     # a bar across every tooth: 2 x teeth splits on its long edges (an edge keeps 22 beside its ends)
     **{f"bar_{n}": ([[comb(n, 40 * S, 4 * S)]], [[[(-S, 2 * S), (41 * S, 2 * S), (41 * S, 2.5 * S), (-S, 2.5 * S), (-S, 2 * S)]]]) for n in (10, 11, 12, 28, 100, 200)},
@@ -37,6 +42,10 @@ SHAPES = {
     "combs_9": ([[comb(9, 10 * S, 10 * S)]], [[comb(9, 10 * S, 10 * S, flip=True)]]),
     "combs_28": ([[comb(28, 10 * S, 10 * S)]], [[comb(28, 10 * S, 10 * S, flip=True)]]),
     "combs_60": ([[comb(60, 10 * S, 10 * S)]], [[comb(60, 10 * S, 10 * S, flip=True)]]),
+    # a whole side against one divided into n: coincident edges beyond the 8 that an edge keeps, and 2 (n - 1) splits
+    **{f"fine_{n}": ([[fine(n)]], [[square(0, -S, S)], [square(0, -0.5 * S, S)]]) for n in (7, 8, 9, 11, 12, 13, 40, 120, 300, 700)},
+    # more cuts than the block bins' lists hold
+    "combs_130": ([[comb(130, 10 * S, 10 * S)]], [[comb(130, 10 * S, 10 * S, flip=True)]]),
     # level neighbours: the overlap box is as thin as its pad
     "touch": ([[square(0, 0, S)]], [[square(0, S, S)], [square(S, S, S)]]),
     "twins": ([[square(0, 0, S)], [comb(9, S, S)]], [[square(0, 0, S)], [comb(9, S, S)]]),
@@ -64,6 +73,16 @@ def test_handed_on_pairs(engine, name, area, relate):
             assert np.array_equal(gp, p)
             assert not area or np.array_equal(ga, oa)
             assert not relate or np.array_equal(gc, oc)
+
+
+@pytest.mark.parametrize("name", [k for k in sorted(SHAPES) if k[:4] in ("bar_", "fine") and int(k.split("_")[1]) < 29])
+@pytest.mark.parametrize("area,relate", [(1, 0), (0, 1), (1, 1)])
+def test_many_cuts_stay(engine, name, area, relate):
+    """However often an edge is cut: pairs whose lists fit are not handed to the bins for larger ones."""
+    lp, lr = (engine.upload_polygons(make_set(g)) for g in SHAPES[name])
+    for a, b in ((lp, lr), (lr, lp)):
+        for m in MODES[1:]:
+            assert engine.join(a, b, want_area=bool(area), want_relate=bool(relate), refine_mode=m).stats["heavy"] == 0
 
 
 @pytest.mark.parametrize("tol", [0.0, 1e-11, 1e-7])
