@@ -200,8 +200,10 @@ int gsj_refine_pairs_noalloc(gsj_ctx* ctx, const gsj_layer* P, const gsj_layer* 
 /* Launch shape of the refinement's size bins, per context. No counterpart in the reference (its k_refine takes a
  * fixed grid, engine.cuh:963-975). Pairs whose local edge lists fit bin_edges per side run in the shared-memory bin
  * (a warp per pair, warps taking `run` consecutive pairs per fetch, at most `runs` fetches each); the others a block per
- * pair (filtered variants, up to 1024 edges per side) or in the global-scratch bin with scratch_warps_per_sm warps per SM. Every shape gives the same results, bit for bit; only
- * the time changes. Defaults: 4, 32, 128, 32. */
+ * pair (filtered variants, up to 1024 edges per side) or in the global-scratch bin with scratch_warps_per_sm warps per
+ * SM. So scratch_warps_per_sm has an effect only where a geometry of the layers has more than 1024 edges (plain:
+ * more than bin_edges); elsewhere the autotuner leaves it as it is. Every shape gives the same results, bit for bit;
+ * only the time changes. Defaults: 4, 32, 128, 32. */
 typedef struct gsj_refine_shape {
   int run;                   /* 1 - 64 */
   int runs;                  /* 1 - 4096 */

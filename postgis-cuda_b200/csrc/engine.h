@@ -122,13 +122,13 @@ KernelArgs<A...> kernel_args(void (*)(A...), V&&... v) {
   return KernelArgs<A...>(static_cast<A>(v)...);
 }
 
-// Launch shape of the refinement's two size bins (set by gsj_set_refine_shape or chosen by gsj_tune_refine):
+// Launch shape of the refinement's size bins (set by gsj_set_refine_shape or chosen by gsj_tune_refine):
 // run / runs = consecutive pairs a warp of the shared-memory bin takes per fetch / fetches per warp (grid size);
 // bin_cap = local edges per side up to which a pair stays in the shared-memory bin (at most its list capacity);
-// scratch_wpsm = warps per SM of the global-scratch bin.
+// scratch_wpsm = warps per SM of the global-scratch bin (launched where uses_scratch_bin).
 struct RefineShape { int run = 4, runs = 32, bin_cap = 128, scratch_wpsm = 32; };
-// The refinement's bins as one CUDA graph per variant (shared-memory bin, then scratch bin), instantiated once per
-// context and re-parameterised per call.
+// The refinement's bins as one CUDA graph per variant (shared-memory bins, then block bins, then scratch bin), instantiated
+// once per context and re-parameterised per call.
 struct RefineGraph {
   cudaGraph_t graph = nullptr; cudaGraphExec_t exec = nullptr;
   cudaGraphNode_t n_main = nullptr, n_scr = nullptr, n_idx = nullptr, n_self = nullptr, n_split = nullptr, n_big = nullptr, n_big2 = nullptr;
@@ -195,6 +195,7 @@ uint64_t refine(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2*
 // caller reads the outputs of pairs with flag 1 alone (flag 2 then counts as 0)
 void refine_enqueue(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, int mode,
                     uint8_t* flag, double* area, double4* ev, uint32_t* evb, bool hits_only = false);
+bool uses_scratch_bin(int mode, uint32_t most, int bin_cap);
 constexpr int REFINE_ROWS = 9;   // a word of c->counters that refine_enqueue sets to 0 and does not use
 uint64_t refine_result(gsj_ctx* c);
 

@@ -1397,6 +1397,9 @@ __global__ void __launch_bounds__(128) k_refine_scratch(DLayer P, DLayer R, cons
   if (lane == 0 && ep) atomicAdd(epairs, ep);
 }
 
+// whether a join of layers whose largest geometry has `most` edges has pairs for the scratch bin (and its launch shape any effect)
+bool uses_scratch_bin(int mode, uint32_t most, int bin_cap) { return most > (uint32_t)(mode == GSJ_REFINE_PLAIN ? bin_cap : CAP_BIG2); }
+
 // Scratch-bin layout for a layer pair: list capacity (rounded to 8 edges, which keeps every double array of the slab
 // 8-byte aligned), candidate entries (indices stay below 2^16) and bytes per warp.
 struct ScratchGeom { int cap, cph; size_t per; };
@@ -1450,7 +1453,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   // block bin, and that bin pairs with more local edges to the next: the bins that no geometry of the layers can need are not
   // launched (stage: 0 - 2, how many behind the first block bin; plain: behind the shared-memory bin).
   const uint32_t most = std::max(P->max_geom_edges, R->max_geom_edges);
-  const bool two = F && most > (uint32_t)CAP_BIG, scr = most > (uint32_t)(F ? CAP_BIG2 : bin_cap), spl = F && W != W_FLAG;
+  const bool two = F && most > (uint32_t)CAP_BIG, scr = uses_scratch_bin(F ? GSJ_REFINE_FILTERED : GSJ_REFINE_PLAIN, most, bin_cap), spl = F && W != W_FLAG;
   const int stage = (two ? 1 : 0) + (scr ? 1 : 0);
   uint32_t* heavy2 = F ? c->heavy2.as<uint32_t>(np) : heavy;   // a pair leaves a bin's list before the next bin runs: the third list is the first's memory
   const ScratchGeom sg = scratch_geom<F>(P, R);

@@ -124,7 +124,7 @@ void tune_refine(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const Refin
       if (field == 0) { if (mode == GSJ_REFINE_PLAIN) continue; vals = {1, 2, 4, 8, 16}; }
       if (field == 1) { if (mode == GSJ_REFINE_PLAIN) continue; vals = {8, 16, 32, 64, 128, 512, 4096}; }
       if (field == 2) vals = {32, 64, 96, 128};
-      if (field == 3) { if (maxe <= (uint32_t)best.bin_cap) continue; vals = {8, 16, 32, 48}; }
+      if (field == 3) { if (!uses_scratch_bin(mode, maxe, best.bin_cap)) continue; vals = {8, 16, 32, 48}; }
       const RefineShape base = best;
       for (int v : vals) {
         RefineShape sh = base;

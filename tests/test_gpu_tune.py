@@ -93,6 +93,17 @@ def test_tuner_small_sample_takes_every_pair(shaped, layers):
     assert t["sample_pairs"] == nc
 
 
+@pytest.mark.parametrize("mode", MODES)
+def test_tuner_times_only_what_has_an_effect(shaped, layers, mode):
+    """The scratch bin's warps are a choice only where a geometry is too large for the bins before it."""
+    plain = mode == gsj.GSJ_REFINE_PLAIN
+    big = shaped.upload_polygons(gen.voronoi(40, gen.LA_BOX, 3, vmin=1100, vmax=1500))
+    for P, scratch in ((layers["zonesA"][0], False), (layers["parcels"][0], plain), (big, True)):
+        t = shaped.tune_refine(P, P, max_pairs=2000, refine_mode=mode, keep=("run", "runs", "bin_edges"))
+        assert (t["shapes_tried"] > 1) == scratch
+        assert scratch or t["best"] == shaped.refine_shape
+
+
 def test_tuner_keeps_named_fields(shaped, layers):
     P = layers["parcels"][0]
     shaped.refine_shape = {"runs": 16, "run": 2}
