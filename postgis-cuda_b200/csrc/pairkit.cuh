@@ -110,8 +110,7 @@ static __device__ bool pip_full_warp(const Frame& B, double mx, double my, int l
 }
 
 // inside(x) = inside(c) xor crossings of c -> x with the local edges (engine.cuh:400-412)
-// S32: the four orientation signs through the certified FP32 filter (the same booleans)
-template <bool F, bool S32 = false, class EL>
+template <bool F, class EL>
 __device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, double cy, bool in_c, double x, double y) {
   bool in = in_c;
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);
@@ -119,17 +118,10 @@ __device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, d
     const double ex0 = L.x0[k], ey0 = L.y0[k], ex1 = L.x1[k], ey1 = L.y1[k];
     if (F ? out_cmp(ex0, ey0, ex1, ey1, sx0, sy0, sx1, sy1)
           : (fmax(ex0, ex1) < sx0 || fmin(ex0, ex1) > sx1 || fmax(ey0, ey1) < sy0 || fmin(ey0, ey1) > sy1)) return false;
-    if constexpr (S32) {
-      const bool sc = left_of32(ex0, ey0, ex1, ey1, cx, cy), sx = left_of32(ex0, ey0, ex1, ey1, x, y);
-      if (sc == sx) return false;
-      const bool su = orient_sign32(cx, cy, x, y, ex0, ey0) > 0, sv = orient_sign32(cx, cy, x, y, ex1, ey1) > 0;
-      if (su != sv) in = !in;
-    } else {
-      bool sc = left_of(ex0, ey0, ex1, ey1, cx, cy), sx = left_of(ex0, ey0, ex1, ey1, x, y);
-      if (sc == sx) return false;
-      bool su = orient(cx, cy, x, y, ex0, ey0) > 0, sv = orient(cx, cy, x, y, ex1, ey1) > 0;
-      if (su != sv) in = !in;
-    }
+    bool sc = left_of(ex0, ey0, ex1, ey1, cx, cy), sx = left_of(ex0, ey0, ex1, ey1, x, y);
+    if (sc == sx) return false;
+    bool su = orient(cx, cy, x, y, ex0, ey0) > 0, sv = orient(cx, cy, x, y, ex1, ey1) > 0;
+    if (su != sv) in = !in;
     return false;
   };
 #pragma unroll 1
@@ -138,7 +130,8 @@ __device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, d
 }
 
 // The same parity for one query point shared by the whole warp: lanes split the edges, a ballot counts crossings
-// (the parity does not depend on the order of the edges).
+// (the parity does not depend on the order of the edges). S32: the four orientation signs through the certified FP32 filter (the same
+// booleans).
 template <bool S32 = false, class EL>
 static __device__ bool inside_from_c_warp(const EL& L, int cnt, double cx, double cy, bool in_c, double x, double y, int lane) {
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);

@@ -596,7 +596,8 @@ struct Nodes { int n; bool full; };   // nodes in use (a warp's own lists; a blo
 // of the pair, behind the same box test), and for either edge what edge_visit finds for it: coincidence (a bit in the
 // masks) or a split point. The two edges' conditions are the same but for their box tests, the order of a product and
 // the end tolerances; r, tn and un change sign together when the edges swap roles, so un / r is B's parameter.
-template <bool SELF, bool CUTS, int SH, class Q, class EL>
+// S32: the contact's signs through the FP32 filter where the contact is all that is wanted; cuts need the orientations' values.
+template <bool S32, bool SELF, bool CUTS, int SH, class Q, class EL>
 __device__ __forceinline__ void classify_pairs(const EL& LA, const EL& LB, const PairGeo& G, const CutLists<Q>& cl, uint32_t e, bool act, int lane, Nodes& nd,
                                                bool& hit, bool& hit_any) {
   const int i = (int)(e >> SH), j = (int)(e & ((1u << SH) - 1u));
@@ -611,7 +612,9 @@ __device__ __forceinline__ void classify_pairs(const EL& LA, const EL& LB, const
     const double ax0 = px < qx ? px : qx, ax1 = px < qx ? qx : px, ay0 = py < qy ? py : qy, ay1 = py < qy ? qy : py;
     const double bx0 = ex0 < ex1 ? ex0 : ex1, bx1 = ex0 < ex1 ? ex1 : ex0, by0 = ey0 < ey1 ? ey0 : ey1, by1 = ey0 < ey1 ? ey1 : ey0;
     const bool near = !(bx1 < ax0 || bx0 > ax1 || by1 < ay0 || by0 > ay1);
-    if (!SELF && near) {
+    if (S32 && !CUTS) {
+      if (near && seg_isect32(px, py, qx, qy, ex0, ey0, ex1, ey1)) { hit_any = true; if (!((fa | fb) & 1u)) hit = true; }
+    } else if (!SELF && near) {
       bool is = ((g0 > 0 && g1 < 0) || (g0 < 0 && g1 > 0)) && ((c0 > 0 && c1 < 0) || (c0 < 0 && c1 > 0));
       is = is || (g0 == 0 && px >= bx0 && px <= bx1 && py >= by0 && py <= by1) || (g1 == 0 && qx >= bx0 && qx <= bx1 && qy >= by0 && qy <= by1) ||
            (c0 == 0 && ex0 >= ax0 && ex0 <= ax1 && ey0 >= ay0 && ey0 <= ay1) || (c1 == 0 && ex1 >= ax0 && ex1 <= ax1 && ey1 >= ay0 && ey1 <= ay1);
@@ -699,7 +702,7 @@ __device__ __forceinline__ void edge_cover(EdgeCuts& C, const EdgeRef& e, const 
 // Candidate edge pairs (boxes within 2 tol of each other, or a little more on the grid) found and classified; CUTS: the cuts
 // are wanted, else the contact alone (the search then ends at the first real one). SELF: only j > i is searched (an edge
 // always coincides with itself); self: a geometry with itself searched in full, less each edge with itself. One warp takes the 32 A edges from ic0 on, then those from ic0 + step on, ...
-template <int MS, bool SELF, bool CUTS, int SH, class Q, class EL>
+template <bool S32, int MS, bool SELF, bool CUTS, int SH, class Q, class EL>
 __device__ Nodes find_pairs(const EL& LA, int na, const EL& LB, int nb, const PairGeo& G, const CutLists<Q>& cl, int ic0, int step, int lane, bool& hit,
                             bool& hit_any, bool self = false) {
   Nodes nd{0, false};
@@ -721,7 +724,7 @@ __device__ Nodes find_pairs(const EL& LA, int na, const EL& LB, int nb, const Pa
         }
       },
       [&](uint32_t e, bool act) {
-        classify_pairs<SELF, CUTS, SH>(LA, LB, G, cl, e, act && !(self && (e >> SH) == (e & ((1u << SH) - 1u))), lane, nd, hit, hit_any);
+        classify_pairs<S32, SELF, CUTS, SH>(LA, LB, G, cl, e, act && !(self && (e >> SH) == (e & ((1u << SH) - 1u))), lane, nd, hit, hit_any);
         return !CUTS && __any_sync(0xffffffffu, hit);
       });
   return nd;
@@ -893,7 +896,7 @@ __device__ Done refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
   if constexpr (SELF == 0 || W != W_FLAG) {
     begin_pairs<MS, (SELF > 0), W != W_FLAG>(LB, na, nb, G, cl, lane, 32);
     __syncwarp();
-    nd = find_pairs<MS, (SELF > 0), W != W_FLAG, 8>(LA, na, LB, nb, G, cl, 0, 32, lane, hit, hit_any);
+    nd = find_pairs<S32, MS, (SELF > 0), W != W_FLAG, 8>(LA, na, LB, nb, G, cl, 0, 32, lane, hit, hit_any);
   }
   if constexpr (SELF > 0) {
 #pragma unroll 1
@@ -973,7 +976,8 @@ template <int W> struct Cfg<true, W> {   // the flag alone needs no room for cut
 
 constexpr int NSPLIT = 12;   // counter of k_refine_split's pairs, behind nheavy
 
-// S32 (filtered only): the contact test's and the gather's orientation signs through the certified FP32 filter
+// S32 (filtered only): the orientation signs of the gather's parity, of the inside tests and, for the flag alone, of the contact test
+// through the certified FP32 filter
 template <bool F, bool S32 = false, int W = W_ALL>
 __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLayer P, DLayer R, const uint2* __restrict__ pairs, uint64_t np,
                                                                         RefineArgs rp, uint8_t* flag, double* area, double4* ev, uint32_t* evb,
@@ -1241,7 +1245,7 @@ __global__ void __launch_bounds__(block_warps(CAP) * 32, 16 / block_warps(CAP)) 
     if (!over) {
       begin_pairs<CAP, false, W != W_FLAG>(LB, na, nb, G, cl, threadIdx.x, NW * 32);
       __syncthreads();
-      const Nodes nd = find_pairs<CAP, false, W != W_FLAG, 16>(LA, na, LB, nb, G, cl, wid * 32, NW * 32, lane, hit, hit_any, self);
+      const Nodes nd = find_pairs<S32, CAP, false, W != W_FLAG, 16>(LA, na, LB, nb, G, cl, wid * 32, NW * 32, lane, hit, hit_any, self);
       if (self)
         for (int i = threadIdx.x; i < na; i += NW * 32) { hit_any = true; if (!(LA.fl[i] & 1u)) hit = true; }
       hit = __syncthreads_or(hit);
