@@ -123,13 +123,37 @@ def test_every_row_arrives(engine, n):
     assert np.array_equal(engine.cluster(la)[0], np.arange(n, dtype=np.uint32))
 
 
-def test_unfolded_pieces_relate(engine):
+def de9im(ev, bits, la, lb):
+    """DE-9IM codes from boundary evidence (lengths of A inside / on B, of B inside / on A) and the whole lengths."""
+    a_in, a_out = ev[:, 0] > 1e-9 * la, la - ev[:, 0] - ev[:, 1] > 1e-9 * la
+    b_in, b_out = ev[:, 2] > 1e-9 * lb, lb - ev[:, 2] - ev[:, 3] > 1e-9 * lb
+    same, opp, touch = (bits & 1) != 0, (bits & 2) != 0, (bits & 4) != 0
+    cells = [3 * (a_in | b_in | same), 2 * b_in, 3 * (a_out | b_in | opp),
+             2 * a_in, np.where(same | opp, 2, touch), 2 * a_out,
+             3 * (b_out | a_in | opp), 2 * b_out, 3]
+    return sum(np.asarray(c, np.uint32) << (2 * k) for k, c in enumerate(cells))
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("maxv,differ", [(12, 4), (64, 92)])
+def test_unfolded_pieces_relate(engine, maxv, differ, mode):
     """no_agg on subdivided layers: piece pairs, whose boundary lengths are their parents' (kept per parent, not per piece)."""
     from gsj import gen
-    P = engine.subdivide(gen.layer_parcels(300, (-118.30, 33.95, -118.29, 33.96), seed=5), 12)
-    lp = engine.upload_polygons(P)
-    assert P.n > P.parent.max() + 1
-    got = [rows(engine.join(lp, lp, want_area=False, want_relate=True, no_agg=True, refine_mode=m)) for m in MODES]
-    assert got[0][0].max() == P.n - 1
-    for p, _, c in got[1:]:
-        assert np.array_equal(p, got[0][0]) and np.array_equal(c, got[0][2])
+    P = engine.subdivide(gen.layer_parcels(300, (-118.30, 33.95, -118.29, 33.96), seed=5), maxv)
+    lp, op = engine.upload_polygons(P), O.OSet(P)
+    p, _, code = rows(engine.join(lp, lp, want_area=False, want_relate=True, no_agg=True, refine_mode=mode))
+    cand = O.candidates(op, op)
+    flag, _, ev, bits = O.refine_pairs(op, op, cand, O.params(0, 1))
+    i = np.lexsort((cand[:, 1], cand[:, 0]))
+    i = i[flag[i] == 1]
+    ev, bits = ev[i], bits[i]
+    assert P.n > P.parent.max() + 1 and np.array_equal(p, cand[i])
+    # boundary lengths: the real edges of all pieces of a parent
+    d = np.hypot(*np.diff(P.xy, axis=0).T) * (P.syn[:-1] == 0)
+    d[P.rvo[1:-1].astype(np.int64) - 1] = 0   # from one ring's end to the next one's start: no edge
+    v0 = P.rvo[P.gro.astype(np.int64)].astype(np.int64)
+    length = np.bincount(P.parent, [d[a:b - 1].sum() for a, b in zip(v0, v0[1:])])
+    assert np.array_equal(code, de9im(ev, bits, length[P.parent[p[:, 0]]], length[P.parent[p[:, 1]]]))
+    # ... which lengths taken by piece would not give
+    by_piece = np.resize(length, P.n)
+    assert (code != de9im(ev, bits, by_piece[p[:, 0]], by_piece[p[:, 1]])).sum() == differ
