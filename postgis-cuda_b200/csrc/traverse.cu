@@ -97,9 +97,14 @@ __global__ void __launch_bounds__(128) k_traverse(const float4* __restrict__ qbb
 }
 
 // Few probes: a warp per probe. Each lane takes one node of the probe's stack (in shared memory, newest first), so the
-// warp walks up to 32 nodes a step and the walk takes about the tree's depth in steps instead of the nodes it visits. The stack
-// grows by at most 32 a step and its top is a level deeper each time: 32 x (depth + 1) entries hold it (depth <= 64).
-constexpr int TW_WARPS = 4, TW_STACK = 32 * 66;
+// warp walks up to 32 nodes a step and the walk takes about the tree's depth in steps instead of the nodes it visits.
+// The stack: let b be the entries below the up to 32 that a step takes. None of these is above level b / 32 (whole part): it holds for the
+// root; their children are a level deeper, and the next step's b is larger by 32 at most; and what a step leaves behind at
+// place p < b' <= b + 32 is a child, at level b / 32 + 1 >= (p + 1) / 32 or deeper, so it holds as well when a later step reaches
+// down to it. The deepest internal nodes are at level 63 (unique 64-bit keys), so a step that pushes has b / 32 <= 62: never more than
+// 62 x 32 + 31 + 64 = 2079 entries.
+constexpr int TW_WARPS = 4, TW_STACK = 32 * 65;
+static_assert(TW_STACK >= 62 * 32 + 31 + 64, "the walk's bound");
 // Against the thread form, ms: 200k parcels, 100 / 1k / 10k / 20k / 40k query boxes 0.029 / 0.029 / 0.054 / 0.077 / 0.127 against
 // 0.078 / 0.090 / 0.103 / 0.103 / 0.113; 50 wide boxes over 20k zones 0.076 against 3.17 (one lane walked a whole box); a
 // tree of 50 leaves under 20k boxes 0.051 against 0.041. Hence the lines:

@@ -13,7 +13,15 @@ def boxes(n, seed, side, size):
     return make_set([[square(x, y, s)] for x, y, s in zip(r.uniform(0, side, n), r.uniform(0, side, n), r.uniform(0.2 * size, size, n))])
 
 
+def nested(n, side, f):
+    """Small boxes at distances side * f^k from a corner: the tree is a chain, then ids alone tell its leaves apart."""
+    k = np.arange(n)
+    return make_set([[square(side * f ** i, side * f ** i, 0.1 * side * f ** i + 1e-12)] for i in k])
+
+
 CASES = {
+    "chain": (boxes(5, 11, 400 * S, 400 * S), nested(3000, 400 * S, 0.97)),
+    "chain_2": (boxes(5, 11, 400 * S, 400 * S), nested(64, 400 * S, 0.5)),
     "one_leaf": (boxes(5, 1, S, S), make_set([[square(0, 0, S)]])),
     "one_probe": (make_set([[square(0, 0, 100 * S)]]), boxes(9000, 2, 100 * S, S)),      # the probe meets every leaf
     "same_boxes": (boxes(3, 3, S, S), make_set([[square(0, 0, S)]] * 3000)),             # leaves told apart by their ids alone
