@@ -5,7 +5,7 @@ import pytest
 
 import gsj
 import pyoracle as O
-from shapes import S, X0, Y0, cw, make_set
+from shapes import S, X0, Y0, cw, make_set, square
 from test_gpu_bins import comb, ngon
 
 pytestmark = pytest.mark.gpu
@@ -73,6 +73,38 @@ def test_polygons_within(engine, mode, d):
     for lr, rs, same in ((lb, b, False), (la, a, True)):
         got, want = engine.dwithin(la, lr, d, same=same, refine_mode=mode)[0], O.dwithin(O.OSet(a), O.OSet(rs), d, same=same)[0]
         assert set(map(tuple, got.tolist())) == set(map(tuple, want.tolist()))
+
+
+def fine_square(n, x0, y0, w, h):
+    """A rectangle of n edges, its sides divided evenly."""
+    c = [(x0, y0), (x0 + w, y0), (x0 + w, y0 + h), (x0, y0 + h), (x0, y0)]
+    pts = []
+    for k in range(4):
+        m = n // 4 + (k < n % 4)
+        pts += [(c[k][0] + (c[k + 1][0] - c[k][0]) * t / m, c[k][1] + (c[k + 1][1] - c[k][1]) * t / m) for t in range(m)]
+    return pts + pts[:1]
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("n,m", [(7, 128), (128, 128), (128, 129), (129, 7), (255, 255), (255, 256), (256, 256), (256, 257), (257, 5), (5, 257), (300, 600)])
+def test_polygons_within_lists(engine, n, m, mode):
+    """Lists around the sizes of the two forms (128 and 256 edges a side): a polygon of n edges in a hole of m, all of them
+    within reach up to the distance, gaps from half of it to just in and out of the band around it."""
+    w = np.sqrt(1 - 0.0066943799901413165 * np.sin(np.radians(Y0)) ** 2)
+    mx, my = 1.0 / (np.radians(6378137.0) / w * np.cos(np.radians(Y0))), 1.0 / (np.radians(6378137.0) * (1 - 0.0066943799901413165) / w ** 3)   # a metre
+    F = [0.5, 0.9, 0.999] + [1 + k * 2e-5 for k in range(-6, 7)] + [1.001]
+    A, B = [], []
+    for k, f in enumerate(F):
+        x, y, g, h = 8 * S * k, 0.0, f * D * mx, f * D * my
+        A.append([fine_square(n, x, y, S, S)])
+        B.append([square(x - S, y - S, 3 * S), cw(fine_square(m, x - g, y - h, S + 2 * g, S + 2 * h))])
+    a, b = make_set(A), make_set(B)
+    pairs, st = engine.dwithin(engine.upload_polygons(a), engine.upload_polygons(b), D, refine_mode=mode)
+    want = O.dwithin(O.OSet(a), O.OSet(b), D)[0]
+    assert set(map(tuple, pairs.tolist())) == set(map(tuple, want.tolist()))
+    assert 3 < len(want) < len(F)
+    if mode != gsj.GSJ_REFINE_PLAIN:   # to the kernel with the geodesic: pairs in the band, or all whose lists are too long
+        assert st["heavy"] >= sum(f < 1 for f in F) if max(n, m) > 256 else 0 < st["heavy"] < 13
 
 
 @pytest.mark.parametrize("mode", MODES)
