@@ -8,7 +8,7 @@ import pytest
 
 import gsj
 import pyoracle as O
-from shapes import S, make_set, square
+from shapes import S, cw, make_set, square
 
 pytestmark = pytest.mark.gpu
 MODES = [gsj.GSJ_REFINE_PLAIN, gsj.GSJ_REFINE_FILTERED, gsj.GSJ_REFINE_FILTERED_FP32]
@@ -46,6 +46,9 @@ SHAPES = {
     **{f"fine_{n}": ([[fine(n)]], [[square(0, -S, S)], [square(0, -0.5 * S, S)]]) for n in (7, 8, 9, 11, 12, 13, 40, 120, 300, 700)},
     # more cuts than the block bins' lists hold
     "combs_130": ([[comb(130, 10 * S, 10 * S)]], [[comb(130, 10 * S, 10 * S, flip=True)]]),
+    # holes and several parts, more than 1024 edges in all: global scratch
+    "parts_1200": ([[ngon(600, S), cw(ngon(300, 0.3 * S, 0.4 * S)), cw(ngon(300, 0.3 * S, -0.4 * S, 0.1 * S)), ngon(60, 0.1 * S, 0.4 * S)]],
+                   [[ngon(600, S, 0.3 * S, 0.2 * S), cw(ngon(500, 0.5 * S, 0.3 * S, 0.2 * S))], [ngon(700, 0.4 * S, 0.1 * S), ngon(400, 0.2 * S, S)]]),
     # level neighbours: the overlap box is as thin as its pad
     "touch": ([[square(0, 0, S)]], [[square(0, S, S)], [square(S, S, S)]]),
     "twins": ([[square(0, 0, S)], [comb(9, S, S)]], [[square(0, 0, S)], [comb(9, S, S)]]),
@@ -83,6 +86,28 @@ def test_many_cuts_stay(engine, name, area, relate):
     for a, b in ((lp, lr), (lr, lp)):
         for m in MODES[1:]:
             assert engine.join(a, b, want_area=bool(area), want_relate=bool(relate), refine_mode=m).stats["heavy"] == 0
+
+
+@pytest.mark.parametrize("area,relate", [(1, 0), (0, 1), (1, 1)])
+def test_large_pieces(engine, area, relate):
+    """Pieces of more than 1024 edges with cut edges among them: global scratch, folded."""
+    def wavy(n, cx):
+        t = 2 * np.pi * np.arange(n) / n
+        r = S * (1 + 0.05 * np.sin(40 * t))
+        return [*zip(cx + r * np.cos(t), r * np.sin(t)), (cx + r[0], 0.0)]
+
+    P, R = (engine.subdivide(make_set([[wavy(6000, x + dx)] for x in (0.0, 1.7 * S)]), 2400) for dx in (0.0, 0.4 * S))
+    assert np.diff(P.rvo.astype(np.int64)).max() > 1025 and P.n > 2 and P.syn.any()
+    for m in MODES:
+        for A, B, up in ((P, R, False), (P, P, True)):
+            la = engine.upload_polygons(A)
+            lb = la if B is A else engine.upload_polygons(B)
+            r = engine.join(la, lb, want_area=bool(area), want_relate=bool(relate), upper=up, refine_mode=m)
+            gp, ga, gc = rows(r)
+            p, oa, oc, _ = O.join(O.OSet(A), O.OSet(B), O.params(area, relate), upper=up)
+            assert r.stats["heavy"] > 0 and np.array_equal(gp, p)
+            assert not area or np.array_equal(ga, oa)
+            assert not relate or np.array_equal(gc, oc)
 
 
 @pytest.mark.parametrize("tol", [0.0, 1e-11, 1e-7])

@@ -1,8 +1,9 @@
 """Refinement launch shapes and the autotuner (gsj_set_refine_shape, gsj_tune_refine) on the GPU.
 
-A shape moves pairs between the two size bins (shared-memory lists up to bin_edges local edges per side, global
-scratch above) and changes how warps take pairs; it never changes a decision. So every shape must give the oracle's
-pair sets, areas and DE-9IM codes bit for bit, including shapes that send nearly every pair to the scratch bin.
+A shape moves pairs between the size bins (a warp's shared-memory lists up to bin_edges local edges per side; above,
+the filtered modes' block bins up to 1024 edges, global scratch for the rest and for the plain mode) and changes how
+warps take pairs; it never changes a decision. So every shape must give the oracle's pair sets, areas and DE-9IM codes bit
+for bit, including shapes that send nearly every pair out of the warp's bin.
 """
 import numpy as np
 import pytest
@@ -17,7 +18,7 @@ SHAPES = [
     {},                                                    # the default shape
     {"run": 1, "runs": 1},                                 # one pair per fetch, one fetch per warp: the largest grid
     {"run": 16, "runs": 4096},                             # few long-lived warps
-    {"bin_edges": 8, "scratch_warps_per_sm": 1},           # nearly every pair in the scratch bin, few scratch warps
+    {"bin_edges": 8, "scratch_warps_per_sm": 1},           # nearly every pair in the bins for larger ones, few scratch warps
     {"bin_edges": 32, "scratch_warps_per_sm": 64},
     {"run": 2, "runs": 8, "bin_edges": 96, "scratch_warps_per_sm": 8},
 ]
@@ -60,7 +61,7 @@ def test_every_shape_gives_the_oracle_rows(shaped, layers, a, b, upper, mode):
         assert np.array_equal(ga, oa), f"shape {sh}: areas differ from the oracle"
         assert np.array_equal(gc, oc), f"shape {sh}: DE-9IM codes differ from the oracle"
         heavy[str(sh)] = r.stats["heavy"]
-    # bin_edges 8 sends most contact pairs of the parcel layers to the scratch bin
+    # bin_edges 8 sends most contact pairs of the parcel layers out of the warp's bin
     if a.startswith("parcels"):
         assert heavy[str(SHAPES[3])] > 10 * max(1, heavy[str(SHAPES[0])])
 
