@@ -854,7 +854,7 @@ def main():
                    "l2": "inputs > L2 (2.2 GB resident layer)"},
         "gen_s": round(t_gen, 2),
         "refine_shape": {"filtered": tune["best"], "plain": default_shape, "autotuner": {k: tune[k] for k in ("start_ms", "best_ms", "sample_pairs", "shapes_tried")},
-                         "what": "launch shape of the refinement's two size bins; the filtered one chosen by gsj_tune_refine (untimed)"},
+                         "what": "launch shape of the refinement's size bins; the filtered one chosen by gsj_tune_refine (untimed)"},
         "latency_ms": ({"p50": serving["filtered"]["p50_ms"], "p99": serving["filtered"]["p99_ms"],
                         "plain_p50": serving["plain"]["p50_ms"], "plain_p99": serving["plain"]["p99_ms"],
                         "what": "gsjd serving the request stream, arrival to end of result stream"} if serving else None),
@@ -873,7 +873,7 @@ def main():
                              "join_and_rows_to_host": float(np.mean([b for _, b in e2e_parts])),
                              "what": "host clock: gsj_layer_upload_polygons (H2D of the arrays, device prep, LBVH), then gsj_join with the "
                                      "rows copied out of the library's pinned buffers"}},
-        "roofline": {"kernel": "k_refine<1> + k_refine_self + k_refine_scratch<1> (the refinement graph)", "bound": "fp64", "achieved": flops / (refine_ms / 1000.0) / 1e12,
+        "roofline": {"kernel": "k_refine<1> + k_refine_self + k_refine_split + k_refine_block (the refinement graph)", "bound": "fp64", "achieved": flops / (refine_ms / 1000.0) / 1e12,
                      "peak": FP64_PEAK_TFLOPS, "unit": "TFLOP/s", "frac": flops / (refine_ms / 1000.0) / 1e12 / FP64_PEAK_TFLOPS,
                      "traffic": traffic, "peak_source": "B200 FP64 specification (HGX B200: 296 TFLOPS / 8 GPUs); not measured here",
                      "work": {"edge_pairs_per_launch": edge_pairs, "flops_per_edge_pair": FLOPS_PER_EDGE_PAIR,

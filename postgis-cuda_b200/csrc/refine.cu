@@ -593,8 +593,8 @@ struct CutLists { uint2* qb; double* val; uint32_t* headA; uint32_t* headB; uint
 struct Nodes { int n; bool full; };   // nodes in use (a warp's own lists; a block counts in *count); full: some did not fit
 
 // Classifies one candidate edge pair (i of A, j of B) per lane: real / any contact (seg_isect on the four orientations
-// of the pair, behind the same box test), and for either edge what edge_visit finds for it: coincidence (a bit in the
-// masks) or a split point. The two edges' conditions are the same but for their box tests, the order of a product and
+// of the pair, behind the same box test), and for either edge what edge_visit finds for it: coincidence (a node that
+// names the edge) or a split point. The two edges' conditions are the same but for their box tests, the order of a product and
 // the end tolerances; r, tn and un change sign together when the edges swap roles, so un / r is B's parameter.
 // S32: the contact's signs through the FP32 filter where the contact is all that is wanted; cuts need the orientations' values.
 template <bool S32, bool SELF, bool CUTS, int SH, class Q, class EL>
@@ -815,7 +815,7 @@ __device__ __forceinline__ bool inside_lanes(bool need, double mx, double my, un
   }
   return need && ((in >> tester) & 1u);
 }
-// link mask of a chunk of edges (see edge_pass): fr = edges without candidates
+// links of a chunk of edges, a bit each (see edge_pass): fr = edges without candidates
 __device__ __forceinline__ unsigned edge_links(const EdgeRef& e, bool valid, unsigned fr, int lane) {
   const double prx = __shfl_up_sync(0xffffffffu, e.qx, 1), pry = __shfl_up_sync(0xffffffffu, e.qy, 1);
   return __ballot_sync(0xffffffffu, valid && lane > 0 && prx == e.px && pry == e.py) & fr & (fr << 1);
@@ -876,7 +876,7 @@ enum Done { LONG = 0, DONE = 1, SPLIT = 2 };
 template <bool S32, int SELF, int W, bool SWEEP = false>
 __device__ Done refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList8 LA, EList8 LB, int cap, int lane,
                               uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const CutLists<uint16_t>& cl, unsigned long long* ep) {
-  constexpr int MS = SELF ? SELF : CAP_F;   // row stride of the masks
+  constexpr int MS = SELF ? SELF : CAP_F;   // edges a side; B's bits of cand follow A's
   constexpr bool AREA = W == W_AREA || W == W_ALL, REL = W >= W_REL;
   Frame A, B;
   const PairGeo G = pair_geo(P, R, a, b, rp, A, B);
@@ -940,15 +940,15 @@ __device__ Done refine_pair_m(const DLayer& P, const DLayer& R, uint32_t a, uint
 // split points and coincident edges of both polygons (about 45 for parcel neighbours); of a self pair, beside each edge itself
 constexpr int NODES = 304, NODES_SELF = 160;
 // (the flag alone: lists, grid boxes, queue, flags)
-__host__ __device__ constexpr size_t mask_warp_bytes(int cap, bool self, bool cuts = true) {
+__host__ __device__ constexpr size_t warp_bytes(int cap, bool self, bool cuts = true) {
   const size_t sides = self ? 1 : 2;
   if (!cuts) return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + QCAP * 2;
   const size_t nodes = self ? NODES_SELF : NODES;
   return sides * cap * EDGE_BYTES_8 + (size_t)cap * 8 + nodes * 8 + sides * cap * 4 + 2 * (cap / 32) * 4 + nodes * 2 + QCAP * 2;
 }
-static_assert(mask_warp_bytes(128, false) % 16 == 0 && mask_warp_bytes(256, true) % 16 == 0, "a warp's part starts on 16 bytes");
+static_assert(warp_bytes(128, false) % 16 == 0 && warp_bytes(256, true) % 16 == 0, "a warp's part starts on 16 bytes");
 template <int MS, bool SELF, bool CUTS>
-__device__ __forceinline__ void carve_mask(unsigned char* base, EList8& LA, EList8& LB, CutLists<uint16_t>& cl) {
+__device__ __forceinline__ void carve_warp(unsigned char* base, EList8& LA, EList8& LB, CutLists<uint16_t>& cl) {
   constexpr int nodes = SELF ? NODES_SELF : NODES;
   double* d = reinterpret_cast<double*>(base);
   auto doubles = [&](EList8& L) { L.x0 = d; L.y0 = d + MS; L.x1 = d + 2 * MS; L.y1 = d + 3 * MS; d += 4 * MS; };
@@ -970,7 +970,7 @@ template <bool F, int W> struct Cfg;
 template <int W> struct Cfg<false, W> { static constexpr int cap = CAP; static constexpr size_t smem = RB_SMEM, warp = 0; static constexpr int minb = 3; };
 template <int W> struct Cfg<true, W> {   // the flag alone needs no room for cuts and fewer registers: 5 blocks per SM
   static constexpr int cap = CAP_F;
-  static constexpr size_t warp = mask_warp_bytes(CAP_F, false, W != W_FLAG), smem = RB_WARPS * warp;
+  static constexpr size_t warp = warp_bytes(CAP_F, false, W != W_FLAG), smem = RB_WARPS * warp;
   static constexpr int minb = W == W_FLAG ? 5 : 4;
 };
 
@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLaye
   EList8 MA, MB;
   CutLists<uint16_t> mbuf;
   if constexpr (F) {
-    carve_mask<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<F, W>::warp, MA, MB, mbuf);
+    carve_warp<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<F, W>::warp, MA, MB, mbuf);
   } else {
     LA = carve(smem + (size_t)wib * 2 * LIST_BYTES, CAP);
     LB = carve(smem + (size_t)wib * 2 * LIST_BYTES + LIST_BYTES, CAP);
@@ -1055,7 +1055,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<true, W>::minb) k_refine_sp
   __syncwarp();
   EList8 LA, LB;
   CutLists<uint16_t> cl;
-  carve_mask<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<true, W>::warp, LA, LB, cl);
+  carve_warp<CAP_F, false, W != W_FLAG>(smem + (size_t)wib * Cfg<true, W>::warp, LA, LB, cl);
   const uint64_t n = *nlist;   // written by k_refine, launched before this kernel
   for (;;) {
     unsigned long long h = 0;
@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<true, W>::minb) k_refine_sp
 // self-join's pairs and the costliest (every edge is local). One list of up to 256 edges per warp (the largest that the
 // queue's bytes index and that keeps 4 blocks of 4 warps per SM), A's gather and contribution pass only (refine_pair_m SELF).
 constexpr int CAP_SELF = 256;
-constexpr size_t SELF_SMEM = RB_WARPS * mask_warp_bytes(CAP_SELF, true);
+constexpr size_t SELF_SMEM = RB_WARPS * warp_bytes(CAP_SELF, true);
 constexpr int SELF_MINB = 4;   // blocks per SM: 4 x 53 KB of shared memory
 
 // positions of the self pairs (a == b) among the candidate pairs, warp-aggregated (order free: outputs go by position)
@@ -1112,7 +1112,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, SELF_MINB) k_refine_self(DLayer
   __syncwarp();
   EList8 L, L2;
   CutLists<uint16_t> mbuf;
-  carve_mask<CAP_SELF, true, true>(smem + (size_t)wib * mask_warp_bytes(CAP_SELF, true), L, L2, mbuf);
+  carve_warp<CAP_SELF, true, true>(smem + (size_t)wib * warp_bytes(CAP_SELF, true), L, L2, mbuf);
   const uint64_t n = *nself;   // written by k_self_index, launched before this kernel
   for (int k = 0; k < runs; k++) {
     unsigned long long h0 = 0;
@@ -1351,7 +1351,7 @@ __global__ void __launch_bounds__(128) k_refine_scratch(DLayer P, DLayer R, cons
                                                        unsigned char* scratch, int cap, int cph, int* err, unsigned long long* epairs,
                                                        unsigned long long* next, int same_layer) {
   const int lane = threadIdx.x & 31;
-  const uint64_t nh = *nheavy;   // written by the shared-memory bin launched before this kernel on the same stream
+  const uint64_t nh = *nheavy;   // written by the bins launched before this kernel
   if (nh == 0) return;
   unsigned long long ep = 0;
   const uint64_t w = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -1417,9 +1417,9 @@ static ScratchGeom scratch_geom(const gsj_layer* P, const gsj_layer* R) {
 }
 
 // One refinement = one graph launch between the counters' reset and their copy to pinned host memory: the
-// shared-memory bin (pairs whose local lists fit bin_cap), then the scratch bin (the pairs the first bin listed as
-// oversized; it reads their count on the device, so no host round trip separates the bins); then one stream sync.
-// The executable graph is built once per context and variant and re-parameterised per call.
+// shared-memory bins (pairs whose local lists fit), then the bins for the pairs that these listed as oversized or rich in
+// cuts; they read their counts on the device, so no host round trip separates the bins; then one stream sync.
+// The executable graph is built once per context, variant and set of bins and re-parameterised per call.
 template <bool F, bool S32 = false, int W = W_ALL>
 static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const uint2* pairs, uint64_t np, const RefineArgs& rp, uint8_t* flag,
                      double* area, double4* ev, uint32_t* evb) {
@@ -1430,7 +1430,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
     GSJ_CK(cudaFuncSetAttribute(k_refine<F, S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
     if (F) {
       GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG)));
-      if (W != W_FLAG) GSJ_CK(cudaFuncSetAttribute(k_refine_split<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
+      if constexpr (W != W_FLAG) GSJ_CK(cudaFuncSetAttribute(k_refine_split<S32, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg<F, W>::smem));
       GSJ_CK(cudaFuncSetAttribute(k_refine_block<S32, W, CAP_BIG2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)block_smem(CAP_BIG2)));
     }
     c->refine_attr |= bit;
@@ -1505,7 +1505,8 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
                            P == R ? 1 : 0);
   auto a_idx = kernel_args(k_self_index, pairs, np, sidx, ctr + 5);
   auto a_self = kernel_args(k_refine_self<S32, W>, P->d, pairs, sidx, ctr + 5, rp, flag, area, ev, evb, heavy, ctr, ctr + 6, ctr + 3, run, runs, self_cap);
-  auto a_split = kernel_args(k_refine_split<S32, W>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr + NSPLIT, ctr + NSPLIT + 1, ctr + 3);
+  constexpr int WS = W == W_FLAG ? W_AREA : W;   // the flag alone has no cuts: not launched
+  auto a_split = kernel_args(k_refine_split<S32, WS>, P->d, R->d, pairs, np, rp, flag, area, ev, evb, heavy, ctr + NSPLIT, ctr + NSPLIT + 1, ctr + 3);
   cudaKernelNodeParams km{}, ks{}, ki{}, kf{}, kb{}, kb2{}, kp{};
   kb.func = (void*)k_refine_block<S32, W, CAP_BIG>;
   kb.gridDim = dim3((unsigned)std::min<uint64_t>(np, (uint64_t)c->sm_count * 4));
@@ -1524,7 +1525,7 @@ static void refine_t(gsj_ctx* c, const gsj_layer* P, const gsj_layer* R, const u
   km.sharedMemBytes = (unsigned)Cfg<F, W>::smem;
   km.kernelParams = a_main.ptr;
   kp = km;
-  kp.func = (void*)k_refine_split<S32, W>;
+  kp.func = (void*)k_refine_split<S32, WS>;
   kp.gridDim = dim3((unsigned)std::min<uint64_t>((np + RB_WARPS - 1) / RB_WARPS, (uint64_t)c->sm_count * Cfg<F, W>::minb));
   kp.kernelParams = a_split.ptr;
   ks.func = (void*)k_refine_scratch<F>;
