@@ -110,7 +110,8 @@ static __device__ bool pip_full_warp(const Frame& B, double mx, double my, int l
 }
 
 // inside(x) = inside(c) xor crossings of c -> x with the local edges (engine.cuh:400-412)
-template <bool F, class EL>
+// U: edges a step (lists in global memory: their loads overlap)
+template <bool F, int U = 1, class EL>
 __device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, double cy, bool in_c, double x, double y) {
   bool in = in_c;
   const double sx0 = fmin(cx, x), sx1 = fmax(cx, x), sy0 = fmin(cy, y), sy1 = fmax(cy, y);
@@ -124,7 +125,7 @@ __device__ __forceinline__ bool inside_from_c(const EL& L, int cnt, double cx, d
     if (su != sv) in = !in;
     return false;
   };
-#pragma unroll 1
+#pragma unroll U
   for (int k = 0; k < cnt; k++) step(k);
   return in;
 }

@@ -25,6 +25,7 @@ constexpr int RB_WARPS = 4;                      // warps per block
 constexpr size_t EDGE_BYTES = 4 * sizeof(double) + sizeof(uint32_t);
 constexpr size_t LIST_BYTES = CAP * EDGE_BYTES;  // one list
 constexpr size_t RB_SMEM = (size_t)RB_WARPS * 2 * LIST_BYTES;
+constexpr int U_GLOBAL = 2;   // edges a step of the sweeps over lists in global memory
 constexpr int CAP_F = 128;                       // filtered: local edges per polygon per warp (a multiple of 32, below 256)
 constexpr size_t EDGE_BYTES_8 = 4 * sizeof(double) + 1;   // filtered shared-memory bins: flags in a byte
 
@@ -336,7 +337,7 @@ __device__ __forceinline__ void edge_segment_add(const Segment& s, const EdgeCut
 
 // One edge by one lane. each_k(visit) calls visit(k) for the other polygon's local edges k in increasing order: all of
 // them, or only those of a candidate list that holds every k passing the box test (the same visits, the same results).
-template <bool F, class EL, class EachK>
+template <bool F, int U, class EL, class EachK>
 __device__ double edge_contrib_k(const EL& LS, int i, const EL& L, int cnt, bool in_c, const PairGeo& G, bool rel, double& l_in, double& l_on, uint32_t& bits,
                                  EachK&& each_k) {
   const EdgeRef e = edge_ref(LS, i, rel);
@@ -351,16 +352,16 @@ __device__ double edge_contrib_k(const EL& LS, int i, const EL& L, int cnt, bool
   for (int k = 0; k + 1 < C.ns; k++) {
     const Segment s = edge_segment(C, e, L, k, G, lens);
     if (!s.valid) continue;
-    const int vin = s.need && inside_from_c<F>(L, cnt, G.cx, G.cy, in_c, s.mx, s.my) ? 1 : 0;
+    const int vin = s.need && inside_from_c<F, U>(L, cnt, G.cx, G.cy, in_c, s.mx, s.my) ? 1 : 0;
     edge_segment_add(s, C, e, L, G, lens, vin, acc, l_in, l_on, bits);
   }
   return acc;
 }
-template <bool F, class EL>
+template <bool F, int U, class EL>
 __device__ __forceinline__ double edge_contrib(const EL& LS, int i, const EL& L, int cnt, bool in_c, const PairGeo& G, bool rel, double& l_in, double& l_on,
                                                uint32_t& bits) {
-  return edge_contrib_k<F>(LS, i, L, cnt, in_c, G, rel, l_in, l_on, bits, [&](auto&& visit) {
-#pragma unroll 1
+  return edge_contrib_k<F, U>(LS, i, L, cnt, in_c, G, rel, l_in, l_on, bits, [&](auto&& visit) {
+#pragma unroll U
     for (int k = 0; k < cnt; k++) visit(k);
   });
 }
@@ -418,7 +419,10 @@ __device__ __forceinline__ PairGeo pair_geo(const DLayer& P, const DLayer& R, ui
 // B's gather and B's contribution pass would repeat A's exactly (the same edges in the same frame, the same candidates
 // in the same order, so the same values): A's pass runs once and each lane adds its recorded values a second time, in
 // the same order, which is the sum the two passes make.
-template <bool F, bool FLAT = false, bool BUCKETS = false, bool SELF = false>
+// U: edges a step of the sweeps. Lists in shared memory are swept one by one (code size), lists in global memory two at a time, so
+// that their loads overlap. Refinement, 1 / 2 / 4 at a time: plain relate self-join of 5k parcels 4.08 / 3.26 / 3.29 ms, of
+// 100k 21.7 / 20.4 / 23.2; pairs of 2000-8000 edges, filtered, 115.5 / 105.6 / 101.0; allocation-free call, 20k parcels, 13.9 / 11.1 / 19.5.
+template <bool F, int U, bool FLAT = false, bool BUCKETS = false, bool SELF = false>
 __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList LA, EList LB, int cap,
                               int lane, uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb, const FlatBuf* fb = nullptr,
                               unsigned long long* ep = nullptr) {
@@ -473,7 +477,7 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
         }
         return false;
       };
-#pragma unroll 1
+#pragma unroll U
       for (int j = 0; j < nb; j++) if (test(j)) break;
     };
 #pragma unroll 1
@@ -499,13 +503,13 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
       for (uint32_t r = A.r0 + lane; r < A.r1 && !h; r += 32) {
         double x, y; const bool real = probe_vertex(A, r, x, y);
         if (!real) A.v(P.rvo[r], x, y);
-        if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c<F>(LB, nb, G.cx, G.cy, inB_c, x, y)) { ha = true; h = real; }
+        if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c<F, U>(LB, nb, G.cx, G.cy, inB_c, x, y)) { ha = true; h = real; }
       }
 #pragma unroll 1
       for (uint32_t r = B.r0 + lane; r < B.r1 && !h; r += 32) {
         double x, y; const bool real = probe_vertex(B, r, x, y);
         if (!real) B.v(R.rvo[r], x, y);
-        if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c<F>(LA, na, G.cx, G.cy, inA_c, x, y)) { ha = true; h = real; }
+        if (x >= G.ov.x0 && x <= G.ov.x1 && y >= G.ov.y0 && y <= G.ov.y1 && inside_from_c<F, U>(LA, na, G.cx, G.cy, inA_c, x, y)) { ha = true; h = real; }
       }
       hit = __any_sync(0xffffffffu, h);
       contain_any = __any_sync(0xffffffffu, ha);
@@ -521,7 +525,7 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
 #pragma unroll 1
       for (int i = lane; i < na; i += 32) {
         const int r0 = (int)fb->sa[i], r1 = (int)fb->sa[i + 1];
-        const double v = edge_contrib_k<F>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits, [&](auto&& visit) {
+        const double v = edge_contrib_k<F, U>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits, [&](auto&& visit) {
 #pragma unroll 1
           for (int e = r0; e < r1; e++) visit((int)(cp[e] >> 16));
         });
@@ -545,7 +549,7 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
         for (int i = lane; i < nself; i += 32) {
           const int r0 = pass ? (i ? (int)fb->sb[i - 1] : 0) : (int)fb->sa[i];
           const int r1 = pass ? (int)fb->sb[i] : (int)fb->sa[i + 1];
-          S.s2 += edge_contrib_k<F>(LS, i, LO, nother, inc, G, rel, lin, lon, bits, [&](auto&& visit) {
+          S.s2 += edge_contrib_k<F, U>(LS, i, LO, nother, inc, G, rel, lin, lon, bits, [&](auto&& visit) {
 #pragma unroll 1
             for (int e = r0; e < r1; e++) visit(pass ? (int)(cp[pj[e]] & 0xFFFFu) : (int)(cp[e] >> 16));
           });
@@ -554,9 +558,9 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
       }
     } else {
 #pragma unroll 1
-      for (int i = lane; i < na; i += 32) S.s2 += edge_contrib<F>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits);
+      for (int i = lane; i < na; i += 32) S.s2 += edge_contrib<F, U>(LA, i, LB, nb, inB_c, G, rel, S.ai, S.ao, bits);
 #pragma unroll 1
-      for (int i = lane; i < nb; i += 32) S.s2 += edge_contrib<F>(LB, i, LA, na, inA_c, G, rel, S.bi, S.bo, bits);
+      for (int i = lane; i < nb; i += 32) S.s2 += edge_contrib<F, U>(LB, i, LA, na, inA_c, G, rel, S.bi, S.bo, bits);
     }
   }
   pair_result(S, sums, hit, rtouch, bits, o_flag, o_area, o_ev, o_evb);
@@ -567,7 +571,7 @@ __device__ bool refine_pair_t(const DLayer& P, const DLayer& R, uint32_t a, uint
 // the plain routine, callable from other translation units (the allocation-free entry point)
 __device__ bool refine_pair(const DLayer& P, const DLayer& R, uint32_t a, uint32_t b, const RefineArgs& rp, EList LA, EList LB, int cap, int lane,
                             uint8_t& o_flag, double& o_area, double4& o_ev, uint32_t& o_evb) {
-  return refine_pair_t<false>(P, R, a, b, rp, LA, LB, cap, lane, o_flag, o_area, o_ev, o_evb);
+  return refine_pair_t<false, U_GLOBAL>(P, R, a, b, rp, LA, LB, cap, lane, o_flag, o_area, o_ev, o_evb);
 }
 
 // ---- the shared-memory bins' pair routine (filtered variants) -----------------------------------------------------------
@@ -1004,7 +1008,7 @@ __global__ void __launch_bounds__(RB_WARPS * 32, Cfg<F, W>::minb) k_refine(DLaye
     uint8_t f; double ar; double4 e4; uint32_t b4;
     Done d;
     if constexpr (F) d = refine_pair_m<S32, 0, W>(P, R, pr.x, pr.y, rp, MA, MB, bin_cap, lane, f, ar, e4, b4, mbuf, &s_ep[wib]);
-    else d = refine_pair_t<false>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &s_ep[wib]) ? DONE : LONG;
+    else d = refine_pair_t<false, 1>(P, R, pr.x, pr.y, rp, LA, LB, bin_cap, lane, f, ar, e4, b4, nullptr, &s_ep[wib]) ? DONE : LONG;
     if (lane == 0) {
       if (d != DONE) {   // the list's front, or its back for k_refine_split
         heavy[d == LONG ? atomicAdd(nheavy, 1ull) : np - 1 - atomicAdd(nheavy + NSPLIT, 1ull)] = (uint32_t)p;
@@ -1381,12 +1385,12 @@ __global__ void __launch_bounds__(128) k_refine_scratch(DLayer P, DLayer R, cons
     bool ok;
     if constexpr (F) {   // candidate entries pack both edge indices in 16 bits each
       if (same_layer && pr.x == pr.y)   // a geometry with itself: one list, one contribution pass (B's list records it)
-        ok = cap <= 0xFFFF && refine_pair_t<F, true, true, true>(P, P, pr.x, pr.y, rp, LA, LA, cap, lane, f, ar, e4, b4, &fb, &ep);
+        ok = cap <= 0xFFFF && refine_pair_t<F, U_GLOBAL, true, true, true>(P, P, pr.x, pr.y, rp, LA, LA, cap, lane, f, ar, e4, b4, &fb, &ep);
       else
-        ok = cap <= 0xFFFF && refine_pair_t<F, true, true>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, &fb, &ep);
-      if (!ok) ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
+        ok = cap <= 0xFFFF && refine_pair_t<F, U_GLOBAL, true, true>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, &fb, &ep);
+      if (!ok) ok = refine_pair_t<F, U_GLOBAL>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
     } else {
-      ok = refine_pair_t<F, false>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
+      ok = refine_pair_t<F, U_GLOBAL>(P, R, pr.x, pr.y, rp, LA, LB, cap, lane, f, ar, e4, b4, nullptr, &ep);
     }
     if (lane == 0) {
       if (!ok) *err = 1;
